@@ -10,13 +10,12 @@
 // matrix and recomputes the rest in every matvec.
 //
 // Here the list lives on the device as records of 2W 64-bit words (up string, then
-// down string; W = 1 for L <= 64, W = 2 for L <= 128). One warp owns one row and
-// streams the list through shared memory in tiles; each lane tests one column
-// (popcount of the XORs, <= 2 excitations) and evaluates the element with the
-// reference's summation order, so the values are bit-identical to the reference's.
-// The full symmetric matrix is built row by row (every row scans the whole list;
-// columns come out ascending, the kept set compacted with a warp ballot), so no
-// transpose is needed and the upper triangle is the reference CRS. Storage:
+// down string; W = 1 for L <= 64, W = 2 for L <= 128). Every row is tested
+// against every column (popcount of the XORs, <= 2 excitations; k_dets_scan), and the
+// elements are evaluated with the reference's summation order, so the values are
+// bit-identical to the reference's. The full symmetric matrix is built row by row with
+// its columns ascending, so no transpose is needed and the upper triangle is the
+// reference CRS. Storage:
 //   CIGPU_DETS_CRS      the CRS (FP64, or FP32 hi/lo for the mixed method);
 //   CIGPU_DETS_ONTHEFLY nothing but the list: every FP64 matvec rescans all pairs
 //                       and applies the elements as it computes them (CI_Big with
@@ -30,6 +29,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "crs.cuh"
@@ -45,6 +45,7 @@ enum DetMode : int { kDetCount = 0, kDetFill64 = 1, kDetFill32 = 2, kDetMatvec =
 
 struct DetParams {
     int L, nup, ndown;
+    uint32_t one = 1;  // see mark()
     int64_t n;
     // rows the pass visits (count / fill: the stored rows; matvec: all n) and the
     // stored block: count / fill take columns below `block` (n for a whole CRS); the
@@ -56,6 +57,7 @@ struct DetParams {
     const double *diag;    // [n]
     // count pass
     uint32_t *row_count, *upper_off;
+    uint32_t *seg_count;  // [nrows][kSegs] kept elements per column segment (the fill reads them)
     // fill pass
     const int64_t *row_ptr;
     uint32_t *col;
@@ -170,18 +172,45 @@ __device__ __forceinline__ double one_diff(const DetParams &p, const uint64_t *s
     }
     const int o0 = pop_lowest<W>(x), o1 = pop_lowest<W>(x);
     double e = Tm(p, o0, o1);
+    // four terms' loads in flight, the terms added in order
+    const int64_t L = p.L, at = (int64_t)o0 * L * L * L + (int64_t)o1 * L * L, ax = (int64_t)o0 * L * L * L + o1;
 #pragma unroll
     for (int w = 0; w < W; ++w)
-        for (uint64_t y = c[w]; y; y &= y - 1) {
-            const int z = 64 * w + __ffsll((long long)y) - 1;
-            e += Vm(p, o0, z, o1, z) - Vm(p, o0, z, z, o1);
+        for (uint64_t y = c[w]; y;) {
+            double t[4], u[4];
+            int n = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (y) {
+                    const int z = 64 * w + __ffsll((long long)y) - 1;
+                    y &= y - 1;
+                    t[k] = __ldg(p.eri + at + z * L + z);       // <o0 z|o1 z>
+                    u[k] = __ldg(p.eri + ax + (z * L + z) * L);  // <o0 z|z o1>
+                    n = k + 1;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < n) e += t[k] - u[k];
         }
     const int diff = nstacked<W>(o0, o1, c);
 #pragma unroll
     for (int w = 0; w < W; ++w)
-        for (uint64_t y = other[w]; y; y &= y - 1) {
-            const int z = 64 * w + __ffsll((long long)y) - 1;
-            e += Vm(p, o0, z, o1, z);
+        for (uint64_t y = other[w]; y;) {
+            double t[4];
+            int n = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (y) {
+                    const int z = 64 * w + __ffsll((long long)y) - 1;
+                    y &= y - 1;
+                    t[k] = __ldg(p.eri + at + z * L + z);
+                    n = k + 1;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < n) e += t[k];
         }
     return negate_if(e, diff & 1);
 }
@@ -254,20 +283,83 @@ __device__ __forceinline__ double two_diff_ab(const DetParams &p, const uint64_t
     return negate_if(e, diff & 1);
 }
 
-// get_ham_element (CIMethod.cpp:459-487), the off-diagonal cases
-template <int W>
-__device__ __forceinline__ double element(const DetParams &p, const uint64_t *u1, const uint64_t *d1,
-                                          const uint64_t *u2, const uint64_t *d2, int nu, int nd) {
-    if (nd > 4 || nu > 4) return 0.0;
-    if (nu == 4 && nd == 0) return two_diff_same<W>(p, u1, u2);
-    if (nu == 2) {
-        if (nd == 0) return one_diff<W>(p, u1, u2, d1);
-        if (nd == 2) return two_diff_ab<W>(p, u1, u2, d1, d2);
-        return 0.0;
+// The same elements for strings of one word U (uint32_t to 32 orbitals, uint64_t to
+// 64): the excitation's orbitals from the words themselves (a lowest or highest set
+// bit each) and the phase from one popcount, the parity of both strings' electrons
+// between the orbitals. The integrals and the order of the additions are those above.
+__device__ __forceinline__ int low_bit(uint32_t x) { return __ffs((int)x) - 1; }
+__device__ __forceinline__ int low_bit(uint64_t x) { return __ffsll((long long)x) - 1; }
+__device__ __forceinline__ int high_bit(uint32_t x) { return 31 - __clz((int)x); }
+__device__ __forceinline__ int high_bit(uint64_t x) { return 63 - __clzll((long long)x); }
+__device__ __forceinline__ int bits(uint32_t x) { return __popc(x); }
+__device__ __forceinline__ int bits(uint64_t x) { return __popcll(x); }
+
+// The orbitals from the lower of two single bits up to, not including, the other.
+template <typename U>
+__device__ __forceinline__ U between(U a, U b) {
+    return (a - 1) ^ (b - 1);
+}
+
+template <typename U>
+__device__ __forceinline__ double word_double_ab(const DetParams &p, U u1, U u2, U d1, U d2) {
+    const U xu = u1 ^ u2, xd = d1 ^ d2;
+    const U a0 = xu & u1, a1 = xu & u2, b0 = xd & d1, b1 = xd & d2;
+    const int odd = bits((U)((u1 & u2 & between(a0, a1)) ^ (d1 & d2 & between(b0, b1)))) & 1;
+    const uint32_t L = (uint32_t)p.L;  // L^4 <= 2^24
+    const double e = __ldg(p.eri + (((uint32_t)low_bit(a0) * L + (uint32_t)low_bit(a1)) * L + (uint32_t)low_bit(b0)) * L +
+                           (uint32_t)low_bit(b1));
+    return negate_if(e, odd);
+}
+
+template <typename U>
+__device__ __forceinline__ double word_double_same(const DetParams &p, U s1, U s2) {
+    const U x = s1 ^ s2, a = x & s1, b = x & s2;
+    const U alo = a & (0 - a), blo = b & (0 - b);
+    const int odd = bits((U)(s1 & s2 & (between(alo, (U)(a ^ alo)) ^ between(blo, (U)(b ^ blo))))) & 1;
+    const uint32_t L = (uint32_t)p.L, a0 = low_bit(a), a1 = high_bit(a), b0 = low_bit(b), b1 = high_bit(b);
+    const double e = __ldg(p.eri + ((a0 * L + b0) * L + a1) * L + b1) - __ldg(p.eri + ((a0 * L + b1) * L + a1) * L + b0);
+    return negate_if(e, odd);
+}
+
+template <typename U>
+__device__ __forceinline__ double word_single(const DetParams &p, U s1, U s2, U other) {
+    const U x = s1 ^ s2, c = s1 & s2;
+    const U lo = x & (0 - x);
+    const uint32_t L = (uint32_t)p.L, o0 = low_bit(x), o1 = high_bit(x);
+    double e = __ldg(p.h + o0 * L + o1);
+    const double *ez = p.eri + (o0 * L + o1) * L * L, *ex = p.eri + o0 * L * L * L + o1;
+    for (U y = c; y;) {  // four terms' loads in flight, the terms added in order
+        double t[4], u[4];
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (y) {
+                const uint32_t z = low_bit(y);
+                y &= y - 1;
+                t[k] = __ldg(ez + z * (L + 1));        // <o0 z|o1 z>
+                u[k] = __ldg(ex + z * (L + 1) * L);    // <o0 z|z o1>
+                n = k + 1;
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < n) e += t[k] - u[k];
     }
-    if (nd == 4 && nu == 0) return two_diff_same<W>(p, d1, d2);
-    if (nd == 2 && nu == 0) return one_diff<W>(p, d1, d2, u1);
-    return 0.0;
+    for (U y = other; y;) {
+        double t[4];
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (y) {
+                const uint32_t z = low_bit(y);
+                y &= y - 1;
+                t[k] = __ldg(ez + z * (L + 1));
+                n = k + 1;
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < n) e += t[k];
+    }
+    return negate_if(e, bits((U)(c & between(lo, (U)(x ^ lo)))) & 1);
 }
 
 template <int W>
@@ -278,92 +370,376 @@ __global__ void k_dets_diag(DetParams p, double *diag) {
     }
 }
 
-// RANGED: a stored block smaller than the list (CI_Big with a kept part), whose
-// passes skip columns outside their range; the whole-list passes carry no test.
-template <int W, int MODE, bool RANGED>
-__global__ void __launch_bounds__(32 * kDetWarps) k_dets_rows(DetParams p, const double *__restrict__ x,
-                                                              double *__restrict__ y) {
-    __shared__ uint64_t tile[kDetTile * 2 * W];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
+// ---------------------------------------------------------------------------
+// The pair scan of the build and of the matvec without a stored matrix.
+//
+// A block owns kScanRows rows, one per lane of every warp; its warps split the
+// columns. A warp stages 32 columns and every lane tests its row against each of
+// them, so a column is one broadcast shared-memory read and 32 pairs are a few
+// integer instructions: the 32-bit words of the two determinants' XOR (each word
+// rotated by its own amount) are OR-ed together and the pair passes when at most 4
+// bits are set. The OR never has more bits than the words together, so no connected
+// pair fails; the few others that pass are dropped below. What bounds it is POPC,
+// 16 lanes per clock and SM: one of them per pair here (a popcount per word before).
+//
+// The pairs that pass, a few in a hundred, go to the warp's queue in shared memory
+// and are evaluated 32 at a time on full warps: doubles first, then the singles, a
+// chain of FP64 additions that costs the warp the same with one lane as with all
+// of them. Evaluated where they were found, one lane or two of a warp at work, they
+// were the time of the pass. (L=32 8a8b CISD list, 52,705 determinants, list to
+// CRS and one product: 23.4 -> 4.6 ms; matvec without a stored matrix of a random 70%
+// of the L=28 7a7b CISD list, 21,500 determinants: 4.53 -> 0.49 ms.)
+//
+// The queue holds a row's columns in ascending order (words in order, a row's bits
+// in order), so the fill writes each row's kept elements in order at the row's
+// start plus the counts of the segments before it, and the matvec adds a row's terms
+// in a fixed order.
+//
+// RANGED: the matvec of a list with a stored block (CI_Big with a kept part) leaves
+// out the pairs of the block; the other passes carry no test.
+constexpr int kScanRows = 32;
+constexpr int kScanWarps = 8;  // the matvec's warps per block
+constexpr int kSegs = 64;      // column segments of the count and fill passes
+constexpr int kQueue = 256;                 // a word of 8 rows fits whatever passes
+constexpr int kQueueColBits = 27;           // queue entry: row << 27 | column - the queue's first column
+constexpr uint32_t kQueueColMask = (1u << kQueueColBits) - 1u;
+
+template <int MODE>
+constexpr int scan_warps() {
+    return MODE == kDetMatvec ? kScanWarps : 1;
+}
+
+// 32-bit words a determinant is tested with: 2 (L <= 32), 4 (L <= 64) or 8.
+template <int W, int NW>
+__device__ __forceinline__ void scan_key(const uint64_t *rec, uint32_t *k) {
+    if constexpr (NW == 2) {
+        k[0] = (uint32_t)rec[0];
+        k[1] = __funnelshift_l((uint32_t)rec[1], (uint32_t)rec[1], 16);
+    } else {
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const uint32_t v = (uint32_t)(rec[w >> 1] >> (32 * (w & 1)));
+            k[w] = __funnelshift_l(v, v, w * (32 / NW));
+        }
+    }
+}
+
+// m += bit where x has at most 4 bits set. The multiply-add (one = 1, not known to
+// the compiler) keeps the add off the ALU pipe, which the XORs and compares fill.
+__device__ __forceinline__ void mark(uint32_t &m, uint32_t x, uint32_t bit, uint32_t one) {
+    asm("{\n\t.reg .pred q;\n\tsetp.le.u32 q, %1, 4;\n\t@q mad.lo.u32 %0, %2, %3, %0;\n\t}"
+        : "+r"(m)
+        : "r"((uint32_t)__popc(x)), "r"(one), "r"(bit));
+}
+
+// Shared memory of one warp.
+template <int W, int NW>
+struct ScanWarp {
+    alignas(16) uint32_t key[32 * NW];  // the staged columns
+    double val[kQueue];
+    uint32_t at[kQueue];
+    uint16_t single[kQueue];  // queue positions of the singles
+    double acc[kScanRows];    // matvec: the row sums
+    uint32_t run[kScanRows], low[kScanRows];  // kept elements so far; those below the diagonal
+};
+
+template <int W>
+struct ScanRow {
+    uint64_t s[kScanRows][2 * W];
+};
+
+// The output of one queue entry's value, lanes in queue order. `live` lanes hold an
+// entry: row, column j, value v.
+template <int MODE, int W, int NW>
+__device__ __forceinline__ void scan_emit(const DetParams &p, ScanWarp<W, NW> &q, const int64_t *rowpos, bool live, int row,
+                                          int64_t j, double v, const double *__restrict__ x) {
+    const int lane = threadIdx.x & 31;
+    const bool keep = live && keep_value(v);
+    const unsigned kb = __ballot_sync(0xffffffffu, keep);
+    if (kb == 0) return;
+    // the kept entries of this lane's row
+    const unsigned same = __match_any_sync(0xffffffffu, live ? row : 32 + lane) & kb;
+    if (MODE == kDetMatvec) {
+        const double xj = keep ? x[j] : 0.0;
+        // the first kept lane of each row adds the row's terms in order
+        const bool lead = keep && (same & ((1u << lane) - 1u)) == 0;
+        unsigned rest = lead ? same : 0u;
+        double a = lead ? q.acc[row] : 0.0;
+        while (__any_sync(0xffffffffu, rest)) {
+            const int src = rest ? __ffs((int)rest) - 1 : lane;
+            const double vs = __shfl_sync(0xffffffffu, v, src), xs = __shfl_sync(0xffffffffu, xj, src);
+            if (rest) a = fma(vs, xs, a);
+            rest &= rest - 1;
+        }
+        if (lead) q.acc[row] = a;
+    } else if (keep) {
+        const int before = __popc(same & ((1u << lane) - 1u));
+        const int64_t pos = rowpos[row] + q.run[row] + before;
+        p.col[pos] = (uint32_t)j;
+        if (MODE == kDetFill64) {
+            p.val64[pos] = v;
+        } else {
+            split_fp32(v, p.val32[pos], p.val32lo[pos]);
+        }
+    }
+    __syncwarp();
+    if (MODE != kDetMatvec && keep && (same >> lane) == 1u) q.run[row] += __popc(same);  // the row's last kept lane
+    __syncwarp();
+}
+
+// Evaluates and outputs the queue's n entries (columns from `first`).
+template <int MODE, int W, int NW>
+__device__ __noinline__ void scan_flush(const DetParams &p, ScanWarp<W, NW> &q, const ScanRow<W> &rows,
+                                        const int64_t *rowpos, int64_t r0, int n, int64_t first,
+                                        const double *__restrict__ x) {
+    using U = std::conditional_t<NW == 2, uint32_t, uint64_t>;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    int ns = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        bool single = false;
+        if (k < n) {
+            const uint32_t e = q.at[k];
+            const int row = (int)(e >> kQueueColBits);
+            const int64_t j = first + (e & kQueueColMask), i = r0 + row;
+            const uint64_t *ui = rows.s[row], *di = ui + W;
+            double v = 0;
+            if constexpr (W == 1) {
+                const ulonglong2 rj = __ldg(reinterpret_cast<const ulonglong2 *>(p.dets) + j);
+                const U u1 = (U)ui[0], d1 = (U)di[0], u2 = (U)rj.x, d2 = (U)rj.y;
+                const int nu = bits((U)(u1 ^ u2)), nd = bits((U)(d1 ^ d2));
+                if (nu + nd == 2) {
+                    single = true;
+                } else if (nu == 2 && nd == 2) {
+                    v = word_double_ab<U>(p, u1, u2, d1, d2);
+                } else if (nu + nd == 4) {
+                    v = word_double_same<U>(p, nu ? u1 : d1, nu ? u2 : d2);
+                } else if (nu + nd == 0) {
+                    v = p.diag[i];  // the row itself, or a repeat of its determinant in the list
+                }
+            } else {
+            uint64_t uj[W], dj[W];
+            int nu = 0, nd = 0;
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                uj[w] = __ldg(p.dets + j * 2 * W + w);
+                dj[w] = __ldg(p.dets + j * 2 * W + W + w);
+                nu += __popcll(ui[w] ^ uj[w]);
+                nd += __popcll(di[w] ^ dj[w]);
+            }
+            if (nu + nd == 0)
+                v = p.diag[i];
+            else if (nu + nd == 2)
+                single = true;
+            else if (nu == 2 && nd == 2)
+                v = two_diff_ab<W>(p, ui, uj, di, dj);
+            else if (nu + nd == 4 && (nu == 4 || nd == 4)) {
+                uint64_t a[W], b[W];
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+                    a[w] = nu ? ui[w] : di[w];
+                    b[w] = nu ? uj[w] : dj[w];
+                }
+                v = two_diff_same<W>(p, a, b);
+            }
+            }
+            if (MODE == kDetCount) {
+                if (keep_value(v)) {
+                    atomicAdd(&q.run[row], 1u);  // integer counts: any order
+                    if (j < i) atomicAdd(&q.low[row], 1u);
+                }
+            } else {
+                q.val[k] = v;
+            }
+        }
+        const unsigned sb = __ballot_sync(0xffffffffu, single);
+        if (single) q.single[ns + __popc(sb & ((1u << lane) - 1u))] = (uint16_t)k;
+        ns += __popc(sb);
+    }
+    __syncwarp();
+    for (int k0 = 0; k0 < ns; k0 += 32) {
+        if (k0 + lane < ns) {
+            const int k = q.single[k0 + lane];
+            const uint32_t e = q.at[k];
+            const int row = (int)(e >> kQueueColBits);
+            const int64_t j = first + (e & kQueueColMask), i = r0 + row;
+            const uint64_t *ui = rows.s[row], *di = ui + W;
+            double v;
+            if constexpr (W == 1) {
+                const ulonglong2 rj = __ldg(reinterpret_cast<const ulonglong2 *>(p.dets) + j);
+                const U u1 = (U)ui[0], d1 = (U)di[0], u2 = (U)rj.x, d2 = (U)rj.y;
+                const bool up = u1 != u2;
+                v = word_single<U>(p, up ? u1 : d1, up ? u2 : d2, up ? d1 : u1);
+            } else {
+            uint64_t a[W], b[W], o[W];
+            bool up = false;
+#pragma unroll
+            for (int w = 0; w < W; ++w) up = up || ui[w] != __ldg(p.dets + j * 2 * W + w);
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                a[w] = up ? ui[w] : di[w];
+                b[w] = __ldg(p.dets + j * 2 * W + (up ? 0 : W) + w);
+                o[w] = up ? di[w] : ui[w];
+            }
+            v = one_diff<W>(p, a, b, o);
+            }
+            if (MODE == kDetCount) {
+                if (keep_value(v)) {
+                    atomicAdd(&q.run[row], 1u);
+                    if (j < i) atomicAdd(&q.low[row], 1u);
+                }
+            } else {
+                q.val[k] = v;
+            }
+        }
+    }
+    __syncwarp();
+    if (MODE != kDetCount) {
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int k = k0 + lane;
+            const bool live = k < n;
+            const uint32_t e = live ? q.at[k] : 0u;
+            scan_emit<MODE, W, NW>(p, q, rowpos, live, (int)(e >> kQueueColBits), first + (e & kQueueColMask),
+                                   live ? q.val[k] : 0.0, x);
+        }
+    }
+    __syncwarp();
+}
+
+// Block: 32 rows x WARPS warps. Counts and fills run one-warp blocks, one per 32 rows
+// and segment of the columns (grid: row groups x kSegs), so that a segment dense in
+// connected pairs holds up no other (the L=32 list's build: 15.7 ms with the segments
+// as the warps of one block, which then wait for the densest; 9.2 ms with 16 one-warp
+// blocks of them, 4.6 with 64 and the single-word element functions). The matvec's warps take every
+// kScanWarps-th word of the columns, which spreads such segments over them, and meet
+// once at the end.
+template <int W, int NW, int MODE, bool RANGED>
+__global__ void __launch_bounds__(32 * scan_warps<MODE>(), MODE == kDetMatvec ? 4 : 32)
+    k_dets_scan(const DetParams p, const double *__restrict__ x, double *__restrict__ y) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int WARPS = scan_warps<MODE>();
     constexpr bool kStoring = MODE != kDetMatvec;
-    for (int64_t r0 = (int64_t)blockIdx.x * kDetWarps; r0 < p.nrows; r0 += (int64_t)gridDim.x * kDetWarps) {
-        const int64_t i = r0 + warp;
-        const bool active = i < p.nrows;
-        // this row's columns [cs, ce): a stored pass takes those of the block; the
-        // matvec of a partly stored matrix takes those outside it
-        const int64_t cs = (RANGED && !kStoring && i < p.block) ? p.block : 0, ce = kStoring ? p.block : p.n;
-        // the warps' common start (rows of one pass below the block skip it together)
-        const int64_t cs_all = (RANGED && !kStoring && r0 + kDetWarps <= p.block) ? p.block : 0;
-        uint64_t ui[W], di[W];
+    __shared__ ScanRow<W> rows;
+    __shared__ int64_t rowpos[kScanRows];
+    ScanWarp<W, NW> *warps = reinterpret_cast<ScanWarp<W, NW> *>(smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    ScanWarp<W, NW> &q = warps[warp];
+    const int64_t group = kStoring ? blockIdx.x / kSegs : blockIdx.x;
+    const int seg = kStoring ? (int)(blockIdx.x - group * kSegs) : 0;
+    const int64_t r0 = group * kScanRows;
+    const int64_t i = r0 + lane;
+    const bool active = i < p.nrows;
+    uint64_t rec[2 * W];
 #pragma unroll
-        for (int w = 0; w < W; ++w) {
-            ui[w] = active ? p.dets[i * 2 * W + w] : 0;
-            di[w] = active ? p.dets[i * 2 * W + W + w] : 0;
-        }
-        uint32_t cnt = 0, lower = 0;
-        int64_t out = (MODE == kDetFill64 || MODE == kDetFill32) && active ? p.row_ptr[i] : 0;
-        double acc = 0;
-        const int64_t cend = kStoring ? p.block : p.n;  // the same for every row of the pass
-        for (int64_t base = cs_all; base < cend; base += kDetTile) {
-            const int tn = (int)(cend - base < kDetTile ? cend - base : kDetTile);
-            __syncthreads();
-            for (int t = threadIdx.x; t < tn * 2 * W; t += blockDim.x) tile[t] = p.dets[base * 2 * W + t];
-            __syncthreads();
-            if (!active) continue;
-            for (int jj0 = 0; jj0 < tn; jj0 += 32) {
-                const int jj = jj0 + lane;
-                const int64_t j = base + jj;
-                double v = 0;
-                bool keep = false;
-                if (jj < tn && (!RANGED || (j >= cs && j < ce))) {
-                    const uint64_t *uj = tile + jj * 2 * W, *dj = uj + W;
-                    int nu = 0, nd = 0;
+    for (int w = 0; w < 2 * W; ++w) rec[w] = active ? p.dets[i * 2 * W + w] : 0;
+    uint32_t rk[NW];
+    scan_key<W, NW>(rec, rk);
+    if (warp == 0) {
 #pragma unroll
-                    for (int w = 0; w < W; ++w) {
-                        nu += __popcll(ui[w] ^ uj[w]);
-                        nd += __popcll(di[w] ^ dj[w]);
-                    }
-                    if (nu + nd <= 4) {
-                        // the row itself, or a repeat of its determinant in the list, is the diagonal
-                        v = (nu + nd == 0) ? p.diag[i] : element<W>(p, ui, di, uj, dj, nu, nd);
-                        keep = keep_value(v);
-                    }
+        for (int w = 0; w < 2 * W; ++w) rows.s[lane][w] = rec[w];
+    }
+    q.acc[lane] = 0.0;
+    q.run[lane] = q.low[lane] = 0;
+    // columns [c_lo, c_end): a stored pass takes those of the block; the matvec of a
+    // partly stored matrix takes, for the block's rows, those outside it
+    const int64_t c_lo = (RANGED && r0 + kScanRows <= p.block) ? p.block : 0;
+    const int64_t c_end = kStoring ? p.block : p.n;
+    const int64_t words = (c_end - c_lo + 31) / 32;
+    const int64_t w0 = kStoring ? words * seg / kSegs : warp, w1 = kStoring ? words * (seg + 1) / kSegs : words;
+    constexpr int kStep = kStoring ? 1 : WARPS;
+    if (MODE == kDetFill64 || MODE == kDetFill32) {
+        int64_t at = 0;
+        if (active) {
+            at = p.row_ptr[i];
+            for (int w = 0; w < seg; ++w) at += p.seg_count[i * kSegs + w];
+        }
+        rowpos[lane] = at;
+    }
+    __syncthreads();
+    const uint32_t one = p.one;
+    int qn = 0;
+    int64_t first = 0;
+    uint64_t next[2 * W];
+    auto load = [&](int64_t word) {
+        const int64_t j = c_lo + word * 32 + lane;
+#pragma unroll
+        for (int w = 0; w < 2 * W; ++w) next[w] = (word < w1 && j < c_end) ? __ldg(p.dets + j * 2 * W + w) : 0;
+    };
+    load(w0);
+    for (int64_t word = w0; word < w1; word += kStep) {
+        const int64_t base = c_lo + word * 32;
+        uint32_t ck[NW];
+        scan_key<W, NW>(next, ck);
+#pragma unroll
+        for (int w = 0; w < NW; ++w) q.key[lane * NW + w] = ck[w];
+        __syncwarp();
+        load(word + kStep);
+        uint32_t m = 0;
+#pragma unroll
+        for (int c = 0; c < 32; c += (NW == 2 ? 2 : 1)) {
+            if constexpr (NW == 2) {
+                const uint4 k = *reinterpret_cast<const uint4 *>(q.key + c * NW);
+                mark(m, (k.x ^ rk[0]) | (k.y ^ rk[1]), 1u << c, one);
+                mark(m, (k.z ^ rk[0]) | (k.w ^ rk[1]), 2u << c, one);
+            } else {
+                uint32_t o = 0;
+#pragma unroll
+                for (int w = 0; w < NW; w += 4) {
+                    const uint4 k = *reinterpret_cast<const uint4 *>(q.key + c * NW + w);
+                    o |= (k.x ^ rk[w]) | (k.y ^ rk[w + 1]);
+                    o |= (k.z ^ rk[w + 2]) | (k.w ^ rk[w + 3]);
                 }
-                if (MODE == kDetCount) {
-                    cnt += keep;
-                    lower += keep && j < i;
-                } else if (MODE == kDetMatvec) {
-                    if (keep) acc = fma(v, x[j], acc);
-                } else {
-                    const unsigned m = __ballot_sync(0xffffffffu, keep);
-                    if (keep) {
-                        const int64_t pos = out + __popc(m & below);
-                        p.col[pos] = (uint32_t)j;
-                        if (MODE == kDetFill64) {
-                            p.val64[pos] = v;
-                        } else {
-                            split_fp32(v, p.val32[pos], p.val32lo[pos]);
-                        }
-                    }
-                    out += __popc(m);
-                }
+                mark(m, o, 1u << c, one);
             }
         }
-        if (!active) continue;
-        if (MODE == kDetCount) {
-            for (int o = 16; o > 0; o >>= 1) {
-                cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-                lower += __shfl_xor_sync(0xffffffffu, lower, o);
+        __syncwarp();  // the staged columns are read; the next word's may be written
+        if (c_end - base < 32) m &= (1u << (int)(c_end - base)) - 1u;
+        if (!active) m = 0;
+        if (RANGED && i < p.block && base < p.block)
+            m = p.block - base >= 32 ? 0u : m & ~((1u << (int)(p.block - base)) - 1u);
+        if (!__any_sync(0xffffffffu, m)) continue;
+        int off = __popc(m);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, off, o);
+            if (lane >= o) off += u;
+        }
+        const int total = __shfl_sync(0xffffffffu, off, 31);
+        off -= __popc(m);
+        if (qn > 0 && (qn + total > kQueue || base - first > (int64_t)(kQueueColMask - 32))) {
+            scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, qn, first, x);
+            qn = 0;
+        }
+        if (qn == 0) first = base;
+        const uint32_t tag = ((uint32_t)lane << kQueueColBits) | (uint32_t)(base - first);
+        if (total <= kQueue) {
+            for (int k = qn + off; m; m &= m - 1) q.at[k++] = tag + (uint32_t)(__ffs((int)m) - 1);
+            qn += total;
+        } else {  // a dense word: eight rows at a time fill the queue at most
+            for (int g = 0; g < 4; ++g) {
+                const int g0 = __shfl_sync(0xffffffffu, off, 8 * g);
+                const int g1 = g < 3 ? __shfl_sync(0xffffffffu, off, (8 * g + 8) & 31) : total;
+                if ((lane >> 3) == g)
+                    for (int k = off - g0; m; m &= m - 1) q.at[k++] = tag + (uint32_t)(__ffs((int)m) - 1);
+                if (g1 > g0) scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, g1 - g0, first, x);
             }
-            if (lane == 0) {
-                p.row_count[i] = cnt;
-                p.upper_off[i] = lower;
-            }
-        } else if (MODE == kDetMatvec) {
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        }
+    }
+    if (qn > 0) scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, qn, first, x);
+    if constexpr (MODE == kDetCount) {
+        if (active) {
+            p.seg_count[i * kSegs + seg] = q.run[lane];
+            if (q.run[lane]) atomicAdd(p.row_count + i, q.run[lane]);  // integer sums: any order
+            if (q.low[lane]) atomicAdd(p.upper_off + i, q.low[lane]);
+        }
+    } else if constexpr (MODE == kDetMatvec) {
+        __syncthreads();
+        if (warp == 0 && active) {
+            double a = 0;
+            for (int w = 0; w < WARPS; ++w) a += warps[w].acc[lane];
             // rows of the stored block add to the stored block's product, already in y
-            if (lane == 0) y[i] = ((RANGED && i < p.block) ? y[i] : 0.0) + acc;
+            y[i] = ((RANGED && i < p.block) ? y[i] : 0.0) + a;
         }
     }
 }
@@ -380,25 +756,39 @@ int rows_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + kDetWarps - 1) / kDetWarps, (int64_t)sm_count() * 16));
 }
 
-template <int W, int MODE>
-void launch_rows(const DetParams &p, const double *x, double *y, cudaStream_t s) {
-    if (p.nrows == 0) return;
-    // the matvec of a partly stored list, or the stored passes of a block smaller than it
-    const bool ranged = MODE == kDetMatvec ? (p.block > 0 && p.block < p.n) : p.block < p.n;
-    if (ranged)
-        k_dets_rows<W, MODE, true><<<rows_grid(p.nrows), 32 * kDetWarps, 0, s>>>(p, x, y);
-    else
-        k_dets_rows<W, MODE, false><<<rows_grid(p.nrows), 32 * kDetWarps, 0, s>>>(p, x, y);
+template <int W, int NW, int MODE, bool RANGED>
+void launch_scan(const DetParams &p, const double *x, double *y, cudaStream_t s) {
+    constexpr int smem = (int)sizeof(ScanWarp<W, NW>) * scan_warps<MODE>();
+    static const cudaError_t attr = cudaFuncSetAttribute(k_dets_scan<W, NW, MODE, RANGED>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    CIGPU_CUDA(attr);
+    const int64_t blocks = (p.nrows + kScanRows - 1) / kScanRows * (MODE == kDetMatvec ? 1 : kSegs);
+    if (blocks > (int64_t)INT32_MAX) throw std::invalid_argument("determinant list too long");
+    k_dets_scan<W, NW, MODE, RANGED><<<(unsigned)blocks, 32 * scan_warps<MODE>(), smem, s>>>(p, x, y);
     CIGPU_CUDA(cudaGetLastError());
     count_launch();
 }
 
+template <int W, int NW, int MODE>
+void launch_rows(const DetParams &p, const double *x, double *y, cudaStream_t s) {
+    if (p.nrows == 0) return;
+    if constexpr (MODE == kDetMatvec) {
+        if (p.block > 0 && p.block < p.n) {  // a partly stored list
+            launch_scan<W, NW, MODE, true>(p, x, y, s);
+            return;
+        }
+    }
+    launch_scan<W, NW, MODE, false>(p, x, y, s);
+}
+
 template <int MODE>
 void rows(const DetParams &p, int W, const double *x, double *y, cudaStream_t s) {
-    if (W == 1)
-        launch_rows<1, MODE>(p, x, y, s);
+    if (W == 2)
+        launch_rows<2, 8, MODE>(p, x, y, s);
+    else if (p.L > 32)
+        launch_rows<1, 4, MODE>(p, x, y, s);
     else
-        launch_rows<2, MODE>(p, x, y, s);
+        launch_rows<1, 2, MODE>(p, x, y, s);
 }
 
 DetParams params_of(const cigpu_crs &c) {
@@ -829,11 +1219,14 @@ int build_dets(cigpu_ham *ham, int64_t ndet, int words, const uint64_t *up, cons
         const int64_t nb = c->det_block;
         p.nrows = nb;
         p.block = nb;
-        DevBuf<uint32_t> count(nb);
+        DevBuf<uint32_t> count(nb), segs((size_t)nb * kSegs);
         c->upper_off.alloc(nb);
         c->row_ptr.alloc(nb + 1);
         p.row_count = count.p;
         p.upper_off = c->upper_off.p;
+        p.seg_count = segs.p;
+        CIGPU_CUDA(cudaMemsetAsync(count.p, 0, count.bytes(), s));
+        CIGPU_CUDA(cudaMemsetAsync(c->upper_off.p, 0, c->upper_off.bytes(), s));
         rows<kDetCount>(p, W, nullptr, nullptr, s);
         exclusive_scan_u32(count.p, c->row_ptr.p, nb, s);
         DevBuf<unsigned long long> lower(1);

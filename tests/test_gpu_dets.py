@@ -176,3 +176,47 @@ def test_dets_rdm_matches_oracle_gkci():
     for x, y in zip(got, ref):
         assert np.max(np.abs(x - y)) < 1e-13
 
+
+
+def random_list(L, na, nb, n, seed):
+    """n determinants: the lowest one, then random excitations of it of up to four
+    electrons (many pairs connected, many not), distinct, in random order."""
+    rng = np.random.default_rng(seed)
+    seen = []
+    ref = ((1 << na) - 1, (1 << nb) - 1)
+    while len(seen) < n:
+        d = list(ref)
+        for _ in range(int(rng.integers(0, 5))):
+            spin = int(rng.integers(0, 2))
+            occ = [o for o in range(L) if (d[spin] >> o) & 1]
+            emp = [o for o in range(L) if not (d[spin] >> o) & 1]
+            if occ and emp:
+                d[spin] ^= (1 << int(rng.choice(occ))) | (1 << int(rng.choice(emp)))
+        if tuple(d) not in seen:
+            seen.append(tuple(d))
+    up, down = np.array([s[0] for s in seen], np.uint64), np.array([s[1] for s in seen], np.uint64)
+    return up, down
+
+
+@pytest.mark.parametrize("L,na,nb,n", [(6, 1, 1, 36), (8, 1, 1, 64), (5, 2, 1, 1), (7, 3, 3, 31), (9, 3, 2, 33), (31, 3, 2, 129),
+                                       (32, 2, 2, 257), (33, 2, 3, 300), (40, 1, 1, 1000)])
+def test_scan_edges(L, na, nb, n):
+    """The pair scan at the edges of its rows, words and queue (lists shorter than a
+    word, one row over it, every pair connected, 32 and 33 orbitals): the CRS equals the
+    oracle's bit for bit, and the matvecs without a stored matrix (none of it, and a
+    leading block) equal the stored one's."""
+    ints = make_integrals(L, na, nb, nchol=4, seed=L + n)
+    up, down = random_list(L, na, nb, n, seed=n)
+    ham = Hamiltonian.from_integrals(ints)
+    cim = FCI_File(ham, up=up, down=down)
+    m = O.build_dets(ints, up, down)
+    assert upper_sha(cim) == crs_sha256(m.row, m.col, m.val)
+    x = np.random.default_rng(3).standard_normal(n)
+    y = cim.get_mat().mvprod(x)
+    y_ref = O.sym_mvprod(m, x)
+    # a row's terms in another order: n roundings of its largest partial sum
+    tol = 2.0 ** -52 * (n + 2) * float(np.abs(m.val).max() * np.abs(x).sum())
+    assert np.abs(y - y_ref).max() <= tol
+    for keep in (0, n // 3):
+        big = CI_Big(ham, up=up, down=down, keep=keep)
+        assert np.abs(big.get_mat().mvprod(x) - y_ref).max() <= tol
