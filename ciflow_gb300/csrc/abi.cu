@@ -512,6 +512,7 @@ void build_crs(cigpu_crs &c, cudaStream_t s) {
             c.kpair64.alloc((size_t)L * L);
             c.kpair32.alloc((size_t)L * L);
             doci_pair_table_launch(L, h.d_eri.p, c.kpair64.p, c.kpair32.p, s);
+            doci_split_make(L, n, dim, c.split, s);
             if (c.precision == CIGPU_MIXED) {
                 c.diag32.alloc(dim);
                 dev_convert(c.diag.p, c.diag32.p, dim, s);
@@ -605,7 +606,7 @@ void crs_mv64(cigpu_crs &c, const double *x, double *y, cudaStream_t s) {
         return;
     }
     if (c.pairs) {
-        doci_mv64(DociMv{c.L, c.nup, c.dim, c.strings.p}, c.kpair64.p, c.diag.p, x, y, s);
+        doci_mv64(DociMv{c.L, c.nup, c.dim, c.strings.p}, c.split, c.kpair64.p, c.diag.p, x, y, s);
         return;
     }
     if (c.slots && c.val64.p) {  // FP64 slot values: the plain method, or MIXED with the sigma vector
@@ -637,7 +638,7 @@ void crs_mv64(cigpu_crs &c, const double *x, double *y, cudaStream_t s) {
 void crs_mv32(cigpu_crs &c, const float *x, float *y, cudaStream_t s) {
     if (c.precision != CIGPU_MIXED || c.onthefly) throw std::invalid_argument("FP32 matvec needs a MIXED CRS");
     if (c.pairs) {
-        doci_mv32(DociMv{c.L, c.nup, c.dim, c.strings.p}, c.kpair32.p, c.diag32.p, x, y, s);
+        doci_mv32(DociMv{c.L, c.nup, c.dim, c.strings.p}, c.split, c.kpair32.p, c.diag32.p, x, y, s);
         return;
     }
     if (c.sig) {

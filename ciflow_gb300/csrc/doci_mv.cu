@@ -1,5 +1,6 @@
 // Matrix-free DOCI matvec: y = H x over the seniority-zero pair space without a
-// stored matrix.
+// stored matrix. k_doci_mv, the general kernel, forms every hop's rank; larger spaces
+// take k_doci_split (below).
 //
 // Replaces SparseMatrix_CRS_Sym::mvprod (SparseMatrix_CRS.cpp:700-723) on the DOCI
 // matrix of DOCI::construct_CI_matrix (CIMethod.cpp:611-660). Every off-diagonal
@@ -35,6 +36,9 @@
 // written once; the hop gathers hit x in L2. The matrix the CRS form streams
 // (145 elements per row at L=24, 12 bytes each in FP64) is not stored at all.
 #include "doci_mv.cuh"
+
+#include <algorithm>
+#include <vector>
 
 namespace cigpu {
 
@@ -182,6 +186,285 @@ __global__ void __launch_bounds__(kMvThreads) k_doci_mv(const DociMv p, const T 
     }
 }
 
+// ---------------------------------------------------------------------------
+// The product by low and high orbitals (larger spaces).
+//
+// With the orbitals split into s low and L - s high ones, the strings of one high
+// part h are a block of consecutive ranks, ordered by their low part l: x is a ragged
+// matrix x(h, l). A pair hop between two high orbitals moves to another block at the
+// same l, one between two low ones stays in the block, and one between a low and a
+// high orbital takes l to a string of one pair less or more. So nothing of a hop's
+// rank depends on the row as a whole:
+//   * high - high: the lanes of a warp (consecutive l) read consecutive x of another
+//     block; its start and K_jk are the same for all of them;
+//   * low - low: the target in the block and the orbital pair come from a table over
+//     l alone;
+//   * low - high: the blocks h + k and h - k are staged in shared memory once and
+//     gathered from there, with the target from a table over l and K from the row of
+//     k (consecutive words over j: no bank conflict).
+// A hop is two or three shared-memory reads and a multiply-add where the general
+// kernel forms a rank (two popcounts' worth of lookups and selects, ~110 issue slots
+// per 32 hops). What bounds it: in FP32 the shared-memory gathers, in FP64 the FP64
+// pipe. L=24, 12 pairs (2,704,156 rows, 144 hops): FP32 1122 -> 227 us, FP64
+// 1.70 -> 0.74 ms (the FP64 pipe's share 0.62); L=20, 8 pairs (125,970): 54 -> 19-23 us and
+// 81 -> 39 us.
+//
+// A thread block takes `group` consecutive high strings of one sector (number of high
+// pairs); a thread takes whole rows, in eight running sums (two per kind of hop) that
+// meet in a fixed order.
+// Threads per block (and rows it aims at): 256 in FP32, 512 in FP64, whose staged
+// blocks leave room for two thread blocks per SM (L=24: 843 us with 256, 751 with 512;
+// FP32 227 and 348).
+template <typename T>
+__host__ __device__ constexpr int split_threads() {
+    return sizeof(T) == 4 ? 256 : 512;
+}
+constexpr size_t kSplitMaxSmem = 112 * 1024;  // two FP64 blocks per SM
+// The split product serves spaces of at least kSplitMinRows rows whose blocks hold at
+// least kSplitMinBlock strings on average. Below, a block's preparation (neighbour
+// starts, staging) shows: L=16 8 pairs, 12,870 rows, FP32 13.5 us against 11.5 of the
+// general kernel, L=17 8 pairs, 24,310 rows, 14.5 against 20.6. Few pairs (or holes) in
+// many orbitals make blocks of a string or two: L=40 4 pairs (3.8 a block) 77.9 against
+// 63.7 us, L=30 26 pairs (6.8) 37.9 against 35.0, L=30 5 pairs (11.3) 51.4 against 74.9.
+constexpr int64_t kSplitMinRows = 20000;
+constexpr int64_t kSplitMinBlock = 10;
+
+// Bytes of shared memory of one thread block (the kernel carves it in this order).
+template <typename T>
+__host__ __device__ inline size_t split_smem(int s, int Lh, const DociSector &c) {
+    const size_t g = c.group[sizeof(T) == 8], nv = Lh - c.nh, nhh = (size_t)c.nh * nv;
+    size_t b = sizeof(T) * ((size_t)s * s + g * (c.nlow + nv * c.nminus + c.nh * c.nplus + (size_t)Lh * s + nhh));
+    b = (b + 7) & ~(size_t)7;
+    return b + 8 * g + 4 * g * (nhh + 1 + Lh);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(split_threads<T>()) k_doci_split(const DociSplitView p, const T *__restrict__ K,
+                                                              const T *__restrict__ diag, const T *__restrict__ x,
+                                                              T *__restrict__ y) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NT = split_threads<T>(), kType = sizeof(T) == 8;
+    const int s = p.s, Lh = p.L - p.s, L = p.L;
+    int q = 0;
+    while (q + 1 < p.nsec && blockIdx.x >= p.sec[q + 1].first_task[kType]) ++q;
+    const DociSector &c = p.sec[q];
+    const int nh = c.nh, nv = Lh - nh, m = c.m, nhh = nh * nv;
+    const int nlow = (int)c.nlow, nminus = (int)c.nminus, nplus = (int)c.nplus;
+    const int gmax = c.group[kType];
+    const uint32_t h0 = (blockIdx.x - c.first_task[kType]) * (uint32_t)gmax;
+    const int g = (int)min((uint32_t)gmax, c.nhigh - h0);
+    T *Kll = reinterpret_cast<T *>(smem);          // [s * s]
+    T *own = Kll + s * s;                          // [g][nlow]
+    T *up = own + (size_t)gmax * nlow;             // [g][nv][nminus]: the blocks h + k
+    T *dn = up + (size_t)gmax * nv * nminus;       // [g][nh][nplus]: the blocks h - k
+    T *Kup = dn + (size_t)gmax * nh * nplus;       // [g][nv][s]: K of the staged blocks' k
+    T *Kdn = Kup + (size_t)gmax * nv * s;          // [g][nh][s]
+    T *Khh = Kdn + (size_t)gmax * nh * s;          // [g][nhh]
+    uint64_t *hb = reinterpret_cast<uint64_t *>((reinterpret_cast<uintptr_t>(Khh + (size_t)gmax * nhh) + 7) & ~(uintptr_t)7);
+    uint32_t *hhb = reinterpret_cast<uint32_t *>(hb + gmax);  // [g][nhh]: starts of the high-high targets
+    uint32_t *rb = hhb + (size_t)gmax * nhh;                  // [g][1 + Lh]: starts of the block, h + k, h - k
+    const int t = threadIdx.x;
+    for (int i = t; i < g; i += NT) {
+        hb[i] = __ldg(p.hbits + c.high0 + h0 + i);
+        rb[i * (1 + Lh)] = __ldg(p.hbase + c.high0 + h0 + i);
+    }
+    for (int i = t; i < s * s; i += NT) Kll[i] = __ldg(K + (i / s) * L + i % s);
+    __syncthreads();
+    // start of the block with high string b and mm low pairs: the high pairs' part of
+    // the rank
+    auto start_of = [&](uint64_t b, int mm) {
+        uint32_t r = 0;
+        for (int k = mm + 1; b; b &= b - 1, ++k) r += __ldg(p.binom + (s + __ffsll((long long)b) - 1) * kSplitBinomRow + k);
+        return r;
+    };
+    // the i-th set bit of b
+    auto nth = [](uint64_t b, int i) {
+        for (; i > 0; --i) b &= b - 1;
+        return __ffsll((long long)b) - 1;
+    };
+    const uint64_t full = (((uint64_t)1) << Lh) - 1;
+    for (int e = t; e < g * Lh; e += NT) {  // the low-high neighbours: nv of h + k, nh of h - k
+        const int i = e / Lh, r = e - i * Lh;
+        const bool add = r < nv;
+        const int k = add ? nth(full & ~hb[i], r) : nth(hb[i], r - nv);
+        const bool any = add ? m > 0 : m < s;
+        rb[i * (1 + Lh) + 1 + r] = any ? start_of(hb[i] ^ ((uint64_t)1 << k), add ? m - 1 : m + 1) : 0u;
+        T *Kr = add ? Kup + ((size_t)i * nv + r) * s : Kdn + ((size_t)i * nh + r - nv) * s;
+        for (int j = 0; j < s; ++j) Kr[j] = __ldg(K + (s + k) * L + j);
+    }
+    for (int e = t; e < g * nhh; e += NT) {
+        const int i = e / nhh, r = e - i * nhh, a = r / nv;
+        const int j = nth(hb[i], a), k = nth(full & ~hb[i], r - a * nv);
+        hhb[e] = start_of(hb[i] ^ ((uint64_t)1 << j) ^ ((uint64_t)1 << k), m);
+        Khh[e] = __ldg(K + (s + j) * L + s + k);
+    }
+    __syncthreads();
+    auto stage = [&](T *dst, const uint32_t *starts, int rows, int per, int len) {
+        // rows = g * per blocks of len entries; row r starts at starts[(r / per) * (1 + Lh) + r % per]
+        const int warp = t >> 5, lane = t & 31;
+        if (len < 32) {
+            for (int e = t; e < rows * len; e += NT) {
+                const int r = e / len;
+                const uint32_t at = starts[(r / per) * (1 + Lh) + r % per] + (uint32_t)(e - r * len);
+                dst[e] = CIGPU_CHECK(p.err, index_ok(at, (uint64_t)p.D), kCheckHopRank, at) ? __ldg(x + at) : (T)0;
+            }
+            return;
+        }
+        for (int r = warp; r < rows; r += NT / 32) {
+            const uint32_t b = starts[(r / per) * (1 + Lh) + r % per];
+            for (int l = lane; l < len; l += 32) {
+                const uint32_t at = b + (uint32_t)l;
+                dst[(size_t)r * len + l] =
+                    CIGPU_CHECK(p.err, index_ok(at, (uint64_t)p.D), kCheckHopRank, at) ? __ldg(x + at) : (T)0;
+            }
+        }
+    };
+    stage(own, rb, g, 1, nlow);
+    if (m > 0 && nv > 0) stage(up, rb + 1, g * nv, nv, nminus);
+    if (m < s && nh > 0) stage(dn, rb + 1 + nv, g * nh, nh, nplus);
+    __syncthreads();
+    const uint32_t *ll = p.ll + c.ll0;
+    const uint16_t *lm = p.lminus + c.minus0, *lp = p.lplus + c.plus0;
+    const int nll = m * (s - m);
+    for (int it = t; it < g * nlow; it += NT) {
+        const int i = it / nlow, l = it - i * nlow;
+        const T *ow = own + (size_t)i * nlow;
+        T a0 = 0, a1 = 0, b0 = 0, b1 = 0, c0 = 0, c1 = 0, d0 = 0, d1 = 0;
+        {
+            const uint32_t *hs = hhb + (size_t)i * nhh;
+            const T *hk = Khh + (size_t)i * nhh;
+            int e = 0;
+            for (; e + 4 <= nhh; e += 4) {  // four loads in flight
+                T v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t at = hs[e + u] + (uint32_t)l;
+                    v[u] = CIGPU_CHECK(p.err, index_ok(at, (uint64_t)p.D), kCheckHopRank, at) ? __ldg(x + at) : (T)0;
+                }
+                a0 += hk[e] * v[0];
+                a1 += hk[e + 1] * v[1];
+                a0 += hk[e + 2] * v[2];
+                a1 += hk[e + 3] * v[3];
+            }
+            for (; e < nhh; ++e) {
+                const uint32_t at = hs[e] + (uint32_t)l;
+                a0 += hk[e] * (CIGPU_CHECK(p.err, index_ok(at, (uint64_t)p.D), kCheckHopRank, at) ? __ldg(x + at) : (T)0);
+            }
+        }
+        {
+            int e = 0;
+            for (; e + 4 <= nll; e += 4) {
+                uint32_t w[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) w[u] = __ldg(ll + (size_t)(e + u) * nlow + l);
+                b0 += Kll[w[0] >> 10] * ow[w[0] & 1023u];
+                b1 += Kll[w[1] >> 10] * ow[w[1] & 1023u];
+                b0 += Kll[w[2] >> 10] * ow[w[2] & 1023u];
+                b1 += Kll[w[3] >> 10] * ow[w[3] & 1023u];
+            }
+            for (; e < nll; ++e) {
+                const uint32_t w = __ldg(ll + (size_t)e * nlow + l);
+                b0 += Kll[w >> 10] * ow[w & 1023u];
+            }
+        }
+        if (nv > 0)
+            for (int e = 0; e < m; ++e) {
+                const uint32_t w = __ldg(lm + (size_t)e * nlow + l);
+                const T *xr = up + (size_t)i * nv * nminus + (w & 1023u), *kr = Kup + (size_t)i * nv * s + (w >> 10);
+                int r = 0;
+                for (; r + 2 <= nv; r += 2) {
+                    c0 += kr[0] * xr[0];
+                    c1 += kr[s] * xr[nminus];
+                    kr += 2 * s;
+                    xr += 2 * nminus;
+                }
+                if (r < nv) c0 += kr[0] * xr[0];
+            }
+        if (nh > 0)
+            for (int e = 0; e < s - m; ++e) {
+                const uint32_t w = __ldg(lp + (size_t)e * nlow + l);
+                const T *xr = dn + (size_t)i * nh * nplus + (w & 1023u), *kr = Kdn + (size_t)i * nh * s + (w >> 10);
+                int r = 0;
+                for (; r + 2 <= nh; r += 2) {
+                    d0 += kr[0] * xr[0];
+                    d1 += kr[s] * xr[nplus];
+                    kr += 2 * s;
+                    xr += 2 * nplus;
+                }
+                if (r < nh) d0 += kr[0] * xr[0];
+            }
+        const uint32_t row = rb[i * (1 + Lh)] + (uint32_t)l;
+        y[row] = ((a0 + a1) + (b0 + b1)) + ((c0 + c1) + (d0 + d1)) + __ldg(diag + row) * ow[l];
+    }
+}
+
+// The plan's tables. Sector q's low strings, by m pairs: thread per low string.
+__device__ __forceinline__ uint32_t low_rank(uint32_t b, const uint32_t *binom) {
+    uint32_t r = 0;
+    for (int k = 1; b; b &= b - 1, ++k) r += binom[(__ffs((int)b) - 1) * kSplitBinomRow + k];
+    return r;
+}
+
+__global__ void k_split_low(const DociSplitView p, uint32_t *__restrict__ ll, uint16_t *__restrict__ lminus,
+                            uint16_t *__restrict__ lplus) {
+    const DociSector &c = p.sec[blockIdx.y];
+    const int s = p.s, m = c.m;
+    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < c.nlow; l += gridDim.x * blockDim.x) {
+        uint32_t b = 0, rest = l;  // the low string of rank l
+        for (int k = m, o = s - 1; k > 0; --o)
+            if (p.binom[o * kSplitBinomRow + k] <= rest) {
+                rest -= p.binom[o * kSplitBinomRow + k];
+                b |= 1u << o;
+                --k;
+            }
+        int e = 0, em = 0, ep = 0;
+        for (int j = s - 1; j >= 0; --j) {
+            const uint32_t bj = b ^ (1u << j);
+            if (!((b >> j) & 1u)) {
+                lplus[c.plus0 + (uint32_t)ep++ * c.nlow + l] = (uint16_t)(low_rank(bj, p.binom) | ((uint32_t)j << 10));
+                continue;
+            }
+            lminus[c.minus0 + (uint32_t)em++ * c.nlow + l] = (uint16_t)(low_rank(bj, p.binom) | ((uint32_t)j << 10));
+            for (int k = s - 1; k >= 0; --k)
+                if (!((b >> k) & 1u))
+                    ll[c.ll0 + (uint32_t)e++ * c.nlow + l] =
+                        low_rank(bj ^ (1u << k), p.binom) | ((uint32_t)(j * s + k) << 10);
+        }
+    }
+}
+
+// High strings and block starts, sector by sector.
+__global__ void k_split_high(const DociSplitView p, uint64_t *__restrict__ hbits, uint32_t *__restrict__ hbase) {
+    const DociSector &c = p.sec[blockIdx.y];
+    const int Lh = p.L - p.s;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.nhigh; i += gridDim.x * blockDim.x) {
+        uint64_t b = 0;
+        uint32_t rest = i, r = 0;
+        for (int k = c.nh, o = Lh - 1; k > 0; --o)
+            if (p.binom[o * kSplitBinomRow + k] <= rest) {
+                rest -= p.binom[o * kSplitBinomRow + k];
+                b |= (uint64_t)1 << o;
+                r += p.binom[(p.s + o) * kSplitBinomRow + c.m + k];
+                --k;
+            }
+        hbits[c.high0 + i] = b;
+        hbase[c.high0 + i] = r;
+    }
+}
+
+template <typename T>
+void launch_split(const DociSplit &sp, const T *K, const T *diag, const T *x, T *y, cudaStream_t s) {
+    static const cudaError_t attr = cudaFuncSetAttribute(k_doci_split<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)kSplitMaxSmem);
+    CIGPU_CUDA(attr);
+    constexpr int kType = sizeof(T) == 8;
+    DociSplitView v = sp.view;
+    v.err = check_word_device();
+    k_doci_split<T><<<v.tasks[kType], split_threads<T>(), sp.smem[kType], s>>>(v, K, diag, x, y);
+    CIGPU_CUDA(cudaGetLastError());
+    count_launch();
+}
+
 // K_jk = (jk|jk) (chemist), zero where |v| <= 1e-14 and on the diagonal; FP64 and FP32.
 __global__ void k_doci_pair_table(int L, const double *__restrict__ eri, double *__restrict__ K64,
                                   float *__restrict__ K32) {
@@ -255,12 +538,95 @@ int64_t count_nonzero(const double *v, int64_t n, cudaStream_t s) {
     return (int64_t)h;
 }
 
-void doci_mv64(const DociMv &p, const double *K, const double *diag, const double *x, double *y, cudaStream_t s) {
-    launch_mv<double>(p, K, diag, x, y, s);
+void doci_split_make(int L, int n, int64_t D, DociSplit &sp, cudaStream_t st) {
+    sp.view = DociSplitView{};
+    if (n < 1 || n >= L || D < kSplitMinRows) return;
+    DociSplitView v{};
+    v.L = L;
+    v.n = n;
+    v.D = D;
+    uint32_t nll = 0, nmi = 0, npl = 0, nhi = 0;
+    for (int s = std::min(kSplitMaxLow, (L + 1) / 2); s >= 4; --s) {
+        const int Lh = L - s;
+        size_t bytes[2] = {0, 0};
+        uint64_t tasks[2] = {0, 0};
+        nll = nmi = npl = nhi = 0;
+        v.nsec = 0;
+        for (int m = std::max(0, n - Lh); m <= std::min(s, n); ++m) {
+            DociSector c{};
+            c.m = m;
+            c.nh = n - m;
+            c.nhigh = (uint32_t)d_binom(Lh, c.nh);
+            c.nlow = (uint32_t)d_binom(s, m);
+            c.nminus = m > 0 ? (uint32_t)d_binom(s, m - 1) : 0u;
+            c.nplus = m < s ? (uint32_t)d_binom(s, m + 1) : 0u;
+            for (int k = 0; k < 2; ++k) {
+                const auto need = [&] { return k ? split_smem<double>(s, Lh, c) : split_smem<float>(s, Lh, c); };
+                const uint32_t want = (uint32_t)(k ? split_threads<double>() : split_threads<float>()) / c.nlow;
+                c.group[k] = (int)std::min({std::max(want, 1u), c.nhigh, 64u});
+                while (c.group[k] > 1 && need() > kSplitMaxSmem / (k ? 1 : 2)) --c.group[k];
+                c.first_task[k] = (uint32_t)tasks[k];
+                tasks[k] += (c.nhigh + c.group[k] - 1) / c.group[k];
+                bytes[k] = std::max(bytes[k], need());
+            }
+            c.high0 = nhi;
+            c.ll0 = nll;
+            c.minus0 = nmi;
+            c.plus0 = npl;
+            nhi += c.nhigh;
+            nll += (uint32_t)(m * (s - m)) * c.nlow;
+            nmi += (uint32_t)m * c.nlow;
+            npl += (uint32_t)(s - m) * c.nlow;
+            v.sec[v.nsec++] = c;
+        }
+        if (std::max(bytes[0], bytes[1]) <= kSplitMaxSmem && std::max(tasks[0], tasks[1]) <= (uint64_t)INT32_MAX) {
+            v.s = s;
+            for (int k = 0; k < 2; ++k) {
+                v.tasks[k] = (uint32_t)tasks[k];
+                sp.smem[k] = bytes[k];
+            }
+            break;
+        }
+    }
+    if (v.s == 0 || (int64_t)nhi * kSplitMinBlock > D) return;
+    std::vector<uint32_t> bin((size_t)64 * kSplitBinomRow);
+    for (int p = 0; p < 64; ++p)
+        for (int k = 0; k < kSplitBinomRow; ++k) bin[(size_t)p * kSplitBinomRow + k] = p <= L && k <= n + 1 ? (uint32_t)d_binom(p, k) : 0u;
+    sp.binom.alloc(bin.size());
+    CIGPU_CUDA(cudaMemcpyAsync(sp.binom.p, bin.data(), bin.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    sp.hbits.alloc(nhi);
+    sp.hbase.alloc(nhi);
+    sp.ll.alloc(std::max(nll, 1u));
+    sp.lminus.alloc(std::max(nmi, 1u));
+    sp.lplus.alloc(std::max(npl, 1u));
+    v.hbits = sp.hbits.p;
+    v.hbase = sp.hbase.p;
+    v.binom = sp.binom.p;
+    v.ll = sp.ll.p;
+    v.lminus = sp.lminus.p;
+    v.lplus = sp.lplus.p;
+    k_split_low<<<dim3(4, v.nsec), 256, 0, st>>>(v, sp.ll.p, sp.lminus.p, sp.lplus.p);
+    k_split_high<<<dim3(64, v.nsec), 256, 0, st>>>(v, sp.hbits.p, sp.hbase.p);
+    CIGPU_CUDA(cudaGetLastError());
+    count_launch(2);
+    CIGPU_CUDA(cudaStreamSynchronize(st));  // the binomial table goes out of scope
+    sp.view = v;
 }
 
-void doci_mv32(const DociMv &p, const float *K, const float *diag, const float *x, float *y, cudaStream_t s) {
-    launch_mv<float>(p, K, diag, x, y, s);
+void doci_mv64(const DociMv &p, const DociSplit &split, const double *K, const double *diag, const double *x,
+               double *y, cudaStream_t s) {
+    if (split)
+        launch_split<double>(split, K, diag, x, y, s);
+    else
+        launch_mv<double>(p, K, diag, x, y, s);
+}
+
+void doci_mv32(const DociMv &p, const DociSplit &split, const float *K, const float *diag, const float *x, float *y,
+               cudaStream_t s) {
+    if (split)
+        launch_split<float>(split, K, diag, x, y, s);
+    else
+        launch_mv<float>(p, K, diag, x, y, s);
 }
 
 }  // namespace cigpu

@@ -275,3 +275,24 @@ def test_mixed_restart_keeps_the_previous_ritz_direction():
     assert abs(m.get_ci_energy() - ref.get_ci_energy()) < 1e-6
     assert m.info["restarts"] >= 1
     assert m.info["matvecs_fp32"] < 150, m.info
+
+
+@pytest.mark.parametrize("L,n", [(17, 8), (18, 11), (21, 5), (22, 17), (24, 18)])
+def test_doci_split_product(L, n):
+    """The DOCI product by low and high orbitals (spaces past its row threshold: odd and
+    even splits, few pairs, few holes), FP64 and FP32, against the oracle's matvec; the
+    bounds are the roundings of a row's terms."""
+    torch = pytest.importorskip("torch")
+    ints = make_integrals(L, n, n, nchol=6, seed=L + n)
+    ref = O.build_upper(O.DOCI, ints)
+    m = build(DOCI, ints, A.MIXED).get_mat()
+    x = np.random.default_rng(5).standard_normal(m.n).astype(np.float32).astype(np.float64)
+    y_ref = O.sym_mvprod(ref, x, threaded=True)
+    terms = n * (L - n) + 3
+    most = np.abs(ref.full_csr()) @ np.abs(x)  # a row's sum of magnitudes
+    for dt, eps in ((torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)):
+        xd = torch.tensor(x, dtype=dt, device="cuda")
+        yd = torch.full_like(xd, float("nan"))
+        m.mvprod_device(xd, yd)
+        torch.cuda.synchronize()
+        assert np.all(np.abs(yd.cpu().numpy().astype(np.float64) - y_ref) <= 2 * terms * eps * most + 1e-300)
