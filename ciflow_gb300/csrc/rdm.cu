@@ -7,19 +7,23 @@
 //
 // FCI. Write C[Ia][Ib] for the CI vector. Every contribution of fill_density_matrix
 // (CIDens.cpp:676-881) with a pair (I, J), I <= J in row order, is one of
-//   * alpha pair (Ia, Ja >= Ia, same Ib): diagonal, single or alpha-alpha double.
-//     Its weight only needs the string-pair densities
-//        Da0[Ia,Ja]    = sum_b C[Ia][b] C[Ja][b]
-//        Daz[Ia,Ja][z] = sum_b C[Ia][b] C[Ja][b] n_z(b)    (beta spectators z)
+//   * alpha pair (Ia, Ja >= Ia, same Ib): diagonal, single or alpha-alpha double. The
+//     same-spin elements only need the string-pair densities
+//        D[Ia,Ja] = sum_b C[Ia][b] C[Ja][b];
 //   * beta pair (Ib, Jb > Ib, same Ia): the mirror image with C transposed;
-//   * alpha-beta double (Ia -> Ja = Ia - ar + ac, ac > ar; Ib -> Jb = Ib - br + bc):
-//        Gamma_ab[(ar,br),(ac,bc)] += s_a s_b C[Ia][Ib] C[Ja][Jb].
-// Step 1 computes the pair densities (one warp per string pair). Step 2 sums, for
-// each RDM element, a host-built list of (density, +/-1) terms -- the list encodes
-// the reference's orbital ordering and antisymmetry signs (add_one_rdm /
-// add_two_rdm, CIDens.cpp:227-292). Step 3 handles the alpha-beta doubles: one
-// block per alpha excitation (ar, ac) (split in a few parts), one thread per beta
-// excitation type (br, bc), looping over the strings that admit it.
+//   * Gamma_ab[(ar,br),(ac,bc)], a product of an alpha and a beta excitation or
+//     occupation.
+// Step 1 computes the pair densities (a warp per eight string pairs). Step 2 sums, for
+// each same-spin RDM element, a host-built list of (density, +/-1) terms -- the list
+// encodes the reference's orbital ordering and antisymmetry signs (add_one_rdm /
+// add_two_rdm, CIDens.cpp:227-292). Step 3, the alpha-beta block: for each alpha
+// excitation (ar < ac) the string sums
+//        g_x[Ib] = sum_(Ia -> Ja) s_a C[Ia][Ib] C[Ja][x(Ib)]
+// over its string pairs, x the identity or one of Ib's single excitations, one thread
+// per Ib with its sums in registers; then the sums of s_b g_x[Ib] over the Ib that
+// belong to each (br, bc). The identity's sums, over the Ib that hold z, are the
+// elements with beta occupation z; the mirror pass (identity only) gives those with
+// alpha occupation.
 //
 // DOCI: one block of L*L threads per slice of pair strings; thread (j, k)
 // accumulates c_I^2 n_j n_k and the pair-hop products c_I c_J (DensDOCI,
@@ -76,28 +80,35 @@ int hnstacked(int a, int b, uint64_t common) {
 // One spin's pair list and its RDM terms.
 struct PairPlan {
     std::vector<uint32_t> I, J;  // pairs: [self..., singles..., doubles...]
-    int nz = 0;                  // the first nz pairs (self + singles) also need Dz
 };
 
 struct Plan {
     int L, np;
     int64_t Da, Db;
     PairPlan a, b;
-    size_t off_ga, off_gb, off_g0, off_g1, off_g2, nslots;
-    // density layout: [Da0 | Daz | Db0 | Dbz]
-    size_t off_da0, off_daz, off_db0, off_dbz, ndens;
+    size_t off_ga, off_gb, off_g0, off_g2, nslots;
+    // density layout: [Da | Db]
+    size_t off_da, off_db, ndens;
     struct Term {
         uint32_t slot, dens;
         int8_t coef;
     };
     std::vector<Term> terms;  // in generation order; grouped by slot (stably) afterwards
-    // alpha-beta doubles
-    std::vector<uint32_t> ap_ptr;   // [np+1] alpha pairs per (ar<ac)
-    std::vector<uint64_t> ap;       // Ia | Ja << 32
-    std::vector<int8_t> ap_sign;
-    std::vector<uint32_t> bx_ptr;   // [L*L+1] beta excitations per (br, bc)
-    std::vector<uint64_t> bx;       // Ib | Jb << 32
-    std::vector<int8_t> bx_sign;
+};
+
+// String pairs of each excitation of one spin: list pidx(r, c), r < c, holds the pairs
+// (I, J = I - r + c) with their signs; with `diag`, list np + u the strings (I, I)
+// holding orbital u.
+struct ExcitationLists {
+    std::vector<uint32_t> ptr;
+    std::vector<uint64_t> pair;  // I | J << 32
+    std::vector<int8_t> sign;
+};
+
+// The members of each sum over strings: place x * D + I in the string sums, the sign in
+// bit 31.
+struct SumLists {
+    std::vector<uint32_t> ptr, at;
 };
 
 void add_term(Plan &P, size_t slot, size_t dens, int coef) {
@@ -117,13 +128,7 @@ void add_two_same(Plan &P, size_t off, int o1, int o2, int o3, int o4, size_t de
     add_term(P, sym_slot(off, P.np, pidx(o1, o2, P.L), pidx(o3, o4, P.L)), dens, coef);
 }
 
-void add_two_ab(Plan &P, int o1, int o2, int o3, int o4, size_t dens, int coef) {
-    const size_t L = P.L;
-    add_term(P, sym_slot(P.off_g1, L * L, o1 * L + o2, o3 * L + o4), dens, coef);
-}
-
-// Pairs and terms of one spin. `alpha` selects which 1-RDM / same-spin block and
-// where the opposite-spin spectators go in Gamma_ab.
+// Pairs and terms of one spin. `alpha` selects which 1-RDM / same-spin block.
 void plan_spin(Plan &P, const SpinTables &t, bool alpha) {
     const int L = P.L, n = t.n;
     PairPlan &pp = alpha ? P.a : P.b;
@@ -152,7 +157,6 @@ void plan_spin(Plan &P, const SpinTables &t, bool alpha) {
         pp.I.push_back(x.I);
         pp.J.push_back(x.J);
     }
-    pp.nz = (int)pp.I.size();
     // upper same-spin doubles
     struct Dbl { uint32_t I, J; int o[4]; int sign; };
     std::vector<Dbl> dbls;
@@ -185,8 +189,7 @@ void plan_spin(Plan &P, const SpinTables &t, bool alpha) {
     }
     (void)n;
     // terms
-    const size_t d0 = alpha ? P.off_da0 : P.off_db0;
-    const size_t dz = alpha ? P.off_daz : P.off_dbz;
+    const size_t d0 = alpha ? P.off_da : P.off_db;
     const size_t g1 = alpha ? P.off_ga : P.off_gb;
     const size_t gs = alpha ? P.off_g0 : P.off_g2;
     for (int64_t I = 0; I < D; ++I) {  // self pairs (fill_diagonal, CIDens.cpp:808-853)
@@ -197,21 +200,13 @@ void plan_spin(Plan &P, const SpinTables &t, bool alpha) {
         for (int i = 0; i < k; ++i) add_term(P, sym_slot(g1, L, o[i], o[i]), d0 + I, 1);
         for (int i = 0; i < k; ++i)
             for (int j = i + 1; j < k; ++j) add_two_same(P, gs, o[i], o[j], o[i], o[j], d0 + I, 1);
-        if (alpha)  // mixed diagonal part, once (alpha side): Gamma_ab(u z, u z) += sum c^2 n_u n_z
-            for (int i = 0; i < k; ++i)
-                for (int z = 0; z < L; ++z) add_two_ab(P, o[i], z, o[i], z, dz + (size_t)I * L + z, 1);
     }
     for (size_t q = 0; q < singles.size(); ++q) {  // fill_one_dense (CIDens.cpp:676-754)
         const Single &x = singles[q];
         const size_t pi = (size_t)D + q;
         add_term(P, sym_slot(g1, L, x.lo, x.hi), d0 + pi, x.sign);
-        for (int z = 0; z < L; ++z) {
+        for (int z = 0; z < L; ++z)
             if ((x.common >> z) & 1) add_two_same(P, gs, x.lo, z, x.hi, z, d0 + pi, x.sign);
-            if (alpha)
-                add_two_ab(P, x.lo, z, x.hi, z, dz + pi * L + z, x.sign);
-            else
-                add_two_ab(P, z, x.lo, z, x.hi, dz + pi * L + z, x.sign);
-        }
     }
     for (size_t q = 0; q < dbls.size(); ++q) {
         const Dbl &x = dbls[q];
@@ -220,86 +215,121 @@ void plan_spin(Plan &P, const SpinTables &t, bool alpha) {
     }
 }
 
-void plan_ab(Plan &P, const SpinTables &ta, const SpinTables &tb) {
-    const int L = P.L;
-    // alpha excitations ar -> ac with ac > ar (the row is the lower-ranked string)
-    std::vector<std::vector<std::pair<uint64_t, int8_t>>> apl(P.np);
-    for (int64_t I = 0; I < ta.D; ++I) {
-        const uint64_t s = ta.strings[I];
-        for (int ar = 0; ar < L; ++ar) {
-            if (!((s >> ar) & 1)) continue;
-            for (int ac = ar + 1; ac < L; ++ac) {
-                if ((s >> ac) & 1) continue;
-                const uint64_t u = s ^ ((uint64_t)1 << ar) ^ ((uint64_t)1 << ac);
-                const int sign = (hnstacked(ar, ac, s & u) & 1) ? -1 : 1;
-                apl[pidx(ar, ac, L)].push_back({(uint64_t)I | ((uint64_t)hrank(u) << 32), (int8_t)sign});
+ExcitationLists excitation_lists(const SpinTables &t, bool diag) {
+    const int L = t.L, np = L * (L - 1) / 2, nl = np + (diag ? L : 0);
+    ExcitationLists e;
+    e.ptr.assign((size_t)nl + 1, 0);
+    auto each = [&](auto &&f) {  // f(list, I, J, odd) in the order of the strings
+        for (int64_t I = 0; I < t.D; ++I) {
+            for (int x = 0; x < t.ns; ++x) {
+                const uint32_t w = t.s_info[(size_t)I * t.ns + x];
+                const int r = (w >> 12) & 63, c = (w >> 18) & 63;
+                if (r < c) f(pidx(r, c, L), I, t.s_target[(size_t)I * t.ns + x], (w >> 24) & 1u);
+            }
+            if (diag)
+                for (int m = 0; m < t.n; ++m) f(np + t.occ[(size_t)I * t.n + m], I, (uint32_t)I, 0u);
+        }
+    };
+    each([&](int q, int64_t, uint32_t, uint32_t) { ++e.ptr[(size_t)q + 1]; });
+    for (int q = 0; q < nl; ++q) e.ptr[(size_t)q + 1] += e.ptr[q];
+    e.pair.resize(e.ptr[nl]);
+    e.sign.resize(e.ptr[nl]);
+    std::vector<uint32_t> fill(e.ptr.begin(), e.ptr.end() - 1);
+    each([&](int q, int64_t I, uint32_t J, uint32_t odd) {
+        e.pair[fill[q]] = (uint64_t)I | ((uint64_t)J << 32);
+        e.sign[fill[q]++] = odd ? -1 : 1;
+    });
+    return e;
+}
+
+// The sums (r, c), r != c, over the single excitations r -> c of one spin's strings
+// (singles), and the sums over the strings that hold z, list z * L + z (or z without
+// singles) of the identity's place.
+SumLists sum_lists(const SpinTables &t, bool singles) {
+    const int L = t.L, nl = singles ? L * L : L;
+    const uint32_t D = (uint32_t)t.D, ident = singles ? (uint32_t)t.ns * D : 0u;
+    SumLists e;
+    e.ptr.assign((size_t)nl + 1, 0);
+    auto each = [&](auto &&f) {
+        for (int64_t I = 0; I < t.D; ++I) {
+            if (singles)
+                for (int x = 0; x < t.ns; ++x) {
+                    const uint32_t w = t.s_info[(size_t)I * t.ns + x];
+                    f((int)((w >> 12) & 63) * L + (int)((w >> 18) & 63), (uint32_t)x * D + (uint32_t)I, (w >> 24) & 1u);
+                }
+            for (int m = 0; m < t.n; ++m) {
+                const int z = t.occ[(size_t)I * t.n + m];
+                f(singles ? z * L + z : z, ident + (uint32_t)I, 0u);
             }
         }
-    }
-    P.ap_ptr.assign(P.np + 1, 0);
-    for (int q = 0; q < P.np; ++q) {
-        P.ap_ptr[q + 1] = P.ap_ptr[q] + (uint32_t)apl[q].size();
-        for (auto &e : apl[q]) {
-            P.ap.push_back(e.first);
-            P.ap_sign.push_back(e.second);
-        }
-    }
-    // beta excitations br -> bc (any order)
-    std::vector<std::vector<std::pair<uint64_t, int8_t>>> bxl((size_t)L * L);
-    for (int64_t I = 0; I < tb.D; ++I) {
-        const uint64_t s = tb.strings[I];
-        for (int br = 0; br < L; ++br) {
-            if (!((s >> br) & 1)) continue;
-            for (int bc = 0; bc < L; ++bc) {
-                if ((s >> bc) & 1) continue;
-                const uint64_t u = s ^ ((uint64_t)1 << br) ^ ((uint64_t)1 << bc);
-                const int sign = (hnstacked(br, bc, s & u) & 1) ? -1 : 1;
-                bxl[(size_t)br * L + bc].push_back({(uint64_t)I | ((uint64_t)hrank(u) << 32), (int8_t)sign});
-            }
-        }
-    }
-    P.bx_ptr.assign((size_t)L * L + 1, 0);
-    for (size_t q = 0; q < (size_t)L * L; ++q) {
-        P.bx_ptr[q + 1] = P.bx_ptr[q] + (uint32_t)bxl[q].size();
-        for (auto &e : bxl[q]) {
-            P.bx.push_back(e.first);
-            P.bx_sign.push_back(e.second);
-        }
-    }
+    };
+    each([&](int q, uint32_t, uint32_t) { ++e.ptr[(size_t)q + 1]; });
+    for (int q = 0; q < nl; ++q) e.ptr[(size_t)q + 1] += e.ptr[q];
+    e.at.resize(e.ptr[nl]);
+    std::vector<uint32_t> fill(e.ptr.begin(), e.ptr.end() - 1);
+    each([&](int q, uint32_t at, uint32_t odd) { e.at[fill[q]++] = at | (odd << 31); });
+    return e;
 }
 
 // ---------------------------------------------------------------------------
-// Step 1: pair densities. C is D1 x D2 row-major; other = strings of the D2 spin.
-__global__ void k_pair_dens(const double *__restrict__ C, int64_t D2, const uint32_t *__restrict__ pI,
-                            const uint32_t *__restrict__ pJ, int64_t npairs, int64_t nz,
-                            const uint64_t *__restrict__ other, int L, double *__restrict__ d0,
-                            double *__restrict__ dz, int64_t D1, unsigned long long *err) {
+// Step 1: pair densities. C is D1 x D2 row-major. A warp takes eight pairs, which
+// mostly share their first string (the lists run over it): nine coalesced loads feed
+// eight multiply-adds, and the eight sums meet in one exchange of halves. Bound by the
+// FP64 pipe (2 lanes per clock and SM): 112 M multiply-adds per spin at L=12 6a6b,
+// 0.18 ms at its rate, 0.20 measured (1.23 ms when the same kernel also formed the
+// densities weighted by the other spin's occupations, 12 of 32 lanes at work).
+constexpr int kPairBatch = 8;
+
+__global__ void __launch_bounds__(kRdmThreads) k_pair_dens(const double *__restrict__ C, int64_t D2,
+                                                           const uint32_t *__restrict__ pI,
+                                                           const uint32_t *__restrict__ pJ, int64_t npairs,
+                                                           double *__restrict__ dens, int64_t D1,
+                                                           unsigned long long *err) {
     const int lane = threadIdx.x & 31;
     const int64_t wid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t p = wid; p < npairs; p += nw) {
-        const uint32_t I = pI[p], J = pJ[p];
-        if (!CIGPU_CHECK(err, index_ok(I, (uint64_t)D1) && index_ok(J, (uint64_t)D1), kCheckRdmPair, p)) {
-            if (lane == 0) d0[p] = 0;  // the same for the whole warp
-            if (p < nz)
-                for (int z = lane; z < L; z += 32) dz[p * L + z] = 0;
-            continue;
+    for (int64_t p0 = wid * kPairBatch; p0 < npairs; p0 += nw * kPairBatch) {
+        const double *ri[kPairBatch], *rj[kPairBatch];
+        bool same = true;
+#pragma unroll
+        for (int k = 0; k < kPairBatch; ++k) {
+            const int64_t p = p0 + k < npairs ? p0 + k : npairs - 1;  // a short last batch repeats its last pair
+            uint32_t I = pI[p], J = pJ[p];
+            if (!CIGPU_CHECK(err, index_ok(I, (uint64_t)D1) && index_ok(J, (uint64_t)D1), kCheckRdmPair, p)) I = J = 0;
+            ri[k] = C + (int64_t)I * D2;
+            rj[k] = C + (int64_t)J * D2;
+            same = same && ri[k] == ri[0];
         }
-        const double *ri = C + (int64_t)I * D2;
-        const double *rj = C + (int64_t)J * D2;
-        double acc = 0;
-        for (int64_t b = lane; b < D2; b += 32) acc += ri[b] * rj[b];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) d0[p] = acc;
-        if (p < nz) {
-            for (int z0 = 0; z0 < L; z0 += 32) {
-                const int z = z0 + lane;
-                double az = 0;
-                for (int64_t b = 0; b < D2; ++b)
-                    if (z < L && ((other[b] >> z) & 1)) az += ri[b] * rj[b];
-                if (z < L) dz[p * L + z] = az;
+        double acc[kPairBatch];
+#pragma unroll
+        for (int k = 0; k < kPairBatch; ++k) acc[k] = 0;
+        if (same) {
+            for (int64_t b = lane; b < D2; b += 32) {
+                const double v = ri[0][b];
+#pragma unroll
+                for (int k = 0; k < kPairBatch; ++k) acc[k] += v * rj[k][b];
+            }
+        } else {
+            for (int64_t b = lane; b < D2; b += 32) {
+#pragma unroll
+                for (int k = 0; k < kPairBatch; ++k) acc[k] += ri[k][b] * rj[k][b];
             }
         }
+        // halves exchanged: after three steps lane l holds a quarter warp's sum of pair l / 4
+#pragma unroll
+        for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
+            const bool hi = lane & o;
+#pragma unroll
+            for (int k = 0; k < h; ++k) {
+                const double give = hi ? acc[k] : acc[k + h];
+                const double keep = hi ? acc[k + h] : acc[k];
+                acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+        double a = acc[0];
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        if ((lane & 3) == 0 && p0 + (lane >> 2) < npairs) dens[p0 + (lane >> 2)] = a;
     }
 }
 
@@ -317,62 +347,145 @@ __global__ void k_slot_gather(const uint32_t *__restrict__ ptr, const uint32_t *
     }
 }
 
-// Step 3: alpha-beta doubles. Block = (alpha excitation q = pidx(ar,ac), split);
-// thread = beta excitation type (br, bc). slices[(q*nsplit + split)*L*L + br*L + bc].
-__global__ void k_ab_doubles(const double *__restrict__ C, int64_t Db, const uint32_t *__restrict__ ap_ptr,
-                             const uint64_t *__restrict__ ap, const int8_t *__restrict__ ap_sign,
-                             const uint32_t *__restrict__ bx_ptr, const uint64_t *__restrict__ bx,
-                             const int8_t *__restrict__ bx_sign, int L, int nsplit, double *__restrict__ slices,
-                             int64_t Da, unsigned long long *err) {
-    extern __shared__ double rows[];  // [2][Db]
-    const int q = blockIdx.x / nsplit, split = blockIdx.x % nsplit;
-    const uint32_t a0 = ap_ptr[q], a1 = ap_ptr[q + 1];
-    const uint32_t cnt = a1 - a0, per = (cnt + nsplit - 1) / nsplit;
-    const uint32_t s0 = a0 + min(cnt, split * per), s1 = a0 + min(cnt, (split + 1) * per);
-    const int ntypes = L * L;
-    constexpr int kMaxTypesPerThread = 8;
-    double acc[kMaxTypesPerThread];
-    for (int i = 0; i < kMaxTypesPerThread; ++i) acc[i] = 0;
-    for (uint32_t e = s0; e < s1; ++e) {
-        const uint64_t pr = ap[e];
-        // the same pair for the whole block, so a skip keeps the barriers aligned
-        if (!CIGPU_CHECK(err, index_ok((uint32_t)pr, (uint64_t)Da) && index_ok((uint32_t)(pr >> 32), (uint64_t)Da),
-                         kCheckRdmPair, e))
-            continue;
-        const double *ri = C + (int64_t)(uint32_t)pr * Db;
-        const double *rj = C + (int64_t)(uint32_t)(pr >> 32) * Db;
-        __syncthreads();
-        for (int64_t b = threadIdx.x; b < Db; b += blockDim.x) {
-            rows[b] = ri[b];
-            rows[Db + b] = rj[b];
-        }
-        __syncthreads();
-        const double sa = (double)ap_sign[e];
-        for (int i = 0; i < kMaxTypesPerThread; ++i) {
-            const int ty = threadIdx.x + i * blockDim.x;
-            if (ty >= ntypes) break;
-            double part = 0;
-            for (uint32_t x = bx_ptr[ty]; x < bx_ptr[ty + 1]; ++x) {
-                const uint64_t bb = bx[x];
-                if (!CIGPU_CHECK(err, index_ok((uint32_t)bb, (uint64_t)Db) && index_ok((uint32_t)(bb >> 32), (uint64_t)Db),
-                                 kCheckRdmExcit, x))
-                    continue;
-                part += (double)bx_sign[x] * rows[(uint32_t)bb] * rows[Db + (uint32_t)(bb >> 32)];
-            }
-            acc[i] += sa * part;
-        }
-    }
-    for (int i = 0; i < kMaxTypesPerThread; ++i) {
-        const int ty = threadIdx.x + i * blockDim.x;
-        if (ty < ntypes) slices[((int64_t)q * nsplit + split) * ntypes + ty] = acc[i];
-    }
+// Step 3: string sums. For each string pair (I, J) of list q (C's first string) the
+// block stages row J and every thread, on its own second string S, adds
+// s C[I][S] C[J][x(S)] to the sums of kAbX of S's single excitations x, and (first
+// chunk) to the identity's. The sums stay in registers over the list's pairs and are
+// stored once, G[q - q0][x][S] (x = ns: the identity). A multiply-add per term and its
+// gather from shared memory: bound by the FP64 pipe, 0.57 G multiply-adds at L=12 6a6b,
+// 0.90 ms at its rate. (One thread per (br, bc) walking lists of string pairs, the
+// sign a second FP64 product, on 264 blocks of 160 threads: 4.36 ms. Now 1.39.)
+constexpr int kAbThreads = 128;
+constexpr int kAbX = 12;
+
+__device__ __forceinline__ void copy8_async(double *dst, const double *src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
 }
 
-// Assemble the outputs: gather sums + alpha-beta double slices, mirrored.
-__global__ void k_rdm_assemble(const double *__restrict__ acc, const double *__restrict__ slices, int nsplit, int L,
-                               int np, size_t off_ga, size_t off_gb, size_t off_g0, size_t off_g1, size_t off_g2,
-                               double *__restrict__ rdm1, double *__restrict__ aa, double *__restrict__ ab,
-                               double *__restrict__ bb) {
+__global__ void __launch_bounds__(kAbThreads) k_string_sums(const double *__restrict__ C, int64_t D2,
+                                                            const uint32_t *__restrict__ target, int ns,
+                                                            const uint32_t *__restrict__ ptr,
+                                                            const uint64_t *__restrict__ pair,
+                                                            const int8_t *__restrict__ sign, int q0,
+                                                            double *__restrict__ G, int64_t D1,
+                                                            unsigned long long *err) {
+    extern __shared__ double rows[];  // [2][D2]
+    const int q = q0 + blockIdx.z, x0 = blockIdx.y * kAbX, nx = min(kAbX, ns - x0);
+    const uint32_t e0 = ptr[q], e1 = ptr[q + 1];
+    const int64_t S = blockIdx.x * (int64_t)kAbThreads + threadIdx.x;
+    const bool act = S < D2;
+    uint32_t at[kAbX];
+#pragma unroll
+    for (int x = 0; x < kAbX; ++x) {
+        at[x] = 0;
+        if (act && x < nx) {
+            at[x] = __ldg(target + S * ns + x0 + x);
+            if (!CIGPU_CHECK(err, index_ok(at[x], (uint64_t)D2), kCheckRdmExcit, S)) at[x] = 0;
+        }
+    }
+    double acc[kAbX], ident = 0;
+#pragma unroll
+    for (int x = 0; x < kAbX; ++x) acc[x] = 0;
+    auto pair_of = [&](uint32_t e, uint32_t &I, uint32_t &J) {
+        const uint64_t pr = __ldg(pair + e);
+        I = (uint32_t)pr;
+        J = (uint32_t)(pr >> 32);
+        if (!CIGPU_CHECK(err, index_ok(I, (uint64_t)D1) && index_ok(J, (uint64_t)D1), kCheckRdmPair, e)) I = J = 0;
+    };
+    auto stage = [&](uint32_t e, double *dst) {
+        uint32_t I, J;
+        pair_of(e, I, J);
+        const double *src = C + (int64_t)J * D2;
+        for (int64_t b = threadIdx.x; b < D2; b += kAbThreads) copy8_async(dst + b, src + b);
+        asm volatile("cp.async.commit_group;");
+    };
+    if (e0 < e1) stage(e0, rows);
+    for (uint32_t e = e0; e < e1; ++e) {
+        const double *row = rows + ((e - e0) & 1) * D2;
+        uint32_t I, J;
+        pair_of(e, I, J);
+        double v = act ? C[(int64_t)I * D2 + S] : 0.0;
+        v = __longlong_as_double(__double_as_longlong(v) ^ ((long long)(__ldg(sign + e) < 0) << 63));
+        asm volatile("cp.async.wait_group 0;");
+        __syncthreads();  // this pair's row is staged; the other buffer is read
+        if (e + 1 < e1) stage(e + 1, rows + ((e + 1 - e0) & 1) * D2);
+        if (act) {
+            if (x0 == 0) ident += v * row[S];
+#pragma unroll
+            for (int x = 0; x < kAbX; ++x)
+                if (x < nx) acc[x] += v * row[at[x]];
+        }
+    }
+    if (!act) return;
+    double *g = G + (int64_t)blockIdx.z * (ns + 1) * D2 + S;
+#pragma unroll
+    for (int x = 0; x < kAbX; ++x)
+        if (x < nx) g[(int64_t)(x0 + x) * D2] = acc[x];
+    if (x0 == 0) g[(int64_t)ns * D2] = ident;
+}
+
+// The identity's string sums alone (no staging: row J is read at S itself).
+__global__ void __launch_bounds__(kAbThreads) k_string_sums_ident(const double *__restrict__ C, int64_t D2,
+                                                                  const uint32_t *__restrict__ ptr,
+                                                                  const uint64_t *__restrict__ pair,
+                                                                  const int8_t *__restrict__ sign, int q0,
+                                                                  double *__restrict__ G, int64_t D1,
+                                                                  unsigned long long *err) {
+    const int q = q0 + blockIdx.z;
+    const uint32_t e0 = ptr[q], e1 = ptr[q + 1];
+    const int64_t S = blockIdx.x * (int64_t)kAbThreads + threadIdx.x;
+    if (S >= D2) return;
+    constexpr int U = 8;  // pairs in flight
+    double acc = 0;
+    for (uint32_t e = e0; e < e1; e += U) {
+        double a[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            a[u] = b[u] = 0.0;
+            if (e + u < e1) {
+                const uint64_t pr = __ldg(pair + e + u);
+                uint32_t I = (uint32_t)pr, J = (uint32_t)(pr >> 32);
+                if (!CIGPU_CHECK(err, index_ok(I, (uint64_t)D1) && index_ok(J, (uint64_t)D1), kCheckRdmPair, e)) I = J = 0;
+                a[u] = C[(int64_t)I * D2 + S];
+                b[u] = C[(int64_t)J * D2 + S];
+                a[u] = __longlong_as_double(__double_as_longlong(a[u]) ^ ((long long)(__ldg(sign + e + u) < 0) << 63));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc += a[u] * b[u];
+    }
+    G[(int64_t)blockIdx.z * D2 + S] = acc;
+}
+
+// out[q][t] = the signed sum of list t over the string sums of q, one warp each.
+__global__ void k_sum_strings(const double *__restrict__ G, int64_t per_q, const uint32_t *__restrict__ ptr,
+                              const uint32_t *__restrict__ at, int nt, int nq, double *__restrict__ out,
+                              unsigned long long *err) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (w >= (int64_t)nq * nt) return;
+    const int64_t q = w / nt;
+    const int t = (int)(w - q * nt);
+    const double *g = G + q * per_q;
+    double v = 0;
+    for (uint32_t e = ptr[t] + lane; e < ptr[t + 1]; e += 32) {
+        const uint32_t k = at[e];
+        if (!CIGPU_CHECK(err, index_ok(k & 0x7FFFFFFFu, (uint64_t)per_q), kCheckRdmTerm, e)) continue;
+        const double x = g[k & 0x7FFFFFFFu];
+        v += __longlong_as_double(__double_as_longlong(x) ^ ((long long)(k >> 31) << 63));
+    }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) out[w] = v;
+}
+
+// Assemble the outputs, mirrored: the same-spin sums, and Gamma_ab's upper triangle
+// from t1[(ar < ac)][br, bc], t2[(br < bc)][z] (alpha occupation z) and, after the np
+// rows of t2, t2[np + u][z] (beta occupation u, alpha occupation z).
+__global__ void k_rdm_assemble(const double *__restrict__ acc, const double *__restrict__ t1,
+                               const double *__restrict__ t2, int L, int np, size_t off_ga, size_t off_gb,
+                               size_t off_g0, size_t off_g2, double *__restrict__ rdm1, double *__restrict__ aa,
+                               double *__restrict__ ab, double *__restrict__ bb) {
     const int64_t L2 = (int64_t)L * L;
     const int64_t n1 = 2 * L2, n2 = (int64_t)np * np, n3 = L2 * L2;
     const int64_t total = n1 + 2 * n2 + n3;
@@ -390,13 +503,14 @@ __global__ void k_rdm_assemble(const double *__restrict__ acc, const double *__r
             const int64_t j = i - n1 - 2 * n2;
             const int64_t A = j / L2, B = j % L2;
             const int64_t lo = min(A, B), hi = max(A, B);
-            double v = acc[off_g1 + (size_t)lo * L2 + hi];
-            const int ar = (int)(lo / L), ac = (int)(hi / L);
-            if (ar < ac) {
-                const int q = ar * L + ac - (ar + 1) * (ar + 2) / 2;
-                const int64_t ty = (lo % L) * L + (hi % L);
-                for (int sp = 0; sp < nsplit; ++sp) v += slices[((int64_t)q * nsplit + sp) * L2 + ty];
-            }
+            const int ar = (int)(lo / L), ac = (int)(hi / L), br = (int)(lo % L), bc = (int)(hi % L);
+            double v;
+            if (ar < ac)
+                v = t1[(int64_t)(ar * L + ac - (ar + 1) * (ar + 2) / 2) * L2 + br * L + bc];
+            else if (br < bc)
+                v = t2[(int64_t)(br * L + bc - (br + 1) * (br + 2) / 2) * L + ar];
+            else
+                v = t2[(int64_t)(np + br) * L + ar];
             ab[j] = v;
         }
     }
@@ -610,24 +724,23 @@ DevBuf<T> upload(const std::vector<T> &v, cudaStream_t s) {
 // term lists and the alpha-beta excitation lists. It depends on the string tables
 // only, so it is made on the first RDM call of a CRS and kept with it.
 struct FciRdmPlan {
-    int64_t npa = 0, nza = 0, npb = 0, nzb = 0;
+    int64_t npa = 0, npb = 0;
     size_t ndens = 0, nslots = 0;
-    size_t off_da0 = 0, off_daz = 0, off_db0 = 0, off_dbz = 0;
-    size_t off_ga = 0, off_gb = 0, off_g0 = 0, off_g1 = 0, off_g2 = 0;
-    int nsplit = 4;
-    DevBuf<uint64_t> sa, sb;                  // alpha / beta strings
+    size_t off_da = 0, off_db = 0;
+    size_t off_ga = 0, off_gb = 0, off_g0 = 0, off_g2 = 0;
     DevBuf<uint32_t> aI, aJ, bI, bJ;          // string pairs per spin
-    DevBuf<uint32_t> dptr, didx;              // terms of every RDM element (CSR)
+    DevBuf<uint32_t> dptr, didx;              // terms of every same-spin RDM element (CSR)
     DevBuf<int8_t> dcf;
-    DevBuf<uint32_t> app, bxp;                // alpha-beta doubles: alpha pairs per (ar<ac), beta per (br,bc)
-    DevBuf<uint64_t> apd, bxd;
-    DevBuf<int8_t> aps, bxs;
+    DevBuf<uint32_t> ap, bp;                  // alpha excitations ar < ac; beta ones and occupations
+    DevBuf<uint64_t> apair, bpair;
+    DevBuf<int8_t> asign, bsign;
+    DevBuf<uint32_t> btp, bta, atp, ata;      // sums over beta strings by (br, bc), over alpha strings by z
 };
 
 std::shared_ptr<FciRdmPlan> make_fci_rdm_plan(cigpu_crs &c, cudaStream_t s) {
     const int L = c.L, np = L * (L - 1) / 2;
     const int64_t L2 = (int64_t)L * L;
-    const int64_t n2 = (int64_t)np * np, n3 = L2 * L2;
+    const int64_t n2 = (int64_t)np * np;
     const SpinTables &ta = c.ta;
     const SpinTables &tb = (c.ndown == c.nup) ? c.ta : c.tb;
     Plan P;
@@ -639,31 +752,22 @@ std::shared_ptr<FciRdmPlan> make_fci_rdm_plan(cigpu_crs &c, cudaStream_t s) {
     P.off_gb = L2;
     P.off_g0 = 2 * L2;
     P.off_g2 = P.off_g0 + n2;
-    P.off_g1 = P.off_g2 + n2;
-    P.nslots = P.off_g1 + n3;
+    P.nslots = P.off_g2 + n2;
     // pair counts first (densities layout needs them)
-    auto count_pairs = [&](const SpinTables &t, size_t &npair, size_t &nz) {
-        size_t ns = 0, nd = 0;
+    auto count_pairs = [&](const SpinTables &t) {
+        size_t n = (size_t)t.D;
         for (int64_t I = 0; I < t.D; ++I) {
-            for (int q = 0; q < t.ns; ++q)
-                if (t.s_target[(size_t)I * t.ns + q] > (uint32_t)I) ++ns;
-            for (int q = 0; q < t.nd; ++q)
-                if (t.d_target[(size_t)I * t.nd + q] > (uint32_t)I) ++nd;
+            for (int q = 0; q < t.ns; ++q) n += t.s_target[(size_t)I * t.ns + q] > (uint32_t)I;
+            for (int q = 0; q < t.nd; ++q) n += t.d_target[(size_t)I * t.nd + q] > (uint32_t)I;
         }
-        nz = (size_t)t.D + ns;
-        npair = nz + nd;
+        return n;
     };
-    size_t npa, nza, npb, nzb;
-    count_pairs(ta, npa, nza);
-    count_pairs(tb, npb, nzb);
-    P.off_da0 = 0;
-    P.off_daz = npa;
-    P.off_db0 = P.off_daz + nza * L;
-    P.off_dbz = P.off_db0 + npb;
-    P.ndens = P.off_dbz + nzb * L;
+    const size_t npa = count_pairs(ta), npb = count_pairs(tb);
+    P.off_da = 0;
+    P.off_db = npa;
+    P.ndens = npa + npb;
     plan_spin(P, ta, true);
     plan_spin(P, tb, false);
-    plan_ab(P, ta, tb);
     if (P.a.I.size() != npa || P.b.I.size() != npb) throw std::runtime_error("rdm plan: pair count mismatch");
     // CSR of the slot terms: a stable counting sort keeps each slot's generation order
     std::vector<uint32_t> ptr(P.nslots + 1, 0), idx(P.terms.size());
@@ -680,22 +784,17 @@ std::shared_ptr<FciRdmPlan> make_fci_rdm_plan(cigpu_crs &c, cudaStream_t s) {
     }
     auto R = std::make_shared<FciRdmPlan>();
     R->npa = (int64_t)npa;
-    R->nza = (int64_t)nza;
     R->npb = (int64_t)npb;
-    R->nzb = (int64_t)nzb;
     R->ndens = P.ndens;
     R->nslots = P.nslots;
-    R->off_da0 = P.off_da0;
-    R->off_daz = P.off_daz;
-    R->off_db0 = P.off_db0;
-    R->off_dbz = P.off_dbz;
+    R->off_da = P.off_da;
+    R->off_db = P.off_db;
     R->off_ga = P.off_ga;
     R->off_gb = P.off_gb;
     R->off_g0 = P.off_g0;
-    R->off_g1 = P.off_g1;
     R->off_g2 = P.off_g2;
-    R->sa = upload(ta.strings, s);
-    R->sb = upload(tb.strings, s);
+    const ExcitationLists ea = excitation_lists(ta, false), eb = excitation_lists(tb, true);
+    const SumLists sb = sum_lists(tb, true), sa = sum_lists(ta, false);
     R->aI = upload(P.a.I, s);
     R->aJ = upload(P.a.J, s);
     R->bI = upload(P.b.I, s);
@@ -703,12 +802,16 @@ std::shared_ptr<FciRdmPlan> make_fci_rdm_plan(cigpu_crs &c, cudaStream_t s) {
     R->dptr = upload(ptr, s);
     R->didx = upload(idx, s);
     R->dcf = upload(cf, s);
-    R->app = upload(P.ap_ptr, s);
-    R->bxp = upload(P.bx_ptr, s);
-    R->apd = upload(P.ap, s);
-    R->bxd = upload(P.bx, s);
-    R->aps = upload(P.ap_sign, s);
-    R->bxs = upload(P.bx_sign, s);
+    R->ap = upload(ea.ptr, s);
+    R->apair = upload(ea.pair, s);
+    R->asign = upload(ea.sign, s);
+    R->bp = upload(eb.ptr, s);
+    R->bpair = upload(eb.pair, s);
+    R->bsign = upload(eb.sign, s);
+    R->btp = upload(sb.ptr, s);
+    R->bta = upload(sb.at, s);
+    R->atp = upload(sa.ptr, s);
+    R->ata = upload(sa.at, s);
     CIGPU_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
     return R;
 }
@@ -752,13 +855,17 @@ void crs_rdm(cigpu_crs &c, const double *c_dev, double *rdm1, double *aa, double
             k_transpose<<<grid, dim3(32, 8), 0, s>>>(c_dev, ta.D, tb.D, Ct.p);
             count_launch();
         }
+        const size_t sm = sizeof(double) * 2 * (size_t)tb.D;
+        if (np > 0 && sm > 200 * 1024) throw std::invalid_argument("FCI RDM: beta string space too large");
         DevBuf<double> dens(R.ndens);
         const int G = sm_count() * 8;
         unsigned long long *ew = check_word_device();
-        k_pair_dens<<<G, kRdmThreads, 0, s>>>(c_dev, tb.D, R.aI.p, R.aJ.p, R.npa, R.nza, R.sb.p, L,
-                                              dens.p + R.off_da0, dens.p + R.off_daz, ta.D, ew);
-        k_pair_dens<<<G, kRdmThreads, 0, s>>>(Ct.p, ta.D, R.bI.p, R.bJ.p, R.npb, R.nzb, R.sa.p, L,
-                                              dens.p + R.off_db0, dens.p + R.off_dbz, tb.D, ew);
+        const auto pair_grid = [](int64_t n) {  // a batch of pairs per warp
+            constexpr int64_t per = kPairBatch * (kRdmThreads / 32);
+            return (unsigned)std::min<int64_t>((n + per - 1) / per, INT32_MAX);
+        };
+        k_pair_dens<<<pair_grid(R.npa), kRdmThreads, 0, s>>>(c_dev, tb.D, R.aI.p, R.aJ.p, R.npa, dens.p + R.off_da, ta.D, ew);
+        k_pair_dens<<<pair_grid(R.npb), kRdmThreads, 0, s>>>(Ct.p, ta.D, R.bI.p, R.bJ.p, R.npb, dens.p + R.off_db, tb.D, ew);
         count_launch(2);
         tr.mark("pair densities");
         DevBuf<double> acc(R.nslots);
@@ -766,24 +873,42 @@ void crs_rdm(cigpu_crs &c, const double *c_dev, double *rdm1, double *aa, double
                                                 (int64_t)R.ndens, ew);
         count_launch();
         tr.mark("slot sums");
-        // alpha-beta doubles
-        const int nsplit = R.nsplit;
-        DevBuf<double> slices((size_t)std::max(np, 1) * nsplit * L2);
-        if (np > 0) {
-            const size_t sm = sizeof(double) * 2 * (size_t)tb.D;
-            if (sm > 200 * 1024) throw std::invalid_argument("FCI RDM: beta string space too large");
+        // the alpha-beta block: string sums of a batch of excitations (at most
+        // kAbBatchBytes of them), then the sums over the strings
+        constexpr size_t kAbBatchBytes = size_t(64) << 20;
+        DevBuf<double> t1((size_t)std::max(np, 1) * L2), t2((size_t)(np + L) * L);
+        auto batches = [&](int nq, size_t per_q, auto &&f) {
+            const int most = (int)std::min<size_t>({(size_t)std::max(nq, 1), 65535,
+                                                    std::max<size_t>(1, kAbBatchBytes / (per_q * sizeof(double)))});
+            DevBuf<double> g((size_t)most * per_q);
+            for (int q0 = 0; q0 < nq; q0 += most) f(g.p, q0, std::min(most, nq - q0));
+        };
+        const int nsb = tb.ns;
+        batches(np, (size_t)(nsb + 1) * tb.D, [&](double *g, int q0, int nq) {
             // one fixed limit, set once: concurrent callers (server workers) must never lower it
             static const cudaError_t attr =
-                cudaFuncSetAttribute(k_ab_doubles, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                cudaFuncSetAttribute(k_string_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
             CIGPU_CUDA(attr);
-            const int th = std::min(1024, (int)((L2 + 31) / 32 * 32));
-            k_ab_doubles<<<np * nsplit, th, sm, s>>>(c_dev, tb.D, R.app.p, R.apd.p, R.aps.p, R.bxp.p, R.bxd.p,
-                                                     R.bxs.p, L, nsplit, slices.p, ta.D, ew);
-            count_launch();
-        }
+            const int64_t per = (int64_t)(nsb + 1) * tb.D;
+            const dim3 grid((unsigned)((tb.D + kAbThreads - 1) / kAbThreads),
+                            (unsigned)std::max(1, (nsb + kAbX - 1) / kAbX), (unsigned)nq);
+            k_string_sums<<<grid, kAbThreads, sm, s>>>(c_dev, tb.D, c.fp.b.s_target, nsb, R.ap.p, R.apair.p, R.asign.p, q0,
+                                                       g, ta.D, ew);
+            k_sum_strings<<<(unsigned)((nq * L2 + 3) / 4), 128, 0, s>>>(g, per, R.btp.p, R.bta.p, (int)L2, nq,
+                                                                        t1.p + (int64_t)q0 * L2, ew);
+            count_launch(2);
+        });
         tr.mark("alpha-beta doubles");
-        k_rdm_assemble<<<G, kRdmThreads, 0, s>>>(acc.p, slices.p, nsplit, L, np, R.off_ga, R.off_gb, R.off_g0, R.off_g1,
-                                                 R.off_g2, o1, oaa, oab, obb);
+        batches(np + L, (size_t)ta.D, [&](double *g, int q0, int nq) {
+            const dim3 grid((unsigned)((ta.D + kAbThreads - 1) / kAbThreads), 1, (unsigned)nq);
+            k_string_sums_ident<<<grid, kAbThreads, 0, s>>>(Ct.p, ta.D, R.bp.p, R.bpair.p, R.bsign.p, q0, g, tb.D, ew);
+            k_sum_strings<<<(unsigned)((nq * L + 3) / 4), 128, 0, s>>>(g, ta.D, R.atp.p, R.ata.p, L, nq,
+                                                                       t2.p + (int64_t)q0 * L, ew);
+            count_launch(2);
+        });
+        tr.mark("alpha occupations");
+        k_rdm_assemble<<<G, kRdmThreads, 0, s>>>(acc.p, t1.p, t2.p, L, np, R.off_ga, R.off_gb, R.off_g0, R.off_g2, o1, oaa,
+                                                 oab, obb);
         CIGPU_CUDA(cudaGetLastError());
         count_launch();
         CIGPU_CUDA(cudaStreamSynchronize(s));
