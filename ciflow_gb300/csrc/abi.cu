@@ -513,6 +513,7 @@ void build_crs(cigpu_crs &c, cudaStream_t s) {
             c.kpair32.alloc((size_t)L * L);
             doci_pair_table_launch(L, h.d_eri.p, c.kpair64.p, c.kpair32.p, s);
             doci_split_make(L, n, dim, c.split, s);
+            c.split_tried = true;
             if (c.precision == CIGPU_MIXED) {
                 c.diag32.alloc(dim);
                 dev_convert(c.diag.p, c.diag32.p, dim, s);

@@ -405,8 +405,15 @@ __device__ __forceinline__ uint32_t low_rank(uint32_t b, const uint32_t *binom) 
     return r;
 }
 
+// b without bit j, the bits above it one place down.
+__device__ __forceinline__ uint32_t squeeze(uint32_t b, int j) {
+    const uint32_t low = (1u << j) - 1u;
+    return (b & low) | ((b >> 1) & ~low);
+}
+
 __global__ void k_split_low(const DociSplitView p, uint32_t *__restrict__ ll, uint16_t *__restrict__ lminus,
-                            uint16_t *__restrict__ lplus) {
+                            uint16_t *__restrict__ lplus, uint32_t *__restrict__ one, uint32_t *__restrict__ two,
+                            uint16_t *__restrict__ lowbits) {
     const DociSector &c = p.sec[blockIdx.y];
     const int s = p.s, m = c.m;
     for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < c.nlow; l += gridDim.x * blockDim.x) {
@@ -417,6 +424,7 @@ __global__ void k_split_low(const DociSplitView p, uint32_t *__restrict__ ll, ui
                 b |= 1u << o;
                 --k;
             }
+        lowbits[c.low0 + l] = (uint16_t)b;
         int e = 0, em = 0, ep = 0;
         for (int j = s - 1; j >= 0; --j) {
             const uint32_t bj = b ^ (1u << j);
@@ -424,7 +432,13 @@ __global__ void k_split_low(const DociSplitView p, uint32_t *__restrict__ ll, ui
                 lplus[c.plus0 + (uint32_t)ep++ * c.nlow + l] = (uint16_t)(low_rank(bj, p.binom) | ((uint32_t)j << 10));
                 continue;
             }
-            lminus[c.minus0 + (uint32_t)em++ * c.nlow + l] = (uint16_t)(low_rank(bj, p.binom) | ((uint32_t)j << 10));
+            const uint32_t without = low_rank(bj, p.binom);
+            lminus[c.minus0 + (uint32_t)em++ * c.nlow + l] = (uint16_t)(without | ((uint32_t)j << 10));
+            one[c.one0 + (uint32_t)j * c.n1 + low_rank(squeeze(bj, j), p.binom)] = l | (without << 16);
+            for (int k = j + 1, q = j * s - j * (j + 1) / 2; k < s; ++k, ++q)  // pair (j, k): row-major, j < k
+                if (!((b >> k) & 1u))
+                    two[c.two0 + (uint32_t)q * c.n2 + low_rank(squeeze(squeeze(bj, k), j), p.binom)] =
+                        l | (low_rank(bj ^ (1u << k), p.binom) << 16);
             for (int k = s - 1; k >= 0; --k)
                 if (!((b >> k) & 1u))
                     ll[c.ll0 + (uint32_t)e++ * c.nlow + l] =
@@ -545,12 +559,12 @@ void doci_split_make(int L, int n, int64_t D, DociSplit &sp, cudaStream_t st) {
     v.L = L;
     v.n = n;
     v.D = D;
-    uint32_t nll = 0, nmi = 0, npl = 0, nhi = 0;
+    uint32_t nll = 0, nmi = 0, npl = 0, nhi = 0, nlo = 0, none = 0, ntwo = 0;
     for (int s = std::min(kSplitMaxLow, (L + 1) / 2); s >= 4; --s) {
         const int Lh = L - s;
         size_t bytes[2] = {0, 0};
         uint64_t tasks[2] = {0, 0};
-        nll = nmi = npl = nhi = 0;
+        nll = nmi = npl = nhi = nlo = none = ntwo = 0;
         v.nsec = 0;
         for (int m = std::max(0, n - Lh); m <= std::min(s, n); ++m) {
             DociSector c{};
@@ -573,7 +587,15 @@ void doci_split_make(int L, int n, int64_t D, DociSplit &sp, cudaStream_t st) {
             c.ll0 = nll;
             c.minus0 = nmi;
             c.plus0 = npl;
+            c.low0 = nlo;
+            c.n1 = m > 0 ? (uint32_t)d_binom(s - 1, m - 1) : 0u;
+            c.n2 = m > 0 && m < s ? (uint32_t)d_binom(s - 2, m - 1) : 0u;
+            c.one0 = none;
+            c.two0 = ntwo;
             nhi += c.nhigh;
+            nlo += c.nlow;
+            none += (uint32_t)s * c.n1;
+            ntwo += (uint32_t)(s * (s - 1) / 2) * c.n2;
             nll += (uint32_t)(m * (s - m)) * c.nlow;
             nmi += (uint32_t)m * c.nlow;
             npl += (uint32_t)(s - m) * c.nlow;
@@ -599,13 +621,21 @@ void doci_split_make(int L, int n, int64_t D, DociSplit &sp, cudaStream_t st) {
     sp.ll.alloc(std::max(nll, 1u));
     sp.lminus.alloc(std::max(nmi, 1u));
     sp.lplus.alloc(std::max(npl, 1u));
+    sp.one.alloc(std::max(none, 1u));
+    sp.two.alloc(std::max(ntwo, 1u));
+    sp.lowbits.alloc(nlo);
+    sp.nlowbits = nlo;
+    v.one = sp.one.p;
+    v.two = sp.two.p;
+    v.lowbits = sp.lowbits.p;
     v.hbits = sp.hbits.p;
     v.hbase = sp.hbase.p;
     v.binom = sp.binom.p;
     v.ll = sp.ll.p;
     v.lminus = sp.lminus.p;
     v.lplus = sp.lplus.p;
-    k_split_low<<<dim3(4, v.nsec), 256, 0, st>>>(v, sp.ll.p, sp.lminus.p, sp.lplus.p);
+    k_split_low<<<dim3(4, v.nsec), 256, 0, st>>>(v, sp.ll.p, sp.lminus.p, sp.lplus.p, sp.one.p, sp.two.p,
+                                               sp.lowbits.p);
     k_split_high<<<dim3(64, v.nsec), 256, 0, st>>>(v, sp.hbits.p, sp.hbase.p);
     CIGPU_CUDA(cudaGetLastError());
     count_launch(2);

@@ -24,6 +24,8 @@ struct DociSector {  // the blocks with nh high and m low pairs
     uint32_t nhigh, high0;            // high strings, and the first one's place in hbits / hbase
     uint32_t nlow, nminus, nplus;     // C(s, m), C(s, m - 1), C(s, m + 1)
     uint32_t ll0, minus0, plus0;      // offsets into the low tables
+    uint32_t low0;                    // the sector's first low string in lowbits
+    uint32_t n1, one0, n2, two0;      // C(s - 1, m - 1), C(s - 2, m - 1) and offsets into one / two
 };
 struct DociSplitView {
     int L, n, s, nsec;
@@ -34,6 +36,10 @@ struct DociSplitView {
     // per low string l of m pairs, entry-major ([entry][C(s, m)]):
     const uint32_t *ll;               // pair hops inside: target rank | (j * s + k) << 10
     const uint16_t *lminus, *lplus;   // a pair taken out of / put into orbital j: rank | j << 10
+    // per orbital j (pair j < k), list-major: the low strings l that hold j (j, not k) and
+    // their targets without j (with k in its place): l | target << 16
+    const uint32_t *one, *two;
+    const uint16_t *lowbits;          // the low strings, sector by sector
     unsigned long long *err;
     int64_t D;
     DociSector sec[kSplitMaxLow + 1];
@@ -43,8 +49,9 @@ struct DociSplit {
     DociSplitView view{};
     size_t smem[2] = {0, 0};          // the product's shared memory, FP32 and FP64
     DevBuf<uint64_t> hbits;
-    DevBuf<uint32_t> hbase, binom, ll;
-    DevBuf<uint16_t> lminus, lplus;
+    DevBuf<uint32_t> hbase, binom, ll, one, two;
+    DevBuf<uint16_t> lminus, lplus, lowbits;
+    uint32_t nlowbits = 0;
     explicit operator bool() const { return view.s > 0; }
 };
 // Makes the plan where the split product is the faster one (plan.view.s stays 0 elsewhere).

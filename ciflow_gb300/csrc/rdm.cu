@@ -660,6 +660,226 @@ __global__ void k_doci_rdm(const double *__restrict__ c, const uint64_t *__restr
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same sums by low and high orbitals (larger spaces; see the split product in
+// doci_mv.cu for the blocks). A pair hop's two coefficients lie in blocks whose starts
+// are shared by all of a block's strings, so the sums are dot products of blocks:
+//   * j, k high: the block h with the block h - j + k, string by string;
+//   * j, k low: inside the block, over the list of the strings that hold j and not k;
+//   * j low, k high: the block h with the staged block h + k, over the list of the
+//     strings that hold j.
+// Every lane of a warp has a product to add (a thread per orbital pair found one in
+// four strings to act on, and formed a rank for each), and A needs only the blocks'
+// sums of squares, per block and per low string. The products and sums are the
+// fixed-point integers above, so the result is the same bit for bit in any order:
+// shared and global integer atomics collect them. Bound by the integer pipe (about 20
+// instructions per product). L=24, 12 pairs: 3.85 -> 0.90 ms per cigpu_rdm,
+// most of the rest the vector's way from host memory.
+constexpr int kSplitRdmThreads = 256;
+constexpr int kSplitRdmWarps = kSplitRdmThreads / 32;
+constexpr int kSplitRdmPairs = (kSplitMaxLow * (kSplitMaxLow - 1) / 2 + kSplitRdmWarps - 1) / kSplitRdmWarps;
+constexpr int kSplitRdmLow = 4;  // low strings per thread: C(12, 6) = 924 <= 4 x 256
+constexpr int kSplitRdmRows = 512;  // rows a block aims at (2048: 1.26 ms per call, 512: 0.90)
+constexpr size_t kSplitRdmMaxSmem = 200 * 1024;
+
+__global__ void k_fix62(const double *__restrict__ c, int64_t n, long long *__restrict__ f) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        f[i] = fx62(c[i]);
+}
+
+__host__ __device__ inline uint32_t split_rdm_group(const DociSector &c) {
+    const uint32_t g = kSplitRdmRows / c.nlow;
+    return g < 1 ? 1u : g > 64 ? 64u : g;
+}
+
+__device__ __forceinline__ long long warp_sum(long long v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ void add_to(long long *at, long long v) {
+    atomicAdd(reinterpret_cast<unsigned long long *>(at), (unsigned long long)v);
+}
+
+// sums: [2][L][L] (A, then B; j <= k), low: [lowbits] sums of squares per low string.
+__global__ void __launch_bounds__(kSplitRdmThreads, 3) k_doci_rdm_split(const DociSplitView p, uint32_t tasks,
+                                                                     const long long *__restrict__ cf,
+                                                                     long long *__restrict__ sums,
+                                                                     long long *__restrict__ low) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int L = p.L, s = p.s, Lh = L - s, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    long long *sA = reinterpret_cast<long long *>(smem);  // [L][L]
+    long long *sB = sA + L * L;                           // [L][L]
+    long long *area = sB + L * L;
+    for (int i = t; i < 2 * L * L; i += kSplitRdmThreads) sA[i] = 0;
+    auto start_of = [&](uint64_t b, int mm) {
+        uint32_t r = 0;
+        for (int k = mm + 1; b; b &= b - 1, ++k) r += __ldg(p.binom + (s + __ffsll((long long)b) - 1) * kSplitBinomRow + k);
+        return r;
+    };
+    auto nth = [](uint64_t b, int i) {
+        for (; i > 0; --i) b &= b - 1;
+        return __ffsll((long long)b) - 1;
+    };
+    auto load = [&](uint32_t at) {
+        return CIGPU_CHECK(p.err, index_ok(at, (uint64_t)p.D), kCheckHopRank, at) ? __ldg(cf + at) : 0ll;
+    };
+    const uint64_t full = (((uint64_t)1) << Lh) - 1;
+    const int np = s * (s - 1) / 2;
+    for (uint32_t task = blockIdx.x; task < tasks; task += gridDim.x) {  // one task, up to INT32_MAX
+        uint32_t first = task;
+        int q = 0;
+        for (; q + 1 < p.nsec; ++q) {
+            const uint32_t g = split_rdm_group(p.sec[q]), nt = (p.sec[q].nhigh + g - 1) / g;
+            if (first < nt) break;
+            first -= nt;
+        }
+        const DociSector &c = p.sec[q];
+        const uint32_t group = split_rdm_group(c);
+        const int nh = c.nh, nv = Lh - nh, m = c.m, nhh = nh * nv;
+        const int nlow = (int)c.nlow, nminus = (int)c.nminus, n1 = (int)c.n1, n2 = (int)c.n2;
+        long long *own = area, *sq = own + nlow, *up = sq + nlow;  // [nlow], [nlow], [nv][nminus]
+        uint32_t *hhb = reinterpret_cast<uint32_t *>(up + (size_t)nv * nminus);  // [nhh]
+        uint32_t *upb = hhb + nhh;                                                // [nv]
+        const uint32_t *one = p.one + c.one0, *two = p.two + c.two0;
+        long long acc[kSplitRdmPairs], sqs[kSplitRdmLow];
+#pragma unroll
+        for (int i = 0; i < kSplitRdmPairs; ++i) acc[i] = 0;
+#pragma unroll
+        for (int i = 0; i < kSplitRdmLow; ++i) sqs[i] = 0;
+        const uint32_t h1 = min((first + 1) * group, c.nhigh);
+        for (uint32_t h = first * group; h < h1; ++h) {
+            const uint64_t hb = __ldg(p.hbits + c.high0 + h);
+            const uint32_t base = __ldg(p.hbase + c.high0 + h);
+            __syncthreads();  // the previous block's coefficients and lists are read
+            for (int e = t; e < nhh; e += kSplitRdmThreads) {
+                const int a = e / nv, j = nth(hb, a), k = nth(full & ~hb, e - a * nv);
+                hhb[e] = k > j ? start_of(hb ^ ((uint64_t)1 << j) ^ ((uint64_t)1 << k), m) : 0xFFFFFFFFu;
+            }
+            if (m > 0)
+                for (int r = t; r < nv; r += kSplitRdmThreads)
+                    upb[r] = start_of(hb | ((uint64_t)1 << nth(full & ~hb, r)), m - 1);
+#pragma unroll
+            for (int i = 0; i < kSplitRdmLow; ++i) {
+                const int l = t + i * kSplitRdmThreads;
+                if (l < nlow) {
+                    const long long v = load(base + (uint32_t)l), v2 = fxmul(v, v);
+                    own[l] = v;
+                    sq[l] = v2;
+                    sqs[i] += v2;
+                }
+            }
+            __syncthreads();
+            if (m > 0)
+                for (int r = warp; r < nv; r += kSplitRdmWarps)
+                    for (int l = lane; l < nminus; l += 32) up[(size_t)r * nminus + l] = load(upb[r] + (uint32_t)l);
+            // high - high
+            for (int e = warp; e < nhh; e += kSplitRdmWarps) {
+                const uint32_t b = hhb[e];
+                if (b == 0xFFFFFFFFu) continue;  // k < j: summed from the other side
+                long long a = 0;
+#pragma unroll 4
+                for (int l = lane; l < nlow; l += 32) a += fxmul(own[l], load(b + (uint32_t)l));
+                a = warp_sum(a);
+                if (lane == 0) {
+                    const int i = e / nv;
+                    add_to(sB + (s + nth(hb, i)) * L + s + nth(full & ~hb, e - i * nv), a);
+                }
+            }
+            // low - low
+            if (n2 > 0) {
+#pragma unroll
+                for (int i = 0; i < kSplitRdmPairs; ++i) {
+                    const int pr = warp + i * kSplitRdmWarps;
+                    if (pr < np) {
+                        const uint32_t *w = two + (size_t)pr * n2;
+#pragma unroll 2
+                        for (int x = lane; x < n2; x += 32) {
+                            const uint32_t e = __ldg(w + x);
+                            acc[i] += fxmul(own[e & 0xFFFFu], own[e >> 16]);
+                        }
+                    }
+                }
+            }
+            // squares: over the block, and over its strings that hold j
+            if (warp == kSplitRdmWarps - 1 && nh > 0) {
+                long long a = 0;
+                for (int l = lane; l < nlow; l += 32) a += sq[l];
+                a = warp_sum(a);
+                for (int e = lane; e < nh * nh; e += 32) {
+                    const int i = e / nh, k = e - i * nh;
+                    if (k >= i) add_to(sA + (s + nth(hb, i)) * L + s + nth(hb, k), a);
+                }
+            }
+            if (m > 0 && nh > 0)
+                for (int j = warp; j < s; j += kSplitRdmWarps) {
+                    long long a = 0;
+                    for (int x = lane; x < n1; x += 32) a += sq[__ldg(one + (size_t)j * n1 + x) & 0xFFFFu];
+                    a = warp_sum(a);
+                    for (int i = lane; i < nh; i += 32) add_to(sA + j * L + s + nth(hb, i), a);
+                }
+            __syncthreads();  // the blocks h + k are staged
+            // low - high
+            if (m > 0)
+                for (int e = warp; e < nv * s; e += kSplitRdmWarps) {
+                    const int r = e / s, j = e - r * s;
+                    const uint32_t *w = one + (size_t)j * n1;
+                    const long long *row = up + (size_t)r * nminus;
+                    long long a = 0;
+#pragma unroll 4
+                    for (int x = lane; x < n1; x += 32) {
+                        const uint32_t v = __ldg(w + x);
+                        a += fxmul(own[v & 0xFFFFu], row[v >> 16]);
+                    }
+                    a = warp_sum(a);
+                    if (lane == 0) add_to(sB + j * L + s + nth(full & ~hb, r), a);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < kSplitRdmPairs; ++i) {
+            const int pr = warp + i * kSplitRdmWarps;
+            const long long a = warp_sum(acc[i]);
+            if (lane == 0 && pr < np) {
+                int j = 0, rem = pr;
+                while (rem >= s - 1 - j) rem -= s - 1 - j++;
+                add_to(sB + j * L + j + 1 + rem, a);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kSplitRdmLow; ++i) {
+            const int l = t + i * kSplitRdmThreads;
+            if (l < nlow) add_to(low + c.low0 + l, sqs[i]);
+        }
+    }
+    __syncthreads();
+    for (int i = t; i < 2 * L * L; i += kSplitRdmThreads)
+        if (sA[i] != 0) add_to(sums + i, sA[i]);
+}
+
+// A of two low orbitals (block.x = j * s + k, j <= k): the sums of squares of the low
+// strings that hold both.
+__global__ void k_doci_rdm_low(const DociSplitView p, uint32_t n, const long long *__restrict__ low,
+                               long long *__restrict__ sums) {
+    const int j = blockIdx.x / p.s, k = blockIdx.x - j * p.s;
+    if (k < j) return;
+    const uint32_t both = (1u << j) | (1u << k);
+    long long a = 0;
+    for (uint32_t l = threadIdx.x; l < n; l += blockDim.x)
+        if ((p.lowbits[l] & both) == both) a += low[l];
+    a = warp_sum(a);
+    if ((threadIdx.x & 31) == 0 && a != 0) add_to(sums + j * p.L + k, a);
+}
+
+size_t split_rdm_smem(const DociSplitView &v) {
+    size_t most = 0;
+    for (int q = 0; q < v.nsec; ++q) {
+        const DociSector &c = v.sec[q];
+        const size_t nv = v.L - v.s - c.nh;
+        most = std::max(most, 8 * (2 * (size_t)c.nlow + nv * c.nminus) + 4 * (c.nh * nv + nv));
+    }
+    return most + 16 * (size_t)v.L * v.L;
+}
+
 __global__ void k_doci_rdm_finish(const double *__restrict__ partial, int G, int L, int np, double *__restrict__ rdm1,
                                   double *__restrict__ aa, double *__restrict__ ab, double *__restrict__ bb) {
     const int L2 = L * L;
@@ -736,6 +956,41 @@ struct FciRdmPlan {
     DevBuf<int8_t> asign, bsign;
     DevBuf<uint32_t> btp, bta, atp, ata;      // sums over beta strings by (br, bc), over alpha strings by z
 };
+
+// The split plan of a DOCI matrix, made on the first call (the mixed builds have it);
+// null where the space is not split.
+const DociSplit *doci_split_of(cigpu_crs &c, cudaStream_t s) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!c.split_tried) {
+        doci_split_make(c.L, c.nup, c.dim, c.split, s);
+        c.split_tried = true;
+    }
+    return c.split && split_rdm_smem(c.split.view) <= kSplitRdmMaxSmem ? &c.split : nullptr;
+}
+
+// Fixed-point sums A, B ([2][L][L], j <= k) of device vector c through the split plan.
+void doci_rdm_split(const DociSplit &sp, const double *c_dev, long long *sums, cudaStream_t s) {
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_doci_rdm_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitRdmMaxSmem);
+    CIGPU_CUDA(attr);
+    DociSplitView v = sp.view;
+    v.err = check_word_device();
+    DevBuf<long long> fixed((size_t)v.D), low(sp.nlowbits);
+    CIGPU_CUDA(cudaMemsetAsync(low.p, 0, low.bytes(), s));
+    CIGPU_CUDA(cudaMemsetAsync(sums, 0, sizeof(long long) * 2 * v.L * v.L, s));
+    uint64_t tasks = 0;
+    for (int q = 0; q < v.nsec; ++q) {
+        const uint32_t g = split_rdm_group(v.sec[q]);
+        tasks += (v.sec[q].nhigh + g - 1) / g;
+    }
+    const int blocks = (int)std::min<uint64_t>(tasks, (uint64_t)INT32_MAX);
+    k_fix62<<<sm_count() * 8, 256, 0, s>>>(c_dev, v.D, fixed.p);
+    k_doci_rdm_split<<<blocks, kSplitRdmThreads, split_rdm_smem(v), s>>>(v, (uint32_t)tasks, fixed.p, sums, low.p);
+    k_doci_rdm_low<<<v.s * v.s, 256, 0, s>>>(v, sp.nlowbits, low.p, sums);
+    CIGPU_CUDA(cudaGetLastError());
+    count_launch(3);
+}
 
 std::shared_ptr<FciRdmPlan> make_fci_rdm_plan(cigpu_crs &c, cudaStream_t s) {
     const int L = c.L, np = L * (L - 1) / 2;
@@ -830,13 +1085,19 @@ void crs_rdm(cigpu_crs &c, const double *c_dev, double *rdm1, double *aa, double
     if (c.method == CIGPU_DOCI) {
         if (L * L > 1024) throw std::invalid_argument("DOCI RDM needs L <= 32");
         CIGPU_CUDA(cudaMemsetAsync(out.p, 0, sizeof(double) * out.n, s));
-        const int G = sm_count() * 4;
+        const DociSplit *sp = doci_split_of(c, s);
+        const int G = sp ? 1 : sm_count() * 4;
         DevBuf<double> partial((size_t)G * 2 * L2);
         const int th = ((L * (L + 1) / 2 + 31) / 32) * 32;  // one thread per pair j <= k
-        k_doci_rdm<<<G, th, 0, s>>>(c_dev, c.strings.p, c.dim, L, c.nup, partial.p, check_word_device());
+        if (sp) {
+            doci_rdm_split(*sp, c_dev, reinterpret_cast<long long *>(partial.p), s);
+        } else {
+            k_doci_rdm<<<G, th, 0, s>>>(c_dev, c.strings.p, c.dim, L, c.nup, partial.p, check_word_device());
+            count_launch();
+        }
         k_doci_rdm_finish<<<(int)((L2 + 255) / 256), 256, 0, s>>>(partial.p, G, L, np, o1, oaa, oab, obb);
         CIGPU_CUDA(cudaGetLastError());
-        count_launch(2);
+        count_launch();
         CIGPU_CUDA(cudaStreamSynchronize(s));
         tr.mark("doci kernels");
     } else {

@@ -121,3 +121,20 @@ def test_python_facade_density():
     # antisymmetry of the same-spin block through the reference getter semantics
     assert d.get_two_rdm(0, 1, 2, 3, 4) == -d.get_two_rdm(0, 2, 1, 3, 4)
     assert d.get_two_rdm(0, 2, 2, 3, 4) == 0.0
+
+
+@pytest.mark.parametrize("L,n", [(17, 8), (18, 11), (21, 5), (22, 17)])
+def test_doci_rdm_split(L, n):
+    """The DOCI RDMs by low and high orbitals (spaces past the split's row threshold),
+    from a mixed matrix and from a plain one (which makes its plan on the first call):
+    the oracle's, and the same bits from both and from a second call."""
+    ints = make_integrals(L, n, n, nchol=4, seed=L + n)
+    ham = Hamiltonian.from_integrals(ints)
+    mixed, plain = DOCI(ham, A.MIXED), DOCI(ham, A.FP64)
+    c = np.random.default_rng(n).standard_normal(mixed.get_mat().n)
+    c /= np.linalg.norm(c)
+    got = rdm_via_abi(mixed, c)
+    assert_rdm_close(got, O.rdm(O.DOCI, L, n, n, c), 1e-13)
+    for other in (rdm_via_abi(plain, c), rdm_via_abi(plain, c), rdm_via_abi(mixed, c)):
+        for g, o in zip(got, other):
+            assert np.array_equal(g, o)
