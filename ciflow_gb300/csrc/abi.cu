@@ -280,7 +280,7 @@ size_t estimate_bytes(int L, int nup, int ndown, int method, int precision) {
     if (method == CIGPU_FCI && precision == CIGPU_MIXED) {  // slot tiles of kTileRows beta strings, hi + lo
         b = (size_t)binom64(L, nup) * ((binom64(L, ndown) + kTileRows - 1) / kTileRows * kTileRows) * (W + 16) * 8;
         if (sigma_applies(L))  // the FP32 sigma operator at its largest rank
-            b += sigma_bytes(L, binom64(L, nup), binom64(L, ndown),
+            b += sigma_bytes(L, nup, ndown,
                              std::min(kSigmaMaxRank, (L * (L + 1) / 2 + kSigmaChunk - 1) / kSigmaChunk * kSigmaChunk));
     }
     if (method == CIGPU_DOCI)  // matrix-free: strings and the FP32 diagonal
@@ -436,7 +436,7 @@ void build_crs(cigpu_crs &c, cudaStream_t s) {
         const int smode = sigma_mode();
         if (c.slots && c.precision == CIGPU_MIXED && c.allow_compact && sigma_applies(c.L) && smode != kSigmaOff) {
             c.sig.reset(new SigmaOp);
-            if (!sigma_prepare(*c.sig, c.L, h.h.data(), h.eri.data(), c.ta, c.ndown == c.nup ? c.ta : c.tb,
+            if (!sigma_prepare(*c.sig, c.L, h.h.data(), h.eri.data(), c.ta, c.ndown == c.nup ? c.ta : c.tb, p,
                                smode == kSigmaForced || c.sigma_any_grid, s))
                 c.sig.reset();
             tr.mark("sigma factors");

@@ -1,44 +1,42 @@
-// FP32 product of the mixed method for FCI: a direct-CI sigma vector from a
-// factorised two-electron part.
+// FP32 product of the mixed method for FCI: a direct-CI sigma vector, the same-spin
+// part from the strings' own matrices and the opposite-spin part factorised.
 //
-// With E_pq = sum over spins of a+_p a_q and real orbitals,
-//   H = sum_pq k_pq E_pq + 1/2 sum_pqrs (pq|rs) E_pq E_rs,   k_ps = h_ps - 1/2 sum_q (pq|qs),
-// and a factorisation (pq|rs) = sum_k s_k F^k_pq F^k_rs with symmetric F^k (a
-// pivoted Cholesky factor of the pair matrix, s_k = 1; eigenpairs with their signs
-// when the integrals are indefinite) gives
-//   1/2 sum (pq|rs) E_pq E_rs = 1/2 sum_k s_k A_k A_k,   A_k = sum_pq F^k_pq E_pq.
-// So y = H x is two one-body passes:
-//   (1) y_k = A_k x for every factor k, and K x;
-//   (2) y = K x + sum_k A_k (1/2 s_k y_k).
-// A one-body pass visits, for every determinant I = (Ia, Ib), its single
-// excitations (Ia -> Ja with Ib fixed, Ib -> Jb with Ia fixed; sign and orbital
-// pair from the string tables) and its diagonal (occupations). Against the stored
-// matrix (about 1,800 elements per row at L=12 6a6b, 4 bytes each) a determinant
-// costs n_a (L - n_a) + n_b (L - n_b) excitations times the rank, and the data it
-// reads (x, the A_k x vectors) stay in L2.
+// With E^s_pq = a+_ps a_qs for spin s and real orbitals,
+//   H = T^a + T^b + sum_pqrs (pq|rs) E^a_pq E^b_rs,
+// T^s the one- and two-electron part of one spin (a sparse matrix over its strings: the
+// diagonal, singles and doubles of the string tables), and a factorisation
+// (pq|rs) = sum_k s_k F^k_pq F^k_rs with symmetric F^k (a pivoted Cholesky factor of the
+// pair matrix, s_k = 1; eigenpairs with their signs when the integrals are indefinite)
+// gives
+//   y = T^a x + x T^b + sum_k A^a_k (s_k A^b_k x),   A^s_k = sum_pq F^k_pq E^s_pq.
+// Only beta excitations form z_k = A^b_k x and only alpha ones act on it: half the
+// factor work of squaring A_k = A^a_k + A^b_k (the form before: 72 excitations x 16
+// factors twice per row at L=12 6a6b, now 36 twice and 522 same-spin elements).
+//
+// The alpha excitations are applied in two steps, so that the R factors of a row are
+// read once and not once per excitation: a row J forms, for each of its alpha
+// excitations (J -> I by pq), the one number
+//   w = sign sum_k s_k F^k_pq z_k(J)
+// into W[I][e'] (e' the excitation of I that leads back to J), and a row I then adds its
+// n_a (L - n_a) numbers, a contiguous read. Gathering the factors instead moved 64 bytes
+// per excitation through L2 (2 x 3.9 GB per product), which bound the product.
+//
+// One product is three launches:
+//   k_sigma_pad    x padded to whole tiles and transposed;
+//   k_sigma_parts  two kinds of block: pairs of blocks form W on 64 x 64 string tiles
+//                  (opposite_tile), others u = x T^b on the transposed vectors
+//                  (same_rows);
+//   k_sigma_sum    y = T^a x + u + the sums of W.
+// L=12 6a6b, rank 16: 308 -> 193 us per product (k_sigma_parts 145, k_sigma_sum 60); L=10 5a5b: the stored
+// values 38.5, the operator 15.9 us.
 //
 // This replaces only the mixed method's FP32 correction products: the operator
 // equals the reference Hamiltonian up to FP32 rounding and the factorisation's
 // truncation (a remaining pair diagonal below 1e-10 of the largest), while the FP64 anchor
 // products and residuals keep using the stored matrix, whose elements are the
 // reference's bit for bit; the residual the solver reports is that exact one.
-//
-// Both passes run on tiles of 32 alpha x 32 beta strings (8 warps in the first
-// pass, 16 in the second). In the alpha
-// phase warp w takes alpha rows of the tile with its lanes on consecutive beta
-// strings: every lane of the warp walks the same alpha excitations (uniform
-// coefficients, broadcast from shared memory) and reads x at consecutive beta
-// strings (coalesced). In the beta phase the warp takes beta columns with its
-// lanes on consecutive alpha strings and reads the transposed vectors. The two
-// phases meet in a shared-memory tile; the A_k x vectors are written in both
-// string orders, in blocks of 32 strings with the factors in groups of four
-// outside the 32 ([Da][Db/32][R/4][32][4] and [Db][Da/32][R/4][32][4]): in the
-// second pass a lane reads four factors of its determinant with one 16-byte load
-// and the warp's load covers 512 contiguous bytes, so one excitation is R/4 loads
-// and its factors one contiguous block. (Measured at L=11: factors innermost per
-// determinant, each 16-byte load of a warp spread over 16 cache lines, 156 us;
-// one factor of 32 strings per 4-byte load, 66 us.) The tile's excitation lists
-// (target, orbital pair, sign) are staged in shared memory.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -51,295 +49,456 @@ namespace cigpu {
 
 namespace {
 
-constexpr int kTile = 32;
-constexpr int kThreads = 256;   // pass 1: 8 warps, 4 rows (columns) of the tile each
+namespace cg = cooperative_groups;
+
+constexpr int kTile = kSigmaTile;
+constexpr int kC = kSigmaChunk;
+constexpr int kPanel = 32;     // columns of a same-spin block
+constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kThreadsB = 512;  // pass 2: 16 warps, 2 rows (columns) each
-constexpr int kWarpsB = kThreadsB / 32;
-constexpr int kYtRow = kSigmaChunk * (kTile + 1) + 1;  // staging tile row (odd: the column phase is conflict-free)
+constexpr int kHalf = kC / 2;  // factors of a pass that one block of a pair forms
+constexpr int kZk = kTile * (kTile + 1);  // one factor of the staged tile
 
-struct SigmaArgs {
-    int L, R, nsa, nsb;
-    int64_t Da, Db;
-    int64_t nTa, nTb;  // 32-string tiles of each spin (the factor blocks of Ya, Yb)
-    const uint32_t *sa_t, *sa_i, *sb_t, *sb_i;  // single excitations: targets and packed info per string
-    unsigned long long *err;                    // checked build: the error word
-};
+// ---- packed FP32 pairs ----
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
-// The single excitations of the tile's 32 strings s0.. in shared memory, as
-// {target J, (lo * L + hi) << 1 | negative}: the orbital pair of E_pq and the sign
-// of <S|E_pq|J> (odd number of electrons between the two orbitals). Strings past
-// the space get {0, 0}.
-// (The checked build tests each target against the string count and stages a
-// failing one as {0, 0}.)
-__device__ __forceinline__ void stage_excitations(const uint32_t *__restrict__ tgt, const uint32_t *__restrict__ info,
-                                                  int64_t s0, int64_t D, int ns, int L, uint2 *dst,
-                                                  unsigned long long *err) {
-    for (int i = threadIdx.x; i < kTile * ns; i += blockDim.x) {
-        const int r = i / ns;
-        const int64_t S = s0 + r;
-        uint2 v = make_uint2(0u, 0u);
-        if (S < D) {
-            const int64_t at = S * ns + (i - r * ns);
-            const uint32_t inf = __ldg(info + at);
-            v.x = __ldg(tgt + at);
-            v.y = (((inf & 63u) * (uint32_t)L + ((inf >> 6) & 63u)) << 1) | ((inf >> 24) & 1u);
-            if (!CIGPU_CHECK(err, index_ok(v.x, (uint64_t)D), kCheckColumn, v.x)) v = make_uint2(0u, 0u);
+__device__ __forceinline__ float signed_by(float v, uint32_t odd) {
+    return __uint_as_float(__float_as_uint(v) ^ (odd << 31));
+}
+
+// ---- string tables of the operator ----
+// Rows of T^s: {self, diagonal}, singles, doubles, padding {self, 0}; `ne` per string.
+__global__ void k_sigma_rows(const SpinDev t, int ne, uint2 *__restrict__ rows, unsigned long long *err) {
+    const int64_t total = t.D * ne;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t S = i / ne;
+        const int e = (int)(i - S * ne);
+        uint32_t J = (uint32_t)S;
+        float v = 0.f;
+        if (e == 0) {
+            v = (float)t.diag[S];
+        } else if (e <= t.ns) {
+            const int64_t at = S * t.ns + e - 1;
+            J = t.s_target[at];
+            v = signed_by((float)t.s_part[at], (t.s_info[at] >> 24) & 1u);
+        } else if (e <= t.ns + t.nd) {
+            const int64_t at = S * t.nd + e - 1 - t.ns;
+            J = t.d_target[at];
+            v = (float)t.d_val[at];
         }
-        dst[i] = v;
+        if (!CIGPU_CHECK(err, index_ok(J, (uint64_t)t.D), kCheckColumn, J)) {
+            J = (uint32_t)S;
+            v = 0.f;
+        }
+        rows[i] = make_uint2(J, __float_as_uint(v));
     }
     (void)err;
 }
-__device__ __forceinline__ float exc_sign(uint32_t packed) { return (packed & 1u) ? -1.f : 1.f; }
-__device__ __forceinline__ float dot4(const float4 a, const float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
 
-__global__ void k_transpose32(const float *__restrict__ a, int64_t rows, int64_t cols, float *__restrict__ t) {
-    __shared__ float tile[kTile][kTile + 1];
-    const int64_t r0 = (int64_t)blockIdx.y * kTile, c0 = (int64_t)blockIdx.x * kTile;
-    for (int i = threadIdx.y; i < kTile; i += blockDim.y) {
+// W row that excitation e of string J feeds: target I, place of the excitation that
+// leads back (I's occupied orbital ascending, then its empty one; see the tables).
+__global__ void k_sigma_back(const SpinDev t, int L, uint32_t *__restrict__ w) {
+    const int64_t total = t.D * t.ns;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t I = t.s_target[i], info = t.s_info[i];
+        const int j = (info >> 12) & 63, l = (info >> 18) & 63;  // J holds j, I holds l in its place
+        int at_l = 0, below_j = 0;
+        for (int m = 0; m < t.n; ++m) {
+            const int o = t.occ[(int64_t)I * t.n + m];
+            at_l += o < l;
+            below_j += o < j;
+        }
+        w[i] = I * (uint32_t)t.ns + (uint32_t)(at_l * (L - t.n) + j - below_j);
+    }
+}
+
+// Single excitations as the opposite-spin tiles read them: {target, pair << 1 | odd},
+// pair = lo * L + hi; with `back`, the W row in place of the target.
+__global__ void k_sigma_singles(const SpinDev t, int L, const uint32_t *__restrict__ back, uint2 *__restrict__ out,
+                                unsigned long long *err) {
+    const int64_t total = t.D * t.ns;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t w = t.s_info[i];
+        uint32_t J = back ? back[i] : t.s_target[i];
+        if (!CIGPU_CHECK(err, index_ok(J, (uint64_t)(back ? total : t.D)), kCheckColumn, J)) J = 0;
+        out[i] = make_uint2(J, (((w & 63u) * (uint32_t)L + ((w >> 6) & 63u)) << 1) | ((w >> 24) & 1u));
+    }
+    (void)err;
+}
+
+struct SigmaArgs {
+    int L, R, nsa, nsb;
+    int64_t Da, Db, Pa, Pb;
+    const uint2 *sa, *sb;             // single excitations: alpha {W row, pair}, beta {target, pair}
+    const float *F, *G, *ga, *fb;     // as in SigmaOp
+    const uint2 *rows;                // the beta strings' same-spin rows
+    int ne;
+    int tiles, panels, chunks, per;   // opposite tiles; same-spin panels and row chunks
+    int panel_rows;                   // rows of xT a same-spin block holds in shared memory (0: none)
+    const float *xT;
+    float *W, *yd, *uT;
+};
+
+// x [Da][Db] into xp [Da][Pb] (zero past Db) and xT [Db][Pa] (zero past Da).
+__global__ void k_sigma_pad(const float *__restrict__ x, int64_t Da, int64_t Db, int64_t Pa, int64_t Pb,
+                            float *__restrict__ xp, float *__restrict__ xT) {
+    constexpr int kSide = 32;
+    __shared__ float tile[kSide][kSide + 1];
+    const int64_t r0 = (int64_t)blockIdx.y * kSide, c0 = (int64_t)blockIdx.x * kSide;
+    for (int i = threadIdx.y; i < kSide; i += blockDim.y) {
         const int64_t r = r0 + i, c = c0 + threadIdx.x;
-        if (r < rows && c < cols) tile[i][threadIdx.x] = a[r * cols + c];
+        const float v = r < Da && c < Db ? x[r * Db + c] : 0.f;
+        tile[i][threadIdx.x] = v;
+        if (r < Da) xp[r * Pb + c] = v;
     }
     __syncthreads();
-    for (int i = threadIdx.y; i < kTile; i += blockDim.y) {
+    for (int i = threadIdx.y; i < kSide; i += blockDim.y) {
         const int64_t c = c0 + i, r = r0 + threadIdx.x;
-        if (r < rows && c < cols) t[c * rows + r] = tile[threadIdx.x][i];
+        if (c < Db) xT[c * Pa + r] = tile[threadIdx.x][i];
     }
 }
 
-// Pass 1: (A_k x)(Ia, Ib) into Ya at (((Ia * nTb + Ib / 32) * R / 4 + k / 4) * 32 + Ib % 32) * 4 + k % 4
-// and into Yb with the spins exchanged, and kx = K x.
-// Per-string diagonal sums fa, fb are factor-major ([R][D]).
-__global__ void __launch_bounds__(kThreads, 2)  // shared memory holds it to two blocks per SM
-    k_sigma_a(const SigmaArgs a, const float *__restrict__ F, const float *__restrict__ K1,
-              const float *__restrict__ fa, const float *__restrict__ fb, const float *__restrict__ ka,
-              const float *__restrict__ kb, const float *__restrict__ x, const float *__restrict__ xT,
-              float *__restrict__ Ya, float *__restrict__ Yb, float *__restrict__ kx) {
-    extern __shared__ __align__(16) float sm[];
-    const int L2 = a.L * a.L, R = a.R;
-    float *Fs = sm;                                                 // [L2][R]
-    float *Ks = Fs + (size_t)L2 * R;                                // [L2] (padded to 4)
-    uint2 *ea = reinterpret_cast<uint2 *>(Ks + ((L2 + 3) & ~3));    // [kTile][nsa]
-    uint2 *eb = ea + kTile * a.nsa;                                 // [kTile][nsb]
-    float *yt = reinterpret_cast<float *>(eb + kTile * a.nsb);      // [kTile][kYtRow]
-    float *kt = yt + kTile * kYtRow;                                // [kTile][kTile + 1]
-    for (int i = threadIdx.x; i < L2 * R; i += kThreads) Fs[i] = F[i];
-    for (int i = threadIdx.x; i < L2; i += kThreads) Ks[i] = K1[i];
-    const int64_t ta = (int64_t)blockIdx.y * kTile, tb = (int64_t)blockIdx.x * kTile;
-    stage_excitations(a.sa_t, a.sa_i, ta, a.Da, a.nsa, a.L, ea, a.err);
-    stage_excitations(a.sb_t, a.sb_i, tb, a.Db, a.nsb, a.L, eb, a.err);
+// Dynamic shared memory of an opposite-spin tile.
+size_t opposite_smem(int L) { return sizeof(float) * ((size_t)L * L * (kHalf + kC) + (size_t)kHalf * kZk); }
+
+// W and yd of a 64 alpha x 64 beta tile, by the two blocks of a cluster. Passes of 16
+// factors: block h forms z_k for its eight of them -- a warp takes a beta string, its
+// lanes the tile's alpha strings, two each, so the excitation and with it F is the same
+// for the warp -- into its shared memory; after the cluster's barrier it takes half the
+// alpha strings, a warp each with its lanes on the beta strings, two each, reads all 16
+// z_k of its rows (half of them from the other block's shared memory) and forms w, the
+// pair and with it s_k F the same for the warp again. A coefficient read from shared
+// memory costs the 128 bytes per clock of its way back to the registers even when all
+// lanes read one address, and that bounds the tile: with two rows per lane it serves
+// two multiply-adds. The excitations' descriptors
+// are read a step ahead (without, their latency cost 20 of 165 us).
+__device__ __forceinline__ void opposite_tile(const SigmaArgs &a, float *sm) {
+    auto cluster = cg::this_cluster();
+    const int half = (int)cluster.block_rank();
+    const int L2 = a.L * a.L, nsa = a.nsa, nsb = a.nsb;
+    float *Fs = sm, *Gs = Fs + L2 * kHalf;  // [L2][8] of this block's factors, [L2][16]
+    float *z = Gs + L2 * kC;                // [8][kTile alpha][kTile + 1 beta]
+    const int tile = blockIdx.x / 2;
+    const int64_t tb = (int64_t)(tile % (int)(a.Pb / kTile)) * kTile, ta = (int64_t)(tile / (int)(a.Pb / kTile)) * kTile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int c = 0; c < R; c += kSigmaChunk) {
-        __syncthreads();  // tables staged / the previous chunk's tile written out
-        // alpha phase: warp rows r, lanes on beta strings
-        for (int r = warp; r < kTile; r += kWarps) {
-            const int64_t Ia = ta + r, Ib = tb + lane;
-            const bool ok = Ia < a.Da && Ib < a.Db;
-            float acc[kSigmaChunk], kacc = 0.f;
-#pragma unroll
-            for (int k = 0; k < kSigmaChunk; ++k) acc[k] = 0.f;
-            if (ok) {
-                const float xi = x[Ia * a.Db + Ib];
-#pragma unroll
-                for (int k = 0; k < kSigmaChunk; ++k)
-                    acc[k] = xi * (fa[(int64_t)(c + k) * a.Da + Ia] + fb[(int64_t)(c + k) * a.Db + Ib]);
-                if (c == 0) kacc = xi * (ka[Ia] + kb[Ib]);
-                const uint2 *ex = ea + r * a.nsa;
-                for (int e = 0; e < a.nsa; ++e) {
-                    const uint2 v = ex[e];
-                    const float xv = exc_sign(v.y) * x[(int64_t)v.x * a.Db + Ib];
-                    const float4 *f4 = reinterpret_cast<const float4 *>(Fs + (size_t)(v.y >> 1) * R + c);
-#pragma unroll
-                    for (int q = 0; q < kSigmaChunk / 4; ++q) {
-                        const float4 f = f4[q];
-                        acc[4 * q] += f.x * xv;
-                        acc[4 * q + 1] += f.y * xv;
-                        acc[4 * q + 2] += f.z * xv;
-                        acc[4 * q + 3] += f.w * xv;
-                    }
-                    if (c == 0) kacc += Ks[v.y >> 1] * xv;
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kSigmaChunk; ++k) yt[r * kYtRow + k * (kTile + 1) + lane] = acc[k];
-            if (c == 0) kt[r * (kTile + 1) + lane] = kacc;
-        }
+    for (int c = 0; c < a.R; c += kC) {
+        if (c > 0) cluster.sync();  // both blocks are done with the factors and z
+        const float4 *F4 = reinterpret_cast<const float4 *>(a.F) + (size_t)(c / kC) * L2 * (kC / 4);
+        const float4 *G4 = reinterpret_cast<const float4 *>(a.G) + (size_t)(c / kC) * L2 * (kC / 4);
+        for (int i = threadIdx.x; i < L2 * (kHalf / 4); i += kThreads)
+            reinterpret_cast<float4 *>(Fs)[i] = __ldg(F4 + (i / 2) * (kC / 4) + half * 2 + (i & 1));
+        for (int i = threadIdx.x; i < L2 * (kC / 4); i += kThreads) reinterpret_cast<float4 *>(Gs)[i] = __ldg(G4 + i);
         __syncthreads();
-        // beta phase: warp columns cl, lanes on alpha strings
+        const int k0 = c + half * kHalf;
         for (int cl = warp; cl < kTile; cl += kWarps) {
-            const int64_t Ib = tb + cl, Ia = ta + lane;
-            const bool ok = Ib < a.Db && Ia < a.Da;
-            float acc[kSigmaChunk], kacc = 0.f;
+            const int64_t Ib = tb + cl;
+            uint64_t acc[2][kHalf / 2];
+            if (Ib < a.Db) {
+                const float *xc = a.xT + ta + lane;  // rows of Pa, zero past Da
+                const float x0 = __ldg(xc + Ib * a.Pa), x1 = __ldg(xc + Ib * a.Pa + 32);
 #pragma unroll
-            for (int k = 0; k < kSigmaChunk; ++k) acc[k] = 0.f;
-            if (ok) {
-                const uint2 *ex = eb + cl * a.nsb;
-                for (int e = 0; e < a.nsb; ++e) {
-                    const uint2 v = ex[e];
-                    const float xv = exc_sign(v.y) * xT[(int64_t)v.x * a.Da + Ia];
-                    const float4 *f4 = reinterpret_cast<const float4 *>(Fs + (size_t)(v.y >> 1) * R + c);
+                for (int k = 0; k < kHalf / 2; ++k) {
+                    const float f0 = __ldg(a.fb + (int64_t)(k0 + 2 * k) * a.Db + Ib),
+                                f1 = __ldg(a.fb + (int64_t)(k0 + 2 * k + 1) * a.Db + Ib);
+                    acc[0][k] = pack2(x0 * f0, x0 * f1);
+                    acc[1][k] = pack2(x1 * f0, x1 * f1);
+                }
+                const uint2 *ex = a.sb + Ib * nsb;
+                uint2 w[4];  // the next four excitations
 #pragma unroll
-                    for (int q = 0; q < kSigmaChunk / 4; ++q) {
-                        const float4 f = f4[q];
-                        acc[4 * q] += f.x * xv;
-                        acc[4 * q + 1] += f.y * xv;
-                        acc[4 * q + 2] += f.z * xv;
-                        acc[4 * q + 3] += f.w * xv;
+                for (int u = 0; u < 4; ++u)
+                    if (u < nsb) w[u] = __ldg(ex + u);
+                for (int e = 0; e < nsb; e += 4) {  // eight loads of x in flight
+                    uint2 v[4];
+                    float u0[4], u1[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = w[u];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (e + 4 + u < nsb) w[u] = __ldg(ex + e + 4 + u);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (e + u < nsb) {
+                            u0[u] = signed_by(__ldg(xc + (int64_t)v[u].x * a.Pa), v[u].y & 1u);
+                            u1[u] = signed_by(__ldg(xc + (int64_t)v[u].x * a.Pa + 32), v[u].y & 1u);
+                        }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (e + u < nsb) {
+                            const uint64_t p0 = pack2(u0[u], u0[u]), p1 = pack2(u1[u], u1[u]);
+                            const ulonglong2 *f = reinterpret_cast<const ulonglong2 *>(Fs + (v[u].y >> 1) * kHalf);
+#pragma unroll
+                            for (int k = 0; k < kHalf / 4; ++k) {
+                                const ulonglong2 f2 = f[k];
+                                acc[0][2 * k] = fma2(f2.x, p0, acc[0][2 * k]);
+                                acc[1][2 * k] = fma2(f2.x, p1, acc[1][2 * k]);
+                                acc[0][2 * k + 1] = fma2(f2.y, p0, acc[0][2 * k + 1]);
+                                acc[1][2 * k + 1] = fma2(f2.y, p1, acc[1][2 * k + 1]);
+                            }
+                        }
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kHalf / 2; ++k) acc[0][k] = acc[1][k] = 0;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float *zc = z + (lane + 32 * h) * (kTile + 1) + cl;
+#pragma unroll
+                for (int k = 0; k < kHalf / 2; ++k) {
+                    float lo, hi;
+                    unpack2(acc[h][k], lo, hi);
+                    zc[2 * k * kZk] = lo;
+                    zc[(2 * k + 1) * kZk] = hi;
+                }
+            }
+        }
+        cluster.sync();
+        const float *z0 = cluster.map_shared_rank(z, 0), *z1 = cluster.map_shared_rank(z, 1);
+        for (int r = half * (kTile / 2) + warp; r < (half + 1) * (kTile / 2); r += kWarps) {
+            const int64_t Ia = ta + r;
+            if (Ia >= a.Da) continue;
+            uint64_t zz[2][kC / 2];
+            float d[2] = {0.f, 0.f};
+#pragma unroll
+            for (int k = 0; k < kC / 2; ++k) {
+                const float *zr = (k < kHalf / 2 ? z0 + 2 * k * kZk : z1 + (2 * k - kHalf) * kZk) + r * (kTile + 1) + lane;
+                const float g0 = __ldg(a.ga + (int64_t)(c + 2 * k) * a.Da + Ia), g1 = __ldg(a.ga + (int64_t)(c + 2 * k + 1) * a.Da + Ia);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float lo = zr[32 * h], hi = zr[kZk + 32 * h];
+                    zz[h][k] = pack2(lo, hi);
+                    d[h] += g0 * lo + g1 * hi;
+                }
+            }
+            float *ydr = a.yd + Ia * a.Pb + tb + lane;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) ydr[32 * h] = c == 0 ? d[h] : ydr[32 * h] + d[h];
+            const uint2 *ex = a.sa + Ia * nsa;
+            float *Wc = a.W + tb + lane;
+            uint2 w[2];  // the next two excitations
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (u < nsa) w[u] = __ldg(ex + u);
+            for (int e = 0; e < nsa; e += 2) {
+                uint2 v[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) v[u] = w[u];
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (e + 2 + u < nsa) w[u] = __ldg(ex + e + 2 + u);
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (e + u < nsa) {
+                        const ulonglong2 *g = reinterpret_cast<const ulonglong2 *>(Gs + (v[u].y >> 1) * kC);
+                        uint64_t s[2][2] = {{0, 0}, {0, 0}};
+#pragma unroll
+                        for (int k = 0; k < kC / 4; ++k) {
+                            const ulonglong2 g2 = g[k];
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                s[h][0] = fma2(g2.x, zz[h][2 * k], s[h][0]);
+                                s[h][1] = fma2(g2.y, zz[h][2 * k + 1], s[h][1]);
+                            }
+                        }
+                        float *at = Wc + (int64_t)v[u].x * a.Pb;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            float p0, p1, p2, p3;
+                            unpack2(s[h][0], p0, p1);
+                            unpack2(s[h][1], p2, p3);
+                            const float x = signed_by((p0 + p1) + (p2 + p3), v[u].y & 1u);
+                            at[32 * h] = c == 0 ? x : at[32 * h] + x;
+                        }
                     }
-                    if (c == 0) kacc += Ks[v.y >> 1] * xv;
+            }
+        }
+    }
+    cluster.sync();  // the other block may still be reading this one's z
+}
+
+// Same-spin rows. A warp takes four rows of T, a group of 8 lanes each, and 32
+// consecutive columns of the other spin, 16 bytes a lane: an element is half a broadcast
+// 16-byte shared-memory read, one 16-byte read of X and four multiply-adds. Bound by the
+// 128 bytes per clock that come back from L1 or shared memory.
+constexpr int kSameE = 16;                // elements staged per warp and row
+constexpr int kSameRow = 2 * kSameE + 4;  // words: rows of a warp's four on different banks
+
+__device__ __forceinline__ void fma4(float4 &a, float s, const float4 x) {
+    a.x += s * x.x;
+    a.y += s * x.y;
+    a.z += s * x.z;
+    a.w += s * x.w;
+}
+
+// sum_e value_e X[target_e] over row S of the lane's group; Xc: X at the lane's columns,
+// rows P apart (in shared or global memory); st: the warp's staging area.
+template <bool SHARED>
+__device__ __forceinline__ float4 same_row(const uint2 *__restrict__ rows, int ne, int64_t S, const float *Xc, int64_t P,
+                                           uint32_t *st) {
+    const int lane = threadIdx.x & 31, g = lane >> 3, l = lane & 7;
+    const uint32_t *mine = st + g * kSameRow;
+    float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+    // each lane brings two elements of its group's row, one step ahead
+    const uint4 *src = reinterpret_cast<const uint4 *>(rows + S * ne) + l;
+    uint4 next = 2 * l < ne ? __ldg(src) : make_uint4(0u, 0u, 0u, 0u);
+    for (int e0 = 0; e0 < ne; e0 += kSameE) {
+        __syncwarp();
+        const int n = min(kSameE, ne - e0);  // a multiple of 8
+        *reinterpret_cast<uint4 *>(st + g * kSameRow + 4 * l) = next;
+        __syncwarp();
+        src += kSameE / 2;
+        if (e0 + kSameE + 2 * l < ne) next = __ldg(src);
+        for (int e = 0; e < n; e += 8) {
+            uint4 d[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) d[u] = *reinterpret_cast<const uint4 *>(mine + 2 * e + 4 * u);
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if constexpr (SHARED) {
+                    v[2 * u] = *reinterpret_cast<const float4 *>(Xc + d[u].x * (uint32_t)P);
+                    v[2 * u + 1] = *reinterpret_cast<const float4 *>(Xc + d[u].z * (uint32_t)P);
+                } else {
+                    v[2 * u] = __ldg(reinterpret_cast<const float4 *>(Xc + (int64_t)d[u].x * P));
+                    v[2 * u + 1] = __ldg(reinterpret_cast<const float4 *>(Xc + (int64_t)d[u].z * P));
                 }
             }
 #pragma unroll
-            for (int k = 0; k < kSigmaChunk; ++k) yt[lane * kYtRow + k * (kTile + 1) + cl] += acc[k];
-            if (c == 0) kt[lane * (kTile + 1) + cl] += kacc;
+            for (int u = 0; u < 4; ++u) {
+                fma4(a0, __uint_as_float(d[u].y), v[2 * u]);
+                fma4(a1, __uint_as_float(d[u].w), v[2 * u + 1]);
+            }
         }
+    }
+    return make_float4(a0.x + a1.x, a0.y + a1.y, a0.z + a1.z, a0.w + a1.w);
+}
+
+// uT rows of one panel (32 alpha columns) and one chunk of beta strings. Where the
+// panel fits, xT's 32 columns are copied to shared memory first.
+__device__ __forceinline__ void same_rows(const SigmaArgs &a, int block, float *sm) {
+    __shared__ __align__(16) uint32_t stage[kWarps][4 * kSameRow];
+    const int panel = block / a.chunks, chunk = block - panel * a.chunks;
+    if (panel >= a.panels) return;  // the odd block of the last cluster
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 3, l = lane & 7;
+    const int64_t col = (int64_t)panel * kPanel;
+    if (a.panel_rows > 0) {
+        for (int i = threadIdx.x; i < (int)a.Db * (kPanel / 4); i += kThreads)
+            reinterpret_cast<float4 *>(sm)[i] =
+                __ldg(reinterpret_cast<const float4 *>(a.xT + (int64_t)(i >> 3) * a.Pa + col) + (i & 7));
         __syncthreads();
-        // write out both orders: per string of the tile, this chunk's four groups of
-        // four factors for 32 strings (512 contiguous bytes per warp store)
-        for (int row = warp; row < kTile * (kSigmaChunk / 4); row += kWarps) {
-            const int r = row / (kSigmaChunk / 4), q = row - r * (kSigmaChunk / 4);
-            const int g = c / 4 + q;  // factor group
-            {
-                const int64_t Ia = ta + r, Ib = tb + lane;
-                if (Ia < a.Da && Ib < a.Db) {
-                    const float *src = yt + r * kYtRow + 4 * q * (kTile + 1) + lane;
-                    reinterpret_cast<float4 *>(Ya)[((Ia * a.nTb + blockIdx.x) * (R / 4) + g) * kTile + lane] =
-                        make_float4(src[0], src[kTile + 1], src[2 * (kTile + 1)], src[3 * (kTile + 1)]);
-                }
-            }
-            {
-                const int64_t Ib = tb + r, Ia = ta + lane;  // r is a beta column here
-                if (Ia < a.Da && Ib < a.Db) {
-                    const float *src = yt + lane * kYtRow + 4 * q * (kTile + 1) + r;
-                    reinterpret_cast<float4 *>(Yb)[((Ib * a.nTa + blockIdx.y) * (R / 4) + g) * kTile + lane] =
-                        make_float4(src[0], src[kTile + 1], src[2 * (kTile + 1)], src[3 * (kTile + 1)]);
-                }
-            }
-        }
-        if (c == 0)
-            for (int r = warp; r < kTile; r += kWarps) {
-                const int64_t Ia = ta + r, Ib = tb + lane;
-                if (Ia < a.Da && Ib < a.Db) kx[Ia * a.Db + Ib] = kt[r * (kTile + 1) + lane];
-            }
+    }
+    const int64_t groups = (a.Db + 3) / 4, g1 = min(groups, (int64_t)(chunk + 1) * a.per);
+    for (int64_t q = (int64_t)chunk * a.per + warp; q < g1; q += kWarps) {
+        const int64_t S = min(4 * q + g, a.Db - 1);  // rows past the last repeat it, and are not written
+        const float4 r = a.panel_rows > 0 ? same_row<true>(a.rows, a.ne, S, sm + 4 * l, kPanel, stage[warp])
+                                          : same_row<false>(a.rows, a.ne, S, a.xT + col + 4 * l, a.Pa, stage[warp]);
+        if (4 * q + g < a.Db) *reinterpret_cast<float4 *>(a.uT + S * a.Pa + col + 4 * l) = r;
     }
 }
 
-// sum_k G^k_pq y_k(J): g the factor row pq (shared memory), yj this lane's first
-// group of four factors in string J's block (group q at yj[32 q]).
-__device__ __forceinline__ float excitation_term(const float4 *__restrict__ g, const float4 *__restrict__ yj, int R4) {
-    float t = 0.f;
-#pragma unroll 4
-    for (int q = 0; q < R4; ++q) t += dot4(g[q], yj[q * kTile]);
-    return t;
-}
-
-// Pass 2: y = K x + sum_k A_k (1/2 s_k y_k), the scaled factors G = 1/2 s_k F^k;
-// ga, gb factor-major ([R][D]).
-__global__ void __launch_bounds__(kThreadsB, 2)
-    k_sigma_b(const SigmaArgs a, const float *__restrict__ G, const float *__restrict__ ga,
-              const float *__restrict__ gb, const float *__restrict__ Ya, const float *__restrict__ Yb,
-              const float *__restrict__ kx, float *__restrict__ y) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) k_sigma_parts(const SigmaArgs a) {
     extern __shared__ __align__(16) float sm[];
-    const int L2 = a.L * a.L, R = a.R, R4 = R / 4;
-    float *Gs = sm;                                              // [L2][R]
-    uint2 *ea = reinterpret_cast<uint2 *>(Gs + (size_t)L2 * R);  // [kTile][nsa]
-    uint2 *eb = ea + kTile * a.nsa;                              // [kTile][nsb]
-    float *st = reinterpret_cast<float *>(eb + kTile * a.nsb);   // [kTile][kTile + 1]
-    for (int i = threadIdx.x; i < L2 * R; i += kThreadsB) Gs[i] = G[i];
-    const int64_t ta = (int64_t)blockIdx.y * kTile, tb = (int64_t)blockIdx.x * kTile;
-    stage_excitations(a.sa_t, a.sa_i, ta, a.Da, a.nsa, a.L, ea, a.err);
-    stage_excitations(a.sb_t, a.sb_i, tb, a.Db, a.nsb, a.L, eb, a.err);
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float4 *G4 = reinterpret_cast<const float4 *>(Gs);
-    // alpha phase with the diagonal and K x
-    for (int r = warp; r < kTile; r += kWarpsB) {
-        const int64_t Ia = ta + r, Ib = tb + lane;
-        float acc = 0.f;
-        if (Ia < a.Da && Ib < a.Db) {
-            acc = kx[Ia * a.Db + Ib];
-            const float4 *yi = reinterpret_cast<const float4 *>(Ya) + (Ia * a.nTb + blockIdx.x) * R4 * kTile + lane;
-            for (int q = 0; q < R4; ++q) {
-                const float4 v = yi[q * kTile];
-                const int k = 4 * q;
-                acc += v.x * (ga[(int64_t)k * a.Da + Ia] + gb[(int64_t)k * a.Db + Ib]) +
-                       v.y * (ga[(int64_t)(k + 1) * a.Da + Ia] + gb[(int64_t)(k + 1) * a.Db + Ib]) +
-                       v.z * (ga[(int64_t)(k + 2) * a.Da + Ia] + gb[(int64_t)(k + 2) * a.Db + Ib]) +
-                       v.w * (ga[(int64_t)(k + 3) * a.Da + Ia] + gb[(int64_t)(k + 3) * a.Db + Ib]);
-            }
-            const uint2 *ex = ea + r * a.nsa;
-            // string J's block: yb + J * js
-            const float4 *yb = reinterpret_cast<const float4 *>(Ya) + (int64_t)blockIdx.x * R4 * kTile + lane;
-            const int64_t js = a.nTb * R4 * kTile;
-            int e = 0;
-            for (; e + 1 < a.nsa; e += 2) {  // two excitations' loads in flight together
-                const uint2 v0 = ex[e], v1 = ex[e + 1];
-                const float t0 = excitation_term(G4 + (size_t)(v0.y >> 1) * R4, yb + v0.x * js, R4);
-                const float t1 = excitation_term(G4 + (size_t)(v1.y >> 1) * R4, yb + v1.x * js, R4);
-                acc += exc_sign(v0.y) * t0 + exc_sign(v1.y) * t1;
-            }
-            if (e < a.nsa) {
-                const uint2 v0 = ex[e];
-                acc += exc_sign(v0.y) * excitation_term(G4 + (size_t)(v0.y >> 1) * R4, yb + v0.x * js, R4);
+    if ((int)blockIdx.x < 2 * a.tiles)
+        opposite_tile(a, sm);
+    else
+        same_rows(a, (int)blockIdx.x - 2 * a.tiles, sm);
+}
+
+// y(Ia, Ib) = (T^a x) + yd + the sum of W's rows of Ia + uT(Ib, Ia), 32 beta columns per
+// panel (blockIdx.y), alpha strings in chunks (blockIdx.x) of `per` groups of four.
+__global__ void __launch_bounds__(kThreads, 1)
+    k_sigma_sum(const SigmaArgs a, const uint2 *__restrict__ rows, int ne, int per, const float *__restrict__ xp,
+                float *__restrict__ y) {
+    __shared__ __align__(16) uint32_t stage[kWarps][4 * kSameRow];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 3, l = lane & 7;
+    const int64_t P = a.Pb, col = (int64_t)blockIdx.y * kPanel + 4 * l;
+    const int64_t groups = (a.Da + 3) / 4, g1 = min(groups, (int64_t)(blockIdx.x + 1) * per);
+    for (int64_t q = (int64_t)blockIdx.x * per + warp; q < g1; q += kWarps) {
+        const int64_t S = min(4 * q + g, a.Da - 1);
+        const float4 r = same_row<false>(rows, ne, S, xp + col, P, stage[warp]);
+        const float *w = a.W + S * a.nsa * P + col;
+        float4 b0 = __ldg(reinterpret_cast<const float4 *>(a.yd + S * P + col)), b1 = make_float4(0.f, 0.f, 0.f, 0.f);
+        int e = 0;
+        for (; e + 8 <= a.nsa; e += 8) {  // read once: streamed past L1
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)(e + u) * P));
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+                fma4(b0, 1.f, v[u]);
+                fma4(b1, 1.f, v[u + 1]);
             }
         }
-        st[r * (kTile + 1) + lane] = acc;
-    }
-    __syncthreads();
-    for (int cl = warp; cl < kTile; cl += kWarpsB) {
-        const int64_t Ib = tb + cl, Ia = ta + lane;
-        float acc = 0.f;
-        if (Ib < a.Db && Ia < a.Da) {
-            const uint2 *ex = eb + cl * a.nsb;
-            const float4 *yb = reinterpret_cast<const float4 *>(Yb) + (int64_t)blockIdx.y * R4 * kTile + lane;
-            const int64_t js = a.nTa * R4 * kTile;
-            int e = 0;
-            for (; e + 1 < a.nsb; e += 2) {
-                const uint2 v0 = ex[e], v1 = ex[e + 1];
-                const float t0 = excitation_term(G4 + (size_t)(v0.y >> 1) * R4, yb + v0.x * js, R4);
-                const float t1 = excitation_term(G4 + (size_t)(v1.y >> 1) * R4, yb + v1.x * js, R4);
-                acc += exc_sign(v0.y) * t0 + exc_sign(v1.y) * t1;
-            }
-            if (e < a.nsb) {
-                const uint2 v0 = ex[e];
-                acc += exc_sign(v0.y) * excitation_term(G4 + (size_t)(v0.y >> 1) * R4, yb + v0.x * js, R4);
-            }
-        }
-        st[lane * (kTile + 1) + cl] += acc;
-    }
-    __syncthreads();
-    for (int r = warp; r < kTile; r += kWarpsB) {
-        const int64_t Ia = ta + r, Ib = tb + lane;
-        if (Ia < a.Da && Ib < a.Db) y[Ia * a.Db + Ib] = st[r * (kTile + 1) + lane];
+        for (; e < a.nsa; ++e) fma4(b0, 1.f, __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)e * P)));
+        const float c[4] = {r.x + (b0.x + b1.x), r.y + (b0.y + b1.y), r.z + (b0.z + b1.z), r.w + (b0.w + b1.w)};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (4 * q + g < a.Da && col + u < a.Db)
+                y[S * a.Db + col + u] = c[u] + __ldg(a.uT + (col + u) * a.Pa + S);
     }
 }
 
-size_t smem_a_bytes(int L, int R, int nsa, int nsb) {
-    const int L2 = L * L;
-    return sizeof(float) * ((size_t)L2 * R + ((L2 + 3) & ~3)) + sizeof(uint2) * (size_t)kTile * (nsa + nsb) +
-           sizeof(float) * ((size_t)kTile * kYtRow + (size_t)kTile * (kTile + 1));
+// Row chunks of the same-spin panels: blocks of 1,024 threads, one per SM, each on one
+// panel of 32 columns (118 KB of x at L=12: it stays in L1 or shared memory); the number
+// of chunks that leaves the fewest row groups on the busiest SM.
+int same_chunks(int64_t groups, int64_t panels) {
+    const int64_t sms = sm_count();
+    int best = 1;
+    int64_t cost = INT64_MAX;
+    for (int c = 1; c <= 64 && (c - 1) * 8 < groups; ++c) {
+        const int64_t per = (groups + c - 1) / c, rounds = (panels * c + sms - 1) / sms;
+        if (per * rounds + 2 * rounds < cost) {  // a block's start and end: about two row groups
+            cost = per * rounds + 2 * rounds;
+            best = c;
+        }
+    }
+    return best;
 }
-size_t smem_b_bytes(int L, int R, int nsa, int nsb) {
-    return sizeof(float) * (size_t)L * L * R + sizeof(uint2) * (size_t)kTile * (nsa + nsb) +
-           sizeof(float) * (size_t)kTile * (kTile + 1);
-}
+
 constexpr size_t kSigmaMaxSmem = 200 * 1024;
+constexpr size_t kSigmaMaxPanel = 192 * 1024;  // a same-spin panel held in shared memory
+// Spaces of fewer 32 x 32 string tiles than SMs: the operator's three launches and its
+// passes of 16 factors take a fixed time each there, the stored values a time by size.
+// Measured per product (operator | stored): rank 16: L=12 3a3b, 48,400 rows, 44 | 47 us;
+// L=10 5a5b, 63,504 rows, 42 | 68; L=9 4a4b, 15,876 rows, 37 | 16; two passes: L=10 5a4b,
+// rank 28, 67 | 63; four: L=10 5a5b, rank 60, 124 | 68. So one pass, from 50,000 rows.
+constexpr int64_t kSigmaMinRows = 50000;
+constexpr size_t kSigmaMaxTables = 132864;  // factors, pairs and excitation lists (bytes): past it, and not
+                                            // measured, the stored values serve
 
 }  // namespace
 
-size_t sigma_bytes(int L, int64_t Da, int64_t Db, int R) {
-    const int64_t dim = Da * Db, padded = Da * ((Db + kTile - 1) / kTile) * kTile + Db * ((Da + kTile - 1) / kTile) * kTile;
-    return sizeof(float) * ((size_t)padded * R + 2 * (size_t)dim + (size_t)(Da + Db) * (2 * R + 1) +
-                            (size_t)L * L * (2 * R + 1));
+size_t sigma_bytes(int L, int na, int nb, int R) {
+    auto dim = [&](int n) { return d_binom(L, n); };
+    auto pad = [](int64_t d) { return (d + kTile - 1) / kTile * kTile; };
+    auto rows = [&](int n) {  // same-spin rows and the excitation places
+        return dim(n) * (8 * (1 + 2 * (int64_t)n * (L - n) + d_binom(n, 2) * d_binom(L - n, 2) + 8));
+    };
+    const int64_t Da = dim(na), Db = dim(nb);
+    return (size_t)(rows(na) + rows(nb)) +
+           sizeof(float) * ((size_t)Da * (na * (L - na) + 2) * pad(Db) + 2 * (size_t)Db * pad(Da) + (size_t)(Da + Db) * R +
+                            2 * (size_t)L * L * R);
 }
 
 bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const SpinTables &ta,
-                   const SpinTables &tb, bool any_grid, cudaStream_t s) {
+                   const SpinTables &tb, const FciParams &p, bool any_grid, cudaStream_t s) {
     op.R = 0;
     if (!sigma_applies(L) || ta.D < 1 || tb.D < 1) return false;
-    // a grid of fewer tiles than SMs leaves the GPU part idle: the stored FP32 slot
-    // values are faster there (L=10 5a5b, 64 tiles: 0.13 against 0.07 ms)
-    if (!any_grid && ((ta.D + kTile - 1) / kTile) * ((tb.D + kTile - 1) / kTile) < sm_count()) return false;
+    const bool small = ((ta.D + 31) / 32) * ((tb.D + 31) / 32) < sm_count();
+    if (!any_grid && small && ta.D * tb.D < kSigmaMinRows) return false;
     const int L2 = L * L;
     const size_t N = (size_t)L2;
     // The factors, in the space of orbital pairs p >= q: with c = 1 on the diagonal
@@ -410,104 +569,118 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
     }
     const int rank = (int)vecs.size();
     const int R = std::max(kSigmaChunk, (rank + kSigmaChunk - 1) / kSigmaChunk * kSigmaChunk);
-    if (R > kSigmaMaxRank || smem_a_bytes(L, R, ta.ns, tb.ns) > kSigmaMaxSmem ||
-        smem_b_bytes(L, R, ta.ns, tb.ns) > kSigmaMaxSmem)
+    if (!any_grid && small && R > kC) return false;
+    if (R > kSigmaMaxRank ||
+        sizeof(float) * N * (R + 1) + sizeof(uint2) * (size_t)kTile * (ta.ns + tb.ns) > kSigmaMaxTables ||
+        opposite_smem(L) > kSigmaMaxSmem || ta.D * std::max(ta.ns, 1) > (int64_t)UINT32_MAX)
         return false;
-    std::vector<float> F(N * R, 0.f), G(N * R, 0.f), K1(N);
+    // [R / 16][L^2][16]
+    std::vector<float> F(N * R, 0.f), G(N * R, 0.f);
+    auto place = [&](size_t pq, int k) { return ((size_t)(k / kC) * N + pq) * kC + k % kC; };
     for (int j = 0; j < rank; ++j)
         for (int i = 0; i < P; ++i) {
             const double f = vecs[j][i] / cP[i];
-            const size_t a = (size_t)(pp[i] * L + pq_[i]) * R + j, b = (size_t)(pq_[i] * L + pp[i]) * R + j;
+            const size_t a = place((size_t)pp[i] * L + pq_[i], j), b = place((size_t)pq_[i] * L + pp[i], j);
             F[a] = F[b] = (float)f;
-            G[a] = G[b] = (float)(0.5 * sgn[j] * f);
-        }
-    for (int p = 0; p < L; ++p)
-        for (int q = 0; q < L; ++q) {
-            double k = h[p * L1 + q];
-            for (int r = 0; r < L; ++r) k -= 0.5 * eri[p * L3 + r * N + r * L1 + q];  // (pr|rq)
-            K1[(size_t)p * L + q] = (float)k;
+            G[a] = G[b] = (float)(sgn[j] * f);
         }
     // per-string diagonal sums over occupied orbitals, factor-major
-    auto diag_sums = [&](const SpinTables &t, std::vector<float> &fs, std::vector<float> &gs, std::vector<float> &ks) {
-        fs.assign((size_t)R * t.D, 0.f);
-        gs.assign((size_t)R * t.D, 0.f);
-        ks.assign((size_t)t.D, 0.f);
-        for (int64_t S = 0; S < t.D; ++S) {
-            double kk = 0;
-            for (int m = 0; m < t.n; ++m) {
-                const int p = t.occ[(size_t)S * t.n + m];
-                kk += K1[(size_t)p * L + p];
+    auto diag_sums = [&](const SpinTables &t, const std::vector<float> &X, std::vector<float> &xs) {
+        xs.assign((size_t)R * t.D, 0.f);
+        for (int j = 0; j < R; ++j)
+            for (int64_t S = 0; S < t.D; ++S) {
+                double v = 0;
+                for (int m = 0; m < t.n; ++m) v += X[place((size_t)t.occ[(size_t)S * t.n + m] * (L + 1), j)];
+                xs[(size_t)j * t.D + S] = (float)v;
             }
-            ks[S] = (float)kk;
-            for (int j = 0; j < R; ++j) {
-                double f = 0, g = 0;
-                for (int m = 0; m < t.n; ++m) {
-                    const int p = t.occ[(size_t)S * t.n + m];
-                    f += F[(size_t)(p * L + p) * R + j];
-                    g += G[(size_t)(p * L + p) * R + j];
-                }
-                fs[(size_t)j * t.D + S] = (float)f;
-                gs[(size_t)j * t.D + S] = (float)g;
-            }
-        }
     };
-    std::vector<float> fa, ga, kav, fb, gb, kbv;
-    diag_sums(ta, fa, ga, kav);
-    diag_sums(tb, fb, gb, kbv);
+    std::vector<float> ga, fb;
+    diag_sums(ta, G, ga);
+    diag_sums(tb, F, fb);
     auto up = [&](DevBuf<float> &buf, const std::vector<float> &v) {
         buf.alloc(v.size());
         if (!v.empty()) CIGPU_CUDA(cudaMemcpyAsync(buf.p, v.data(), v.size() * sizeof(float), cudaMemcpyHostToDevice, s));
     };
     up(op.F, F);
     up(op.G, G);
-    up(op.K1, K1);
-    up(op.fa, fa);
-    up(op.fb, fb);
     up(op.ga, ga);
-    up(op.gb, gb);
-    up(op.ka, kav);
-    up(op.kb, kbv);
-    const int64_t dim = ta.D * tb.D;
-    op.xT.alloc((size_t)dim);
-    const int64_t nTa = (ta.D + kTile - 1) / kTile, nTb = (tb.D + kTile - 1) / kTile;
-    op.Ya.alloc((size_t)ta.D * nTb * kTile * R);  // factor blocks of 32 strings, the last one padded
-    op.Yb.alloc((size_t)tb.D * nTa * kTile * R);
-    op.kx.alloc((size_t)dim);
+    up(op.fb, fb);
     op.L = L;
     op.rank = rank;
     op.Da = ta.D;
     op.Db = tb.D;
-    op.smem_a = smem_a_bytes(L, R, ta.ns, tb.ns);
-    op.smem_b = smem_b_bytes(L, R, ta.ns, tb.ns);
+    op.Pa = (ta.D + kTile - 1) / kTile * kTile;
+    op.Pb = (tb.D + kTile - 1) / kTile * kTile;
+    op.nea = (p.a.nfull + 7) / 8 * 8;
+    op.neb = (p.b.nfull + 7) / 8 * 8;
+    op.ea.alloc((size_t)op.Da * op.nea);
+    op.eb.alloc((size_t)op.Db * op.neb);
+    op.sa.alloc(std::max<size_t>((size_t)op.Da * ta.ns, 1));
+    op.sb.alloc(std::max<size_t>((size_t)op.Db * tb.ns, 1));
+    const int g = sm_count() * 8;
+    unsigned long long *ew = check_word_device();
+    k_sigma_rows<<<g, 256, 0, s>>>(p.a, op.nea, op.ea.p, ew);
+    k_sigma_rows<<<g, 256, 0, s>>>(p.b, op.neb, op.eb.p, ew);
+    count_launch(2);
+    if (ta.ns > 0) {
+        DevBuf<uint32_t> back((size_t)op.Da * ta.ns);
+        k_sigma_back<<<g, 256, 0, s>>>(p.a, L, back.p);
+        k_sigma_singles<<<g, 256, 0, s>>>(p.a, L, back.p, op.sa.p, ew);
+        count_launch(2);
+    }
+    if (tb.ns > 0) {
+        k_sigma_singles<<<g, 256, 0, s>>>(p.b, L, nullptr, op.sb.p, ew);
+        count_launch();
+    }
+    CIGPU_CUDA(cudaGetLastError());
+    op.xp.alloc((size_t)op.Da * op.Pb);
+    op.xT.alloc((size_t)op.Db * op.Pa);
+    op.uT.alloc((size_t)op.Db * op.Pa);
+    op.yd.alloc((size_t)op.Da * op.Pb);
+    op.W.alloc(std::max<size_t>((size_t)op.Da * ta.ns * op.Pb, 1));
     op.R = R;
     return true;
 }
 
 void sigma_mv32(SigmaOp &op, const FciParams &p, const float *x, float *y, cudaStream_t s) {
-    static const bool attr_set = [] {  // thread-safe one-time init
-        cudaFuncSetAttribute(k_sigma_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSigmaMaxSmem);
-        cudaFuncSetAttribute(k_sigma_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSigmaMaxSmem);
-        return true;
-    }();
-    (void)attr_set;
-    const SigmaArgs a{op.L,
-                      op.R,
-                      p.a.ns,
-                      p.b.ns,
-                      op.Da,
-                      op.Db,
-                      (op.Da + kTile - 1) / kTile,
-                      (op.Db + kTile - 1) / kTile,
-                      p.a.s_target,
-                      p.a.s_info,
-                      p.b.s_target,
-                      p.b.s_info,
-                      check_word_device()};
-    const dim3 tgrid((unsigned)((op.Db + kTile - 1) / kTile), (unsigned)((op.Da + kTile - 1) / kTile));
-    k_transpose32<<<tgrid, dim3(kTile, 8), 0, s>>>(x, op.Da, op.Db, op.xT.p);
-    k_sigma_a<<<tgrid, kThreads, op.smem_a, s>>>(a, op.F.p, op.K1.p, op.fa.p, op.fb.p, op.ka.p, op.kb.p, x, op.xT.p,
-                                                  op.Ya.p, op.Yb.p, op.kx.p);
-    k_sigma_b<<<tgrid, kThreadsB, op.smem_b, s>>>(a, op.G.p, op.ga.p, op.gb.p, op.Ya.p, op.Yb.p, op.kx.p, y);
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_sigma_parts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSigmaMaxSmem);
+    CIGPU_CUDA(attr);
+    SigmaArgs a{};
+    a.L = op.L;
+    a.R = op.R;
+    a.nsa = p.a.ns;
+    a.nsb = p.b.ns;
+    a.Da = op.Da;
+    a.Db = op.Db;
+    a.Pa = op.Pa;
+    a.Pb = op.Pb;
+    a.sa = op.sa.p;
+    a.sb = op.sb.p;
+    a.F = op.F.p;
+    a.G = op.G.p;
+    a.ga = op.ga.p;
+    a.fb = op.fb.p;
+    a.rows = op.eb.p;
+    a.ne = op.neb;
+    a.tiles = (int)((op.Pa / kTile) * (op.Pb / kTile));
+    a.panels = (int)((op.Da + kPanel - 1) / kPanel);
+    const int64_t gb = (op.Db + 3) / 4, ga = (op.Da + 3) / 4;
+    a.chunks = same_chunks(gb, a.panels);
+    a.per = (int)((gb + a.chunks - 1) / a.chunks);
+    const size_t panel = sizeof(float) * kPanel * (size_t)op.Db;
+    a.panel_rows = panel <= kSigmaMaxPanel ? (int)op.Db : 0;
+    a.xT = op.xT.p;
+    a.W = op.W.p;
+    a.yd = op.yd.p;
+    a.uT = op.uT.p;
+    const size_t smem = std::max(opposite_smem(op.L), a.panel_rows ? panel : 0);
+    const int64_t blocks = 2 * (int64_t)a.tiles + ((int64_t)a.panels * a.chunks + 1) / 2 * 2;
+    k_sigma_pad<<<dim3((unsigned)(op.Pb / 32), (unsigned)(op.Pa / 32)), dim3(32, 8), 0, s>>>(x, op.Da, op.Db, op.Pa, op.Pb,
+                                                                                             op.xp.p, op.xT.p);
+    k_sigma_parts<<<(unsigned)blocks, kThreads, smem, s>>>(a);
+    const int pb = (int)((op.Db + kPanel - 1) / kPanel), c = same_chunks(ga, pb);
+    k_sigma_sum<<<dim3((unsigned)c, (unsigned)pb), kThreads, 0, s>>>(a, op.ea.p, op.nea, (int)((ga + c - 1) / c), op.xp.p, y);
     CIGPU_CUDA(cudaGetLastError());
     count_launch(3);
 }
