@@ -700,6 +700,12 @@ int solve_crs(cigpu_crs &crs, double tol, int64_t max_matvec, double *c_dev, boo
     if (crs.precision == CIGPU_MIXED)
         P.mv32 = [cp](const float *x, float *y, cudaStream_t st) { crs_mv32(*cp, x, y, st); };
     P.fp32_first_anchor = crs.sig != nullptr;
+    if (crs.precision == CIGPU_FP64 && !crs.slots && !crs.pairs && !crs.onthefly && crs.val64.p) {
+        P.row_ptr = crs.row_ptr.p;
+        P.col = crs.col.p;
+        P.val = crs.val64.p;
+        P.nnz = crs.nnz_full;
+    }
     SolveOptions o;
     o.tol = tol;
     o.max_matvec = max_matvec;

@@ -26,6 +26,9 @@
 #include <exception>
 #include <mutex>
 
+#include <cooperative_groups.h>
+
+#include "checked.cuh"
 #include "lanczos.cuh"
 #include "small_eigh.h"
 #include <type_traits>
@@ -646,11 +649,148 @@ __global__ void k_convert(const S *__restrict__ s, D *__restrict__ d, int64_t n)
 }
 
 // ---------------------------------------------------------------------------
+// Several whole Lanczos steps of a small problem in one launch: product, two classical
+// Gram-Schmidt passes, norm and scaling, on one cluster of 16 blocks. A block owns a
+// slice of the rows and keeps its slice of every basis vector in shared memory over the
+// steps; the product's vector is copied whole into shared memory first. The dot products
+// meet through distributed shared memory, every block adding the 16 parts in the same
+// order. A step of the separate kernels is six launches of a few microseconds each for
+// work of less than one, so the launches, not the arithmetic, were the solve (DOCI L=12,
+// 924 rows, residual 1e-11, ~66 steps: whole call 5.46 -> 2.14 ms, half of the rest the
+// host's eigensolves of T, one per launch). Up to kSmallRows rows and kSmallNnz
+// elements, past which the product or the dots take longer on 16 SMs than the launches
+// on all of them.
+constexpr int kSmallCluster = 16;
+constexpr int kSmallThreads = 256;
+constexpr int64_t kSmallRows = 4096;
+constexpr int64_t kSmallNnz = 400000;
+constexpr int kSmallSteps = 4;                 // steps per launch
+constexpr int kSmallOut = 2 * (kMaxBasis + 1) + 1;  // first pass, second pass, norm^2
+
+// Basis slices are rows of a pitch that puts eight of them on different banks.
+__host__ __device__ inline int small_pitch(int64_t n) {
+    const int slice = (int)((n + kSmallCluster - 1) / kSmallCluster);
+    return (slice + 15) / 16 * 16 + 4;
+}
+inline size_t small_smem(int64_t n, int m) {
+    return sizeof(double) * ((size_t)n + (size_t)(m + 2) * small_pitch(n) + 3 * (kMaxBasis + 1) + kSmallThreads + 1);
+}
+
+__global__ void __launch_bounds__(kSmallThreads) k_lanczos_steps(int64_t n, double *__restrict__ V, int j0, int steps,
+                                                                 int m, const int64_t *__restrict__ row_ptr,
+                                                                 const uint32_t *__restrict__ col,
+                                                                 const double *__restrict__ val,
+                                                                 double *__restrict__ out, unsigned long long *err) {
+    namespace cg = cooperative_groups;
+    auto cluster = cg::this_cluster();
+    extern __shared__ __align__(16) double small_sm[];
+    const int pitch = small_pitch(n), slice = (int)((n + kSmallCluster - 1) / kSmallCluster);
+    double *x = small_sm;                      // [n] the vector the matrix acts on
+    double *Vs = x + n;                        // [m + 1][pitch] this block's slices of the basis
+    double *w = Vs + (size_t)(m + 1) * pitch;  // [pitch]
+    double *part = w + pitch;                  // [2][kMaxBasis + 1] this block's dots, one set per pass
+    double *h = part + 2 * (kMaxBasis + 1);    // [kMaxBasis + 1] their sums
+    double *scr = h + (kMaxBasis + 1);         // [kSmallThreads]
+    double *nrm = scr + kSmallThreads;         // this block's ||w||^2
+    const int t = threadIdx.x, rank = (int)cluster.block_rank();
+    const int64_t r0 = (int64_t)rank * slice;
+    const int mine = (int)max((int64_t)0, min((int64_t)slice, n - r0));
+    for (int i = t; i < (j0 + 1) * mine; i += kSmallThreads) {
+        const int v = i / mine, r = i - v * mine;
+        Vs[(size_t)v * pitch + r] = V[(int64_t)v * n + r0 + r];
+    }
+    // threads per row of the updates: they share the basis vectors
+    const int rows = mine <= 64 ? 64 : mine <= 128 ? 128 : 256, share = kSmallThreads / rows;
+    for (int s = 0; s < steps; ++s) {
+        const int j = j0 + s, nv = j + 1;
+        for (int64_t i = t; i < n; i += kSmallThreads) x[i] = __ldcg(V + (int64_t)j * n + i);  // written by the cluster
+        __syncthreads();
+        // w = H v_j: eight lanes per row
+        for (int r = t >> 3; r < (slice + 3) / 4 * 4; r += kSmallThreads / 8) {  // whole warps: four rows each
+            double a = 0;
+            if (r < mine) {
+                const int64_t b = __ldg(row_ptr + r0 + r), e = __ldg(row_ptr + r0 + r + 1);
+                for (int64_t k = b + (t & 7); k < e; k += 8) {
+                    const uint32_t c = __ldg(col + k);
+                    if (CIGPU_CHECK(err, index_ok(c, (uint64_t)n), kCheckColumn, c)) a += __ldg(val + k) * x[c];
+                }
+            }
+            for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if ((t & 7) == 0 && r < mine) w[r] = a;
+        }
+        __syncthreads();
+        double *o = out + (size_t)s * kSmallOut;
+        for (int pass = 0; pass < 2; ++pass) {
+            double *p = part + pass * (kMaxBasis + 1);
+            // dots: four lanes per basis vector
+            for (int i = t >> 2; i < (nv + 7) / 8 * 8; i += kSmallThreads / 4) {
+                double a = 0;
+                if (i < nv)
+                    for (int r = t & 3; r < mine; r += 4) a += Vs[(size_t)i * pitch + r] * w[r];
+                a += __shfl_xor_sync(0xffffffffu, a, 2);
+                a += __shfl_xor_sync(0xffffffffu, a, 1);
+                if ((t & 3) == 0 && i < nv) p[i] = a;
+            }
+            cluster.sync();
+            for (int i = t; i < nv; i += kSmallThreads) {
+                double a[kSmallCluster];
+#pragma unroll
+                for (int b = 0; b < kSmallCluster; ++b) a[b] = cluster.map_shared_rank(p, b)[i];
+                double sum = 0;
+#pragma unroll
+                for (int b = 0; b < kSmallCluster; ++b) sum += a[b];
+                h[i] = sum;
+                if (rank == 0) o[pass * (kMaxBasis + 1) + i] = sum;
+            }
+            __syncthreads();
+            // w -= sum_i h_i V_i; the second pass also ||w||^2
+            const int r = t % rows, g = t / rows;
+            double a = 0;
+            if (r < mine)
+                for (int i = g; i < nv; i += share) a += Vs[(size_t)i * pitch + r] * h[i];
+            scr[t] = a;
+            __syncthreads();
+            double sq = 0;
+            if (t < rows) {
+                double y = t < mine ? w[t] : 0.0;
+                for (int q = 0; q < share; ++q) y -= scr[q * rows + t];
+                if (t < mine) w[t] = y;
+                sq = t < mine ? y * y : 0.0;
+            }
+            __syncthreads();
+            if (pass == 1) {
+                for (int d = 16; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
+                if ((t & 31) == 0) scr[t >> 5] = sq;
+                __syncthreads();
+                if (t == 0) {
+                    double a2 = 0;
+                    for (int q = 0; q < kSmallThreads / 32; ++q) a2 += scr[q];
+                    *nrm = a2;
+                }
+            }
+        }
+        cluster.sync();
+        double total = 0;
+#pragma unroll
+        for (int b = 0; b < kSmallCluster; ++b) total += *cluster.map_shared_rank(nrm, b);
+        if (rank == 0 && t == 0) o[2 * (kMaxBasis + 1)] = total;
+        const double inv = 1.0 / sqrt(total);
+        for (int r = t; r < mine; r += kSmallThreads) {
+            const double v = w[r] * inv;
+            Vs[(size_t)(j + 1) * pitch + r] = v;
+            V[(int64_t)(j + 1) * n + r0 + r] = v;
+        }
+        cluster.sync();  // the vector is whole, and every block's sums are read
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Host-side helpers around the kernels.
 
 // Pinned result buffers are pooled for the life of the process: cudaFreeHost
 // synchronises the whole device, which would stall every concurrent solve.
-constexpr size_t kPinnedDoubles = 4 * (kMaxBasis + 2);
+constexpr int kSmallDepth = 2;  // launches of several steps in flight
+constexpr size_t kPinnedDoubles = std::max<size_t>(4 * (kMaxBasis + 2), kSmallDepth * kSmallSteps * kSmallOut);
 std::mutex g_pinned_mutex;
 std::vector<double *> g_pinned_pool;
 
@@ -678,6 +818,33 @@ void pinned_put(double *p) {
 // 16-byte aligned start.
 inline bool vec4_ok(const float *p, int64_t ld, int64_t n) {
     return n % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+}
+
+// Whether the device runs a cluster of k_lanczos_steps with this much shared memory.
+bool small_cluster_ok(size_t smem) {
+    static const bool attr = [] {  // thread-safe one-time init
+        const bool ok = cudaFuncSetAttribute(k_lanczos_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
+                        cudaFuncSetAttribute(k_lanczos_steps, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }();
+    if (!attr || smem > 227 * 1024) return false;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kSmallCluster);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kSmallCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_lanczos_steps, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return clusters > 0;
 }
 
 struct VecOps {
@@ -922,6 +1089,101 @@ struct TRLanczos {
         CIGPU_CUDA(cudaStreamSynchronize(s));
     }
 
+    // run() for a small problem on a stored CRS: kSmallSteps steps per launch
+    // (k_lanczos_steps, which leaves their coefficients in pinned memory), kSmallDepth
+    // launches in flight while the host analyses T after each of them. The steps past
+    // the one that meets the target are discarded, as run()'s speculative one.
+    bool run_small(const SolveProblem &P, double abs_target, double rel_target, int64_t budget) {
+        double best = 1e300;
+        int64_t best_at = matvecs;
+        auto target = [&] { return std::max(abs_target, rel_target * std::max(1.0, std::fabs(theta0))); };
+        struct Events {
+            cudaEvent_t e[kSmallDepth] = {};
+            Events() {
+                for (auto &x : e) CIGPU_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+            }
+            ~Events() {
+                for (auto x : e)
+                    if (x) cudaEventDestroy(x);
+            }
+        } ev;
+        int count[kSmallDepth] = {}, queued = j;  // steps per launch in flight; vectors once they are done
+        int64_t head = 0, tail = 0;               // launches made, launches read
+        auto launch = [&] {
+            const int steps = (int)std::min<int64_t>({kSmallSteps, m - queued, n - queued, budget - matvecs});
+            if (steps < 1 || head - tail >= kSmallDepth) return false;
+            const int slot = (int)(head % kSmallDepth);
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(kSmallCluster);
+            cfg.blockDim = dim3(kSmallThreads);
+            cfg.dynamicSmemBytes = small_smem(n, m);
+            cfg.stream = s;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = kSmallCluster;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            CIGPU_CUDA(cudaLaunchKernelEx(&cfg, k_lanczos_steps, n, V.p, queued, steps, m, P.row_ptr, P.col, P.val,
+                                          ops.h_out + (size_t)slot * kSmallSteps * kSmallOut, check_word_device()));
+            count_launch();
+            CIGPU_CUDA(cudaEventRecord(ev.e[slot], s));
+            count[slot] = steps;
+            queued += steps;
+            matvecs += steps;
+            ++head;
+            return true;
+        };
+        auto drain = [&] {
+            CIGPU_CUDA(cudaStreamSynchronize(s));
+            tail = head;
+        };
+        for (;;) {
+            while (launch()) {
+            }
+            if (head == tail) break;  // out of budget
+            const int slot = (int)(tail % kSmallDepth);
+            const double t0 = wall();
+            CIGPU_CUDA(cudaEventSynchronize(ev.e[slot]));
+            g_clk.wait += wall() - t0;
+            ++g_clk.n_wait;
+            const double *h = ops.h_out + (size_t)slot * kSmallSteps * kSmallOut;
+            bool breakdown = false;
+            for (int k = 0; k < count[slot] && !breakdown; ++k, h += kSmallOut) {
+                for (int i = 0; i <= j; ++i) t(i, j) = t(j, i) = h[i] + h[kMaxBasis + 1 + i];
+                const double beta = std::sqrt(h[2 * (kMaxBasis + 1)]);
+                t(j + 1, j) = t(j, j + 1) = beta;
+                ++j;
+                // not a number once the space is exhausted: nothing is left to expand
+                breakdown = !(beta > 1e-13 * std::max(1.0, std::fabs(theta0)));
+            }
+            ++tail;
+            if (!breakdown) launch();  // runs beside the analysis
+            analyse();
+            if (breakdown) resid_est = 0.0;
+            bool stop = resid_est <= target();
+            if (!stop) {
+                if (resid_est < 0.9 * best) {
+                    best = resid_est;
+                    best_at = matvecs;
+                } else if (matvecs - best_at > 3 * m) {
+                    stop = true;  // stagnated
+                }
+            }
+            if (stop || j >= n || breakdown) {
+                drain();
+                return resid_est <= target() || j >= n;
+            }
+            if (j == m) {
+                drain();
+                restart();
+                queued = j;
+            }
+        }
+        analyse();
+        return resid_est <= target();
+    }
+
     // Iterate until resid_est <= max(abs_target, rel_target * max(1, |theta0|)), the
     // matvec budget is spent, breakdown, or stagnation (no 10% gain in 3 cycles).
     // The step after the current one is already running on the device while the host
@@ -1039,10 +1301,11 @@ int solve_fp64(const SolveProblem &P, const SolveOptions &o, double *c_dev, bool
     TRLanczos<double> lz(n, m, keep, s, ops);
     lz.mv = [&](const double *x, double *y, cudaStream_t st) { P.mv64(x, y, st); };
     lz.start(c_dev);
+    const bool small = P.val && n <= kSmallRows && P.nnz <= kSmallNnz && small_cluster_ok(small_smem(n, m));
     double target = o.tol;
     std::pair<double, double> er{0, 1e300};
     for (int attempt = 0; attempt < 8; ++attempt) {
-        const bool ok = lz.run(target, 0.0, budget);
+        const bool ok = small ? lz.run_small(P, target, 0.0, budget) : lz.run(target, 0.0, budget);
         lz.ritz_vector(c_dev);
         er = ref.eval(P, c_dev);
         if (er.second <= o.tol || !ok) break;

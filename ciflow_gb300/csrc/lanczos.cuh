@@ -30,6 +30,12 @@ struct SolveProblem {
     // mixed cold starts: the first anchor from the FP32 product (worth it where that is
     // several times cheaper than the FP64 one: the FCI sigma vector)
     bool fp32_first_anchor = false;
+    // an FP64 matrix stored as a whole CRS (null otherwise): small problems run several
+    // Lanczos steps per launch on it
+    const int64_t *row_ptr = nullptr;
+    const uint32_t *col = nullptr;
+    const double *val = nullptr;
+    int64_t nnz = 0;
     cudaStream_t stream = nullptr;
 };
 

@@ -296,3 +296,25 @@ def test_doci_split_product(L, n):
         m.mvprod_device(xd, yd)
         torch.cuda.synchronize()
         assert np.all(np.abs(yd.cpu().numpy().astype(np.float64) - y_ref) <= 2 * terms * eps * most + 1e-300)
+
+
+@pytest.mark.parametrize("L,n", [(2, 1), (3, 1), (5, 2), (10, 2), (11, 5), (14, 5), (15, 5)])
+def test_small_lanczos(L, n):
+    """Plain DOCI solves whose Lanczos steps run several to a launch: spaces below one
+    restart (exhausted inside a launch), slices of one row and of many, against the
+    dense eigenvalue; a budget is kept to the matvec."""
+    ints = make_integrals(L, n, n, nchol=6, seed=3 * L + n)
+    w = np.linalg.eigvalsh(O.build_upper(O.DOCI, ints).full_csr().toarray())
+    cim = build(DOCI, ints)
+    cim.solve(tol=1e-9)
+    # the Rayleigh quotient's error is at most the residual squared over the gap, plus
+    # its own rounding
+    tol = 64 * 2.0 ** -52 * np.abs(w).max() + (1e-18 / max(w[1] - w[0], 1e-9) if len(w) > 1 else 0.0)
+    assert abs(cim.get_ci_energy() - ints.econst - w[0]) <= tol
+    c = cim.get_eigvec()
+    r = cim.get_mat().mvprod(c) - (cim.get_ci_energy() - ints.econst) * c
+    assert np.linalg.norm(r) <= 2e-9
+    for budget in (1, 3, 6):
+        short = build(DOCI, ints)
+        short.solve(tol=1e-13, max_matvec=budget)
+        assert short.info["matvecs_fp64"] <= budget + 1  # and the residual's own
