@@ -123,7 +123,7 @@ int solve_crs(cigpu_crs &crs, double tol, int64_t max_matvec, double *c_dev, boo
 void rotate_ham(const cigpu_ham &base, const double *U, cigpu_ham &H, cudaStream_t s);
 // exp(X) of an antisymmetric L x L generator (host).
 void unitary_exp(int L, const double *X, double *U);
-// DOCI: blocks of partial sums doci_pair_matrices needs (partial holds 2 L^2 doubles per block).
+// DOCI: sets of sums doci_pair_matrices needs (partial holds 2 L^2 doubles per set).
 int doci_pair_partials();
 // DOCI pair matrices of device vector c (normalised): Pm[j][k] = Gamma_ab(jj,kk),
 // Dm[j][k] = Gamma_aa(jk,jk) (zero diagonal); device outputs, L x L each.

@@ -574,8 +574,12 @@ __device__ __forceinline__ long long fxmul(long long a, long long b) {
     return hi + (long long)(lo >> 63);
 }
 
+__device__ __forceinline__ void add_to(long long *at, long long v) {
+    atomicAdd(reinterpret_cast<unsigned long long *>(at), (unsigned long long)v);
+}
+
 __global__ void k_doci_rdm(const double *__restrict__ c, const uint64_t *__restrict__ strings, int64_t D, int L,
-                           int n, double *__restrict__ partial, unsigned long long *err) {
+                           int n, long long *__restrict__ sums, unsigned long long *err) {
     __shared__ uint32_t binom[(kDociMaxL + 1) * (kDociMaxL + 2)];  // C(nn, kk), nn <= L, kk <= n + 1
     __shared__ uint64_t ss[kDociChunk];
     __shared__ long long cs[kDociChunk], cs2[kDociChunk];  // c_I * 2^62, c_I^2 * 2^60
@@ -651,12 +655,12 @@ __global__ void k_doci_rdm(const double *__restrict__ c, const uint64_t *__restr
             }
         }
     }
-    // fixed-point sums at (j, k), j <= k, of the block's [2][L][L] partials (the
-    // lower triangle is not written and not read), read back by the finishing kernels
+    // added at (j, k), j <= k, of the [2][L][L] sums (zero before the launch; the lower
+    // triangle is not written and not read): integer sums, the same in any order. A
+    // finishing kernel that summed 608 blocks' partials, a thread per element, took 181 us.
     if (work) {
-        long long *pl = reinterpret_cast<long long *>(partial);
-        pl[((int64_t)blockIdx.x * 2) * L * L + j * L + k] = A;
-        pl[((int64_t)blockIdx.x * 2 + 1) * L * L + j * L + k] = B;
+        add_to(sums + j * L + k, A);
+        add_to(sums + L * L + j * L + k, B);
     }
 }
 
@@ -695,10 +699,6 @@ __host__ __device__ inline uint32_t split_rdm_group(const DociSector &c) {
 __device__ __forceinline__ long long warp_sum(long long v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-__device__ __forceinline__ void add_to(long long *at, long long v) {
-    atomicAdd(reinterpret_cast<unsigned long long *>(at), (unsigned long long)v);
 }
 
 // sums: [2][L][L] (A, then B; j <= k), low: [lowbits] sums of squares per low string.
@@ -880,20 +880,14 @@ size_t split_rdm_smem(const DociSplitView &v) {
     return most + 16 * (size_t)v.L * v.L;
 }
 
-__global__ void k_doci_rdm_finish(const double *__restrict__ partial, int G, int L, int np, double *__restrict__ rdm1,
+__global__ void k_doci_rdm_finish(const long long *__restrict__ sums, int L, int np, double *__restrict__ rdm1,
                                   double *__restrict__ aa, double *__restrict__ ab, double *__restrict__ bb) {
     const int L2 = L * L;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= L2) return;
     const int j = t / L, k = t % L;
-    const int tu = j <= k ? t : k * L + j;  // the partials hold j <= k
-    const long long *pl = reinterpret_cast<const long long *>(partial);  // fixed point, 2^60
-    long long Af = 0, Bf = 0;
-    for (int b = 0; b < G; ++b) {
-        Af += pl[((int64_t)b * 2) * L2 + tu];
-        Bf += pl[((int64_t)b * 2 + 1) * L2 + tu];
-    }
-    const double A = (double)Af * 0x1p-60, B = (double)Bf * 0x1p-60;
+    const int tu = j <= k ? t : k * L + j;  // the sums hold j <= k
+    const double A = (double)sums[tu] * 0x1p-60, B = (double)sums[L2 + tu] * 0x1p-60;  // fixed point, 2^60
     // 1-RDM (both spins): gamma_jj = A_jj
     if (j == k) {
         rdm1[j * L + j] = A;
@@ -913,20 +907,14 @@ __global__ void k_doci_rdm_finish(const double *__restrict__ partial, int G, int
 // The two L x L matrices a DOCI state's RDMs reduce to, in CIDens element terms:
 //   Pm[j][k] = get_two_rdm(1, j, j, k, k)   (pair hop B_jk; A_jj on the diagonal)
 //   Dm[j][k] = get_two_rdm(0, j, k, j, k)   (A_jk; zero on the diagonal)
-__global__ void k_doci_pairs_finish(const double *__restrict__ partial, int G, int L, double *__restrict__ Pm,
+__global__ void k_doci_pairs_finish(const long long *__restrict__ sums, int L, double *__restrict__ Pm,
                                     double *__restrict__ Dm) {
     const int L2 = L * L;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= L2) return;
     const int j = t / L, k = t % L;
-    const int tu = j <= k ? t : k * L + j;  // the partials hold j <= k (B: j < k)
-    const long long *pl = reinterpret_cast<const long long *>(partial);  // fixed point, 2^60
-    long long Af = 0, Bf = 0;
-    for (int b = 0; b < G; ++b) {
-        Af += pl[((int64_t)b * 2) * L2 + tu];
-        Bf += pl[((int64_t)b * 2 + 1) * L2 + tu];
-    }
-    const double A = (double)Af * 0x1p-60, B = (double)Bf * 0x1p-60;
+    const int tu = j <= k ? t : k * L + j;  // the sums hold j <= k (B: j < k)
+    const double A = (double)sums[tu] * 0x1p-60, B = (double)sums[L2 + tu] * 0x1p-60;  // fixed point, 2^60
     Pm[t] = j == k ? A : B;
     Dm[t] = j == k ? 0.0 : A;
 }
@@ -969,7 +957,16 @@ const DociSplit *doci_split_of(cigpu_crs &c, cudaStream_t s) {
     return c.split && split_rdm_smem(c.split.view) <= kSplitRdmMaxSmem ? &c.split : nullptr;
 }
 
-// Fixed-point sums A, B ([2][L][L], j <= k) of device vector c through the split plan.
+// Adds the fixed-point sums A, B ([2][L][L], j <= k, zero before) of device vector c:
+// by the general kernel, and through the split plan.
+void doci_rdm_sums(const cigpu_crs &c, const double *c_dev, long long *sums, unsigned long long *err, cudaStream_t s) {
+    const int th = ((c.L * (c.L + 1) / 2 + 31) / 32) * 32;  // one thread per pair j <= k
+    const int64_t chunks = (c.dim + kDociChunk - 1) / kDociChunk;
+    k_doci_rdm<<<(int)std::min<int64_t>(chunks, (int64_t)sm_count() * 4), th, 0, s>>>(c_dev, c.strings.p, c.dim, c.L, c.nup,
+                                                                                      sums, err);
+    count_launch();
+}
+
 void doci_rdm_split(const DociSplit &sp, const double *c_dev, long long *sums, cudaStream_t s) {
     static const cudaError_t attr =
         cudaFuncSetAttribute(k_doci_rdm_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitRdmMaxSmem);
@@ -978,7 +975,6 @@ void doci_rdm_split(const DociSplit &sp, const double *c_dev, long long *sums, c
     v.err = check_word_device();
     DevBuf<long long> fixed((size_t)v.D), low(sp.nlowbits);
     CIGPU_CUDA(cudaMemsetAsync(low.p, 0, low.bytes(), s));
-    CIGPU_CUDA(cudaMemsetAsync(sums, 0, sizeof(long long) * 2 * v.L * v.L, s));
     uint64_t tasks = 0;
     for (int q = 0; q < v.nsec; ++q) {
         const uint32_t g = split_rdm_group(v.sec[q]);
@@ -1085,17 +1081,13 @@ void crs_rdm(cigpu_crs &c, const double *c_dev, double *rdm1, double *aa, double
     if (c.method == CIGPU_DOCI) {
         if (L * L > 1024) throw std::invalid_argument("DOCI RDM needs L <= 32");
         CIGPU_CUDA(cudaMemsetAsync(out.p, 0, sizeof(double) * out.n, s));
-        const DociSplit *sp = doci_split_of(c, s);
-        const int G = sp ? 1 : sm_count() * 4;
-        DevBuf<double> partial((size_t)G * 2 * L2);
-        const int th = ((L * (L + 1) / 2 + 31) / 32) * 32;  // one thread per pair j <= k
-        if (sp) {
-            doci_rdm_split(*sp, c_dev, reinterpret_cast<long long *>(partial.p), s);
-        } else {
-            k_doci_rdm<<<G, th, 0, s>>>(c_dev, c.strings.p, c.dim, L, c.nup, partial.p, check_word_device());
-            count_launch();
-        }
-        k_doci_rdm_finish<<<(int)((L2 + 255) / 256), 256, 0, s>>>(partial.p, G, L, np, o1, oaa, oab, obb);
+        DevBuf<long long> sums((size_t)2 * L2);
+        CIGPU_CUDA(cudaMemsetAsync(sums.p, 0, sums.bytes(), s));
+        if (const DociSplit *sp = doci_split_of(c, s))
+            doci_rdm_split(*sp, c_dev, sums.p, s);
+        else
+            doci_rdm_sums(c, c_dev, sums.p, check_word_device(), s);
+        k_doci_rdm_finish<<<(int)((L2 + 255) / 256), 256, 0, s>>>(sums.p, L, np, o1, oaa, oab, obb);
         CIGPU_CUDA(cudaGetLastError());
         count_launch();
         CIGPU_CUDA(cudaStreamSynchronize(s));
@@ -1182,16 +1174,17 @@ void crs_rdm(cigpu_crs &c, const double *c_dev, double *rdm1, double *aa, double
     tr.mark("assemble + copy out");
 }
 
-int doci_pair_partials() { return sm_count() * 4; }
+int doci_pair_partials() { return 1; }
 
 void doci_pair_matrices(cigpu_crs &c, const double *c_dev, double *partial, double *Pm, double *Dm, cudaStream_t s) {
     if (c.method != CIGPU_DOCI || c.L > 32) throw std::invalid_argument("DOCI pair matrices need a DOCI CRS, L <= 32");
-    const int L = c.L, G = doci_pair_partials();
-    const int th = ((L * (L + 1) / 2 + 31) / 32) * 32;  // one thread per pair j <= k
-    k_doci_rdm<<<G, th, 0, s>>>(c_dev, c.strings.p, c.dim, L, c.nup, partial, check_word_device());
-    k_doci_pairs_finish<<<(L * L + 255) / 256, 256, 0, s>>>(partial, G, L, Pm, Dm);
+    const int L = c.L;
+    long long *sums = reinterpret_cast<long long *>(partial);
+    CIGPU_CUDA(cudaMemsetAsync(sums, 0, sizeof(long long) * 2 * L * L, s));
+    doci_rdm_sums(c, c_dev, sums, check_word_device(), s);
+    k_doci_pairs_finish<<<(L * L + 255) / 256, 256, 0, s>>>(sums, L, Pm, Dm);
     CIGPU_CUDA(cudaGetLastError());
-    count_launch(2);
+    count_launch();
 }
 
 }  // namespace cigpu
@@ -1203,11 +1196,11 @@ void doci_pair_matrices(cigpu_crs &c, const double *c_dev, double *partial, doub
 // RDMs: a host framework that hands out all device memory from its own fixed
 // pool and forbids cudaMalloc on its request path, or a latency-bound loop where
 // the implicit device synchronisation of cudaMalloc/cudaFree would stall work
-// queued by others. For them the per-block partial sums of the DOCI RDM kernel
-// live in a fixed array inside this library instead of in allocated scratch.
+// queued by others. For them the sums of the DOCI RDM kernel live in a fixed
+// array inside this library instead of in allocated scratch.
 //
 // The array below is file-scope device memory: every GPU that loads the library
-// holds it (4 MiB) until the process exits. Host code must not take its name as
+// holds it (16 KiB) until the process exits. Host code must not take its name as
 // a device address; the address is looked up once per device with
 // cudaGetSymbolAddress (on the first call on that device, which should therefore
 // come before any stream capture) and kept for the life of the process, so it
@@ -1218,17 +1211,16 @@ void doci_pair_matrices(cigpu_crs &c, const double *c_dev, double *partial, doub
 namespace cigpu {
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = size_t(4) << 20;  // 4 MiB
-constexpr int kNoAllocMaxBlocks = 256;
+constexpr int kNoAllocSums = 2 * kDociMaxL * kDociMaxL;  // 16 KiB: [2][L][L], L <= 32
 
-static __device__ __align__(256) double g_doci_rdm_scratch[kNoAllocScratchBytes / sizeof(double)];
+static __device__ __align__(256) long long g_doci_rdm_scratch[kNoAllocSums];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mutex;
-double *g_scratch_addr[kMaxDevices] = {nullptr};
+long long *g_scratch_addr[kMaxDevices] = {nullptr};
 
 // Device address of the scratch array on the current device (set up once per device).
-cudaError_t scratch_address(double **out) {
+cudaError_t scratch_address(long long **out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1238,7 +1230,7 @@ cudaError_t scratch_address(double **out) {
         void *p = nullptr;
         e = cudaGetSymbolAddress(&p, g_doci_rdm_scratch);
         if (e != cudaSuccess) return e;
-        g_scratch_addr[dev] = static_cast<double *>(p);
+        g_scratch_addr[dev] = static_cast<long long *>(p);
     }
     *out = g_scratch_addr[dev];
     return cudaSuccess;
@@ -1254,15 +1246,13 @@ extern "C" int cigpu_rdm_doci_noalloc(cigpu_crs *crs, const double *c, double *r
     if (crs->method != CIGPU_DOCI) return CIGPU_EINVAL;
     const int L = crs->L, np = L * (L - 1) / 2;
     const int64_t L2 = (int64_t)L * L;
-    // one thread per orbital pair (j, k) and 2 L^2 partial sums per block must fit
+    // one thread per orbital pair (j, k), and 2 L^2 sums must fit
     if (L2 > 1024) return CIGPU_ENOTSUP;
-    const int G = (int)std::min<int64_t>(kNoAllocMaxBlocks, kNoAllocScratchBytes / (sizeof(double) * 2 * L2));
-    if (G < 1) return CIGPU_ENOTSUP;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess) return CIGPU_ECUDA;
     if (dev != crs->device) return CIGPU_EINVAL;  // the matrix and the scratch must share a device
-    double *scratch = nullptr;
-    cudaError_t e = scratch_address(&scratch);
+    long long *sums = nullptr;
+    cudaError_t e = scratch_address(&sums);
     if (e != cudaSuccess) {
         std::fprintf(stderr, "cigpu: scratch address lookup failed: %s\n", cudaGetErrorString(e));
         return CIGPU_ECUDA;
@@ -1274,10 +1264,10 @@ extern "C" int cigpu_rdm_doci_noalloc(cigpu_crs *crs, const double *c, double *r
         cudaMemsetAsync(rdm2_bb, 0, sizeof(double) * np * np, s) != cudaSuccess ||
         cudaMemsetAsync(rdm2_ab, 0, sizeof(double) * L2 * L2, s) != cudaSuccess)
         return CIGPU_ECUDA;
-    const int th = (int)((L2 + 31) / 32 * 32);
-    k_doci_rdm<<<G, th, 0, s>>>(c, crs->strings.p, crs->dim, L, crs->nup, scratch, nullptr);  // no error word: allocates nothing
-    k_doci_rdm_finish<<<(int)((L2 + 255) / 256), 256, 0, s>>>(scratch, G, L, np, rdm1, rdm2_aa, rdm2_ab, rdm2_bb);
+    if (cudaMemsetAsync(sums, 0, sizeof(long long) * 2 * L2, s) != cudaSuccess) return CIGPU_ECUDA;
+    doci_rdm_sums(*crs, c, sums, nullptr, s);  // no error word: allocates nothing
+    k_doci_rdm_finish<<<(int)((L2 + 255) / 256), 256, 0, s>>>(sums, L, np, rdm1, rdm2_aa, rdm2_ab, rdm2_bb);
     if (cudaGetLastError() != cudaSuccess) return CIGPU_ECUDA;
-    count_launch(2);
+    count_launch();
     return CIGPU_OK;
 }

@@ -196,7 +196,7 @@ int cigpu_rdm(cigpu_crs *crs, const double *c, double *rdm1, double *rdm2_aa, do
  * For callers that cannot allocate device memory on their request path (a host
  * framework that owns all device memory through its own fixed pool, or a
  * latency-bound loop that cannot afford the device synchronisation cudaMalloc
- * implies): the block partial sums live in a fixed 4 MiB array inside the
+ * implies): the sums live in a fixed 16 KiB array inside the
  * library, so this call allocates nothing. crs must be a DOCI CRS with L <= 32
  * (CIGPU_ENOTSUP otherwise). c (dim) and the outputs, laid out as in cigpu_rdm,
  * are DEVICE buffers; the work is queued on `stream` (NULL: the CRS stream) and
