@@ -292,6 +292,8 @@ size_t estimate_bytes(int L, int nup, int ndown, int method, int precision) {
     return b;
 }
 
+constexpr int64_t kSplitPlainRows = 500000;  // plain DOCI spaces whose products use the split plan
+
 // Per-row single-excitation tables of an FCI CRS (FP64, plus the FP32 splits of
 // them and of the diagonal for MIXED); only the fill passes read them.
 struct RowSingles {
@@ -498,10 +500,8 @@ void build_crs(cigpu_crs &c, cudaStream_t s) {
         doci_diag_launch(p, c.diag.p, s);
         p.row_count = count.p;
         p.upper_off = c.upper_off.p;
-        // MIXED is matrix-free (its FP32 product costs about what the FP32 CRS costs,
-        // and the build drops from a CRS count + sort + fill to the pair table); the
-        // FP64 form keeps the CRS, whose FP64 product is the faster one (1.24 against
-        // 1.70 ms at L=24, 12 pairs), and its 120-odd matvecs outweigh the build
+        // MIXED is matrix-free (the build drops from a CRS count + sort + fill to the pair
+        // table); the FP64 form stores the CRS
         if (c.allow_compact && c.precision == CIGPU_MIXED) {
             // matrix-free: the pair-hop table and, for MIXED, the FP32 diagonal; the
             // stored-element counts follow from K: a pair (j, k) with K_jk != 0 hops in
@@ -537,6 +537,19 @@ void build_crs(cigpu_crs &c, cudaStream_t s) {
         }
         doci_launch(kCount, p, s);
         tr.mark("strings + diag + count");
+        // large plain spaces: the products by low and high orbitals, from no matrix at all,
+        // beat the stored rows (12 bytes per element at two thirds of HBM's rate): L=24, 12
+        // pairs 745 against 1,068 us, L=26, 8 pairs (1,562,275) 469 against 607; L=20, 10
+        // pairs (184,756), whose rows lie in L2 in part, 60.3 against 63.5, L=30, 5 pairs
+        // (142,506) 80 against 57.
+        if (c.allow_compact && c.precision == CIGPU_FP64 && dim >= kSplitPlainRows) {
+            c.kpair64.alloc((size_t)c.L * c.L);
+            c.kpair32.alloc((size_t)c.L * c.L);
+            doci_pair_table_launch(c.L, h.d_eri.p, c.kpair64.p, c.kpair32.p, s);
+            doci_split_make(c.L, c.nup, dim, c.split, s);
+            c.split_tried = true;
+            c.split_product = (bool)c.split;
+        }
     }
     if (c.side) {
         // deferred: the scans on the side stream, the counts read by finish_deferred
@@ -623,8 +636,12 @@ void crs_mv64(cigpu_crs &c, const double *x, double *y, cudaStream_t s) {
         spmv_slots_hilo(c.fp, c.val32.p, c.val32lo.p, x, c.x32.p, y, s);
         return;
     }
+    if (c.split_product) {
+        doci_mv64(DociMv{c.L, c.nup, c.dim, c.strings.p}, c.split, c.kpair64.p, c.diag.p, x, y, s);
+        return;
+    }
     if (c.precision == CIGPU_FP64) {
-        spmv_f64(c.dim, c.nnz_full, c.row_ptr.p, c.col.p, c.val64.p, x, y, s);
+        spmv_f64(c.dim, c.nnz_full, c.row_ptr.p, c.col.p, c.val64.p, x, y, s, c.method == CIGPU_FCI);
         return;
     }
     if (c.val32lo.p || c.nnz_full == 0) {

@@ -51,6 +51,7 @@ struct cigpu_crs {
     cigpu::DevBuf<float> kpair32, diag32;
     cigpu::DociSplit split;  // the plan of the product and RDM by low / high orbitals (larger spaces)
     bool split_tried = false;
+    bool split_product = false;  // plain DOCI: the FP64 products use it too
     cigpu::DevBuf<uint64_t> slot_desc;  // the slot matvecs' staging tables (slot_tables_launch)
     cigpu::DevBuf<uint32_t> slot_st;
     cigpu::DevBuf<float> x32;  // MIXED: FP32 copy of x for the FP64 product from hi + lo

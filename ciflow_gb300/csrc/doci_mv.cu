@@ -411,12 +411,19 @@ __device__ __forceinline__ uint32_t squeeze(uint32_t b, int j) {
     return (b & low) | ((b >> 1) & ~low);
 }
 
-__global__ void k_split_low(const DociSplitView p, uint32_t *__restrict__ ll, uint16_t *__restrict__ lminus,
-                            uint16_t *__restrict__ lplus, uint32_t *__restrict__ one, uint32_t *__restrict__ two,
-                            uint16_t *__restrict__ lowbits) {
+constexpr int kSplitLowThreads = 128;
+
+__global__ void __launch_bounds__(kSplitLowThreads) k_split_low(const DociSplitView p, uint32_t *__restrict__ ll,
+                                                                uint16_t *__restrict__ lminus,
+                                                                uint16_t *__restrict__ lplus,
+                                                                uint32_t *__restrict__ one, uint32_t *__restrict__ two,
+                                                                uint16_t *__restrict__ lowbits) {
+    __shared__ uint16_t rank[1 << kSplitMaxLow];  // of every low string among those of its size
     const DociSector &c = p.sec[blockIdx.y];
     const int s = p.s, m = c.m;
-    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < c.nlow; l += gridDim.x * blockDim.x) {
+    for (int b = threadIdx.x; b < (1 << s); b += kSplitLowThreads) rank[b] = (uint16_t)low_rank((uint32_t)b, p.binom);
+    __syncthreads();
+    for (uint32_t l = blockIdx.x * kSplitLowThreads + threadIdx.x; l < c.nlow; l += gridDim.x * kSplitLowThreads) {
         uint32_t b = 0, rest = l;  // the low string of rank l
         for (int k = m, o = s - 1; k > 0; --o)
             if (p.binom[o * kSplitBinomRow + k] <= rest) {
@@ -427,22 +434,20 @@ __global__ void k_split_low(const DociSplitView p, uint32_t *__restrict__ ll, ui
         lowbits[c.low0 + l] = (uint16_t)b;
         int e = 0, em = 0, ep = 0;
         for (int j = s - 1; j >= 0; --j) {
-            const uint32_t bj = b ^ (1u << j);
+            const uint32_t bj = b ^ (1u << j), at = rank[bj];
             if (!((b >> j) & 1u)) {
-                lplus[c.plus0 + (uint32_t)ep++ * c.nlow + l] = (uint16_t)(low_rank(bj, p.binom) | ((uint32_t)j << 10));
+                lplus[c.plus0 + (uint32_t)ep++ * c.nlow + l] = (uint16_t)(at | ((uint32_t)j << 10));
                 continue;
             }
-            const uint32_t without = low_rank(bj, p.binom);
-            lminus[c.minus0 + (uint32_t)em++ * c.nlow + l] = (uint16_t)(without | ((uint32_t)j << 10));
-            one[c.one0 + (uint32_t)j * c.n1 + low_rank(squeeze(bj, j), p.binom)] = l | (without << 16);
+            lminus[c.minus0 + (uint32_t)em++ * c.nlow + l] = (uint16_t)(at | ((uint32_t)j << 10));
+            one[c.one0 + (uint32_t)j * c.n1 + rank[squeeze(bj, j)]] = l | (at << 16);
             for (int k = j + 1, q = j * s - j * (j + 1) / 2; k < s; ++k, ++q)  // pair (j, k): row-major, j < k
                 if (!((b >> k) & 1u))
-                    two[c.two0 + (uint32_t)q * c.n2 + low_rank(squeeze(squeeze(bj, k), j), p.binom)] =
-                        l | (low_rank(bj ^ (1u << k), p.binom) << 16);
+                    two[c.two0 + (uint32_t)q * c.n2 + rank[squeeze(squeeze(bj, k), j)]] =
+                        l | ((uint32_t)rank[bj ^ (1u << k)] << 16);
             for (int k = s - 1; k >= 0; --k)
                 if (!((b >> k) & 1u))
-                    ll[c.ll0 + (uint32_t)e++ * c.nlow + l] =
-                        low_rank(bj ^ (1u << k), p.binom) | ((uint32_t)(j * s + k) << 10);
+                    ll[c.ll0 + (uint32_t)e++ * c.nlow + l] = rank[bj ^ (1u << k)] | ((uint32_t)(j * s + k) << 10);
         }
     }
 }
@@ -634,7 +639,7 @@ void doci_split_make(int L, int n, int64_t D, DociSplit &sp, cudaStream_t st) {
     v.ll = sp.ll.p;
     v.lminus = sp.lminus.p;
     v.lplus = sp.lplus.p;
-    k_split_low<<<dim3(4, v.nsec), 256, 0, st>>>(v, sp.ll.p, sp.lminus.p, sp.lplus.p, sp.one.p, sp.two.p,
+    k_split_low<<<dim3(8, v.nsec), kSplitLowThreads, 0, st>>>(v, sp.ll.p, sp.lminus.p, sp.lplus.p, sp.one.p, sp.two.p,
                                                sp.lowbits.p);
     k_split_high<<<dim3(64, v.nsec), 256, 0, st>>>(v, sp.hbits.p, sp.hbase.p);
     CIGPU_CUDA(cudaGetLastError());

@@ -4,7 +4,7 @@
 // serial symmetric scatter over the upper triangle. The device keeps the full
 // symmetric matrix, so y = H x is a plain row gather with no atomics and a
 // fixed summation order (bit-reproducible run to run):
-//   * a group of 8-32 lanes per row, rows dealt round-robin to a persistent grid;
+//   * a group of 4-32 lanes per row, rows dealt round-robin to a persistent grid;
 //   * col/val are streamed once (ld.global.cs: they are not reused, so they
 //     must not evict x from L2); x is gathered through the read-only path and
 //     stays L2-resident (853,776 doubles = 6.8 MB for the L=12 FCI space);
@@ -16,6 +16,7 @@
 #include "spmv_formats.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cigpu {
 
@@ -130,26 +131,40 @@ int sm_count_spmv() {
     return sms;
 }
 
-// lanes per row from the mean row length (in 4-element chunks: 32 lanes for FCI
-// rows of hundreds, 8 for the DOCI rows of ~36); the grid covers
-// the rows once (at most a full persistent grid), so a small matrix leaves SMs
-// free for the kernels of concurrent solves on other streams.
+// Lanes per row from the mean row length (in 4-element chunks), and chunks per lane and
+// round. FP64 products are bound by the FP64 pipe as much as by memory: a lane without an
+// element in a round, and every step of a row's final sum, costs the pipe a full warp.
+//   * DOCI rows (18-36 chunks): 4 lanes in FP64 from 12,000 rows (L=20 8 pairs, 125,970
+//     rows: 52 us with 8 lanes, 41 with 4; L=24: 1,241 and 1,068; L=14, 3,432 rows, 5.2
+//     and 6.2: too few warps), else 8, five chunks each (one round covers a row's 36).
+//   * longer rows: 32 lanes, four chunks each; FCI rows, all of one length, two in FP64
+//     (fewer registers: L=9 4a3b, 504 elements, 22.7 -> 18.6 us, L=8 4a4b 12.4 -> 11.3;
+//     determinant lists' uneven rows lose by it: 20.6 and 24.5 at 595).
+// The grid covers the rows once (at most a full persistent grid), so a small matrix
+// leaves SMs free for the kernels of concurrent solves on other streams.
+constexpr int64_t kFourLaneRows = 12000;
+
 template <typename F>
 static void launch_rows(int64_t n, int64_t nnz, const int64_t *row_ptr, const uint32_t *col, const F &f0,
-                        typename F::X *y, cudaStream_t s) {
+                        typename F::X *y, cudaStream_t s, bool equal_rows = false) {
     F f = f0;
     f.nx = (uint64_t)n;
     f.err = check_word_device();
+    constexpr bool kFp64 = std::is_same<F, Plain<double>>::value;
     const double chunks = n > 0 ? (double)nnz / n / 4.0 : 0;
-    const int G = chunks >= 48 ? 32 : 8;  // DOCI L=24 (36 chunks): 8 lanes 19% over 16
+    const int G = chunks >= 48 ? 32 : (kFp64 && n >= kFourLaneRows) ? 4 : 8;
     const int64_t need = (n * G + kSpmvThreads - 1) / kSpmvThreads;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(spmv_grid(), need));
-    if (G == 32)
-        k_spmv_rows<F, 32, 4><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
-    else if (G == 16)
-        k_spmv_rows<F, 16, 4><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
-    else  // five chunks per lane: one round covers a DOCI row's 36 (FP32 5% over four)
+    if (G == 32) {
+        if (kFp64 && equal_rows)
+            k_spmv_rows<F, 32, 2><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
+        else
+            k_spmv_rows<F, 32, 4><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
+    } else if (G == 4) {
+        k_spmv_rows<F, 4, 2><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
+    } else {
         k_spmv_rows<F, 8, 5><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
+    }
     CIGPU_CUDA(cudaGetLastError());
     count_launch();
 }
@@ -181,8 +196,8 @@ void spmv_f64_shape(int64_t n, const int64_t *row_ptr, const uint32_t *col, cons
 }
 
 void spmv_f64(int64_t n, int64_t nnz, const int64_t *row_ptr, const uint32_t *col, const double *val, const double *x,
-              double *y, cudaStream_t s) {
-    launch_rows(n, nnz, row_ptr, col, Plain<double>{val, x}, y, s);
+              double *y, cudaStream_t s, bool equal_rows) {
+    launch_rows(n, nnz, row_ptr, col, Plain<double>{val, x}, y, s, equal_rows);
 }
 
 void spmv_f32(int64_t n, int64_t nnz, const int64_t *row_ptr, const uint32_t *col, const float *val, const float *x,

@@ -318,3 +318,23 @@ def test_small_lanczos(L, n):
         short = build(DOCI, ints)
         short.solve(tol=1e-13, max_matvec=budget)
         assert short.info["matvecs_fp64"] <= budget + 1  # and the residual's own
+
+
+def test_plain_doci_split_product():
+    """A plain DOCI matrix past kSplitPlainRows multiplies through the split plan and
+    still exports the CRS: its product equals the exported rows'."""
+    torch = pytest.importorskip("torch")
+    # 490,314 rows (below it) and 735,471
+    for L, n in ((23, 8), (24, 8)):
+        ints = make_integrals(L, n, n, nchol=4, seed=L)
+        m = build(DOCI, ints).get_mat()
+        row, col, val = m.full()
+        x = np.random.default_rng(1).standard_normal(m.n)
+        import scipy.sparse as sp
+        H = sp.csr_matrix((val, col.astype(np.int64), row.astype(np.int64)), shape=(m.n, m.n))
+        y = torch.empty(m.n, dtype=torch.float64, device="cuda")
+        m.mvprod_device(torch.tensor(x, device="cuda"), y)
+        torch.cuda.synchronize()
+        terms = n * (L - n) + 3
+        most = abs(H) @ np.abs(x)
+        assert np.all(np.abs(y.cpu().numpy() - H @ x) <= 2 * terms * 2.0 ** -53 * most)
