@@ -146,6 +146,7 @@ struct SigmaArgs {
     const uint2 *rows;                // the beta strings' same-spin rows
     int ne;
     int tiles, panels, chunks, per;   // opposite tiles; same-spin panels and row chunks
+    int slabs, slab_r;                // sets of W and yd, each of slab_r factors (see sigma_slabs)
     int panel_rows;                   // rows of xT a same-spin block holds in shared memory (0: none)
     const float *xT;
     float *W, *yd, *uT;
@@ -190,11 +191,13 @@ __device__ __forceinline__ void opposite_tile(const SigmaArgs &a, float *sm) {
     const int L2 = a.L * a.L, nsa = a.nsa, nsb = a.nsb;
     float *Fs = sm, *Gs = Fs + L2 * kHalf;  // [L2][8] of this block's factors, [L2][16]
     float *z = Gs + L2 * kC;                // [8][kTile alpha][kTile + 1 beta]
-    const int tile = blockIdx.x / 2;
+    const int slab = (int)(blockIdx.x / 2) / a.tiles, tile = (int)(blockIdx.x / 2) - slab * a.tiles;
+    const int c_begin = slab * a.slab_r, c_end = min(a.R, c_begin + a.slab_r);
+    float *W = a.W + (int64_t)slab * a.Da * nsa * a.Pb, *yd = a.yd + (int64_t)slab * a.Da * a.Pb;
     const int64_t tb = (int64_t)(tile % (int)(a.Pb / kTile)) * kTile, ta = (int64_t)(tile / (int)(a.Pb / kTile)) * kTile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int c = 0; c < a.R; c += kC) {
-        if (c > 0) cluster.sync();  // both blocks are done with the factors and z
+    for (int c = c_begin; c < c_end; c += kC) {
+        if (c > c_begin) cluster.sync();  // both blocks are done with the factors and z
         const float4 *F4 = reinterpret_cast<const float4 *>(a.F) + (size_t)(c / kC) * L2 * (kC / 4);
         const float4 *G4 = reinterpret_cast<const float4 *>(a.G) + (size_t)(c / kC) * L2 * (kC / 4);
         for (int i = threadIdx.x; i < L2 * (kHalf / 4); i += kThreads)
@@ -283,11 +286,11 @@ __device__ __forceinline__ void opposite_tile(const SigmaArgs &a, float *sm) {
                     d[h] += g0 * lo + g1 * hi;
                 }
             }
-            float *ydr = a.yd + Ia * a.Pb + tb + lane;
+            float *ydr = yd + Ia * a.Pb + tb + lane;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) ydr[32 * h] = c == 0 ? d[h] : ydr[32 * h] + d[h];
+            for (int h = 0; h < 2; ++h) ydr[32 * h] = c == c_begin ? d[h] : ydr[32 * h] + d[h];
             const uint2 *ex = a.sa + Ia * nsa;
-            float *Wc = a.W + tb + lane;
+            float *Wc = W + tb + lane;
             uint2 w[2];  // the next two excitations
 #pragma unroll
             for (int u = 0; u < 2; ++u)
@@ -320,7 +323,7 @@ __device__ __forceinline__ void opposite_tile(const SigmaArgs &a, float *sm) {
                             unpack2(s[h][0], p0, p1);
                             unpack2(s[h][1], p2, p3);
                             const float x = signed_by((p0 + p1) + (p2 + p3), v[u].y & 1u);
-                            at[32 * h] = c == 0 ? x : at[32 * h] + x;
+                            at[32 * h] = c == c_begin ? x : at[32 * h] + x;
                         }
                     }
             }
@@ -411,10 +414,11 @@ __device__ __forceinline__ void same_rows(const SigmaArgs &a, int block, float *
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) k_sigma_parts(const SigmaArgs a) {
     extern __shared__ __align__(16) float sm[];
-    if ((int)blockIdx.x < 2 * a.tiles)
+    const int opposite = 2 * a.tiles * a.slabs;
+    if ((int)blockIdx.x < opposite)
         opposite_tile(a, sm);
     else
-        same_rows(a, (int)blockIdx.x - 2 * a.tiles, sm);
+        same_rows(a, (int)blockIdx.x - opposite, sm);
 }
 
 // y(Ia, Ib) = (T^a x) + yd + the sum of W's rows of Ia + uT(Ib, Ia), 32 beta columns per
@@ -429,20 +433,23 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int64_t q = (int64_t)blockIdx.x * per + warp; q < g1; q += kWarps) {
         const int64_t S = min(4 * q + g, a.Da - 1);
         const float4 r = same_row<false>(rows, ne, S, xp + col, P, stage[warp]);
-        const float *w = a.W + S * a.nsa * P + col;
-        float4 b0 = __ldg(reinterpret_cast<const float4 *>(a.yd + S * P + col)), b1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        int e = 0;
-        for (; e + 8 <= a.nsa; e += 8) {  // read once: streamed past L1
-            float4 v[8];
+        float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;
+        for (int slab = 0; slab < a.slabs; ++slab) {
+            const float *w = a.W + ((int64_t)slab * a.Da + S) * a.nsa * P + col;
+            fma4(b0, 1.f, __ldg(reinterpret_cast<const float4 *>(a.yd + ((int64_t)slab * a.Da + S) * P + col)));
+            int e = 0;
+            for (; e + 8 <= a.nsa; e += 8) {  // read once: streamed past L1
+                float4 v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)(e + u) * P));
+                for (int u = 0; u < 8; ++u) v[u] = __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)(e + u) * P));
 #pragma unroll
-            for (int u = 0; u < 8; u += 2) {
-                fma4(b0, 1.f, v[u]);
-                fma4(b1, 1.f, v[u + 1]);
+                for (int u = 0; u < 8; u += 2) {
+                    fma4(b0, 1.f, v[u]);
+                    fma4(b1, 1.f, v[u + 1]);
+                }
             }
+            for (; e < a.nsa; ++e) fma4(b0, 1.f, __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)e * P)));
         }
-        for (; e < a.nsa; ++e) fma4(b0, 1.f, __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)e * P)));
         const float c[4] = {r.x + (b0.x + b1.x), r.y + (b0.y + b1.y), r.z + (b0.z + b1.z), r.w + (b0.w + b1.w)};
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -468,14 +475,27 @@ int same_chunks(int64_t groups, int64_t panels) {
     return best;
 }
 
+// Sets of W: a grid of fewer pairs of blocks than SMs runs passes of 16 factors side by
+// side, each set's sums in its own W, and k_sigma_sum adds the sets (one after the other
+// a pass costs such a grid about 25 us whatever the space: L=10 5a5b, 16 tiles, rank 60:
+// 124 -> 50 us).
+int sigma_slabs(int64_t tiles, int R, int64_t sms) {
+    const int64_t passes = R / kC, most = std::max<int64_t>(1, std::min<int64_t>(passes, sms / (2 * tiles)));
+    const int64_t per = (passes + most - 1) / most;
+    return (int)((passes + per - 1) / per);  // no set without a pass
+}
+
 constexpr size_t kSigmaMaxSmem = 200 * 1024;
 constexpr size_t kSigmaMaxPanel = 192 * 1024;  // a same-spin panel held in shared memory
-// Spaces of fewer 32 x 32 string tiles than SMs: the operator's three launches and its
-// passes of 16 factors take a fixed time each there, the stored values a time by size.
-// Measured per product (operator | stored): rank 16: L=12 3a3b, 48,400 rows, 44 | 47 us;
-// L=10 5a5b, 63,504 rows, 42 | 68; L=9 4a4b, 15,876 rows, 37 | 16; two passes: L=10 5a4b,
-// rank 28, 67 | 63; four: L=10 5a5b, rank 60, 124 | 68. So one pass, from 50,000 rows.
-constexpr int64_t kSigmaMinRows = 50000;
+// Spaces of fewer 32 x 32 string tiles than SMs: the operator's three launches take about
+// 40 us one after the other, the stored values a time by size; with other products beside
+// them only the work counts. Measured per product alone, and among others, operator |
+// stored: L=10 4a4b, 44,100 rows, rank 12, 40 | 38 and 12 | 28 us, rank 20, 42 | 38 and
+// 15 | 28, rank 60, 47 | 38 (whole mixed solve 27.8 | 25.5 ms; rank 20: 19.4 | 20.7);
+// L=10 5a5b, 63,504, rank 60, 50 | 67 and 32 | 39 (solve 25.4 | 28.3 ms); L=9 4a4b,
+// 15,876, 37 | 16 and 11 | 7.
+constexpr int64_t kSigmaMinRows = 40000;
+constexpr int64_t kSigmaMinRowsAnyRank = 50000;  // ranks above two passes of factors
 constexpr size_t kSigmaMaxTables = 132864;  // factors, pairs and excitation lists (bytes): past it, and not
                                             // measured, the stored values serve
 
@@ -487,9 +507,9 @@ size_t sigma_bytes(int L, int na, int nb, int R) {
     auto rows = [&](int n) {  // same-spin rows and the excitation places
         return dim(n) * (8 * (1 + 2 * (int64_t)n * (L - n) + d_binom(n, 2) * d_binom(L - n, 2) + 8));
     };
-    const int64_t Da = dim(na), Db = dim(nb);
+    const int64_t Da = dim(na), Db = dim(nb), slabs = sigma_slabs(pad(Da) / kTile * (pad(Db) / kTile), R, 152);
     return (size_t)(rows(na) + rows(nb)) +
-           sizeof(float) * ((size_t)Da * (na * (L - na) + 2) * pad(Db) + 2 * (size_t)Db * pad(Da) + (size_t)(Da + Db) * R +
+           sizeof(float) * ((size_t)Da * (slabs * (na * (L - na) + 1) + 1) * pad(Db) + 2 * (size_t)Db * pad(Da) + (size_t)(Da + Db) * R +
                             2 * (size_t)L * L * R);
 }
 
@@ -569,7 +589,7 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
     }
     const int rank = (int)vecs.size();
     const int R = std::max(kSigmaChunk, (rank + kSigmaChunk - 1) / kSigmaChunk * kSigmaChunk);
-    if (!any_grid && small && R > kC) return false;
+    if (!any_grid && small && R > 2 * kC && ta.D * tb.D < kSigmaMinRowsAnyRank) return false;
     if (R > kSigmaMaxRank ||
         sizeof(float) * N * (R + 1) + sizeof(uint2) * (size_t)kTile * (ta.ns + tb.ns) > kSigmaMaxTables ||
         opposite_smem(L) > kSigmaMaxSmem || ta.D * std::max(ta.ns, 1) > (int64_t)UINT32_MAX)
@@ -636,8 +656,9 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
     op.xp.alloc((size_t)op.Da * op.Pb);
     op.xT.alloc((size_t)op.Db * op.Pa);
     op.uT.alloc((size_t)op.Db * op.Pa);
-    op.yd.alloc((size_t)op.Da * op.Pb);
-    op.W.alloc(std::max<size_t>((size_t)op.Da * ta.ns * op.Pb, 1));
+    op.slabs = sigma_slabs((op.Pa / kTile) * (op.Pb / kTile), R, sm_count());
+    op.yd.alloc((size_t)op.slabs * op.Da * op.Pb);
+    op.W.alloc(std::max<size_t>((size_t)op.slabs * op.Da * ta.ns * op.Pb, 1));
     op.R = R;
     return true;
 }
@@ -665,6 +686,8 @@ void sigma_mv32(SigmaOp &op, const FciParams &p, const float *x, float *y, cudaS
     a.ne = op.neb;
     a.tiles = (int)((op.Pa / kTile) * (op.Pb / kTile));
     a.panels = (int)((op.Da + kPanel - 1) / kPanel);
+    a.slabs = op.slabs;
+    a.slab_r = (op.R / kC + op.slabs - 1) / op.slabs * kC;
     const int64_t gb = (op.Db + 3) / 4, ga = (op.Da + 3) / 4;
     a.chunks = same_chunks(gb, a.panels);
     a.per = (int)((gb + a.chunks - 1) / a.chunks);
@@ -675,7 +698,7 @@ void sigma_mv32(SigmaOp &op, const FciParams &p, const float *x, float *y, cudaS
     a.yd = op.yd.p;
     a.uT = op.uT.p;
     const size_t smem = std::max(opposite_smem(op.L), a.panel_rows ? panel : 0);
-    const int64_t blocks = 2 * (int64_t)a.tiles + ((int64_t)a.panels * a.chunks + 1) / 2 * 2;
+    const int64_t blocks = 2 * (int64_t)a.tiles * a.slabs + ((int64_t)a.panels * a.chunks + 1) / 2 * 2;
     k_sigma_pad<<<dim3((unsigned)(op.Pb / 32), (unsigned)(op.Pa / 32)), dim3(32, 8), 0, s>>>(x, op.Da, op.Db, op.Pa, op.Pb,
                                                                                              op.xp.p, op.xT.p);
     k_sigma_parts<<<(unsigned)blocks, kThreads, smem, s>>>(a);

@@ -16,6 +16,7 @@ struct SigmaOp {
     int rank = 0;  // factors kept
     int R = 0;     // rank padded to a multiple of kSigmaChunk; 0: the operator is not in use
     int64_t Da = 0, Db = 0, Pa = 0, Pb = 0;  // strings of each spin, and padded to kSigmaTile
+    int slabs = 1;                           // sets of W and yd
     int nea = 0, neb = 0;                    // same-spin elements per string (padded to 8)
     DevBuf<float> F, G;                  // [R/16][L*L][16]: factors F^k and s_k F^k
     DevBuf<float> ga, fb;                // per-string diagonal sums of G (alpha), F (beta): [R][Da], [R][Db]

@@ -338,3 +338,23 @@ def test_plain_doci_split_product():
         terms = n * (L - n) + 3
         most = abs(H) @ np.abs(x)
         assert np.all(np.abs(y.cpu().numpy() - H @ x) <= 2 * terms * 2.0 ** -53 * most)
+
+
+@pytest.mark.parametrize("L,na,nb,rank", [(11, 3, 4, 70), (11, 4, 4, 70), (9, 2, 5, 40), (12, 2, 1, 12)])
+def test_sigma_sets(L, na, nb, rank, monkeypatch):
+    """The factorised FP32 product on grids small enough to run its passes of 16 factors
+    side by side: five passes on three sets and on two, three passes on three, one tile
+    of a few strings; the bound of test_sigma_fp32_matvec."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("CIGPU_FP32_PRODUCT", "sigma")
+    ints = make_integrals(L, na, nb, nchol=rank, seed=rank + L)
+    ref = O.build_upper(O.FCI, ints)
+    m = build(FCI, ints, A.MIXED).get_mat()
+    x = np.random.default_rng(5).standard_normal(m.n).astype(np.float32).astype(np.float64)
+    y_ref = O.sym_mvprod(ref, x)
+    xd = torch.tensor(x, dtype=torch.float32, device="cuda")
+    yd = torch.full_like(xd, float("nan"))
+    m.mvprod_device(xd, yd)
+    torch.cuda.synchronize()
+    y = yd.cpu().numpy().astype(np.float64)
+    assert np.abs(y - y_ref).max() <= 2e-5 * np.abs(y_ref).max()
