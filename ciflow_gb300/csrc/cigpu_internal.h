@@ -173,6 +173,7 @@ struct cigpu_ham {
     // false: h/eri are not filled (a Hamiltonian made on the device for a DOCI
     // build, which reads the device tables only); the device tables are current
     bool host_valid = true;
+    bool eri_zero = true;  // some |(pq|rs)| <= 1e-14 (or not known)
     cigpu::DevBuf<double> d_h;
     cigpu::DevBuf<double> d_eri;
     cigpu::DevBuf<float> d_eri_hi, d_eri_lo;  // FP32 split, zero where |v| <= 1e-14

@@ -220,3 +220,26 @@ def test_scan_edges(L, na, nb, n):
     for keep in (0, n // 3):
         big = CI_Big(ham, up=up, down=down, keep=keep)
         assert np.abs(big.get_mat().mvprod(x) - y_ref).max() <= tol
+
+
+@pytest.mark.parametrize("kind", ["no zero", "zeros", "vanishing differences"])
+@pytest.mark.parametrize("precision", [A.FP64, A.MIXED])
+def test_dropped_elements(kind, precision):
+    """Lists whose elements are all kept, dropped by zero integrals, and dropped though no
+    integral is zero (equal integrals whose difference vanishes: the build that takes the
+    connected pairs for the structure has to start again): the oracle's CRS."""
+    ints = make_integrals(12, 3, 3, nchol=5, seed=8)
+    if kind == "zeros":
+        odd = np.arange(12) % 2  # two symmetry classes: (pq|rs) with p q r s odd in all vanish
+        ints.eri[((odd[:, None, None, None] + odd[:, None, None] + odd[:, None] + odd) % 2) == 1] = 0.0
+    elif kind == "vanishing differences":
+        ints.eri[...] = 0.125
+    up, down = random_list(12, 3, 3, 400, seed=4)
+    m = O.build_dets(ints, up, down)
+    cim = FCI_File(Hamiltonian.from_integrals(ints), up=up, down=down, precision=precision)
+    row, col, val = cim.get_mat().upper()
+    assert np.array_equal(row.astype(np.int64), m.row) and np.array_equal(col, m.col)
+    if precision == A.FP64:
+        assert np.array_equal(val, m.val)
+    else:
+        assert np.array_equal(val, m.val.astype(np.float32).astype(np.float64))
