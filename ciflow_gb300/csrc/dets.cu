@@ -41,7 +41,7 @@ namespace {
 
 constexpr int kDetWarps = 8;   // rows per block (one warp each)
 constexpr int kDetTile = 256;  // determinants per shared-memory tile
-enum DetMode : int { kDetCount = 0, kDetFill64 = 1, kDetFill32 = 2, kDetMatvec = 3 };
+enum DetMode : int { kDetCount = 0, kDetFill64 = 1, kDetFill32 = 2 };
 
 struct DetParams {
     int L, nup, ndown;
@@ -393,23 +393,13 @@ __global__ void k_dets_diag(DetParams p, double *diag) {
 // of the L=28 7a7b CISD list, 21,500 determinants: 4.53 -> 0.49 ms.)
 //
 // The queue holds a row's columns in ascending order (words in order, a row's bits
-// in order), so the fill writes each row's kept elements in order at the row's
-// start plus the counts of the segments before it, and the matvec adds a row's terms
-// in a fixed order.
-//
-// RANGED: the matvec of a list with a stored block (CI_Big with a kept part) leaves
-// out the pairs of the block; the other passes carry no test.
+// in order), so the fill writes each row's kept elements in order at the row's start
+// plus the counts of the segments before it.
 constexpr int kScanRows = 32;
-constexpr int kScanWarps = 8;  // the matvec's warps per block
-constexpr int kSegs = 64;      // column segments of the count and fill passes
+constexpr int kSegs = 64;  // column segments of the count and fill passes
 constexpr int kQueue = 256;                 // a word of 8 rows fits whatever passes
 constexpr int kQueueColBits = 27;           // queue entry: row << 27 | column - the queue's first column
 constexpr uint32_t kQueueColMask = (1u << kQueueColBits) - 1u;
-
-template <int MODE>
-constexpr int scan_warps() {
-    return MODE == kDetMatvec ? kScanWarps : 1;
-}
 
 // 32-bit words a determinant is tested with: 2 (L <= 32), 4 (L <= 64) or 8.
 template <int W, int NW>
@@ -441,7 +431,6 @@ struct ScanWarp {
     double val[kQueue];
     uint32_t at[kQueue];
     uint16_t single[kQueue];  // queue positions of the singles
-    double acc[kScanRows];    // matvec: the row sums
     uint32_t run[kScanRows], low[kScanRows];  // kept elements so far; those below the diagonal
 };
 
@@ -450,31 +439,18 @@ struct ScanRow {
     uint64_t s[kScanRows][2 * W];
 };
 
-// The output of one queue entry's value, lanes in queue order. `live` lanes hold an
+// The fill's output of one queue entry's value, lanes in queue order. `live` lanes hold an
 // entry: row, column j, value v.
 template <int MODE, int W, int NW>
 __device__ __forceinline__ void scan_emit(const DetParams &p, ScanWarp<W, NW> &q, const int64_t *rowpos, bool live, int row,
-                                          int64_t j, double v, const double *__restrict__ x) {
+                                          int64_t j, double v) {
     const int lane = threadIdx.x & 31;
     const bool keep = live && keep_value(v);
     const unsigned kb = __ballot_sync(0xffffffffu, keep);
     if (kb == 0) return;
     // the kept entries of this lane's row
     const unsigned same = __match_any_sync(0xffffffffu, live ? row : 32 + lane) & kb;
-    if (MODE == kDetMatvec) {
-        const double xj = keep ? x[j] : 0.0;
-        // the first kept lane of each row adds the row's terms in order
-        const bool lead = keep && (same & ((1u << lane) - 1u)) == 0;
-        unsigned rest = lead ? same : 0u;
-        double a = lead ? q.acc[row] : 0.0;
-        while (__any_sync(0xffffffffu, rest)) {
-            const int src = rest ? __ffs((int)rest) - 1 : lane;
-            const double vs = __shfl_sync(0xffffffffu, v, src), xs = __shfl_sync(0xffffffffu, xj, src);
-            if (rest) a = fma(vs, xs, a);
-            rest &= rest - 1;
-        }
-        if (lead) q.acc[row] = a;
-    } else if (keep) {
+    if (keep) {
         const int before = __popc(same & ((1u << lane) - 1u));
         const int64_t pos = rowpos[row] + q.run[row] + before;
         p.col[pos] = (uint32_t)j;
@@ -485,7 +461,7 @@ __device__ __forceinline__ void scan_emit(const DetParams &p, ScanWarp<W, NW> &q
         }
     }
     __syncwarp();
-    if (MODE != kDetMatvec && keep && (same >> lane) == 1u) q.run[row] += __popc(same);  // the row's last kept lane
+    if (keep && (same >> lane) == 1u) q.run[row] += __popc(same);  // the row's last kept lane
     __syncwarp();
 }
 
@@ -563,8 +539,7 @@ __device__ __forceinline__ double single_of(const DetParams &p, const uint64_t *
 // Evaluates and outputs the queue's n entries (columns from `first`).
 template <int MODE, int W, int NW>
 __device__ __noinline__ void scan_flush(const DetParams &p, ScanWarp<W, NW> &q, const ScanRow<W> &rows,
-                                        const int64_t *rowpos, int64_t r0, int n, int64_t first,
-                                        const double *__restrict__ x) {
+                                        const int64_t *rowpos, int64_t r0, int n, int64_t first) {
     using U = std::conditional_t<NW == 2, uint32_t, uint64_t>;
     const int lane = threadIdx.x & 31;
     auto put = [&](int k, int row, int64_t j, double v) {
@@ -608,7 +583,7 @@ __device__ __noinline__ void scan_flush(const DetParams &p, ScanWarp<W, NW> &q, 
             const bool live = k < n;
             const uint32_t e = live ? q.at[k] : 0u;
             scan_emit<MODE, W, NW>(p, q, rowpos, live, (int)(e >> kQueueColBits), first + (e & kQueueColMask),
-                                   live ? q.val[k] : 0.0, x);
+                                   live ? q.val[k] : 0.0);
         }
     }
     __syncwarp();
@@ -653,26 +628,19 @@ __device__ __forceinline__ uint32_t connected(const uint32_t *key, const uint32_
     return x;
 }
 
-// Block: 32 rows x WARPS warps. Counts and fills run one-warp blocks, one per 32 rows
-// and segment of the columns (grid: row groups x kSegs), so that a segment dense in
-// connected pairs holds up no other (the L=32 list's build: 15.7 ms with the segments
-// as the warps of one block, which then wait for the densest; 9.2 ms with 16 one-warp
-// blocks of them, 4.6 with 64 and the single-word element functions). The matvec's warps take every
-// kScanWarps-th word of the columns, which spreads such segments over them, and meet
-// once at the end.
-template <int W, int NW, int MODE, bool RANGED>
-__global__ void __launch_bounds__(32 * scan_warps<MODE>(), MODE == kDetMatvec ? 4 : 32)
-    k_dets_scan(const DetParams p, const double *__restrict__ x, double *__restrict__ y) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int WARPS = scan_warps<MODE>();
-    constexpr bool kStoring = MODE != kDetMatvec;
+// One-warp blocks, one per 32 rows and segment of the columns (grid: row groups x kSegs),
+// so that a segment dense in connected pairs holds up no other (the L=32 list's build:
+// 15.7 ms with the segments as the warps of one block, which then wait for the densest;
+// 9.2 ms with 16 one-warp blocks of them, 4.6 with 64 and the single-word element
+// functions).
+template <int W, int NW, int MODE>
+__global__ void __launch_bounds__(32, 32) k_dets_scan(const DetParams p) {
+    __shared__ ScanWarp<W, NW> q;
     __shared__ ScanRow<W> rows;
     __shared__ int64_t rowpos[kScanRows];
-    ScanWarp<W, NW> *warps = reinterpret_cast<ScanWarp<W, NW> *>(smem);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    ScanWarp<W, NW> &q = warps[warp];
-    const int64_t group = kStoring ? blockIdx.x / kSegs : blockIdx.x;
-    const int seg = kStoring ? (int)(blockIdx.x - group * kSegs) : 0;
+    const int lane = threadIdx.x;
+    const int64_t group = blockIdx.x / kSegs;
+    const int seg = (int)(blockIdx.x - group * kSegs);
     const int64_t r0 = group * kScanRows;
     const int64_t i = r0 + lane;
     const bool active = i < p.nrows;
@@ -681,19 +649,10 @@ __global__ void __launch_bounds__(32 * scan_warps<MODE>(), MODE == kDetMatvec ? 
     for (int w = 0; w < 2 * W; ++w) rec[w] = active ? p.dets[i * 2 * W + w] : 0;
     uint32_t rk[NW];
     scan_key<W, NW>(rec, rk);
-    if (warp == 0) {
 #pragma unroll
-        for (int w = 0; w < 2 * W; ++w) rows.s[lane][w] = rec[w];
-    }
-    q.acc[lane] = 0.0;
+    for (int w = 0; w < 2 * W; ++w) rows.s[lane][w] = rec[w];
     q.run[lane] = q.low[lane] = 0;
-    // columns [c_lo, c_end): a stored pass takes those of the block; the matvec of a
-    // partly stored matrix takes, for the block's rows, those outside it
-    const int64_t c_lo = (RANGED && r0 + kScanRows <= p.block) ? p.block : 0;
-    const int64_t c_end = kStoring ? p.block : p.n;
-    const int64_t words = (c_end - c_lo + 31) / 32;
-    const int64_t w0 = kStoring ? words * seg / kSegs : warp, w1 = kStoring ? words * (seg + 1) / kSegs : words;
-    constexpr int kStep = kStoring ? 1 : WARPS;
+    const int64_t words = (p.block + 31) / 32, w0 = words * seg / kSegs, w1 = words * (seg + 1) / kSegs;
     if (MODE == kDetFill64 || MODE == kDetFill32) {
         int64_t at = 0;
         if (active) {
@@ -702,31 +661,29 @@ __global__ void __launch_bounds__(32 * scan_warps<MODE>(), MODE == kDetMatvec ? 
         }
         rowpos[lane] = at;
     }
-    __syncthreads();
+    __syncwarp();
     const uint32_t one = p.one;
     int qn = 0;
     int64_t first = 0;
     uint64_t next[2 * W];
     auto load = [&](int64_t word) {
-        const int64_t j = c_lo + word * 32 + lane;
+        const int64_t j = word * 32 + lane;
 #pragma unroll
-        for (int w = 0; w < 2 * W; ++w) next[w] = (word < w1 && j < c_end) ? __ldg(p.dets + j * 2 * W + w) : 0;
+        for (int w = 0; w < 2 * W; ++w) next[w] = (word < w1 && j < p.block) ? __ldg(p.dets + j * 2 * W + w) : 0;
     };
     load(w0);
-    for (int64_t word = w0; word < w1; word += kStep) {
-        const int64_t base = c_lo + word * 32;
+    for (int64_t word = w0; word < w1; ++word) {
+        const int64_t base = word * 32;
         uint32_t ck[NW];
         scan_key<W, NW>(next, ck);
 #pragma unroll
         for (int w = 0; w < NW; ++w) q.key[lane * NW + w] = ck[w];
         __syncwarp();
-        load(word + kStep);
+        load(word + 1);
         uint32_t m = scan_word<NW>(q.key, rk, one);
         __syncwarp();  // the staged columns are read; the next word's may be written
-        if (c_end - base < 32) m &= (1u << (int)(c_end - base)) - 1u;
+        if (p.block - base < 32) m &= (1u << (int)(p.block - base)) - 1u;
         if (!active) m = 0;
-        if (RANGED && i < p.block && base < p.block)
-            m = p.block - base >= 32 ? 0u : m & ~((1u << (int)(p.block - base)) - 1u);
         if (!__any_sync(0xffffffffu, m)) continue;
         int off = __popc(m);
 #pragma unroll
@@ -737,7 +694,7 @@ __global__ void __launch_bounds__(32 * scan_warps<MODE>(), MODE == kDetMatvec ? 
         const int total = __shfl_sync(0xffffffffu, off, 31);
         off -= __popc(m);
         if (qn > 0 && (qn + total > kQueue || base - first > (int64_t)(kQueueColMask - 32))) {
-            scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, qn, first, x);
+            scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, qn, first);
             qn = 0;
         }
         if (qn == 0) first = base;
@@ -751,24 +708,16 @@ __global__ void __launch_bounds__(32 * scan_warps<MODE>(), MODE == kDetMatvec ? 
                 const int g1 = g < 3 ? __shfl_sync(0xffffffffu, off, (8 * g + 8) & 31) : total;
                 if ((lane >> 3) == g)
                     for (int k = off - g0; m; m &= m - 1) q.at[k++] = tag + (uint32_t)(__ffs((int)m) - 1);
-                if (g1 > g0) scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, g1 - g0, first, x);
+                if (g1 > g0) scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, g1 - g0, first);
             }
         }
     }
-    if (qn > 0) scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, qn, first, x);
+    if (qn > 0) scan_flush<MODE, W, NW>(p, q, rows, rowpos, r0, qn, first);
     if constexpr (MODE == kDetCount) {
         if (active) {
             p.seg_count[i * kSegs + seg] = q.run[lane];
             if (q.run[lane]) atomicAdd(p.row_count + i, q.run[lane]);  // integer sums: any order
             if (q.low[lane]) atomicAdd(p.upper_off + i, q.low[lane]);
-        }
-    } else if constexpr (MODE == kDetMatvec) {
-        __syncthreads();
-        if (warp == 0 && active) {
-            double a = 0;
-            for (int w = 0; w < WARPS; ++w) a += warps[w].acc[lane];
-            // rows of the stored block add to the stored block's product, already in y
-            y[i] = ((RANGED && i < p.block) ? y[i] : 0.0) + a;
         }
     }
 }
@@ -950,6 +899,258 @@ __global__ void __launch_bounds__(32, 32) k_dets_pairs(const DetParams p) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// The matvec without a stored matrix: y_i = sum_j H_ij x_j, every element recomputed. A
+// block owns 32 rows; its warps take every kMvWarps-th word of the columns, which spreads
+// dense stretches over them, and meet once at the end. A warp keeps the masks of up to
+// kMvSpan words and queues their pairs row by row, so that after the evaluation every
+// lane adds its own row's products, one after the other: about as many FP64 additions for
+// the warp as the longest row has elements in the queue. (Words queued one by one, the
+// lanes of a row finding each other for each 32 entries: 600 instructions per 32
+// elements, 0.49 ms for the L=28 list; now
+// 0.48.)
+//
+// RANGED: a list with a stored block (CI_Big with a kept part) leaves out the block's
+// pairs.
+constexpr int kMvWarps = 8;
+constexpr int kMvSpan = 16;
+
+template <int W, int NW>
+struct MatvecWarp {
+    alignas(16) uint32_t key[32 * NW];
+    double val[kQueue], xv[kQueue];
+    uint32_t mask[kMvSpan][32];
+    int64_t base[kMvSpan];
+    uint16_t at[kQueue], single[kQueue];  // row << 9 | word << 5 | column; queue positions of the singles
+};
+
+// Evaluates the queued words (n pairs in all, `mine` of the lane's row) and adds them.
+template <int W, int NW>
+__device__ __noinline__ double matvec_flush(const DetParams &p, MatvecWarp<W, NW> &q, const ScanRow<W> &rows, int64_t r0,
+                                            int span, int n, int mine, const double *__restrict__ x, double acc) {
+    using U = std::conditional_t<NW == 2, uint32_t, uint64_t>;
+    const int lane = threadIdx.x & 31;
+    int start = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, start, o);
+        if (lane >= o) start += u;
+    }
+    start -= mine;
+    for (int s = 0, k = start; s < span; ++s)
+        for (uint32_t m = q.mask[s][lane]; m; m &= m - 1)
+            q.at[k++] = (uint16_t)(lane << 9 | s << 5 | (__ffs((int)m) - 1));
+    __syncwarp();
+    auto place = [&](int k, int &row, int64_t &j) {
+        const int e = q.at[k];
+        row = e >> 9;
+        j = q.base[(e >> 5) & 15] + (e & 31);
+    };
+    int ns = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        bool single = false;
+        if (k < n) {
+            int row;
+            int64_t j;
+            place(k, row, j);
+            const double xj = __ldg(x + j);
+            const double v = pair_of<W, U>(p, rows.s[row], r0 + row, j, single);
+            if (!single) q.val[k] = v;
+            q.xv[k] = xj;
+        }
+        const unsigned sb = __ballot_sync(0xffffffffu, single);
+        if (single) q.single[ns + __popc(sb & ((1u << lane) - 1u))] = (uint16_t)k;
+        ns += __popc(sb);
+    }
+    __syncwarp();
+    for (int k0 = 0; k0 < ns; k0 += 32) {
+        if (k0 + lane < ns) {
+            const int k = q.single[k0 + lane];
+            int row;
+            int64_t j;
+            place(k, row, j);
+            q.val[k] = single_of<W, U>(p, rows.s[row], j);
+        }
+    }
+    __syncwarp();
+    for (int k = start; k < start + mine; ++k) {
+        const double v = q.val[k];
+        if (keep_value(v)) acc = fma(v, q.xv[k], acc);
+    }
+    __syncwarp();
+    return acc;
+}
+
+template <int W, int NW, bool RANGED>
+__global__ void __launch_bounds__(32 * kMvWarps, 3) k_dets_matvec(const DetParams p, const double *__restrict__ x,
+                                                                  double *__restrict__ y) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ ScanRow<W> rows;
+    __shared__ double part[kMvWarps][kScanRows];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    MatvecWarp<W, NW> &q = reinterpret_cast<MatvecWarp<W, NW> *>(smem)[warp];
+    const int64_t r0 = (int64_t)blockIdx.x * kScanRows, i = r0 + lane;
+    const bool active = i < p.n;
+    uint64_t rec[2 * W];
+#pragma unroll
+    for (int w = 0; w < 2 * W; ++w) rec[w] = active ? p.dets[i * 2 * W + w] : 0;
+    uint32_t rk[NW];
+    scan_key<W, NW>(rec, rk);
+    if (warp == 0) {
+#pragma unroll
+        for (int w = 0; w < 2 * W; ++w) rows.s[lane][w] = rec[w];
+    }
+    __syncthreads();
+    const int64_t c_lo = (RANGED && r0 + kScanRows <= p.block) ? p.block : 0;  // the stored rows' pairs outside the block
+    const int64_t words = (p.n - c_lo + 31) / 32;
+    const uint32_t one = p.one;
+    uint64_t next[2 * W];
+    auto load = [&](int64_t word) {
+        const int64_t j = c_lo + word * 32 + lane;
+#pragma unroll
+        for (int w = 0; w < 2 * W; ++w) next[w] = (word < words && j < p.n) ? __ldg(p.dets + j * 2 * W + w) : 0;
+    };
+    int span = 0, n = 0, mine = 0;
+    double acc = 0;
+    auto flush = [&] {
+        acc = matvec_flush<W, NW>(p, q, rows, r0, span, n, mine, x, acc);
+        span = n = mine = 0;
+    };
+    auto add = [&](int64_t base, uint32_t m, int total) {
+        q.mask[span][lane] = m;
+        if (lane == 0) q.base[span] = base;
+        ++span;
+        n += total;
+        mine += __popc(m);
+    };
+    load(warp);
+    for (int64_t word = warp; word < words; word += kMvWarps) {
+        const int64_t base = c_lo + word * 32;
+        uint32_t ck[NW];
+        scan_key<W, NW>(next, ck);
+#pragma unroll
+        for (int w = 0; w < NW; ++w) q.key[lane * NW + w] = ck[w];
+        __syncwarp();
+        load(word + kMvWarps);
+        uint32_t m = scan_word<NW>(q.key, rk, one);
+        if (p.n - base < 32) m &= (1u << (int)(p.n - base)) - 1u;
+        if (!active) m = 0;
+        if (RANGED && i < p.block && base < p.block)
+            m = p.block - base >= 32 ? 0u : m & ~((1u << (int)(p.block - base)) - 1u);
+        m = connected<NW>(q.key, rk, m);
+        const int total = __reduce_add_sync(0xffffffffu, __popc(m));  // the staged columns are read
+        if (total == 0) continue;
+        if (span == kMvSpan || n + total > kQueue) flush();
+        if (total <= kQueue) {
+            add(base, m, total);
+            continue;
+        }
+        for (int g = 0; g < 4; ++g) {  // a dense word: eight rows at a time fill the queue at most
+            const uint32_t mg = (lane >> 3) == g ? m : 0u;
+            add(base, mg, __reduce_add_sync(0xffffffffu, __popc(mg)));
+            flush();
+        }
+    }
+    if (n > 0) flush();
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && active) {
+        double a = 0;
+        for (int w = 0; w < kMvWarps; ++w) a += part[w][lane];
+        // rows of the stored block add to the stored block's product, already in y
+        y[i] = ((RANGED && i < p.block) ? y[i] : 0.0) + a;
+    }
+}
+
+// The same for short lists: a warp owns one row and its lanes test 32 columns at a time, so
+// that a few thousand rows make enough warps; the pairs found are queued and evaluated 32
+// at a time, and every 32nd of them is added by one lane. Half the pairs per instruction of
+// the kernel above, whose 32 rows to a warp leave a short list's blocks too few. Alone,
+// and among other products, this | that: 1,577 rows of L=36 44 | 199 and 17 | 70 us; 5,665
+// of L=20 133 | 491 and 107 | 173; 6,189 of L=24 236 | 253 and 129 | 98; 12,290 of L=28
+// 623 | 428 and 400 | 181.
+constexpr int64_t kMvShort = 6000;
+
+template <int W>
+struct RowQueue {
+    double val[kQueue];
+    uint32_t at[kQueue];  // columns
+    uint16_t single[kQueue];
+};
+
+template <int W, int NW>
+__device__ __noinline__ double row_flush(const DetParams &p, RowQueue<W> &q, const uint64_t *row, int64_t i, int n,
+                                         const double *__restrict__ x, double acc) {
+    using U = std::conditional_t<NW == 2, uint32_t, uint64_t>;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    int ns = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        bool single = false;
+        if (k < n) {
+            const double v = pair_of<W, U>(p, row, i, q.at[k], single);
+            if (!single) q.val[k] = v;
+        }
+        const unsigned sb = __ballot_sync(0xffffffffu, single);
+        if (single) q.single[ns + __popc(sb & ((1u << lane) - 1u))] = (uint16_t)k;
+        ns += __popc(sb);
+    }
+    __syncwarp();
+    for (int k0 = 0; k0 < ns; k0 += 32)
+        if (k0 + lane < ns) {
+            const int k = q.single[k0 + lane];
+            q.val[k] = single_of<W, U>(p, row, q.at[k]);
+        }
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) {
+        const double v = q.val[k];
+        if (keep_value(v)) acc = fma(v, __ldg(x + q.at[k]), acc);
+    }
+    __syncwarp();
+    return acc;
+}
+
+template <int W, int NW, bool RANGED>
+__global__ void __launch_bounds__(32 * kMvWarps) k_dets_matvec_rows(const DetParams p, const double *__restrict__ x,
+                                                                    double *__restrict__ y) {
+    __shared__ RowQueue<W> queues[kMvWarps];
+    __shared__ uint64_t rows[kMvWarps][2 * W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t i = (int64_t)blockIdx.x * kMvWarps + warp;
+    if (i >= p.n) return;
+    RowQueue<W> &q = queues[warp];
+    uint64_t ri[2 * W];
+#pragma unroll
+    for (int w = 0; w < 2 * W; ++w) ri[w] = __ldg(p.dets + i * 2 * W + w);
+    if (lane < 2 * W) rows[warp][lane] = __ldg(p.dets + i * 2 * W + lane);
+    const int64_t c_lo = (RANGED && i < p.block) ? p.block : 0;  // a stored row's pairs outside the block
+    int n = 0;
+    double acc = 0;
+    for (int64_t base = c_lo; base < p.n; base += 32) {
+        const int64_t j = base + lane;
+        int d = 0;
+#pragma unroll
+        for (int w = 0; w < 2 * W; ++w) {
+            const uint64_t v = (j < p.n ? __ldg(p.dets + j * 2 * W + w) : ~ri[w]) ^ ri[w];
+            d += NW == 2 ? __popc((uint32_t)v) : __popcll(v);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, d <= 4);  // past the list: every bit differs
+        if (m == 0) continue;
+        if (n + 32 > kQueue) {
+            acc = row_flush<W, NW>(p, q, rows[warp], i, n, x, acc);
+            n = 0;
+        }
+        if (d <= 4) q.at[n + __popc(m & ((1u << lane) - 1u))] = (uint32_t)j;
+        n += __popc(m);
+    }
+    if (n > 0) acc = row_flush<W, NW>(p, q, rows[warp], i, n, x, acc);
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    // rows of the stored block add to the stored block's product, already in y
+    if (lane == 0) y[i] = ((RANGED && i < p.block) ? y[i] : 0.0) + acc;
+}
+
 __global__ void k_sum_u32(const uint32_t *a, int64_t n, unsigned long long *out) {
     unsigned long long s = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -962,61 +1163,67 @@ int rows_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + kDetWarps - 1) / kDetWarps, (int64_t)sm_count() * 16));
 }
 
-template <int W, int NW, int MODE, bool RANGED>
-void launch_scan(const DetParams &p, const double *x, double *y, cudaStream_t s) {
-    constexpr int smem = (int)sizeof(ScanWarp<W, NW>) * scan_warps<MODE>();
-    static const cudaError_t attr = cudaFuncSetAttribute(k_dets_scan<W, NW, MODE, RANGED>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    CIGPU_CUDA(attr);
-    const int64_t blocks = (p.nrows + kScanRows - 1) / kScanRows * (MODE == kDetMatvec ? 1 : kSegs);
+unsigned segment_blocks(const DetParams &p) {
+    const int64_t blocks = (p.nrows + kScanRows - 1) / kScanRows * kSegs;
     if (blocks > (int64_t)INT32_MAX) throw std::invalid_argument("determinant list too long");
-    k_dets_scan<W, NW, MODE, RANGED><<<(unsigned)blocks, 32 * scan_warps<MODE>(), smem, s>>>(p, x, y);
-    CIGPU_CUDA(cudaGetLastError());
-    count_launch();
+    return (unsigned)blocks;
 }
 
-template <int W, int NW, int MODE>
-void launch_rows(const DetParams &p, const double *x, double *y, cudaStream_t s) {
-    if (p.nrows == 0) return;
-    if constexpr (MODE == kDetMatvec) {
-        if (p.block > 0 && p.block < p.n) {  // a partly stored list
-            launch_scan<W, NW, MODE, true>(p, x, y, s);
-            return;
-        }
-    }
-    launch_scan<W, NW, MODE, false>(p, x, y, s);
+// f with the words of 64 and of 32 bits a determinant of the list takes.
+template <typename F>
+void by_words(const DetParams &p, int W, F &&f) {
+    if (W == 2)
+        f(std::integral_constant<int, 2>{}, std::integral_constant<int, 8>{});
+    else if (p.L > 32)
+        f(std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{});
+    else
+        f(std::integral_constant<int, 1>{}, std::integral_constant<int, 2>{});
 }
 
 template <int MODE>
-void rows(const DetParams &p, int W, const double *x, double *y, cudaStream_t s) {
-    if (W == 2)
-        launch_rows<2, 8, MODE>(p, x, y, s);
-    else if (p.L > 32)
-        launch_rows<1, 4, MODE>(p, x, y, s);
-    else
-        launch_rows<1, 2, MODE>(p, x, y, s);
-}
-
-template <int W, int NW, int MODE>
-void launch_pairs(const DetParams &p, cudaStream_t s) {
-    const int64_t blocks = (p.nrows + kScanRows - 1) / kScanRows * kSegs;
-    if (blocks > (int64_t)INT32_MAX) throw std::invalid_argument("determinant list too long");
-    if (p.masks)
-        k_dets_pairs<W, NW, MODE, true><<<(unsigned)blocks, 32, 0, s>>>(p);
-    else
-        k_dets_pairs<W, NW, MODE, false><<<(unsigned)blocks, 32, 0, s>>>(p);
+void rows(const DetParams &p, int W, cudaStream_t s) {
+    by_words(p, W, [&](auto w, auto nw) { k_dets_scan<w(), nw(), MODE><<<segment_blocks(p), 32, 0, s>>>(p); });
     CIGPU_CUDA(cudaGetLastError());
     count_launch();
 }
 
 template <int MODE>
 void pairs(const DetParams &p, int W, cudaStream_t s) {
-    if (W == 2)
-        launch_pairs<2, 8, MODE>(p, s);
-    else if (p.L > 32)
-        launch_pairs<1, 4, MODE>(p, s);
-    else
-        launch_pairs<1, 2, MODE>(p, s);
+    by_words(p, W, [&](auto w, auto nw) {
+        if (p.masks)
+            k_dets_pairs<w(), nw(), MODE, true><<<segment_blocks(p), 32, 0, s>>>(p);
+        else
+            k_dets_pairs<w(), nw(), MODE, false><<<segment_blocks(p), 32, 0, s>>>(p);
+    });
+    CIGPU_CUDA(cudaGetLastError());
+    count_launch();
+}
+
+void matvec(const DetParams &p, int W, const double *x, double *y, cudaStream_t s) {
+    const bool ranged = p.block > 0 && p.block < p.n;  // a partly stored list
+    by_words(p, W, [&](auto w, auto nw) {
+        if (p.n < kMvShort) {
+            const unsigned blocks = (unsigned)((p.n + kMvWarps - 1) / kMvWarps);
+            if (ranged)
+                k_dets_matvec_rows<w(), nw(), true><<<blocks, 32 * kMvWarps, 0, s>>>(p, x, y);
+            else
+                k_dets_matvec_rows<w(), nw(), false><<<blocks, 32 * kMvWarps, 0, s>>>(p, x, y);
+            return;
+        }
+        const unsigned blocks = (unsigned)((p.n + kScanRows - 1) / kScanRows);
+        constexpr int smem = (int)sizeof(MatvecWarp<w(), nw()>) * kMvWarps;
+        auto go = [&](auto kern) {
+            // the same value at every call: concurrent callers never lower it
+            CIGPU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            kern<<<blocks, 32 * kMvWarps, smem, s>>>(p, x, y);
+        };
+        if (ranged)
+            go(k_dets_matvec<w(), nw(), true>);
+        else
+            go(k_dets_matvec<w(), nw(), false>);
+    });
+    CIGPU_CUDA(cudaGetLastError());
+    count_launch();
 }
 
 DetParams params_of(const cigpu_crs &c) {
@@ -1333,7 +1540,7 @@ void dets_mv64(cigpu_crs &c, const double *x, double *y, cudaStream_t s) {
     // the stored leading block first (rows and columns below det_block), then every
     // pair outside it recomputed (CI_Big::mvprod, CIMethod.cpp:943-984)
     if (c.det_block > 0) spmv_f64(c.det_block, c.nnz_full, c.row_ptr.p, c.col.p, c.val64.p, x, y, s);
-    if (c.det_block < c.dim) rows<kDetMatvec>(p, c.det_words, x, y, s);  // nothing outside a whole-list block
+    if (c.det_block < c.dim) matvec(p, c.det_words, x, y, s);  // nothing outside a whole-list block
 }
 
 }  // namespace cigpu
@@ -1469,7 +1676,7 @@ int build_dets(cigpu_ham *ham, int64_t ndet, int words, const uint64_t *up, cons
             if (structure)
                 pairs<kDetCount>(p, W, s);
             else
-                rows<kDetCount>(p, W, nullptr, nullptr, s);
+                rows<kDetCount>(p, W, s);
             exclusive_scan_u32(count.p, c->row_ptr.p, nb, s);
             k_sum_u32<<<(int)std::min<int64_t>((nb + 255) / 256, 1024), 256, 0, s>>>(c->upper_off.p, nb, lower.p);
             CIGPU_CUDA(cudaGetLastError());
@@ -1497,9 +1704,9 @@ int build_dets(cigpu_ham *ham, int64_t ndet, int words, const uint64_t *up, cons
             else if (structure)
                 pairs<kDetFill32>(p, W, s);
             else if (precision == CIGPU_FP64)
-                rows<kDetFill64>(p, W, nullptr, nullptr, s);
+                rows<kDetFill64>(p, W, s);
             else
-                rows<kDetFill32>(p, W, nullptr, nullptr, s);
+                rows<kDetFill32>(p, W, s);
             if (!structure) return true;
             uint32_t d = 0;
             CIGPU_CUDA(cudaMemcpyAsync(&d, dropped.p, sizeof(d), cudaMemcpyDeviceToHost, s));

@@ -243,3 +243,21 @@ def test_dropped_elements(kind, precision):
         assert np.array_equal(val, m.val)
     else:
         assert np.array_equal(val, m.val.astype(np.float32).astype(np.float64))
+
+
+@pytest.mark.parametrize("L,na,nb,n,repeat", [(14, 3, 3, 6100, 1), (36, 4, 3, 6001, 1), (40, 1, 1, 1600, 5)])
+def test_matvec_of_a_longer_list(L, na, nb, n, repeat):
+    """The matvec without a stored matrix past the short lists' kernel: 32 and 64-bit
+    strings, and a list of repeated determinants whose pairs are all connected (words that
+    overflow the queue), whole and with a stored leading block, against the stored CRS."""
+    ints = make_integrals(L, na, nb, nchol=3, seed=L)
+    up, down = random_list(L, na, nb, n, seed=n)
+    up, down = np.tile(up, repeat), np.tile(down, repeat)
+    ham = Hamiltonian.from_integrals(ints)
+    x = np.random.default_rng(6).standard_normal(len(up))
+    stored = FCI_File(ham, up=up, down=down).get_mat()
+    y = stored.mvprod(x)
+    _, _, val = stored.full()
+    tol = 2.0 ** -52 * (len(up) + 2) * float(np.abs(val).max() * np.abs(x).max()) * np.sqrt(len(up))
+    for keep in (0, 777):
+        assert np.abs(CI_Big(ham, up=up, down=down, keep=keep).get_mat().mvprod(x) - y).max() <= tol
