@@ -550,8 +550,8 @@ def run_cigpu(args, rank: int, world: int, dist):
         shape = f"{cfg['method'].lower()}_L{cfg['L']}_{cfg['nup']}a{cfg['ndown']}b"
         if kind[0] == A.FP32_SIGMA:
             # the factorised sigma vector reads the matrix from no DRAM stream: its work
-            # is FP32 FMAs over every determinant's single excitations times the rank,
-            # on vectors that stay in L2; its roofline is the FP32 FMA rate
+            # is FP32 FMAs (the strings' same-spin elements, and every determinant's
+            # single excitations times the rank); its roofline is the FP32 FMA rate
             w = A.sigma_work(cfg["L"], cfg["nup"], cfg["ndown"], kind[1], kind[2])
             sms = torch.cuda.get_device_properties(0).multi_processor_count
             peak_tf = sms * 128 * 2 * 2070e6 / 1e12
@@ -559,10 +559,10 @@ def run_cigpu(args, rank: int, world: int, dist):
             roof[tag] = {"bound": "fp32", "achieved": ach, "peak": peak_tf, "unit": "TFLOP/s", "frac": ach / peak_tf,
                          "traffic": ncu_traffic(f"sigma_fp32_{shape}"), "algorithmic_flops": w["flops"],
                          "l2_bytes_per_launch": w["l2_bytes"], "l2_gbs": w["l2_bytes"] / t / 1e9,
-                         "l2_note": "the factor vectors the kernels read per excitation live in L2 (about half of "
-                                    "those reads hit L1); ncu: L2 27% busy, issue 46-50% at L=11",
+                         "l2_note": "one number per alpha excitation written and read; the same-spin part reads x "
+                                    "through L1 and shared memory, whose data path bounds the kernels",
                          "layout": f"sigma-fp32 (rank {kind[1]}, padded {kind[2]})",
-                         "kernels": "k_transpose32 + k_sigma_a + k_sigma_b", "ms_per_launch": t * 1000,
+                         "kernels": "k_sigma_pad + k_sigma_parts + k_sigma_sum", "ms_per_launch": t * 1000,
                          "nnz_full": nf.value,
                          "peak_source": "nominal FP32 FMA rate: SMs x 128 lanes x 2 flops x 2070 MHz "
                                         "(no measured FP32 figure)"}

@@ -213,17 +213,18 @@ def fp32_product(handle) -> tuple[int, int, int]:
 
 def sigma_work(L: int, nup: int, ndown: int, rank: int, padded: int) -> dict:
     """Algorithmic work of one FP32 sigma product on the FCI space (nup, ndown) of L
-    orbitals with `rank` factors: FP32 FMAs per determinant (pass 1: (R + 1) per
-    single excitation and on the diagonal, the one-body matrix included; pass 2: R
-    per excitation and on the diagonal) and the bytes the passes move through L2
-    (x read per excitation, the padded factor vectors written twice and read per
-    excitation, y written)."""
+    orbitals with `rank` factors: FP32 FMAs per determinant (the same-spin elements of
+    both strings; `rank` per beta single excitation and on the diagonal for the factor
+    sums, `rank` per alpha one for its number, one per alpha one to add it) and the bytes
+    that move through L2 (x in two orders written and read, the alpha numbers written
+    and read once, the beta part written and read, y written)."""
     from math import comb
-    ns = nup * (L - nup) + ndown * (L - ndown)
+    sa, sb = nup * (L - nup), ndown * (L - ndown)
+    same = 2 + sa + sb + comb(nup, 2) * comb(L - nup, 2) + comb(ndown, 2) * comb(L - ndown, 2)
     dim = comb(L, nup) * comb(L, ndown)
-    fma = dim * (ns * (rank + 1) + rank + 1 + rank + ns * rank)
-    l2 = dim * 4 * ((1 + ns) + 2 * padded + (1 + ns) * padded + 2)
-    return {"fma": fma, "flops": 2 * fma, "l2_bytes": l2, "dim": dim, "excitations_per_det": ns}
+    fma = dim * (same + rank * (sb + 1) + rank * (sa + 1) + sa)
+    l2 = dim * 4 * (1 + 4 + 2 * (sa + 1) + 2 + 1)
+    return {"fma": fma, "flops": 2 * fma, "l2_bytes": l2, "dim": dim, "excitations_per_det": sa + sb}
 
 
 def matvec_bytes(handle, fp32: bool) -> tuple[int, str]:

@@ -784,6 +784,149 @@ __global__ void __launch_bounds__(kSmallThreads) k_lanczos_steps(int64_t n, doub
     }
 }
 
+// The mixed solver's step on small spaces: what k_dav_residual32, two k_multidot / k_update
+// passes and k_scale do in seven launches, each of a few microseconds for less than one of
+// work, on one cluster of 16 blocks; the couplings and the fetch of their results in one
+// more, which writes them to pinned memory. A block owns a slice of the rows, keeps its
+// slices of the basis in shared memory after the residual has read them, and the sums meet
+// through distributed shared memory in a fixed order (FP32 sums per warp, FP64 above, as
+// the separate kernels). Up to kDavRows rows, past which the basis is read faster by all
+// SMs. FCI L=8 4a4b (4,900 rows) to 1e-11: 9.9 -> 6.7 ms.
+constexpr int kDavThreads = 512;
+constexpr int64_t kDavRows = 16384;
+
+struct DavCoef {
+    double y[kMaxBasis];  // y_1..y_k
+};
+
+inline size_t dav_smem(int64_t n, int mmax) {
+    const size_t slice = (size_t)((n + kSmallCluster - 1) / kSmallCluster);
+    return sizeof(float) * slice * (mmax + 3);
+}
+
+// Adds the cluster's parts of `count` sums (part: each block's, at the same place), the
+// same order in every block.
+template <typename C>
+__device__ __forceinline__ void cluster_sums(C &cluster, double *part, int count, double *sum) {
+    cluster.sync();
+    for (int i = threadIdx.x; i < count; i += kDavThreads) {
+        double a = 0;
+#pragma unroll
+        for (int b = 0; b < kSmallCluster; ++b) a += cluster.map_shared_rank(part, b)[i];
+        sum[i] = a;
+    }
+    __syncthreads();
+}
+
+// Direction k + 1 of the basis, orthonormalised against slots 0..k. `given`: V's slot
+// k + 1 holds the direction already (the first one after an anchor).
+__global__ void __launch_bounds__(kDavThreads) k_dav_step(int64_t n, float *__restrict__ V, const float *__restrict__ HV,
+                                                          int k, bool given, const DavCoef coef, double a0, double a0_de,
+                                                          double theta, const double *__restrict__ dmin,
+                                                          const float *__restrict__ r32, const float *__restrict__ c32,
+                                                          const float *__restrict__ diag32, double *__restrict__ out_r,
+                                                          double *__restrict__ out_n) {
+    namespace cg = cooperative_groups;
+    auto cluster = cg::this_cluster();
+    extern __shared__ __align__(16) float dav_sm[];
+    __shared__ float ys[kMaxBasis];
+    __shared__ double part[2][kMaxBasis + 2], sum[kMaxBasis + 2], wsum[kDavThreads / 32];
+    const int slice = (int)((n + kSmallCluster - 1) / kSmallCluster), t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int rank = (int)cluster.block_rank();
+    const int64_t r0 = (int64_t)rank * slice;
+    const int mine = (int)max((int64_t)0, min((int64_t)slice, n - r0));
+    float *Vs = dav_sm;                         // [k + 1][slice]
+    float *w = Vs + (size_t)(k + 1) * slice;    // [slice] the direction
+    float *out = V + (int64_t)(k + 1) * n + r0;
+    for (int i = t; i < k; i += kDavThreads) ys[i] = (float)coef.y[i];
+    __syncthreads();
+    const float fa0 = (float)a0, fa0de = (float)a0_de, fth = (float)theta, fsig = (float)fmin(theta, *dmin);
+    float rr = 0.f;
+    for (int e = t; e < mine; e += kDavThreads) {
+        const int64_t r = r0 + e;
+        float ru = 0.f;
+        if (!given) ru = fa0 * r32[r] + fa0de * c32[r];
+        Vs[e] = V[r];
+        for (int i = 0; i < k; ++i) {
+            const float v = V[(int64_t)(i + 1) * n + r];
+            Vs[(size_t)(i + 1) * slice + e] = v;
+            if (!given) ru += ys[i] * (HV[(int64_t)(i + 1) * n + r] - fth * v);
+        }
+        rr += ru * ru;
+        w[e] = given ? out[e] : dav_precond(ru, fsig, diag32[r]);
+    }
+    auto block_sum = [&](float v) {  // FP32 per warp, FP64 above; the result on thread 0
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        __syncthreads();
+        if (lane == 0) wsum[warp] = (double)v;
+        __syncthreads();
+        double a = 0;
+        if (t == 0)
+            for (int q = 0; q < kDavThreads / 32; ++q) a += wsum[q];
+        return a;
+    };
+    const double rrs = block_sum(rr);
+    if (t == 0) part[0][k + 2] = rrs;
+    double norm = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        double *p = part[pass];
+        // the dots with slots 0..k, and w with itself (place k + 1)
+        for (int i = warp; i < k + 2; i += kDavThreads / 32) {
+            const float *v = i <= k ? Vs + (size_t)i * slice : w;
+            float a = 0.f;
+            for (int e = lane; e < mine; e += 32) a += v[e] * w[e];
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0) p[i] = (double)a;
+        }
+        cluster_sums(cluster, p, k + 2 + (pass == 0), sum);
+        const double before = sum[k + 1];
+        if (pass == 0 && rank == 0 && t == 0) *out_r = sum[k + 2];
+        float nn = 0.f;
+        for (int e = t; e < mine; e += kDavThreads) {
+            float x = w[e];
+            for (int i = 0; i <= k; ++i) x -= Vs[(size_t)i * slice + e] * (float)sum[i];
+            w[e] = x;
+            nn += x * x;
+        }
+        const double ns = block_sum(nn);
+        // every block has read the other parts of this pass before one is written again
+        cluster.sync();
+        if (t == 0) p[0] = ns;
+        cluster_sums(cluster, p, 1, sum);
+        norm = sum[0];
+        if (norm >= 0.5 * before) break;  // the DGKS test: a second pass is not needed (the same in every block)
+        cluster.sync();
+    }
+    if (rank == 0 && t == 0) *out_n = norm;
+    const float inv = (float)(1.0 / sqrt(norm));
+    for (int e = t; e < mine; e += kDavThreads) out[e] = w[e] * inv;
+    cluster.sync();  // no block leaves while another reads its parts
+}
+
+// h[0..k] = V_1..V_{k+1} . hv, h[k + 1] = c . v, h[k + 2] = r . v (v = V_{k+1}).
+__global__ void __launch_bounds__(kDavThreads) k_dav_couple(int64_t n, const float *__restrict__ V, int k,
+                                                            const float *__restrict__ hv, const float *__restrict__ c32,
+                                                            const float *__restrict__ r32, double *__restrict__ h) {
+    namespace cg = cooperative_groups;
+    auto cluster = cg::this_cluster();
+    __shared__ double part[kMaxBasis + 2], sum[kMaxBasis + 2];
+    const int slice = (int)((n + kSmallCluster - 1) / kSmallCluster), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t r0 = (int64_t)cluster.block_rank() * slice;
+    const int mine = (int)max((int64_t)0, min((int64_t)slice, n - r0));
+    const float *v = V + (int64_t)(k + 1) * n + r0;
+    for (int i = warp; i < k + 3; i += kDavThreads / 32) {
+        const float *x = i <= k ? V + (int64_t)(i + 1) * n + r0 : v, *y = (i <= k ? hv : i == k + 1 ? c32 : r32) + r0;
+        float a = 0.f;
+        for (int e = lane; e < mine; e += 32) a += x[e] * y[e];
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) part[i] = (double)a;
+    }
+    cluster_sums(cluster, part, k + 3, sum);
+    if (cluster.block_rank() == 0)
+        for (int i = threadIdx.x; i < k + 3; i += kDavThreads) h[i] = sum[i];
+    cluster.sync();
+}
+
 // ---------------------------------------------------------------------------
 // Host-side helpers around the kernels.
 
@@ -820,27 +963,40 @@ inline bool vec4_ok(const float *p, int64_t ld, int64_t n) {
     return n % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
 }
 
-// Whether the device runs a cluster of k_lanczos_steps with this much shared memory.
-bool small_cluster_ok(size_t smem) {
-    static const bool attr = [] {  // thread-safe one-time init
-        const bool ok = cudaFuncSetAttribute(k_lanczos_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
-                        cudaFuncSetAttribute(k_lanczos_steps, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-        if (!ok) cudaGetLastError();
-        return ok;
-    }();
-    if (!attr || smem > 227 * 1024) return false;
+// One cluster of kSmallCluster blocks.
+struct ClusterLaunch {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kSmallCluster);
-    cfg.blockDim = dim3(kSmallThreads);
-    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kSmallCluster;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    ClusterLaunch(int threads, size_t smem, cudaStream_t s) {
+        cfg.gridDim = dim3(kSmallCluster);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kSmallCluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+    }
+    ClusterLaunch(const ClusterLaunch &) = delete;
+    template <typename... P, typename... X>
+    void operator()(void (*kern)(P...), X &&...x) {
+        CIGPU_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<X>(x)...));
+        count_launch();
+    }
+};
+
+// Whether the device runs such a cluster of `kern` with this much shared memory.
+template <typename K>
+bool cluster_ok(K kern, int threads, size_t smem) {
+    constexpr size_t kStatic = 4 * 1024;  // the kernels' static shared memory, at most
+    if (smem > 227 * 1024 - kStatic) return false;
+    // the same values at every call: concurrent callers never lower them
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, k_lanczos_steps, &cfg) != cudaSuccess) {
+    ClusterLaunch l(threads, smem, nullptr);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - kStatic)) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kern, &l.cfg) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -926,6 +1082,10 @@ struct VecOps {
     // fetch out[0..cnt) to the host (synchronises the stream)
     const double *fetch(int cnt) {
         CIGPU_CUDA(cudaMemcpyAsync(h_out, out.p, sizeof(double) * cnt, cudaMemcpyDeviceToHost, s));
+        return wait();
+    }
+    // the results that kernels left in h_out themselves
+    const double *wait() {
         const double t0 = wall();
         CIGPU_CUDA(cudaStreamSynchronize(s));
         g_clk.wait += wall() - t0;
@@ -1113,20 +1273,9 @@ struct TRLanczos {
             const int steps = (int)std::min<int64_t>({kSmallSteps, m - queued, n - queued, budget - matvecs});
             if (steps < 1 || head - tail >= kSmallDepth) return false;
             const int slot = (int)(head % kSmallDepth);
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(kSmallCluster);
-            cfg.blockDim = dim3(kSmallThreads);
-            cfg.dynamicSmemBytes = small_smem(n, m);
-            cfg.stream = s;
-            cudaLaunchAttribute at{};
-            at.id = cudaLaunchAttributeClusterDimension;
-            at.val.clusterDim.x = kSmallCluster;
-            at.val.clusterDim.y = at.val.clusterDim.z = 1;
-            cfg.attrs = &at;
-            cfg.numAttrs = 1;
-            CIGPU_CUDA(cudaLaunchKernelEx(&cfg, k_lanczos_steps, n, V.p, queued, steps, m, P.row_ptr, P.col, P.val,
-                                          ops.h_out + (size_t)slot * kSmallSteps * kSmallOut, check_word_device()));
-            count_launch();
+            ClusterLaunch(kSmallThreads, small_smem(n, m), s)(k_lanczos_steps, n, V.p, queued, steps, m, P.row_ptr, P.col,
+                                                              P.val, ops.h_out + (size_t)slot * kSmallSteps * kSmallOut,
+                                                              check_word_device());
             CIGPU_CUDA(cudaEventRecord(ev.e[slot], s));
             count[slot] = steps;
             queued += steps;
@@ -1301,7 +1450,8 @@ int solve_fp64(const SolveProblem &P, const SolveOptions &o, double *c_dev, bool
     TRLanczos<double> lz(n, m, keep, s, ops);
     lz.mv = [&](const double *x, double *y, cudaStream_t st) { P.mv64(x, y, st); };
     lz.start(c_dev);
-    const bool small = P.val && n <= kSmallRows && P.nnz <= kSmallNnz && small_cluster_ok(small_smem(n, m));
+    const bool small = P.val && n <= kSmallRows && P.nnz <= kSmallNnz && 
+                       cluster_ok(k_lanczos_steps, kSmallThreads, small_smem(n, m));
     double target = o.tol;
     std::pair<double, double> er{0, 1e300};
     for (int attempt = 0; attempt < 8; ++attempt) {
@@ -1475,6 +1625,8 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
     double a0p = 0;
     int kept = 0;
     const int SLOT_R = 3 * (kMaxBasis + 1), SLOT_N = SLOT_R + 1, SLOT_G = SLOT_R + 2;
+    const bool small = n <= kDavRows && cluster_ok(k_dav_step, kDavThreads, dav_smem(n, mmax)) &&
+                       cluster_ok(k_dav_couple, kDavThreads, 0);
     while (rho > o.tol && mv32 + mv64 < budget) {
         float *vnew = V.p + (size_t)(k + 1) * n;
         float *hvnew = HV.p + (size_t)(k + 1) * n;
@@ -1482,7 +1634,7 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
         if (k == 0) {
             k_precond32<<<ops.G, kVecThreads, 0, s>>>(ref.r.p, P.diag, E, dmin, vnew, n);
             count_launch();
-        } else {
+        } else if (!small) {
             CIGPU_CUDA(cudaMemcpyAsync(yd.p, y.data() + 1, sizeof(double) * k, cudaMemcpyHostToDevice, s));
             if (vec4_ok(cr32.p + n, n, n) && vec4_ok(V.p, n, n) && vec4_ok(HV.p, n, n) && vec4_ok(diag32.p, 0, n) &&
                 vec4_ok(vnew, 0, n)) {
@@ -1504,17 +1656,31 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
         // more than half of ||t||^2 (DGKS, decided on the device: the second pass's
         // kernels return at once otherwise). The first dots include t itself (slot
         // k + 1), giving ||t||^2 in out[k + 1].
-        ops.dots<float, float, float>(V.p, n, k + 2, vnew, n, 0);
-        ops.update<float, float, float>(V.p, n, k + 1, 0, vnew, n, SLOT_N, -1, k + 1, SLOT_G);
-        ops.dots<float, float, float>(V.p, n, k + 1, vnew, n, 0, SLOT_G);
-        ops.update<float, float, float>(V.p, n, k + 1, 0, vnew, n, SLOT_N, SLOT_G);
-        ops.scale(vnew, n, SLOT_N);
+        if (small) {
+            DavCoef coef{};
+            std::copy(y.begin() + 1, y.begin() + 1 + k, coef.y);
+            ClusterLaunch(kDavThreads, dav_smem(n, mmax), s)(k_dav_step, n, V.p, HV.p, k, k == 0, coef, a0, a0 * (E - theta), theta,
+                                                            dmin, cr32.p + n, cr32.p, diag32.p, ops.h_out + SLOT_R,
+                                                            ops.h_out + SLOT_N);
+        } else {
+            ops.dots<float, float, float>(V.p, n, k + 2, vnew, n, 0);
+            ops.update<float, float, float>(V.p, n, k + 1, 0, vnew, n, SLOT_N, -1, k + 1, SLOT_G);
+            ops.dots<float, float, float>(V.p, n, k + 1, vnew, n, 0, SLOT_G);
+            ops.update<float, float, float>(V.p, n, k + 1, 0, vnew, n, SLOT_N, SLOT_G);
+            ops.scale(vnew, n, SLOT_N);
+        }
         P.mv32(vnew, hvnew, s);
         ++mv32;
         // projection column and couplings: V[1..k+1].Hv_new, then c32.v_new, r32.v_new
-        ops.dots<float, float, float>(V.p + n, n, k + 1, hvnew, n, 0);
-        ops.dots<float, float, float>(cr32.p, n, 2, vnew, n, k + 1);
-        const double *h = ops.fetch(SLOT_N + 1);
+        const double *h;
+        if (small) {
+            ClusterLaunch(kDavThreads, 0, s)(k_dav_couple, n, V.p, k, hvnew, cr32.p, cr32.p + n, ops.h_out);
+            h = ops.wait();
+        } else {
+            ops.dots<float, float, float>(V.p + n, n, k + 1, hvnew, n, 0);
+            ops.dots<float, float, float>(cr32.p, n, 2, vnew, n, k + 1);
+            h = ops.fetch(SLOT_N + 1);
+        }
         const double tn2 = h[SLOT_N];
         const double rho_u = (k > 0) ? std::sqrt(h[SLOT_R]) : 1e300;
         if (!(tn2 > 1e-28)) {
