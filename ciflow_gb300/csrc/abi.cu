@@ -840,11 +840,10 @@ int cigpu_ham_create(int L, int nup, int ndown, double econst, const double *h, 
     CIGPU_CUDA(cudaMemcpy(H->d_eri.p, H->eri.data(), L4 * sizeof(double), cudaMemcpyHostToDevice));
     {
         std::vector<float> hi(L4), lo(L4);
-        H->eri_zero = false;
-        for (size_t i = 0; i < L4; ++i) {
-            split_fp32(H->eri[i], hi[i], lo[i]);
-            H->eri_zero |= !(std::fabs(H->eri[i]) > 1e-14);
-        }
+        for (size_t i = 0; i < L4; ++i) split_fp32(H->eri[i], hi[i], lo[i]);
+        int64_t zeros = 0;  // hi is 0 where |v| <= 1e-14
+        for (size_t i = 0; i < L4; ++i) zeros += hi[i] == 0.f;
+        H->eri_zero = zeros > 0;
         H->d_eri_hi.alloc(L4);
         H->d_eri_lo.alloc(L4);
         CIGPU_CUDA(cudaMemcpy(H->d_eri_hi.p, hi.data(), L4 * sizeof(float), cudaMemcpyHostToDevice));

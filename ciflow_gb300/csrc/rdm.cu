@@ -677,13 +677,15 @@ __global__ void k_doci_rdm(const double *__restrict__ c, const uint64_t *__restr
 // sums of squares, per block and per low string. The products and sums are the
 // fixed-point integers above, so the result is the same bit for bit in any order:
 // shared and global integer atomics collect them. Bound by the integer pipe (about 20
-// instructions per product). L=24, 12 pairs: 3.85 -> 0.90 ms per cigpu_rdm,
-// most of the rest the vector's way from host memory.
+// instructions per product). L=24, 12 pairs: 3.80 -> 0.74 ms per cigpu_rdm,
+// the vector's way from host memory among it.
 constexpr int kSplitRdmThreads = 256;
 constexpr int kSplitRdmWarps = kSplitRdmThreads / 32;
-constexpr int kSplitRdmPairs = (kSplitMaxLow * (kSplitMaxLow - 1) / 2 + kSplitRdmWarps - 1) / kSplitRdmWarps;
-constexpr int kSplitRdmLow = 4;  // low strings per thread: C(12, 6) = 924 <= 4 x 256
-constexpr int kSplitRdmRows = 512;  // rows a block aims at (2048: 1.26 ms per call, 512: 0.90)
+// Spaces whose blocks hold at least this many strings on average take it: a block of
+// strings costs a thread block some microseconds whatever its length (L=27, 19 pairs, 76
+// strings a block: 3.72 -> 2.42 ms per call; L=19, 12 pairs, 98: 280 -> 134 us; L=30, 24
+// pairs, 19 strings: 1.44 ms against 2.43; L=30, 5 pairs, 11: 0.49 against 0.83).
+constexpr int64_t kSplitRdmBlock = 40;
 constexpr size_t kSplitRdmMaxSmem = 200 * 1024;
 
 __global__ void k_fix62(const double *__restrict__ c, int64_t n, long long *__restrict__ f) {
@@ -691,18 +693,15 @@ __global__ void k_fix62(const double *__restrict__ c, int64_t n, long long *__re
         f[i] = fx62(c[i]);
 }
 
-__host__ __device__ inline uint32_t split_rdm_group(const DociSector &c) {
-    const uint32_t g = kSplitRdmRows / c.nlow;
-    return g < 1 ? 1u : g > 64 ? 64u : g;
-}
-
 __device__ __forceinline__ long long warp_sum(long long v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
+// A thread block per block of strings (several to one thread block left its last ones, and
+// the sectors of short blocks, to run alone: 0.90 ms at L=24 with a few, 0.74 with one).
 // sums: [2][L][L] (A, then B; j <= k), low: [lowbits] sums of squares per low string.
-__global__ void __launch_bounds__(kSplitRdmThreads, 3) k_doci_rdm_split(const DociSplitView p, uint32_t tasks,
+__global__ void __launch_bounds__(kSplitRdmThreads, 4) k_doci_rdm_split(const DociSplitView p,
                                                                      const long long *__restrict__ cf,
                                                                      long long *__restrict__ sums,
                                                                      long long *__restrict__ low) {
@@ -726,131 +725,96 @@ __global__ void __launch_bounds__(kSplitRdmThreads, 3) k_doci_rdm_split(const Do
     };
     const uint64_t full = (((uint64_t)1) << Lh) - 1;
     const int np = s * (s - 1) / 2;
-    for (uint32_t task = blockIdx.x; task < tasks; task += gridDim.x) {  // one task, up to INT32_MAX
-        uint32_t first = task;
-        int q = 0;
-        for (; q + 1 < p.nsec; ++q) {
-            const uint32_t g = split_rdm_group(p.sec[q]), nt = (p.sec[q].nhigh + g - 1) / g;
-            if (first < nt) break;
-            first -= nt;
-        }
-        const DociSector &c = p.sec[q];
-        const uint32_t group = split_rdm_group(c);
-        const int nh = c.nh, nv = Lh - nh, m = c.m, nhh = nh * nv;
-        const int nlow = (int)c.nlow, nminus = (int)c.nminus, n1 = (int)c.n1, n2 = (int)c.n2;
-        long long *own = area, *sq = own + nlow, *up = sq + nlow;  // [nlow], [nlow], [nv][nminus]
-        uint32_t *hhb = reinterpret_cast<uint32_t *>(up + (size_t)nv * nminus);  // [nhh]
-        uint32_t *upb = hhb + nhh;                                                // [nv]
-        const uint32_t *one = p.one + c.one0, *two = p.two + c.two0;
-        long long acc[kSplitRdmPairs], sqs[kSplitRdmLow];
-#pragma unroll
-        for (int i = 0; i < kSplitRdmPairs; ++i) acc[i] = 0;
-#pragma unroll
-        for (int i = 0; i < kSplitRdmLow; ++i) sqs[i] = 0;
-        const uint32_t h1 = min((first + 1) * group, c.nhigh);
-        for (uint32_t h = first * group; h < h1; ++h) {
-            const uint64_t hb = __ldg(p.hbits + c.high0 + h);
-            const uint32_t base = __ldg(p.hbase + c.high0 + h);
-            __syncthreads();  // the previous block's coefficients and lists are read
-            for (int e = t; e < nhh; e += kSplitRdmThreads) {
-                const int a = e / nv, j = nth(hb, a), k = nth(full & ~hb, e - a * nv);
-                hhb[e] = k > j ? start_of(hb ^ ((uint64_t)1 << j) ^ ((uint64_t)1 << k), m) : 0xFFFFFFFFu;
-            }
-            if (m > 0)
-                for (int r = t; r < nv; r += kSplitRdmThreads)
-                    upb[r] = start_of(hb | ((uint64_t)1 << nth(full & ~hb, r)), m - 1);
-#pragma unroll
-            for (int i = 0; i < kSplitRdmLow; ++i) {
-                const int l = t + i * kSplitRdmThreads;
-                if (l < nlow) {
-                    const long long v = load(base + (uint32_t)l), v2 = fxmul(v, v);
-                    own[l] = v;
-                    sq[l] = v2;
-                    sqs[i] += v2;
-                }
-            }
-            __syncthreads();
-            if (m > 0)
-                for (int r = warp; r < nv; r += kSplitRdmWarps)
-                    for (int l = lane; l < nminus; l += 32) up[(size_t)r * nminus + l] = load(upb[r] + (uint32_t)l);
-            // high - high
-            for (int e = warp; e < nhh; e += kSplitRdmWarps) {
-                const uint32_t b = hhb[e];
-                if (b == 0xFFFFFFFFu) continue;  // k < j: summed from the other side
-                long long a = 0;
+    uint32_t h = blockIdx.x;
+    int q = 0;
+    for (; q + 1 < p.nsec && h >= p.sec[q].nhigh; ++q) h -= p.sec[q].nhigh;
+    const DociSector &c = p.sec[q];
+    const int nh = c.nh, nv = Lh - nh, m = c.m, nhh = nh * nv;
+    const int nlow = (int)c.nlow, nminus = (int)c.nminus, n1 = (int)c.n1, n2 = (int)c.n2;
+    long long *own = area, *sq = own + nlow, *up = sq + nlow;  // [nlow], [nlow], [nv][nminus]
+    uint32_t *hhb = reinterpret_cast<uint32_t *>(up + (size_t)nv * nminus);  // [nhh]
+    uint32_t *upb = hhb + nhh;                                                // [nv]
+    const uint32_t *one = p.one + c.one0, *two = p.two + c.two0;
+    const uint64_t hb = __ldg(p.hbits + c.high0 + h);
+    const uint32_t base = __ldg(p.hbase + c.high0 + h);
+    for (int e = t; e < nhh; e += kSplitRdmThreads) {
+        const int a = e / nv, j = nth(hb, a), k = nth(full & ~hb, e - a * nv);
+        hhb[e] = k > j ? start_of(hb ^ ((uint64_t)1 << j) ^ ((uint64_t)1 << k), m) : 0xFFFFFFFFu;
+    }
+    if (m > 0)
+        for (int r = t; r < nv; r += kSplitRdmThreads)
+            upb[r] = start_of(hb | ((uint64_t)1 << nth(full & ~hb, r)), m - 1);
+    for (int l = t; l < nlow; l += kSplitRdmThreads) {
+        const long long v = load(base + (uint32_t)l), v2 = fxmul(v, v);
+        own[l] = v;
+        sq[l] = v2;
+        add_to(low + c.low0 + l, v2);
+    }
+    __syncthreads();
+    if (m > 0)
+        for (int r = warp; r < nv; r += kSplitRdmWarps)
+            for (int l = lane; l < nminus; l += 32) up[(size_t)r * nminus + l] = load(upb[r] + (uint32_t)l);
+    // high - high
+    for (int e = warp; e < nhh; e += kSplitRdmWarps) {
+        const uint32_t b = hhb[e];
+        if (b == 0xFFFFFFFFu) continue;  // k < j: summed from the other side
+        long long a = 0;
 #pragma unroll 4
-                for (int l = lane; l < nlow; l += 32) a += fxmul(own[l], load(b + (uint32_t)l));
-                a = warp_sum(a);
-                if (lane == 0) {
-                    const int i = e / nv;
-                    add_to(sB + (s + nth(hb, i)) * L + s + nth(full & ~hb, e - i * nv), a);
-                }
-            }
-            // low - low
-            if (n2 > 0) {
-#pragma unroll
-                for (int i = 0; i < kSplitRdmPairs; ++i) {
-                    const int pr = warp + i * kSplitRdmWarps;
-                    if (pr < np) {
-                        const uint32_t *w = two + (size_t)pr * n2;
-#pragma unroll 2
-                        for (int x = lane; x < n2; x += 32) {
-                            const uint32_t e = __ldg(w + x);
-                            acc[i] += fxmul(own[e & 0xFFFFu], own[e >> 16]);
-                        }
-                    }
-                }
-            }
-            // squares: over the block, and over its strings that hold j
-            if (warp == kSplitRdmWarps - 1 && nh > 0) {
-                long long a = 0;
-                for (int l = lane; l < nlow; l += 32) a += sq[l];
-                a = warp_sum(a);
-                for (int e = lane; e < nh * nh; e += 32) {
-                    const int i = e / nh, k = e - i * nh;
-                    if (k >= i) add_to(sA + (s + nth(hb, i)) * L + s + nth(hb, k), a);
-                }
-            }
-            if (m > 0 && nh > 0)
-                for (int j = warp; j < s; j += kSplitRdmWarps) {
-                    long long a = 0;
-                    for (int x = lane; x < n1; x += 32) a += sq[__ldg(one + (size_t)j * n1 + x) & 0xFFFFu];
-                    a = warp_sum(a);
-                    for (int i = lane; i < nh; i += 32) add_to(sA + j * L + s + nth(hb, i), a);
-                }
-            __syncthreads();  // the blocks h + k are staged
-            // low - high
-            if (m > 0)
-                for (int e = warp; e < nv * s; e += kSplitRdmWarps) {
-                    const int r = e / s, j = e - r * s;
-                    const uint32_t *w = one + (size_t)j * n1;
-                    const long long *row = up + (size_t)r * nminus;
-                    long long a = 0;
-#pragma unroll 4
-                    for (int x = lane; x < n1; x += 32) {
-                        const uint32_t v = __ldg(w + x);
-                        a += fxmul(own[v & 0xFFFFu], row[v >> 16]);
-                    }
-                    a = warp_sum(a);
-                    if (lane == 0) add_to(sB + j * L + s + nth(full & ~hb, r), a);
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < kSplitRdmPairs; ++i) {
-            const int pr = warp + i * kSplitRdmWarps;
-            const long long a = warp_sum(acc[i]);
-            if (lane == 0 && pr < np) {
-                int j = 0, rem = pr;
-                while (rem >= s - 1 - j) rem -= s - 1 - j++;
-                add_to(sB + j * L + j + 1 + rem, a);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kSplitRdmLow; ++i) {
-            const int l = t + i * kSplitRdmThreads;
-            if (l < nlow) add_to(low + c.low0 + l, sqs[i]);
+        for (int l = lane; l < nlow; l += 32) a += fxmul(own[l], load(b + (uint32_t)l));
+        a = warp_sum(a);
+        if (lane == 0) {
+            const int i = e / nv;
+            add_to(sB + (s + nth(hb, i)) * L + s + nth(full & ~hb, e - i * nv), a);
         }
     }
+    // low - low
+    if (n2 > 0) {
+        for (int pr = warp, j = 0, k0 = 0; pr < np; pr += kSplitRdmWarps) {  // pair (j, k), row-major, j < k
+            while (pr - k0 >= s - 1 - j) k0 += s - 1 - j++;
+            const uint32_t *w = two + (size_t)pr * n2;
+            long long a = 0;
+#pragma unroll 4
+            for (int x = lane; x < n2; x += 32) {
+                const uint32_t e = __ldg(w + x);
+                a += fxmul(own[e & 0xFFFFu], own[e >> 16]);
+            }
+            a = warp_sum(a);
+            if (lane == 0) add_to(sB + j * L + j + 1 + pr - k0, a);
+        }
+    }
+    // squares: over the block, and over its strings that hold j
+    if (warp == kSplitRdmWarps - 1 && nh > 0) {
+        long long a = 0;
+        for (int l = lane; l < nlow; l += 32) a += sq[l];
+        a = warp_sum(a);
+        for (int e = lane; e < nh * nh; e += 32) {
+            const int i = e / nh, k = e - i * nh;
+            if (k >= i) add_to(sA + (s + nth(hb, i)) * L + s + nth(hb, k), a);
+        }
+    }
+    if (m > 0 && nh > 0)
+        for (int j = warp; j < s; j += kSplitRdmWarps) {
+            long long a = 0;
+            for (int x = lane; x < n1; x += 32) a += sq[__ldg(one + (size_t)j * n1 + x) & 0xFFFFu];
+            a = warp_sum(a);
+            for (int i = lane; i < nh; i += 32) add_to(sA + j * L + s + nth(hb, i), a);
+        }
+    __syncthreads();  // the blocks h + k are staged
+    // low - high
+    if (m > 0)
+        for (int e = warp; e < nv * s; e += kSplitRdmWarps) {
+            const int r = e / s, j = e - r * s;
+            const uint32_t *w = one + (size_t)j * n1;
+            const long long *row = up + (size_t)r * nminus;
+            long long a = 0;
+#pragma unroll 4
+            for (int x = lane; x < n1; x += 32) {
+                const uint32_t v = __ldg(w + x);
+                a += fxmul(own[v & 0xFFFFu], row[v >> 16]);
+            }
+            a = warp_sum(a);
+            if (lane == 0) add_to(sB + j * L + s + nth(full & ~hb, r), a);
+        }
     __syncthreads();
     for (int i = t; i < 2 * L * L; i += kSplitRdmThreads)
         if (sA[i] != 0) add_to(sums + i, sA[i]);
@@ -868,6 +832,13 @@ __global__ void k_doci_rdm_low(const DociSplitView p, uint32_t n, const long lon
         if ((p.lowbits[l] & both) == both) a += low[l];
     a = warp_sum(a);
     if ((threadIdx.x & 31) == 0 && a != 0) add_to(sums + j * p.L + k, a);
+}
+
+// Blocks of strings of the plan.
+uint32_t split_blocks(const DociSplitView &v) {
+    uint32_t n = 0;
+    for (int q = 0; q < v.nsec; ++q) n += v.sec[q].nhigh;
+    return n;
 }
 
 size_t split_rdm_smem(const DociSplitView &v) {
@@ -954,7 +925,10 @@ const DociSplit *doci_split_of(cigpu_crs &c, cudaStream_t s) {
         doci_split_make(c.L, c.nup, c.dim, c.split, s);
         c.split_tried = true;
     }
-    return c.split && split_rdm_smem(c.split.view) <= kSplitRdmMaxSmem ? &c.split : nullptr;
+    return c.split && (int64_t)split_blocks(c.split.view) * kSplitRdmBlock <= c.dim &&
+                   split_rdm_smem(c.split.view) <= kSplitRdmMaxSmem
+               ? &c.split
+               : nullptr;
 }
 
 // Adds the fixed-point sums A, B ([2][L][L], j <= k, zero before) of device vector c:
@@ -975,14 +949,8 @@ void doci_rdm_split(const DociSplit &sp, const double *c_dev, long long *sums, c
     v.err = check_word_device();
     DevBuf<long long> fixed((size_t)v.D), low(sp.nlowbits);
     CIGPU_CUDA(cudaMemsetAsync(low.p, 0, low.bytes(), s));
-    uint64_t tasks = 0;
-    for (int q = 0; q < v.nsec; ++q) {
-        const uint32_t g = split_rdm_group(v.sec[q]);
-        tasks += (v.sec[q].nhigh + g - 1) / g;
-    }
-    const int blocks = (int)std::min<uint64_t>(tasks, (uint64_t)INT32_MAX);
     k_fix62<<<sm_count() * 8, 256, 0, s>>>(c_dev, v.D, fixed.p);
-    k_doci_rdm_split<<<blocks, kSplitRdmThreads, split_rdm_smem(v), s>>>(v, (uint32_t)tasks, fixed.p, sums, low.p);
+    k_doci_rdm_split<<<split_blocks(v), kSplitRdmThreads, split_rdm_smem(v), s>>>(v, fixed.p, sums, low.p);
     k_doci_rdm_low<<<v.s * v.s, 256, 0, s>>>(v, sp.nlowbits, low.p, sums);
     CIGPU_CUDA(cudaGetLastError());
     count_launch(3);

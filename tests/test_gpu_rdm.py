@@ -123,7 +123,7 @@ def test_python_facade_density():
     assert d.get_two_rdm(0, 2, 2, 3, 4) == 0.0
 
 
-@pytest.mark.parametrize("L,n", [(17, 8), (18, 11), (21, 5), (22, 17)])
+@pytest.mark.parametrize("L,n", [(17, 8), (18, 11), (20, 13), (21, 5), (22, 17)])
 def test_doci_rdm_split(L, n):
     """The DOCI RDMs by low and high orbitals (spaces past the split's row threshold),
     from a mixed matrix and from a plain one (which makes its plan on the first call):
