@@ -333,17 +333,23 @@ __global__ void __launch_bounds__(kRdmThreads) k_pair_dens(const double *__restr
     }
 }
 
-// Step 2: per-slot ordered sums of +/- densities.
+// Step 2: per-slot sums of +/- densities, a warp per slot (lanes over the terms, then the
+// warp tree: a fixed order). A thread per slot took 79 us for the 243,000 terms of L=12
+// 6a6b, the longest lists one after the other: 60 us more per call.
 __global__ void k_slot_gather(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ idx,
                               const int8_t *__restrict__ coef, const double *__restrict__ dens, int64_t nslots,
                               double *__restrict__ acc, int64_t ndens, unsigned long long *err) {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < nslots; s += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < nslots; s += nw) {
         double v = 0;
-        for (uint32_t e = ptr[s]; e < ptr[s + 1]; ++e) {
+        for (uint32_t e = ptr[s] + lane; e < ptr[s + 1]; e += 32) {
             const uint32_t k = idx[e];
-            if (CIGPU_CHECK(err, index_ok(k, (uint64_t)ndens), kCheckRdmTerm, e)) v += (double)coef[e] * dens[k];
+            if (!CIGPU_CHECK(err, index_ok(k, (uint64_t)ndens), kCheckRdmTerm, e)) continue;
+            v += __longlong_as_double(__double_as_longlong(dens[k]) ^ ((long long)(coef[e] < 0) << 63));
         }
-        acc[s] = v;
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) acc[s] = v;
     }
 }
 
@@ -354,15 +360,19 @@ __global__ void k_slot_gather(const uint32_t *__restrict__ ptr, const uint32_t *
 // stored once, G[q - q0][x][S] (x = ns: the identity). A multiply-add per term and its
 // gather from shared memory: bound by the FP64 pipe, 0.57 G multiply-adds at L=12 6a6b,
 // 0.90 ms at its rate. (One thread per (br, bc) walking lists of string pairs, the
-// sign a second FP64 product, on 264 blocks of 160 threads: 4.36 ms. Now 1.39.)
+// sign a second FP64 product, on 264 blocks of 160 threads: 4.36 ms. Now 1.25.)
 constexpr int kAbThreads = 128;
-constexpr int kAbX = 12;
+// Excitations per thread: 36 where the strings alone make three blocks per SM (L=12 6a6b:
+// each row staged once, 1.25 against 1.39 ms), else 12, whose chunks make up to three
+// times as many blocks (L=10 5a5b would have 110).
+constexpr int kAbWide = 36, kAbNarrow = 12;
 
 __device__ __forceinline__ void copy8_async(double *dst, const double *src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
 }
 
+template <int kAbX>
 __global__ void __launch_bounds__(kAbThreads) k_string_sums(const double *__restrict__ C, int64_t D2,
                                                             const uint32_t *__restrict__ target, int ns,
                                                             const uint32_t *__restrict__ ptr,
@@ -1106,15 +1116,18 @@ void crs_rdm(cigpu_crs &c, const double *c_dev, double *rdm1, double *aa, double
         };
         const int nsb = tb.ns;
         batches(np, (size_t)(nsb + 1) * tb.D, [&](double *g, int q0, int nq) {
-            // one fixed limit, set once: concurrent callers (server workers) must never lower it
-            static const cudaError_t attr =
-                cudaFuncSetAttribute(k_string_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            CIGPU_CUDA(attr);
             const int64_t per = (int64_t)(nsb + 1) * tb.D;
-            const dim3 grid((unsigned)((tb.D + kAbThreads - 1) / kAbThreads),
-                            (unsigned)std::max(1, (nsb + kAbX - 1) / kAbX), (unsigned)nq);
-            k_string_sums<<<grid, kAbThreads, sm, s>>>(c_dev, tb.D, c.fp.b.s_target, nsb, R.ap.p, R.apair.p, R.asign.p, q0,
-                                                       g, ta.D, ew);
+            const unsigned tiles = (unsigned)((tb.D + kAbThreads - 1) / kAbThreads);
+            auto go = [&](auto kern, int x) {
+                // one fixed limit: concurrent callers (server workers) never lower it
+                CIGPU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+                kern<<<dim3(tiles, (unsigned)std::max(1, (nsb + x - 1) / x), (unsigned)nq), kAbThreads, sm, s>>>(
+                    c_dev, tb.D, c.fp.b.s_target, nsb, R.ap.p, R.apair.p, R.asign.p, q0, g, ta.D, ew);
+            };
+            if ((int64_t)tiles * nq >= 3 * (int64_t)sm_count())
+                go(k_string_sums<kAbWide>, kAbWide);
+            else
+                go(k_string_sums<kAbNarrow>, kAbNarrow);
             k_sum_strings<<<(unsigned)((nq * L2 + 3) / 4), 128, 0, s>>>(g, per, R.btp.p, R.bta.p, (int)L2, nq,
                                                                         t1.p + (int64_t)q0 * L2, ew);
             count_launch(2);

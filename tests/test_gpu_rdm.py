@@ -74,6 +74,16 @@ def test_fci_rdm_facade_and_unequal_spins():
     assert_rdm_close(got, ref, 1e-13)
 
 
+@pytest.mark.parametrize("L,na,nb", [(12, 1, 6), (13, 2, 6), (13, 2, 7)])
+def test_fci_rdm_many_beta_strings(L, na, nb):
+    # enough blocks for 36 excitations per thread: one whole set, and a ragged second one
+    ints = make_integrals(L, na, nb, nchol=4, seed=3)
+    cim = FCI(Hamiltonian.from_integrals(ints))
+    c = np.random.default_rng(L + nb).standard_normal(cim.get_dim())
+    c /= np.linalg.norm(c)
+    assert_rdm_close(rdm_via_abi(cim, c), O.rdm(O.FCI, L, na, nb, c), 1e-13)
+
+
 def test_c1_rdm_against_oracle():
     ints = integrals("c1")
     cim = FCI(Hamiltonian.from_integrals(ints), precision=A.MIXED)
