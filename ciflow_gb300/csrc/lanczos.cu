@@ -201,18 +201,31 @@ __global__ void __launch_bounds__(kVecThreads) k_multidot(const VT *__restrict__
     reduce_chunk_in_last_block(partial + (int64_t)v0 * G, nv, out + v0, tickets + blockIdx.y);
 }
 
+// Other vectors' dots (at most kDotChunk) taken by one more row of blocks, stored behind
+// the first ones.
+struct DotTail {
+    const float4 *V;
+    int nvec;
+    const float4 *w;
+};
+
 // The FP32 dots of k_multidot<float, float, float> with 16-byte loads: V rows and w
 // as float4 (a length divisible by 4, rows 16-byte aligned), four elements per
-// thread and step (at most 64 registers: the grid is four blocks per SM).
+// thread and step (at most 64 registers: the grid is four blocks per SM, all chunks').
+// Bound by L2 and HBM: between the products the basis (100 MB at L=12) shares the L2 with
+// the sigma product's sums.
 __global__ void __launch_bounds__(kVecThreads, 4) k_multidot_f4(const float4 *__restrict__ V, int64_t ld4, int nvec,
                                                              const float4 *__restrict__ w, int64_t n4,
                                                              double *__restrict__ partial, double *__restrict__ out,
                                                              unsigned *__restrict__ tickets,
-                                                             const double *__restrict__ skip) {
+                                                             const double *__restrict__ skip, const DotTail tail) {
     if (skip && *skip != 0.0) return;  // a second orthogonalisation pass that the first made unnecessary
     const int G = gridDim.x;
-    const int v0 = blockIdx.y * kDotChunk;
-    const int nv = min(kDotChunk, nvec - v0);
+    const int row = blockIdx.y * kDotChunk;  // of the chunk's partial sums
+    const bool last = tail.nvec > 0 && blockIdx.y == gridDim.y - 1;
+    const int nv = last ? tail.nvec : min(kDotChunk, nvec - row);
+    V = last ? tail.V : V + row * ld4;
+    w = last ? tail.w : w;
     float acc[kDotChunk];
 #pragma unroll
     for (int i = 0; i < kDotChunk; ++i) acc[i] = 0.f;
@@ -221,7 +234,7 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_multidot_f4(const float4 *__
         float4 va[kDotChunk];
 #pragma unroll
         for (int i = 0; i < kDotChunk; ++i)
-            if (i < nv) va[i] = V[(int64_t)(v0 + i) * ld4 + r];
+            if (i < nv) va[i] = V[i * ld4 + r];
 #pragma unroll
         for (int i = 0; i < kDotChunk; ++i)
             if (i < nv) acc[i] += (va[i].x * wr.x + va[i].y * wr.y) + (va[i].z * wr.z + va[i].w * wr.w);
@@ -234,9 +247,9 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_multidot_f4(const float4 *__
     if (threadIdx.x < nv) {
         double t = 0;
         for (int k = 0; k < kVecThreads / 32; ++k) t += sh[threadIdx.x][k];
-        partial[(int64_t)(v0 + threadIdx.x) * G + blockIdx.x] = t;
+        partial[(int64_t)(row + threadIdx.x) * G + blockIdx.x] = t;
     }
-    reduce_chunk_in_last_block(partial + (int64_t)v0 * G, nv, out + v0, tickets + blockIdx.y);
+    reduce_chunk_in_last_block(partial + (int64_t)row * G, nv, out + (last ? nvec : row), tickets + blockIdx.y);
 }
 
 // k_update<float, float, float> with 16-byte loads (the same per-element order of
@@ -441,16 +454,16 @@ __global__ void __launch_bounds__(kVecThreads) k_dav_residual32_f4(const float4 
         float4 ru = make_float4(fa0 * rr.x + fa0de * cc.x, fa0 * rr.y + fa0de * cc.y, fa0 * rr.z + fa0de * cc.z,
                                 fa0 * rr.w + fa0de * cc.w);
         int i = 0;
-        for (; i + 2 <= k; i += 2) {  // four 16-byte loads in flight, terms added in order
-            float4 hv[2], vv[2];
+        for (; i + 4 <= k; i += 4) {  // eight 16-byte loads in flight, terms added in order
+            float4 hv[4], vv[4];
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
+            for (int q = 0; q < 4; ++q) {
                 const int64_t o = (int64_t)(i + q + 1) * ld4 + r;  // corrections live in slots 1..k
                 hv[q] = HV[o];
                 vv[q] = V[o];
             }
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
+            for (int q = 0; q < 4; ++q) {
                 const float yq = ys[i + q];
                 ru.x += yq * (hv[q].x - fth * vv[q].x);
                 ru.y += yq * (hv[q].y - fth * vv[q].y);
@@ -1036,20 +1049,33 @@ struct VecOps {
     }
     // out[dst .. dst+nvec) = V_i . w   (AT: arithmetic type of the products)
     // skip_at >= 0: the kernel does nothing when out[skip_at] != 0
+    // V2 . w2 (nvec2 vectors of the same pitch, FP32) follow in out[dst + nvec ..)
     template <typename VT, typename WT, typename AT = double>
-    void dots(const VT *V, int64_t ld, int nvec, const WT *w, int64_t n, int dst, int skip_at = -1) {
+    void dots(const VT *V, int64_t ld, int nvec, const WT *w, int64_t n, int dst, int skip_at = -1,
+              const VT *V2 = nullptr, int nvec2 = 0, const WT *w2 = nullptr) {
         dim3 grid(Gd, (nvec + kDotChunk - 1) / kDotChunk);
         if constexpr (std::is_same<VT, float>::value && std::is_same<WT, float>::value &&
                       std::is_same<AT, float>::value) {
-            if (vec4_ok(V, ld, n) && vec4_ok(w, 0, n)) {
-                k_multidot_f4<<<grid, kVecThreads, 0, s>>>(reinterpret_cast<const float4 *>(V), ld / 4, nvec,
-                                                           reinterpret_cast<const float4 *>(w), n / 4, partial.p,
-                                                           out.p + dst, ticket.p,
-                                                           skip_at >= 0 ? out.p + skip_at : nullptr);
+            const bool tail = nvec2 > 0 && nvec2 <= kDotChunk && (int)grid.y < kTickets && vec4_ok(V2, ld, n) && vec4_ok(w2, 0, n);
+            if (vec4_ok(V, ld, n) && vec4_ok(w, 0, n) && (nvec2 == 0 || tail)) {
+                using F4 = const float4 *;
+                grid.y += tail;
+                // all chunks' blocks resident at once, several elements per thread: a block's
+                // reduction costs as much as an element's loads (L=12 6a6b, 15 vectors: 22 us
+                // with four waves of blocks, one element per thread)
+                grid.x = std::min<unsigned>(grid.x, ((unsigned)sm_count() * 4 + grid.y - 1) / grid.y);
+                k_multidot_f4<<<grid, kVecThreads, 0, s>>>(F4(V), ld / 4, nvec, F4(w), n / 4, partial.p, out.p + dst, ticket.p,
+                                                           skip_at >= 0 ? out.p + skip_at : nullptr,
+                                                           DotTail{F4(V2), nvec2, F4(w2)});
                 CIGPU_CUDA(cudaGetLastError());
                 count_launch();
                 return;
             }
+        }
+        if (nvec2 > 0) {
+            dots<VT, WT, AT>(V, ld, nvec, w, n, dst, skip_at);
+            dots<VT, WT, AT>(V2, ld, nvec2, w2, n, dst + nvec, skip_at);
+            return;
         }
         k_multidot<VT, WT, AT><<<grid, kVecThreads, 0, s>>>(V, ld, nvec, w, n, partial.p, out.p + dst, ticket.p,
                                                             skip_at >= 0 ? out.p + skip_at : nullptr);
@@ -1687,8 +1713,7 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
             ClusterLaunch(kDavThreads, 0, s)(k_dav_couple, n, V.p, k, hvnew, cr32.p, cr32.p + n, ops.h_out);
             h = ops.wait();
         } else {
-            ops.dots<float, float, float>(V.p + n, n, k + 1, hvnew, n, 0);
-            ops.dots<float, float, float>(cr32.p, n, 2, vnew, n, k + 1);
+            ops.dots<float, float, float>(V.p + n, n, k + 1, hvnew, n, 0, -1, cr32.p, 2, vnew);
             h = ops.fetch(SLOT_N + 1);
         }
         const double tn2 = h[SLOT_N];
