@@ -184,6 +184,25 @@ def test_compact_fp64_tiles_equal_full_tiles(L, nup, ndown, monkeypatch):
         np.testing.assert_array_equal(col, ref.col)
 
 
+@pytest.mark.parametrize("L,nup,ndown", [(7, 3, 3), (6, 2, 3), (7, 2, 1), (5, 4, 1), (6, 1, 5), (23, 1, 1), (0, 0, 0)])
+def test_full_fp64_tiles_of_small_spaces(L, nup, ndown, monkeypatch):
+    """The full tiles' fill walks the alpha singles with four beta singles at hand: 12, 9
+    (odd), 6 and 4 beta singles, a last quad that is not full, more orbital pairs than the
+    counts have room for (23 orbitals: the walk by slots), and a molecule with vanishing
+    integrals (0: BeH2). Against the plain build's rows."""
+    ints = make_integrals(L, nup, ndown, nchol=6, seed=L + nup) if L else beh2_integrals()[0]
+    monkeypatch.setenv("CIGPU_FP32_PRODUCT", "sigma")
+    monkeypatch.setenv("CIGPU_SLOTS64", "full")
+    full = build(FCI, ints, precision=A.MIXED).get_mat()
+    plain = build(FCI, ints).get_mat()
+    assert (full.nnz_upper, full.nnz_full) == (plain.nnz_upper, plain.nnz_full)
+    x = np.random.default_rng(1).standard_normal(full.n)
+    y, ref = full.mvprod(x), plain.mvprod(x)
+    assert np.abs(y - ref).max() <= 1e-12 * np.abs(ref).max()
+    for a, b in zip(full.full(), plain.full()):  # a mixed matrix exports FP32 values
+        np.testing.assert_array_equal(a, b.astype(np.float32) if b.dtype == np.float64 else b)
+
+
 def test_symmetry_zeros_dropped_like_reference():
     # BeH2 in D2h: many elements are exactly zero and must be dropped (|v| <= 1e-14)
     ints, meta, _ = beh2_integrals()
