@@ -32,6 +32,8 @@
 #include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "crs.cuh"
 #include "spmv.cuh"
 
@@ -911,7 +913,11 @@ __global__ void __launch_bounds__(32, 32) k_dets_pairs(const DetParams p) {
 // 0.48.)
 //
 // RANGED: a list with a stored block (CI_Big with a kept part) leaves out the block's
-// pairs.
+// pairs. CL: the blocks (a cluster) that share 32 rows' columns. Two where one would leave
+// the SMs fewer than four, three of which an SM holds at a time. One | two, alone and among
+// other products: 6,189 rows of L=24 254 | 138 and 100 | 76 us, 16,471 of L=24 956 | 536
+// alone, 12,290 of L=28 453 | 262 and 182 | 173, 21,507 853 | 613 and 492 | 505, 52,705 of
+// L=32 2.89 | 3.43 ms; four or eight were slower among others everywhere.
 constexpr int kMvWarps = 8;
 constexpr int kMvSpan = 16;
 
@@ -982,15 +988,16 @@ __device__ __noinline__ double matvec_flush(const DetParams &p, MatvecWarp<W, NW
     return acc;
 }
 
-template <int W, int NW, bool RANGED>
-__global__ void __launch_bounds__(32 * kMvWarps, 3) k_dets_matvec(const DetParams p, const double *__restrict__ x,
+template <int W, int NW, bool RANGED, int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * kMvWarps, 3) k_dets_matvec(const DetParams p, const double *__restrict__ x,
                                                                   double *__restrict__ y) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ScanRow<W> rows;
     __shared__ double part[kMvWarps][kScanRows];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x % CL;  // of the rows' blocks
     MatvecWarp<W, NW> &q = reinterpret_cast<MatvecWarp<W, NW> *>(smem)[warp];
-    const int64_t r0 = (int64_t)blockIdx.x * kScanRows, i = r0 + lane;
+    const int64_t r0 = (int64_t)(blockIdx.x / CL) * kScanRows, i = r0 + lane;
     const bool active = i < p.n;
     uint64_t rec[2 * W];
 #pragma unroll
@@ -1024,15 +1031,15 @@ __global__ void __launch_bounds__(32 * kMvWarps, 3) k_dets_matvec(const DetParam
         n += total;
         mine += __popc(m);
     };
-    load(warp);
-    for (int64_t word = warp; word < words; word += kMvWarps) {
+    load(rank * kMvWarps + warp);
+    for (int64_t word = rank * kMvWarps + warp; word < words; word += CL * kMvWarps) {
         const int64_t base = c_lo + word * 32;
         uint32_t ck[NW];
         scan_key<W, NW>(next, ck);
 #pragma unroll
         for (int w = 0; w < NW; ++w) q.key[lane * NW + w] = ck[w];
         __syncwarp();
-        load(word + kMvWarps);
+        load(word + CL * kMvWarps);
         uint32_t m = scan_word<NW>(q.key, rk, one);
         if (p.n - base < 32) m &= (1u << (int)(p.n - base)) - 1u;
         if (!active) m = 0;
@@ -1054,22 +1061,27 @@ __global__ void __launch_bounds__(32 * kMvWarps, 3) k_dets_matvec(const DetParam
     }
     if (n > 0) flush();
     part[warp][lane] = acc;
-    __syncthreads();
-    if (warp == 0 && active) {
+    auto cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    if (rank == 0 && warp == 0 && active) {
         double a = 0;
-        for (int w = 0; w < kMvWarps; ++w) a += part[w][lane];
+        for (int b = 0; b < CL; ++b) {
+            const double *sums = cluster.map_shared_rank(&part[0][0], b);
+            for (int w = 0; w < kMvWarps; ++w) a += sums[w * kScanRows + lane];
+        }
         // rows of the stored block add to the stored block's product, already in y
         y[i] = ((RANGED && i < p.block) ? y[i] : 0.0) + a;
     }
+    cluster.sync();  // the sums are read
 }
 
 // The same for short lists: a warp owns one row and its lanes test 32 columns at a time, so
 // that a few thousand rows make enough warps; the pairs found are queued and evaluated 32
 // at a time, and every 32nd of them is added by one lane. Half the pairs per instruction of
 // the kernel above, whose 32 rows to a warp leave a short list's blocks too few. Alone,
-// and among other products, this | that: 1,577 rows of L=36 44 | 199 and 17 | 70 us; 5,665
-// of L=20 133 | 491 and 107 | 173; 6,189 of L=24 236 | 253 and 129 | 98; 12,290 of L=28
-// 623 | 428 and 400 | 181.
+// and among other products, this | that: 1,577 rows of L=36 44 | 126 and 17 | 46 us; 5,665
+// of L=20 133 | 280 and 107 | 123; 6,189 of L=24 236 | 138 and 129 | 76; 12,290 of L=28
+// 623 | 262 and 400 | 173.
 constexpr int64_t kMvShort = 6000;
 
 template <int W>
@@ -1210,17 +1222,22 @@ void matvec(const DetParams &p, int W, const double *x, double *y, cudaStream_t 
                 k_dets_matvec_rows<w(), nw(), false><<<blocks, 32 * kMvWarps, 0, s>>>(p, x, y);
             return;
         }
-        const unsigned blocks = (unsigned)((p.n + kScanRows - 1) / kScanRows);
+        const unsigned groups = (unsigned)((p.n + kScanRows - 1) / kScanRows);
         constexpr int smem = (int)sizeof(MatvecWarp<w(), nw()>) * kMvWarps;
-        auto go = [&](auto kern) {
+        auto go = [&](auto kern, unsigned blocks) {
             // the same value at every call: concurrent callers never lower it
             CIGPU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             kern<<<blocks, 32 * kMvWarps, smem, s>>>(p, x, y);
         };
-        if (ranged)
-            go(k_dets_matvec<w(), nw(), true>);
+        const bool two = groups < 4 * (unsigned)sm_count();
+        if (ranged && two)
+            go(k_dets_matvec<w(), nw(), true, 2>, 2 * groups);
+        else if (ranged)
+            go(k_dets_matvec<w(), nw(), true, 1>, groups);
+        else if (two)
+            go(k_dets_matvec<w(), nw(), false, 2>, 2 * groups);
         else
-            go(k_dets_matvec<w(), nw(), false>);
+            go(k_dets_matvec<w(), nw(), false, 1>, groups);
     });
     CIGPU_CUDA(cudaGetLastError());
     count_launch();

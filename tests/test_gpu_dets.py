@@ -245,7 +245,8 @@ def test_dropped_elements(kind, precision):
         assert np.array_equal(val, m.val.astype(np.float32).astype(np.float64))
 
 
-@pytest.mark.parametrize("L,na,nb,n,repeat", [(14, 3, 3, 6100, 1), (36, 4, 3, 6001, 1), (40, 1, 1, 1600, 5)])
+@pytest.mark.parametrize("L,na,nb,n,repeat", [(14, 3, 3, 6100, 1), (36, 4, 3, 6001, 1), (40, 1, 1, 1600, 5),
+                                              (28, 4, 3, 19500, 1)])
 def test_matvec_of_a_longer_list(L, na, nb, n, repeat):
     """The matvec without a stored matrix past the short lists' kernel: 32 and 64-bit
     strings, and a list of repeated determinants whose pairs are all connected (words that
