@@ -424,9 +424,9 @@ __global__ void __launch_bounds__(kSlotThreads, 3) k_spmv_slots_fly(const FciPar
 // lower-triangle count.
 // FP64, slices staged and at most 512 orbital pairs (their counts take the place of the
 // sums): the alpha-single x beta-single block, two thirds of the slots, is walked with four
-// beta singles at hand and written 32 bytes at a time. L=12 6a6b, whole build 8.27 -> 7.26 ms
-// (13 GB written, 1.9 ms at the copy rate); the waits left are for the singles' and doubles'
-// values.
+// beta singles at hand and written 32 bytes at a time (L=12 6a6b, whole build 8.27 -> 7.26
+// ms), and the other slots' values are read a quad ahead (7.35 -> 6.97; 13 GB written, 1.9 ms
+// at the copy rate).
 template <bool F64>
 struct FillVals;
 template <>
@@ -558,9 +558,8 @@ __global__ void __launch_bounds__(kSlotThreads) k_fill_slots(const FciParams p, 
     const int64_t r = ia * p.Db + ib;
     const bool fly = F64 && p.fly;
     const int Qs = fly ? m.s4 >> 2 : Q;  // stored quads per row
-    const int Qr = wide ? m.s4 >> 2 : Q;  // quads shared out here
-    const int c0 = (int)((int64_t)Qr * ks / kSplits), c1 = (int)((int64_t)Qr * (ks + 1) / kSplits);
-    const int cs = min(c1, Qs);
+    const int c0 = (int)((int64_t)Q * ks / kSplits), c1 = (int)((int64_t)Q * (ks + 1) / kSplits);
+    const int cs = wide ? 0 : min(c1, Qs);
     const int64_t qbase = (ia * T + t) * (int64_t)Qs;
     const int nsb = p.b.ns, ndb = p.b.nd, nda = p.a.nd, nsr = nsa + nsb, L = p.L;
     uint32_t n_keep = 0, n_low = 0;
@@ -681,6 +680,62 @@ __global__ void __launch_bounds__(kSlotThreads) k_fill_slots(const FciParams p, 
         }
     if constexpr (F64) {
         if (wide) {
+            // S0 to S3: the values of a quad and the columns they stand in, read a step ahead
+            struct Quad {
+                uint64_t v[4];
+                uint32_t col[4];
+            };
+            const int e1 = (int)((int64_t)(m.s4 >> 2) * (ks + 1) / kSplits);
+            auto fetch = [&](int c, Quad &q) {
+                const int k0 = 4 * c;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    q.v[j] = 0;
+                    q.col[j] = 0xFFFFFFFFu;
+                }
+                auto take = [&](int j, const double *at, uint32_t col) {
+                    q.v[j] = (uint64_t)__double_as_longlong(__ldg(at));
+                    q.col[j] = col;
+                };
+                if (k0 < m.s1) {  // the diagonal
+                    take(0, p.diag + r, 0xFFFFFFFFu);
+                } else if (k0 < m.s2) {  // beta singles
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int x = k0 - m.s1 + j;
+                        if (x < nsb) take(j, p.sgl64 + (size_t)r * nsr + nsa + x, st[x * kTileRows + rr]);
+                    }
+                } else if (k0 < m.s3) {  // beta-beta doubles
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int x = k0 - m.s2 + j;
+                        if (x < ndb) take(j, p.b.d_val + ib * ndb + x, __ldg(p.b.d_target + ib * ndb + x));
+                    }
+                } else {  // alpha singles, alpha-alpha doubles
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int x = k0 - m.s3 + j;
+                        if (x < nsa) take(j, p.sgl64 + (size_t)r * nsr + x, (uint32_t)desc[k0 + j]);
+                        else if (x < nsa + nda) take(j, p.a.d_val + ia * nda + (x - nsa), (uint32_t)desc[k0 + j]);
+                    }
+                }
+            };
+            Quad next;
+            int c = (int)((int64_t)(m.s4 >> 2) * ks / kSplits);
+            if (c < e1) fetch(c, next);
+            for (; c < e1; ++c) {
+                Quad q = next;
+                if (c + 1 < e1) fetch(c + 1, next);
+                const uint32_t here = 4 * c < m.s3 ? (uint32_t)ib : (uint32_t)ia;  // columns below it: the lower triangle
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const bool keep = active && above_drop(q.v[j]);
+                    if (!keep) q.v[j] = 0;
+                    n_keep += keep;
+                    n_low += keep && q.col[j] < here;
+                }
+                store_quad(v64 + ((qbase + c) * kTileRows + rr) * 4, q.v);
+            }
             // S4 slot i of a row is alpha single i / nsb, beta single i % nsb: quads P apart
             // hold the same four beta singles, A alpha singles on, so a thread takes a
             // quad's four pairs of orbitals once and walks the alpha singles
