@@ -584,6 +584,25 @@ __device__ __forceinline__ long long fxmul(long long a, long long b) {
     return hi + (long long)(lo >> 63);
 }
 
+// A fixed-point value as two signed 32-bit digits, hi 2^32 + lo: the four products of a
+// multiplication are then signed 32 x 32 -> 64 bit, with no corrections.
+__device__ __forceinline__ long long fxdigits(long long a) {
+    const uint32_t lo = (uint32_t)a, hi = (uint32_t)((unsigned long long)a >> 32) + (lo >> 31);
+    return (long long)((unsigned long long)hi << 32 | lo);
+}
+
+// sum += fxmul(a, b) of two values in digits: of a b = hh 2^64 + mid 2^32 + ll, rounded to
+// nearest at 2^64, the low half of ll changes nothing.
+__device__ __forceinline__ void fxadd(long long &sum, long long a, long long b) {
+    const int ah = (int)(a >> 32), al = (int)a, bh = (int)(b >> 32), bl = (int)b;
+    const long long ll = (long long)al * bl;  // within +-2^62
+    long long mid = (long long)((uint32_t)(ll >> 32) + 0x80000000u);
+    mid += (long long)ah * bl;
+    mid += (long long)al * bh;
+    sum += (long long)ah * bh;
+    sum += mid >> 32;
+}
+
 __device__ __forceinline__ void add_to(long long *at, long long v) {
     atomicAdd(reinterpret_cast<unsigned long long *>(at), (unsigned long long)v);
 }
@@ -686,21 +705,23 @@ __global__ void k_doci_rdm(const double *__restrict__ c, const uint64_t *__restr
 // four strings to act on, and formed a rank for each), and A needs only the blocks'
 // sums of squares, per block and per low string. The products and sums are the
 // fixed-point integers above, so the result is the same bit for bit in any order:
-// shared and global integer atomics collect them. Bound by the integer pipe (about 20
-// instructions per product). L=24, 12 pairs: 3.80 -> 0.74 ms per cigpu_rdm,
-// the vector's way from host memory among it.
+// shared and global integer atomics collect them. Bound by instruction issue (49 for 32
+// products, ALU 41%) and, at three blocks per SM, the barriers around the staging. L=24,
+// 12 pairs: 3.80 -> 0.74 ms per cigpu_rdm with a sum at a time for every warp, 0.66 with
+// four and in digits (the kernel 490 -> 423 us; the vector's way from host memory is 150).
 constexpr int kSplitRdmThreads = 256;
 constexpr int kSplitRdmWarps = kSplitRdmThreads / 32;
 // Spaces whose blocks hold at least this many strings on average take it: a block of
 // strings costs a thread block some microseconds whatever its length (L=27, 19 pairs, 76
-// strings a block: 3.72 -> 2.42 ms per call; L=19, 12 pairs, 98: 280 -> 134 us; L=30, 24
-// pairs, 19 strings: 1.44 ms against 2.43; L=30, 5 pairs, 11: 0.49 against 0.83).
+// strings a block: 3.72 -> 1.40 ms per call; L=19, 12 pairs, 98: 280 -> 121 us; L=30, 24
+// pairs, 19 strings: 1.44 ms against 2.43 when the split took 2.42 and 134 in those; L=30, 5
+// pairs, 11: 0.49 against 0.83).
 constexpr int64_t kSplitRdmBlock = 40;
 constexpr size_t kSplitRdmMaxSmem = 200 * 1024;
 
 __global__ void k_fix62(const double *__restrict__ c, int64_t n, long long *__restrict__ f) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        f[i] = fx62(c[i]);
+        f[i] = fxdigits(fx62(c[i]));
 }
 
 __device__ __forceinline__ long long warp_sum(long long v) {
@@ -708,8 +729,19 @@ __device__ __forceinline__ long long warp_sum(long long v) {
     return v;
 }
 
+// The sums over the warp of four values per lane, by exchange of halves: lane's is that of
+// a[lane >> 3].
+__device__ __forceinline__ long long sum_four(const long long (&a)[4], int lane) {
+    const bool h = lane & 16, q = lane & 8;
+    const long long b0 = (h ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, h ? a[0] : a[2], 16);
+    const long long b1 = (h ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, h ? a[1] : a[3], 16);
+    long long v = (q ? b1 : b0) + __shfl_xor_sync(0xffffffffu, q ? b0 : b1, 8);
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // A thread block per block of strings (several to one thread block left its last ones, and
-// the sectors of short blocks, to run alone: 0.90 ms at L=24 with a few, 0.74 with one).
+// the sectors of short blocks, to run alone: 0.90 ms per call at L=24 with a few, 0.74 with one).
 // sums: [2][L][L] (A, then B; j <= k), low: [lowbits] sums of squares per low string.
 __global__ void __launch_bounds__(kSplitRdmThreads, 4) k_doci_rdm_split(const DociSplitView p,
                                                                      const long long *__restrict__ cf,
@@ -743,19 +775,28 @@ __global__ void __launch_bounds__(kSplitRdmThreads, 4) k_doci_rdm_split(const Do
     const int nlow = (int)c.nlow, nminus = (int)c.nminus, n1 = (int)c.n1, n2 = (int)c.n2;
     long long *own = area, *sq = own + nlow, *up = sq + nlow;  // [nlow], [nlow], [nv][nminus]
     uint32_t *hhb = reinterpret_cast<uint32_t *>(up + (size_t)nv * nminus);  // [nhh]
-    uint32_t *upb = hhb + nhh;                                                // [nv]
+    uint32_t *hhe = hhb + nhh;                                                // [nhh]
+    uint32_t *upb = hhe + nhh;                                                // [nv]
     const uint32_t *one = p.one + c.one0, *two = p.two + c.two0;
     const uint64_t hb = __ldg(p.hbits + c.high0 + h);
     const uint32_t base = __ldg(p.hbase + c.high0 + h);
+    __shared__ int nhop, job;
+    if (t == 0) nhop = job = 0;
+    __syncthreads();
     for (int e = t; e < nhh; e += kSplitRdmThreads) {
         const int a = e / nv, j = nth(hb, a), k = nth(full & ~hb, e - a * nv);
-        hhb[e] = k > j ? start_of(hb ^ ((uint64_t)1 << j) ^ ((uint64_t)1 << k), m) : 0xFFFFFFFFu;
+        if (k < j) continue;  // summed from the other side
+        const int at = atomicAdd(&nhop, 1);  // in any order
+        hhb[at] = start_of(hb ^ ((uint64_t)1 << j) ^ ((uint64_t)1 << k), m);
+        hhe[at] = (uint32_t)(j * L + k);
     }
     if (m > 0)
         for (int r = t; r < nv; r += kSplitRdmThreads)
             upb[r] = start_of(hb | ((uint64_t)1 << nth(full & ~hb, r)), m - 1);
     for (int l = t; l < nlow; l += kSplitRdmThreads) {
-        const long long v = load(base + (uint32_t)l), v2 = fxmul(v, v);
+        const long long v = load(base + (uint32_t)l);
+        long long v2 = 0;
+        fxadd(v2, v, v);
         own[l] = v;
         sq[l] = v2;
         add_to(low + c.low0 + l, v2);
@@ -764,67 +805,89 @@ __global__ void __launch_bounds__(kSplitRdmThreads, 4) k_doci_rdm_split(const Do
     if (m > 0)
         for (int r = warp; r < nv; r += kSplitRdmWarps)
             for (int l = lane; l < nminus; l += 32) up[(size_t)r * nminus + l] = load(upb[r] + (uint32_t)l);
-    // high - high
-    for (int e = warp; e < nhh; e += kSplitRdmWarps) {
-        const uint32_t b = hhb[e];
-        if (b == 0xFFFFFFFFu) continue;  // k < j: summed from the other side
-        long long a = 0;
-#pragma unroll 4
-        for (int l = lane; l < nlow; l += 32) a += fxmul(own[l], load(b + (uint32_t)l));
-        a = warp_sum(a);
-        if (lane == 0) {
-            const int i = e / nv;
-            add_to(sB + (s + nth(hb, i)) * L + s + nth(full & ~hb, e - i * nv), a);
-        }
-    }
-    // low - low
-    if (n2 > 0) {
-        for (int pr = warp, j = 0, k0 = 0; pr < np; pr += kSplitRdmWarps) {  // pair (j, k), row-major, j < k
-            while (pr - k0 >= s - 1 - j) k0 += s - 1 - j++;
-            const uint32_t *w = two + (size_t)pr * n2;
-            long long a = 0;
-#pragma unroll 4
-            for (int x = lane; x < n2; x += 32) {
-                const uint32_t e = __ldg(w + x);
-                a += fxmul(own[e & 0xFFFFu], own[e >> 16]);
-            }
-            a = warp_sum(a);
-            if (lane == 0) add_to(sB + j * L + j + 1 + pr - k0, a);
-        }
-    }
-    // squares: over the block, and over its strings that hold j
-    if (warp == kSplitRdmWarps - 1 && nh > 0) {
-        long long a = 0;
-        for (int l = lane; l < nlow; l += 32) a += sq[l];
-        a = warp_sum(a);
-        for (int e = lane; e < nh * nh; e += 32) {
-            const int i = e / nh, k = e - i * nh;
-            if (k >= i) add_to(sA + (s + nth(hb, i)) * L + s + nth(hb, k), a);
-        }
-    }
-    if (m > 0 && nh > 0)
-        for (int j = warp; j < s; j += kSplitRdmWarps) {
-            long long a = 0;
-            for (int x = lane; x < n1; x += 32) a += sq[__ldg(one + (size_t)j * n1 + x) & 0xFFFFu];
-            a = warp_sum(a);
-            for (int i = lane; i < nh; i += 32) add_to(sA + j * L + s + nth(hb, i), a);
-        }
     __syncthreads();  // the blocks h + k are staged
-    // low - high
-    if (m > 0)
-        for (int e = warp; e < nv * s; e += kSplitRdmWarps) {
-            const int r = e / s, j = e - r * s;
-            const uint32_t *w = one + (size_t)j * n1;
-            const long long *row = up + (size_t)r * nminus;
-            long long a = 0;
-#pragma unroll 4
-            for (int x = lane; x < n1; x += 32) {
-                const uint32_t v = __ldg(w + x);
-                a += fxmul(own[v & 0xFFFFu], row[v >> 16]);
+    // Four sums at a time, the next four for whichever warp is free, the longest first: one
+    // sum at a time, its reduction, its place and its atomic cost as much as its products.
+    const int hops = (nhop + 3) / 4, mixed = m > 0 ? (nv * s + 3) / 4 : 0, pairs = n2 > 0 ? (np + 3) / 4 : 0;
+    const int squares = m > 0 && nh > 0 ? s : 0, jobs = hops + mixed + pairs + squares + (nh > 0);
+    for (;;) {
+        int g = lane == 0 ? atomicAdd(&job, 1) : 0;
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (g >= jobs) break;
+        long long a[4] = {0, 0, 0, 0};
+        const int mine = lane >> 3;  // of the four, after the reduction
+        const bool writes = (lane & 7) == 0;
+        if (g < hops) {  // high - high
+            uint32_t b[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) b[u] = hhb[min(4 * g + u, nhop - 1)];
+            for (int l = lane; l < nlow; l += 32) {
+                const long long v = own[l];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) fxadd(a[u], v, load(b[u] + (uint32_t)l));
             }
-            a = warp_sum(a);
-            if (lane == 0) add_to(sB + j * L + s + nth(full & ~hb, r), a);
+            const long long sum = sum_four(a, lane);
+            const int e = 4 * g + mine;
+            if (writes && e < nhop) add_to(sB + (hhe[e] / L + s) * L + s + hhe[e] % L, sum);
+            continue;
         }
+        g -= hops;
+        if (g < mixed) {  // low - high
+            const uint32_t *w[4];
+            const long long *row[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = min(4 * g + u, nv * s - 1), r = e / s;
+                w[u] = one + (size_t)(e - r * s) * n1;
+                row[u] = up + (size_t)r * nminus;
+            }
+            for (int x = lane; x < n1; x += 32) {
+                uint32_t v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = __ldg(w[u] + x);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) fxadd(a[u], own[v[u] & 0xFFFFu], row[u][v[u] >> 16]);
+            }
+            const long long sum = sum_four(a, lane);
+            const int e = 4 * g + mine, r = e / s;
+            if (writes && e < nv * s) add_to(sB + (e - r * s) * L + s + nth(full & ~hb, r), sum);
+            continue;
+        }
+        g -= mixed;
+        if (g < pairs) {  // low - low: pairs (j, k), row-major, j < k
+            const uint32_t *w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[u] = two + (size_t)min(4 * g + u, np - 1) * n2;
+            for (int x = lane; x < n2; x += 32) {
+                uint32_t v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = __ldg(w[u] + x);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) fxadd(a[u], own[v[u] & 0xFFFFu], own[v[u] >> 16]);
+            }
+            const long long sum = sum_four(a, lane);
+            int e = 4 * g + mine, j = 0;
+            if (writes && e < np) {
+                for (; e >= s - 1 - j; ++j) e -= s - 1 - j;
+                add_to(sB + j * L + j + 1 + e, sum);
+            }
+            continue;
+        }
+        g -= pairs;
+        long long v = 0;
+        if (g < squares) {  // squares of the block's strings that hold g
+            for (int x = lane; x < n1; x += 32) v += sq[__ldg(one + (size_t)g * n1 + x) & 0xFFFFu];
+            v = warp_sum(v);
+            for (int i = lane; i < nh; i += 32) add_to(sA + g * L + s + nth(hb, i), v);
+        } else {  // squares of the block
+            for (int l = lane; l < nlow; l += 32) v += sq[l];
+            v = warp_sum(v);
+            for (int e = lane; e < nh * nh; e += 32) {
+                const int i = e / nh, k = e - i * nh;
+                if (k >= i) add_to(sA + (s + nth(hb, i)) * L + s + nth(hb, k), v);
+            }
+        }
+    }
     __syncthreads();
     for (int i = t; i < 2 * L * L; i += kSplitRdmThreads)
         if (sA[i] != 0) add_to(sums + i, sA[i]);
@@ -856,7 +919,7 @@ size_t split_rdm_smem(const DociSplitView &v) {
     for (int q = 0; q < v.nsec; ++q) {
         const DociSector &c = v.sec[q];
         const size_t nv = v.L - v.s - c.nh;
-        most = std::max(most, 8 * (2 * (size_t)c.nlow + nv * c.nminus) + 4 * (c.nh * nv + nv));
+        most = std::max(most, 8 * (2 * (size_t)c.nlow + nv * c.nminus) + 4 * (2 * c.nh * nv + nv));
     }
     return most + 16 * (size_t)v.L * v.L;
 }

@@ -148,3 +148,26 @@ def test_doci_rdm_split(L, n):
     for other in (rdm_via_abi(plain, c), rdm_via_abi(plain, c), rdm_via_abi(mixed, c)):
         for g, o in zip(got, other):
             assert np.array_equal(g, o)
+
+
+@pytest.mark.parametrize("kind", ["unit", "minus", "pair", "tiny", "halves"])
+def test_doci_rdm_split_values(kind):
+    # the ends of the fixed point: +-1, entries below a unit of the low digit, and digits at
+    # their own ends (multiples of 2^-31 and of 2^-30 plus half a low digit)
+    L, n = 17, 8
+    ints = make_integrals(L, n, n, nchol=4, seed=5)
+    cim = DOCI(Hamiltonian.from_integrals(ints))
+    rng = np.random.default_rng(3)
+    c = np.zeros(cim.get_dim())
+    if kind in ("unit", "minus"):
+        c[1234] = 1.0 if kind == "unit" else -1.0
+    elif kind == "pair":
+        c[[100, 101]] = 0.6, -0.8
+    elif kind == "tiny":
+        c[:] = rng.standard_normal(c.size) * 2.0 ** -45
+        c[7] = 1.0
+    else:
+        c[:] = rng.integers(-3, 4, c.size) * 2.0 ** -30 + rng.integers(-1, 2, c.size) * 2.0 ** -31
+        c[11] = -0.5
+    got = rdm_via_abi(cim, c)
+    assert_rdm_close(got, O.rdm(O.DOCI, L, n, n, c), 1e-13)
