@@ -230,7 +230,9 @@ def sigma_work(L: int, nup: int, ndown: int, rank: int, padded: int) -> dict:
 def matvec_bytes(handle, fp32: bool) -> tuple[int, str]:
     """Algorithmic bytes of one matvec for the stored layout: one read of the stored
     matrix and of x, one write of y. FP32: FP32 values/x/y; FP64: FP64 x/y with FP64
-    values (plain CRS) or the split hi + lo values (MIXED)."""
+    values (plain CRS) or the split hi + lo values (MIXED). Plain DOCI matrices from
+    500,000 rows keep their CRS but multiply matrix-free: these are the bytes of the rows
+    that such a product does not read."""
     dim, nu, nf = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int64()
     check(lib().cigpu_crs_dims(handle, ctypes.byref(dim), ctypes.byref(nu), ctypes.byref(nf)))
     lay, stored = ctypes.c_int(), ctypes.c_int64()
