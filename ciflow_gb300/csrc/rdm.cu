@@ -705,15 +705,16 @@ __global__ void k_doci_rdm(const double *__restrict__ c, const uint64_t *__restr
 // four strings to act on, and formed a rank for each), and A needs only the blocks'
 // sums of squares, per block and per low string. The products and sums are the
 // fixed-point integers above, so the result is the same bit for bit in any order:
-// shared and global integer atomics collect them. Bound by instruction issue (49 for 32
+// integer atomics collect them. Bound by instruction issue (49 for 32
 // products, ALU 41%) and, at three blocks per SM, the barriers around the staging. L=24,
 // 12 pairs: 3.80 -> 0.74 ms per cigpu_rdm with a sum at a time for every warp, 0.66 with
-// four and in digits (the kernel 490 -> 423 us; the vector's way from host memory is 150).
-constexpr int kSplitRdmThreads = 256;
+// four and in digits, 0.65 without the block's own matrices of sums (the kernel 490 -> 418
+// us; the vector's way from host memory is 150).
+constexpr int kSplitRdmThreads = 256;  // 384: L=24 0.63, L=27 19 pairs 1.47 against 1.36 ms; 512: 0.68, 1.80
 constexpr int kSplitRdmWarps = kSplitRdmThreads / 32;
 // Spaces whose blocks hold at least this many strings on average take it: a block of
 // strings costs a thread block some microseconds whatever its length (L=27, 19 pairs, 76
-// strings a block: 3.72 -> 1.40 ms per call; L=19, 12 pairs, 98: 280 -> 121 us; L=30, 24
+// strings a block: 3.72 -> 1.36 ms per call; L=19, 12 pairs, 98: 280 -> 121 us; L=30, 24
 // pairs, 19 strings: 1.44 ms against 2.43 when the split took 2.42 and 134 in those; L=30, 5
 // pairs, 11: 0.49 against 0.83).
 constexpr int64_t kSplitRdmBlock = 40;
@@ -749,10 +750,9 @@ __global__ void __launch_bounds__(kSplitRdmThreads, 4) k_doci_rdm_split(const Do
                                                                      long long *__restrict__ low) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int L = p.L, s = p.s, Lh = L - s, t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    long long *sA = reinterpret_cast<long long *>(smem);  // [L][L]
-    long long *sB = sA + L * L;                           // [L][L]
-    long long *area = sB + L * L;
-    for (int i = t; i < 2 * L * L; i += kSplitRdmThreads) sA[i] = 0;
+    long long *area = reinterpret_cast<long long *>(smem);
+    // a block of strings has one sum for an element of either: added to memory as it is formed
+    long long *sA = sums, *sB = sums + L * L;
     auto start_of = [&](uint64_t b, int mm) {
         uint32_t r = 0;
         for (int k = mm + 1; b; b &= b - 1, ++k) r += __ldg(p.binom + (s + __ffsll((long long)b) - 1) * kSplitBinomRow + k);
@@ -888,9 +888,6 @@ __global__ void __launch_bounds__(kSplitRdmThreads, 4) k_doci_rdm_split(const Do
             }
         }
     }
-    __syncthreads();
-    for (int i = t; i < 2 * L * L; i += kSplitRdmThreads)
-        if (sA[i] != 0) add_to(sums + i, sA[i]);
 }
 
 // A of two low orbitals (block.x = j * s + k, j <= k): the sums of squares of the low
@@ -921,7 +918,7 @@ size_t split_rdm_smem(const DociSplitView &v) {
         const size_t nv = v.L - v.s - c.nh;
         most = std::max(most, 8 * (2 * (size_t)c.nlow + nv * c.nminus) + 4 * (2 * c.nh * nv + nv));
     }
-    return most + 16 * (size_t)v.L * v.L;
+    return most;
 }
 
 __global__ void k_doci_rdm_finish(const long long *__restrict__ sums, int L, int np, double *__restrict__ rdm1,
