@@ -1623,37 +1623,7 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
     // FP32 steps than it saved (L=24 12 pairs: 24 + 2 against 21 + 3 products). A
     // warm start may already be near the tolerance and takes the FP64 product.
     anchor(!have_start && P.fp32_first_anchor);
-    // A fold of a full basis far above the FP32 floor moves the anchor without a product:
-    // H c follows with c as the same combination of H c and the H v_i, its error the FP32
-    // rounding of the corrections' products, which the residual of every step of the cycle
-    // held already. `carried` sums the corrections moved that way since the last exact
-    // anchor and counts in the floor; the anchor is exact again where the residual reaches
-    // it, at a fold that made no progress, and before the solver returns. (FCI L=12 6a6b to
-    // 1e-11, three seeds: 9 FP64 products of 2.65 ms in all, 17 with an exact anchor at every
-    // fold.)
-    bool exact = have_start || !P.fp32_first_anchor;
-    double carried = exact ? 0.0 : 1.0;  // a first anchor from the FP32 product carries c itself
-    if (!exact && rho <= o.tol) {
-        anchor(false);
-        exact = true;
-        carried = 0;
-    }
-    auto move_anchor = [&](int k, double a0) {  // c has moved already; yd holds y_1..y_k
-        k_combine<float, double, 1><<<ops.G, kVecThreads, 0, s>>>(HV.p + n, n, k, yd.p, 1, ref.t.p, n, n);
-        k_axpby64<<<ops.G, kVecThreads, 0, s>>>(1.0, ref.t.p, a0, ref.w.p, n);
-        CIGPU_CUDA(cudaGetLastError());
-        count_launch(2);
-        ops.dots(c_dev, n, 1, c_dev, n, 0);
-        ops.scale(c_dev, n, 0);
-        ops.scale(ref.w.p, n, 0);
-        ops.dots(c_dev, n, 1, ref.w.p, n, 0);
-        E = ops.fetch(1)[0];
-        rho = ops.residual(ref.w.p, c_dev, E, ref.r.p, n);
-        dev_convert(c_dev, V.p, n, s);
-        dev_convert(ref.w.p, HV.p, n, s);
-        dev_convert(c_dev, cr32.p, n, s);
-        dev_convert(ref.r.p, cr32.p + n, n, s);
-    };
+    if (!have_start && P.fp32_first_anchor && rho <= o.tol) anchor(false);  // no convergence on the FP32 residual
     int k = 0;  // corrections in the basis
     double theta = E, a0 = 1.0, yv = 0;
     std::vector<double> y(kMaxBasis + 1, 0.0), yp(kMaxBasis + 1, 0.0), d(kMaxBasis + 1, 0.0);
@@ -1752,9 +1722,8 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
         // fold when the previous approximate residual reached the FP32 floor of the
         // correction (the new solution, with one more vector, is at least as good),
         // when the basis is full, or on breakdown
-        const auto floor_of = [&](double size) { return std::max(0.5 * o.tol, 30.0 * 6e-8 * std::max(1.0, std::fabs(theta)) * size); };
-        const double floor = floor_of(std::hypot(yv, carried));
-        const bool fold = rho_u <= floor || k >= mmax || !(tn2 > 1e-28);
+        const double floor = 30.0 * 6e-8 * std::max(1.0, std::fabs(theta)) * yv;
+        const bool fold = rho_u <= std::max(0.5 * o.tol, floor) || k >= mmax || !(tn2 > 1e-28);
         yv = 0;
         for (int i = 1; i <= k; ++i) yv += y[i] * y[i];
         yv = std::sqrt(yv);
@@ -1766,7 +1735,7 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
             // correction restarts clean (the kept direction would carry that floor
             // into the next cycle, and at tight tolerances the cycles then stall)
             bool keep = false;
-            if (kp >= 0 && kp <= k && k >= mmax && !(rho_u <= floor) && tn2 > 1e-28) {
+            if (kp >= 0 && kp <= k && k >= mmax && !(rho_u <= std::max(0.5 * o.tol, floor)) && tn2 > 1e-28) {
                 double uu = a0 * a0, up = a0 * a0p;
                 for (int i = 1; i <= k; ++i) {
                     uu += y[i] * y[i];
@@ -1798,17 +1767,7 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
             CIGPU_CUDA(cudaGetLastError());
             count_launch(2);
             const int kf = k;
-            const double noise = std::hypot(yv, carried);
-            exact = !(tn2 > 1e-28) || rho_u <= 4.0 * floor_of(noise);
-            if (!exact) {
-                move_anchor(k, a0);
-                carried = noise;
-                exact = rho <= std::max(o.tol, floor_of(noise)) || rho > 0.7 * last_rho;
-            }
-            if (exact) {
-                anchor(false);
-                carried = 0;
-            }
+            anchor(false);
             ++collapses;
             k = 0;
             yv = 0;
@@ -1848,7 +1807,6 @@ int solve_mixed(const SolveProblem &P, const SolveOptions &o, double *c_dev, boo
             }
         }
     }
-    if (!exact) anchor(false);
     info.e0 = E;
     info.residual = rho;
     info.gap = gap;

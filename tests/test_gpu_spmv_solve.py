@@ -358,3 +358,26 @@ def test_sigma_sets(L, na, nb, rank, monkeypatch):
     torch.cuda.synchronize()
     y = yd.cpu().numpy().astype(np.float64)
     assert np.abs(y - y_ref).max() <= 2e-5 * np.abs(y_ref).max()
+
+
+@pytest.mark.parametrize("case,form", [("11x4x4x16", "sigma"), ("11x4x4x16", "slots"), ("8x4x4x16", "slots"),
+                                       ("7x3x3-indefinite", "sigma")])
+def test_mixed_folds_take_an_fp64_product(case, form, monkeypatch):
+    """Every correction cycle of a mixed solve ends in an FP64 product of the stored
+    matrix, also where it ends because the basis is full (the spaces of 4,900 rows and
+    less run the solver's small form): as many FP64 products as cycles, and one more where
+    the first residual is not the FP32 product's. A budget that ends inside a cycle is
+    passed by the closing fold's product at most."""
+    monkeypatch.setenv("CIGPU_FP32_PRODUCT", form)
+    ints = _ints_case(case)
+    ref = build(FCI, ints)
+    ref.solve(tol=1e-10)
+    m = build(FCI, ints, A.MIXED)
+    m.solve(tol=1e-10)
+    assert m.info["converged"] and m.info["corrections"] >= 2
+    assert m.info["matvecs_fp64"] == m.info["corrections"] + (form == "slots")
+    # both energies are Rayleigh quotients of residuals below 1e-10
+    assert abs(m.get_ci_energy() - ref.get_ci_energy()) <= 1e-12 * max(1.0, abs(ref.get_ci_energy()))
+    for budget in (9, 14, 40):
+        m.solve(tol=1e-13, max_matvec=budget)
+        assert m.info["matvecs_fp32"] + m.info["matvecs_fp64"] <= budget + 1
