@@ -148,6 +148,48 @@ __device__ __forceinline__ T warp_sums8(T (&a)[kDotChunk], int lane) {
     return v + __shfl_xor_sync(0xffffffffu, v, 1);
 }
 
+// s + e, a sum of FP32 terms with the roundings of its additions (Knuth's TwoSum; the
+// rounding intrinsics keep the compiler from contracting a product into it). Threads that
+// add several terms keep one: the length of a thread's chain then costs no accuracy, and
+// the basis kernels are bound by loads, not by FP32 additions.
+__device__ __forceinline__ void add_exact(float &s, float &e, float p) {
+    const float t = __fadd_rn(s, p), b = __fsub_rn(t, s);
+    e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(p, b)));
+    s = t;
+}
+
+// The warp's sum of s + e, on every lane.
+__device__ __forceinline__ double warp_sum_exact(float s, float e) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const float rs = __shfl_xor_sync(0xffffffffu, s, o), re = __shfl_xor_sync(0xffffffffu, e, o);
+        e = __fadd_rn(e, re);
+        add_exact(s, e, rs);
+    }
+    return (double)s + (double)e;
+}
+
+// warp_sums8 of such sums.
+__device__ __forceinline__ double warp_sums8_exact(float (&a)[kDotChunk], float (&e)[kDotChunk], int lane) {
+#pragma unroll
+    for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
+        const bool hi = lane & o;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const float rs = __shfl_xor_sync(0xffffffffu, hi ? a[k] : a[k + h], o);
+            const float re = __shfl_xor_sync(0xffffffffu, hi ? e[k] : e[k + h], o);
+            a[k] = hi ? a[k + h] : a[k];
+            e[k] = __fadd_rn(hi ? e[k + h] : e[k], re);
+            add_exact(a[k], e[k], rs);
+        }
+    }
+    for (int o = 2; o > 0; o >>= 1) {
+        const float rs = __shfl_xor_sync(0xffffffffu, a[0], o), re = __shfl_xor_sync(0xffffffffu, e[0], o);
+        e[0] = __fadd_rn(e[0], re);
+        add_exact(a[0], e[0], rs);
+    }
+    return (double)a[0] + (double)e[0];
+}
+
 // Per-block partial dots V_i . w (i < nvec, chunks of kDotChunk on blockIdx.y, one
 // ticket per chunk). AT is the arithmetic type of the products and of the
 // per-thread sums (float for FP32 vectors: GB300 issues FP64 at 1/64 of the FP32
@@ -226,9 +268,9 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_multidot_f4(const float4 *__
     const int nv = last ? tail.nvec : min(kDotChunk, nvec - row);
     V = last ? tail.V : V + row * ld4;
     w = last ? tail.w : w;
-    float acc[kDotChunk];
+    float acc[kDotChunk], err[kDotChunk];
 #pragma unroll
-    for (int i = 0; i < kDotChunk; ++i) acc[i] = 0.f;
+    for (int i = 0; i < kDotChunk; ++i) acc[i] = err[i] = 0.f;
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n4; r += (int64_t)gridDim.x * blockDim.x) {
         const float4 wr = w[r];
         float4 va[kDotChunk];
@@ -237,12 +279,13 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_multidot_f4(const float4 *__
             if (i < nv) va[i] = V[i * ld4 + r];
 #pragma unroll
         for (int i = 0; i < kDotChunk; ++i)
-            if (i < nv) acc[i] += (va[i].x * wr.x + va[i].y * wr.y) + (va[i].z * wr.z + va[i].w * wr.w);
+            if (i < nv)
+                add_exact(acc[i], err[i], (va[i].x * wr.x + va[i].y * wr.y) + (va[i].z * wr.z + va[i].w * wr.w));
     }
     __shared__ double sh[kDotChunk][kVecThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float a = warp_sums8(acc, lane);  // warp sums in FP32, block and grid sums in FP64
-    if ((lane & 3) == 0) sh[lane >> 2][warp] = (double)a;
+    const double a = warp_sums8_exact(acc, err, lane);  // block and grid sums in FP64
+    if ((lane & 3) == 0) sh[lane >> 2][warp] = a;
     __syncthreads();
     if (threadIdx.x < nv) {
         double t = 0;
@@ -812,8 +855,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_lanczos_steps(int64_t n, doub
 // work, on one cluster of 16 blocks; the couplings and the fetch of their results in one
 // more, which writes them to pinned memory. A block owns a slice of the rows, keeps its
 // slices of the basis in shared memory after the residual has read them, and the sums meet
-// through distributed shared memory in a fixed order (FP32 sums per warp, FP64 above, as
-// the separate kernels). Up to kDavRows rows, past which the basis is read faster by all
+// through distributed shared memory in a fixed order (FP32 terms, their sums exact to the
+// warp, see add_exact, and FP64 above). Up to kDavRows rows, past which the basis is read faster by all
 // SMs. FCI L=8 4a4b (4,900 rows) to 1e-11: 9.9 -> 6.7 ms.
 constexpr int kDavThreads = 512;
 constexpr int64_t kDavRows = 16384;
@@ -864,7 +907,7 @@ __global__ void __launch_bounds__(kDavThreads) k_dav_step(int64_t n, float *__re
     for (int i = t; i < k; i += kDavThreads) ys[i] = (float)coef.y[i];
     __syncthreads();
     const float fa0 = (float)a0, fa0de = (float)a0_de, fth = (float)theta, fsig = (float)fmin(theta, *dmin);
-    float rr = 0.f;
+    float rr = 0.f, rr_err = 0.f;
     for (int e = t; e < mine; e += kDavThreads) {
         const int64_t r = r0 + e;
         float ru = 0.f;
@@ -875,20 +918,20 @@ __global__ void __launch_bounds__(kDavThreads) k_dav_step(int64_t n, float *__re
             Vs[(size_t)(i + 1) * slice + e] = v;
             if (!given) ru += ys[i] * (HV[(int64_t)(i + 1) * n + r] - fth * v);
         }
-        rr += ru * ru;
+        add_exact(rr, rr_err, ru * ru);
         w[e] = given ? out[e] : dav_precond(ru, fsig, diag32[r]);
     }
-    auto block_sum = [&](float v) {  // FP32 per warp, FP64 above; the result on thread 0
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    auto block_sum = [&](float s, float err) {  // FP64 above a warp; the result on thread 0
+        const double v = warp_sum_exact(s, err);
         __syncthreads();
-        if (lane == 0) wsum[warp] = (double)v;
+        if (lane == 0) wsum[warp] = v;
         __syncthreads();
         double a = 0;
         if (t == 0)
             for (int q = 0; q < kDavThreads / 32; ++q) a += wsum[q];
         return a;
     };
-    const double rrs = block_sum(rr);
+    const double rrs = block_sum(rr, rr_err);
     if (t == 0) part[0][k + 2] = rrs;
     double norm = 0;
     for (int pass = 0; pass < 2; ++pass) {
@@ -896,22 +939,22 @@ __global__ void __launch_bounds__(kDavThreads) k_dav_step(int64_t n, float *__re
         // the dots with slots 0..k, and w with itself (place k + 1)
         for (int i = warp; i < k + 2; i += kDavThreads / 32) {
             const float *v = i <= k ? Vs + (size_t)i * slice : w;
-            float a = 0.f;
-            for (int e = lane; e < mine; e += 32) a += v[e] * w[e];
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (lane == 0) p[i] = (double)a;
+            float a = 0.f, err = 0.f;
+            for (int e = lane; e < mine; e += 32) add_exact(a, err, v[e] * w[e]);
+            const double dot = warp_sum_exact(a, err);
+            if (lane == 0) p[i] = dot;
         }
         cluster_sums(cluster, p, k + 2 + (pass == 0), sum);
         const double before = sum[k + 1];
         if (pass == 0 && rank == 0 && t == 0) *out_r = sum[k + 2];
-        float nn = 0.f;
+        float nn = 0.f, nn_err = 0.f;
         for (int e = t; e < mine; e += kDavThreads) {
             float x = w[e];
             for (int i = 0; i <= k; ++i) x -= Vs[(size_t)i * slice + e] * (float)sum[i];
             w[e] = x;
-            nn += x * x;
+            add_exact(nn, nn_err, x * x);
         }
-        const double ns = block_sum(nn);
+        const double ns = block_sum(nn, nn_err);
         // every block has read the other parts of this pass before one is written again
         cluster.sync();
         if (t == 0) p[0] = ns;
@@ -939,10 +982,10 @@ __global__ void __launch_bounds__(kDavThreads) k_dav_couple(int64_t n, const flo
     const float *v = V + (int64_t)(k + 1) * n + r0;
     for (int i = warp; i < k + 3; i += kDavThreads / 32) {
         const float *x = i <= k ? V + (int64_t)(i + 1) * n + r0 : v, *y = (i <= k ? hv : i == k + 1 ? c32 : r32) + r0;
-        float a = 0.f;
-        for (int e = lane; e < mine; e += 32) a += x[e] * y[e];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) part[i] = (double)a;
+        float a = 0.f, err = 0.f;
+        for (int e = lane; e < mine; e += 32) add_exact(a, err, x[e] * y[e]);
+        const double dot = warp_sum_exact(a, err);
+        if (lane == 0) part[i] = dot;
     }
     cluster_sums(cluster, part, k + 3, sum);
     if (cluster.block_rank() == 0)
