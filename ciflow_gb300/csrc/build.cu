@@ -527,13 +527,10 @@ void fci_launch(int mode, const FciParams &p0, cudaStream_t s) {
     const int64_t blocks = p.a.D * nchunks;
     if (mode == kFill32 && (!p.eri_hi || !p.eri_lo))
         throw CudaError{cudaErrorInvalidValue, "FP32 integral tables missing"};
-    static const bool attr_set = [] {  // thread-safe one-time init
-        cudaFuncSetAttribute(k_fci_rows<kCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFciMaxSmem);
-        cudaFuncSetAttribute(k_fci_rows<kFill64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFciMaxSmem);
-        cudaFuncSetAttribute(k_fci_rows<kFill32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFciMaxSmem);
-        return true;
-    }();
-    (void)attr_set;
+    static SmemLimit limit[3];
+    CIGPU_CUDA(limit[0].raise(k_fci_rows<kCount>, kFciMaxSmem));
+    CIGPU_CUDA(limit[1].raise(k_fci_rows<kFill64>, kFciMaxSmem));
+    CIGPU_CUDA(limit[2].raise(k_fci_rows<kFill32>, kFciMaxSmem));
     switch (mode) {
         case kCount: k_fci_rows<kCount><<<(unsigned)blocks, kFciThreads, sm, s>>>(p); break;
         case kFill64: k_fci_rows<kFill64><<<(unsigned)blocks, kFciThreads, sm, s>>>(p); break;
@@ -578,13 +575,10 @@ void doci_diag_launch(const DociParams &p, double *diag, cudaStream_t s) {
 void doci_launch(int mode, const DociParams &p, cudaStream_t s) {
     const int warps = kDociThreads / 32;
     const size_t sm = doci_smem_bytes(p.W, warps);
-    static const bool attr_set = [] {  // thread-safe one-time init
-        cudaFuncSetAttribute(k_doci_rows<kCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_doci_rows<kFill64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_doci_rows<kFill32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        return true;
-    }();
-    (void)attr_set;
+    static SmemLimit limit[3];
+    CIGPU_CUDA(limit[0].raise(k_doci_rows<kCount>, 200 * 1024));
+    CIGPU_CUDA(limit[1].raise(k_doci_rows<kFill64>, 200 * 1024));
+    CIGPU_CUDA(limit[2].raise(k_doci_rows<kFill32>, 200 * 1024));
     const int blocks = grid_for(p.D * 32, kDociThreads, 16);
     switch (mode) {
         case kCount: k_doci_rows<kCount><<<blocks, kDociThreads, sm, s>>>(p); break;

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/cigpu.h"
+#include "smem_limit.cuh"
 
 namespace cigpu {
 

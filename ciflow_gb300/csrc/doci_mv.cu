@@ -473,9 +473,8 @@ __global__ void k_split_high(const DociSplitView p, uint64_t *__restrict__ hbits
 
 template <typename T>
 void launch_split(const DociSplit &sp, const T *K, const T *diag, const T *x, T *y, cudaStream_t s) {
-    static const cudaError_t attr = cudaFuncSetAttribute(k_doci_split<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)kSplitMaxSmem);
-    CIGPU_CUDA(attr);
+    static SmemLimit limit;
+    CIGPU_CUDA(limit.raise(k_doci_split<T>, kSplitMaxSmem));
     constexpr int kType = sizeof(T) == 8;
     DociSplitView v = sp.view;
     v.err = check_word_device();
@@ -512,11 +511,8 @@ void launch_mv_g(const DociMv &p0, const T *K, const T *diag, const T *x, T *y, 
     DociMv p = p0;
     p.err = check_word_device();
     const size_t sm = sizeof(T) * (size_t)p.L * p.L;
-    static const bool attr_set = [] {  // thread-safe one-time init (L = 63: 31 KB of FP64 K)
-        cudaFuncSetAttribute(k_doci_mv<T, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        return true;
-    }();
-    (void)attr_set;
+    static SmemLimit limit;  // L = 63: 31 KB of FP64 K
+    CIGPU_CUDA(limit.raise(k_doci_mv<T, G>, 64 * 1024));
     constexpr int rows_per_block = kMvWarps * (32 / G);
     const int64_t blocks = std::min<int64_t>((p.D + rows_per_block - 1) / rows_per_block, (int64_t)sm_count() * 8);
     k_doci_mv<T, G><<<(unsigned)std::max<int64_t>(blocks, 1), kMvThreads, sm, s>>>(p, K, diag, x, y);

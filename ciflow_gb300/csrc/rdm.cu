@@ -1012,9 +1012,8 @@ void doci_rdm_sums(const cigpu_crs &c, const double *c_dev, long long *sums, uns
 }
 
 void doci_rdm_split(const DociSplit &sp, const double *c_dev, long long *sums, cudaStream_t s) {
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_doci_rdm_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitRdmMaxSmem);
-    CIGPU_CUDA(attr);
+    static SmemLimit limit;
+    CIGPU_CUDA(limit.raise(k_doci_rdm_split, kSplitRdmMaxSmem));
     DociSplitView v = sp.view;
     v.err = check_word_device();
     DevBuf<long long> fixed((size_t)v.D), low(sp.nlowbits);

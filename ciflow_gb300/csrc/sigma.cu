@@ -664,9 +664,8 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
 }
 
 void sigma_mv32(SigmaOp &op, const FciParams &p, const float *x, float *y, cudaStream_t s) {
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_sigma_parts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSigmaMaxSmem);
-    CIGPU_CUDA(attr);
+    static SmemLimit limit;
+    CIGPU_CUDA(limit.raise(k_sigma_parts, kSigmaMaxSmem));
     SigmaArgs a{};
     a.L = op.L;
     a.R = op.R;

@@ -812,11 +812,8 @@ void launch_slots(const FciParams &p, const F &f0, typename F::X *y, cudaStream_
     F f = f0;
     f.nx = (uint64_t)(p.a.D * p.Db);
     f.err = check_word_device();
-    static const bool attr_set = [] {  // thread-safe one-time init
-        cudaFuncSetAttribute(k_spmv_slots<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlotsMaxSmem);
-        return true;
-    }();
-    (void)attr_set;
+    static SmemLimit limit;
+    CIGPU_CUDA(limit.raise(k_spmv_slots<F>, kSlotsMaxSmem));
     const int64_t T = (p.Db + kTileRows - 1) / kTileRows;
     k_spmv_slots<F><<<(unsigned)(p.a.D * T), kSlotThreads, tile_smem(p), s>>>(p, f, y);
     CIGPU_CUDA(cudaGetLastError());
@@ -847,11 +844,8 @@ void fill_slots_launch(const FciParams &p0, float *hi, float *lo, uint32_t *coun
     FciParams p = p0;
     const size_t base = fill_smem(p), sl = slice_smem(p);
     p.staged = base + sl <= kSlotsMaxSmem ? 1 : 0;
-    static const bool attr_set = [] {  // thread-safe one-time init
-        cudaFuncSetAttribute(k_fill_slots<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlotsMaxSmem);
-        return true;
-    }();
-    (void)attr_set;
+    static SmemLimit limit;
+    CIGPU_CUDA(limit.raise(k_fill_slots<false>, kSlotsMaxSmem));
     const int64_t T = (p.Db + kTileRows - 1) / kTileRows;
     k_fill_slots<false><<<(unsigned)(p.a.D * T), kSlotThreads, p.staged ? base + sl : base, s>>>(p, hi, lo, nullptr,
                                                                                                 count, lower);
@@ -869,11 +863,8 @@ void fill_slots64_launch(const FciParams &p0, double *v64, uint32_t *count, uint
         p.staged = 0;
         smem = fly_smem(p);
     }
-    static const bool attr_set = [] {  // thread-safe one-time init
-        cudaFuncSetAttribute(k_fill_slots<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlotsMaxSmem);
-        return true;
-    }();
-    (void)attr_set;
+    static SmemLimit limit;
+    CIGPU_CUDA(limit.raise(k_fill_slots<true>, kSlotsMaxSmem));
     const int64_t T = (p.Db + kTileRows - 1) / kTileRows;
     k_fill_slots<true><<<(unsigned)(p.a.D * T), kSlotThreads, smem, s>>>(p, nullptr, nullptr, v64, count, lower);
     CIGPU_CUDA(cudaGetLastError());
@@ -908,13 +899,9 @@ void spmv_slots_f64(const FciParams &p, const double *val, const double *x, doub
     Plain<double> f{val, x};
     f.nx = (uint64_t)(p.a.D * p.Db);
     f.err = check_word_device();
-    static const bool attr_set = [] {  // thread-safe one-time init; three blocks of ~76 KB per SM at L=12 6a6b
-        cudaFuncSetAttribute(k_spmv_slots_fly, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlotsMaxSmem);
-        cudaFuncSetAttribute(k_spmv_slots_fly, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-        return true;
-    }();
-    (void)attr_set;
+    // three blocks of ~76 KB per SM at L=12 6a6b
+    static SmemLimit limit;
+    CIGPU_CUDA(limit.raise(k_spmv_slots_fly, kSlotsMaxSmem, cudaSharedmemCarveoutMaxShared));
     const int64_t T = (p.Db + kTileRows - 1) / kTileRows;
     k_spmv_slots_fly<<<(unsigned)(p.a.D * T), kSlotThreads, fly_mv_smem(p), s>>>(p, f, y);
     CIGPU_CUDA(cudaGetLastError());
