@@ -346,24 +346,25 @@ __device__ __forceinline__ void fma4(float4 &a, float s, const float4 x) {
     a.w += s * x.w;
 }
 
-// sum_e value_e X[target_e] over row S of the lane's group; Xc: X at the lane's columns,
-// rows P apart (in shared or global memory); st: the warp's staging area.
+// sum_e value_e X[target_e] over the elements [eb, ee), multiples of 8, of row S of the
+// lane's group (rows of ne elements); Xc: X at the lane's columns, rows P apart (in shared
+// or global memory); st: the warp's staging area.
 template <bool SHARED>
-__device__ __forceinline__ float4 same_row(const uint2 *__restrict__ rows, int ne, int64_t S, const float *Xc, int64_t P,
-                                           uint32_t *st) {
+__device__ __forceinline__ float4 same_row(const uint2 *__restrict__ rows, int ne, int eb, int ee, int64_t S,
+                                           const float *Xc, int64_t P, uint32_t *st) {
     const int lane = threadIdx.x & 31, g = lane >> 3, l = lane & 7;
     const uint32_t *mine = st + g * kSameRow;
     float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
     // each lane brings two elements of its group's row, one step ahead
-    const uint4 *src = reinterpret_cast<const uint4 *>(rows + S * ne) + l;
-    uint4 next = 2 * l < ne ? __ldg(src) : make_uint4(0u, 0u, 0u, 0u);
-    for (int e0 = 0; e0 < ne; e0 += kSameE) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(rows + S * ne + eb) + l;
+    uint4 next = eb + 2 * l < ee ? __ldg(src) : make_uint4(0u, 0u, 0u, 0u);
+    for (int e0 = eb; e0 < ee; e0 += kSameE) {
         __syncwarp();
-        const int n = min(kSameE, ne - e0);  // a multiple of 8
+        const int n = min(kSameE, ee - e0);  // a multiple of 8
         *reinterpret_cast<uint4 *>(st + g * kSameRow + 4 * l) = next;
         __syncwarp();
         src += kSameE / 2;
-        if (e0 + kSameE + 2 * l < ne) next = __ldg(src);
+        if (e0 + kSameE + 2 * l < ee) next = __ldg(src);
         for (int e = 0; e < n; e += 8) {
             uint4 d[4];
 #pragma unroll
@@ -406,8 +407,8 @@ __device__ __forceinline__ void same_rows(const SigmaArgs &a, int block, float *
     const int64_t groups = (a.Db + 3) / 4, g1 = min(groups, (int64_t)(chunk + 1) * a.per);
     for (int64_t q = (int64_t)chunk * a.per + warp; q < g1; q += kWarps) {
         const int64_t S = min(4 * q + g, a.Db - 1);  // rows past the last repeat it, and are not written
-        const float4 r = a.panel_rows > 0 ? same_row<true>(a.rows, a.ne, S, sm + 4 * l, kPanel, stage[warp])
-                                          : same_row<false>(a.rows, a.ne, S, a.xT + col + 4 * l, a.Pa, stage[warp]);
+        const float4 r = a.panel_rows > 0 ? same_row<true>(a.rows, a.ne, 0, a.ne, S, sm + 4 * l, kPanel, stage[warp])
+                                          : same_row<false>(a.rows, a.ne, 0, a.ne, S, a.xT + col + 4 * l, a.Pa, stage[warp]);
         if (4 * q + g < a.Db) *reinterpret_cast<float4 *>(a.uT + S * a.Pa + col + 4 * l) = r;
     }
 }
@@ -422,50 +423,84 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) k_sigma
 }
 
 // y(Ia, Ib) = (T^a x) + yd + the sum of W's rows of Ia + uT(Ib, Ia), 32 beta columns per
-// panel (blockIdx.y), alpha strings in chunks (blockIdx.x) of `per` groups of four.
+// panel (blockIdx.y), alpha strings in chunks (blockIdx.x) of `per` groups of four. SPLIT:
+// chunks of at most half as many groups as a block has warps give each group two warps,
+// which take half of its elements and of its numbers each: such a block is one chain of
+// gathers per warp, and half of it is half the time (L=20 4a1b, 792 elements a row: the
+// product among others 101 -> 78 us with it).
+template <bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
     k_sigma_sum(const SigmaArgs a, const uint2 *__restrict__ rows, int ne, int per, const float *__restrict__ xp,
                 float *__restrict__ y) {
     __shared__ __align__(16) uint32_t stage[kWarps][4 * kSameRow];
+    __shared__ float4 second[SPLIT ? kWarps / 2 : 1][32];
+    constexpr int kGroups = SPLIT ? kWarps / 2 : kWarps;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 3, l = lane & 7;
+    const int part = SPLIT ? warp / kGroups : 0;
+    const int eb = part ? ne / 16 * 8 : 0, ee = SPLIT && !part ? ne / 16 * 8 : ne;
+    const int wb = part ? a.nsa / 2 : 0, we = SPLIT && !part ? a.nsa / 2 : a.nsa;
     const int64_t P = a.Pb, col = (int64_t)blockIdx.y * kPanel + 4 * l;
     const int64_t groups = (a.Da + 3) / 4, g1 = min(groups, (int64_t)(blockIdx.x + 1) * per);
-    for (int64_t q = (int64_t)blockIdx.x * per + warp; q < g1; q += kWarps) {
-        const int64_t S = min(4 * q + g, a.Da - 1);
-        const float4 r = same_row<false>(rows, ne, S, xp + col, P, stage[warp]);
-        float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;
-        for (int slab = 0; slab < a.slabs; ++slab) {
-            const float *w = a.W + ((int64_t)slab * a.Da + S) * a.nsa * P + col;
-            fma4(b0, 1.f, __ldg(reinterpret_cast<const float4 *>(a.yd + ((int64_t)slab * a.Da + S) * P + col)));
-            int e = 0;
-            for (; e + 8 <= a.nsa; e += 8) {  // read once: streamed past L1
-                float4 v[8];
+    for (int64_t q = (int64_t)blockIdx.x * per + warp % kGroups; SPLIT || q < g1; q += kGroups) {
+        const bool live = !SPLIT || q < g1;
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        if (live) {
+            const int64_t S = min(4 * q + g, a.Da - 1);
+            const float4 r = same_row<false>(rows, ne, eb, ee, S, xp + col, P, stage[warp]);
+            float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = b0;
+            for (int slab = 0; slab < a.slabs; ++slab) {
+                const float *w = a.W + ((int64_t)slab * a.Da + S) * a.nsa * P + col;
+                if (!part) fma4(b0, 1.f, __ldg(reinterpret_cast<const float4 *>(a.yd + ((int64_t)slab * a.Da + S) * P + col)));
+                int e = wb;
+                for (; e + 8 <= we; e += 8) {  // read once: streamed past L1
+                    float4 v[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)(e + u) * P));
+                    for (int u = 0; u < 8; ++u) v[u] = __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)(e + u) * P));
 #pragma unroll
-                for (int u = 0; u < 8; u += 2) {
-                    fma4(b0, 1.f, v[u]);
-                    fma4(b1, 1.f, v[u + 1]);
+                    for (int u = 0; u < 8; u += 2) {
+                        fma4(b0, 1.f, v[u]);
+                        fma4(b1, 1.f, v[u + 1]);
+                    }
                 }
+                for (; e < we; ++e) fma4(b0, 1.f, __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)e * P)));
             }
-            for (; e < a.nsa; ++e) fma4(b0, 1.f, __ldcs(reinterpret_cast<const float4 *>(w + (int64_t)e * P)));
+            c[0] = r.x + (b0.x + b1.x);
+            c[1] = r.y + (b0.y + b1.y);
+            c[2] = r.z + (b0.z + b1.z);
+            c[3] = r.w + (b0.w + b1.w);
         }
-        const float c[4] = {r.x + (b0.x + b1.x), r.y + (b0.y + b1.y), r.z + (b0.z + b1.z), r.w + (b0.w + b1.w)};
+        if constexpr (SPLIT) {
+            if (part) second[warp % kGroups][lane] = make_float4(c[0], c[1], c[2], c[3]);
+            __syncthreads();
+            if (part) return;
+            const float4 v = second[warp][lane];
+            c[0] += v.x;
+            c[1] += v.y;
+            c[2] += v.z;
+            c[3] += v.w;
+        }
+        if (live) {
+            const int64_t S = min(4 * q + g, a.Da - 1);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (4 * q + g < a.Da && col + u < a.Db)
-                y[S * a.Db + col + u] = c[u] + __ldg(a.uT + (col + u) * a.Pa + S);
+            for (int u = 0; u < 4; ++u)
+                if (4 * q + g < a.Da && col + u < a.Db)
+                    y[S * a.Db + col + u] = c[u] + __ldg(a.uT + (col + u) * a.Pa + S);
+        }
+        if (SPLIT) return;  // one group per pair of warps
     }
 }
 
-// Row chunks of the same-spin panels: blocks of 1,024 threads, one per SM, each on one
-// panel of 32 columns (118 KB of x at L=12: it stays in L1 or shared memory); the number
-// of chunks that leaves the fewest row groups on the busiest SM.
+// Row chunks of the same-spin panels: blocks of 512 threads, one per SM, each on one panel
+// of 32 columns (118 KB of x at L=12: it stays in L1 or shared memory); the number of
+// chunks that leaves the fewest row groups on the busiest SM. One panel (few strings of
+// the other spin) takes a chunk for every SM: L=20 4a1b, 1,212 row groups in at most 64
+// chunks left 88 SMs idle and its warps a second round (k_sigma_sum 113 us, the product 155;
+// with a chunk for every SM 101).
 int same_chunks(int64_t groups, int64_t panels) {
     const int64_t sms = sm_count();
     int best = 1;
     int64_t cost = INT64_MAX;
-    for (int c = 1; c <= 64 && (c - 1) * 8 < groups; ++c) {
+    for (int c = 1; c <= sms && (c - 1) * 8 < groups; ++c) {
         const int64_t per = (groups + c - 1) / c, rounds = (panels * c + sms - 1) / sms;
         if (per * rounds + 2 * rounds < cost) {  // a block's start and end: about two row groups
             cost = per * rounds + 2 * rounds;
@@ -702,7 +737,9 @@ void sigma_mv32(SigmaOp &op, const FciParams &p, const float *x, float *y, cudaS
                                                                                              op.xp.p, op.xT.p);
     k_sigma_parts<<<(unsigned)blocks, kThreads, smem, s>>>(a);
     const int pb = (int)((op.Db + kPanel - 1) / kPanel), c = same_chunks(ga, pb);
-    k_sigma_sum<<<dim3((unsigned)c, (unsigned)pb), kThreads, 0, s>>>(a, op.ea.p, op.nea, (int)((ga + c - 1) / c), op.xp.p, y);
+    const int per = (int)((ga + c - 1) / c);
+    const auto sum = 2 * per <= kWarps ? k_sigma_sum<true> : k_sigma_sum<false>;
+    sum<<<dim3((unsigned)c, (unsigned)pb), kThreads, 0, s>>>(a, op.ea.p, op.nea, per, op.xp.p, y);
     CIGPU_CUDA(cudaGetLastError());
     count_launch(3);
 }

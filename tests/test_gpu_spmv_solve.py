@@ -381,3 +381,23 @@ def test_mixed_folds_take_an_fp64_product(case, form, monkeypatch):
     for budget in (9, 14, 40):
         m.solve(tol=1e-13, max_matvec=budget)
         assert m.info["matvecs_fp32"] + m.info["matvecs_fp64"] <= budget + 1
+
+
+@pytest.mark.parametrize("L,na,nb", [(18, 4, 0), (15, 5, 0), (18, 0, 4), (15, 4, 1), (20, 1, 2)])
+def test_sigma_one_panel(L, na, nb, monkeypatch):
+    """The factorised FP32 product with few strings of one spin (down to none of its
+    electrons): one panel of columns, whose row chunks cover the SMs; the bound of
+    test_sigma_fp32_matvec."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("CIGPU_FP32_PRODUCT", "sigma")
+    ints = make_integrals(L, na, nb, nchol=12, seed=L + na)
+    ref = O.build_upper(O.FCI, ints)
+    m = build(FCI, ints, A.MIXED).get_mat()
+    x = np.random.default_rng(5).standard_normal(m.n).astype(np.float32).astype(np.float64)
+    y_ref = O.sym_mvprod(ref, x)
+    xd = torch.tensor(x, dtype=torch.float32, device="cuda")
+    yd = torch.full_like(xd, float("nan"))
+    m.mvprod_device(xd, yd)
+    torch.cuda.synchronize()
+    y = yd.cpu().numpy().astype(np.float64)
+    assert np.abs(y - y_ref).max() <= 2e-5 * np.abs(y_ref).max()
