@@ -531,8 +531,23 @@ constexpr size_t kSigmaMaxPanel = 192 * 1024;  // a same-spin panel held in shar
 // 15,876, 37 | 16 and 11 | 7.
 constexpr int64_t kSigmaMinRows = 40000;
 constexpr int64_t kSigmaMinRowsAnyRank = 50000;  // ranks above two passes of factors
-constexpr size_t kSigmaMaxTables = 132864;  // factors, pairs and excitation lists (bytes): past it, and not
-                                            // measured, the stored values serve
+
+// Whether the operator is the faster product on a grid that fills the GPU. Its time (us): 22
+// for the launches and the same-spin part, and for every pass of 16 factors and wave of
+// blocks 5 and 0.43 per single excitation of a row (fitted to 27.5 to 43 us a pass at 52
+// to 88 excitations). The stored values come at about 5.5 TB/s, rows padded to whole tiles
+// of beta strings. Measured, operator | stored, among others: L=15 3a3b (207,025 rows)
+// padded rank 112 272 | 311 us, 128 308 | 311; L=16 4a2b (218,400) 96 252 | 299, 128 326 |
+// 299; L=20 3a2b (216,600) 64 198 | 398, 128 364 | 398; L=12 6a6b 32 316 | 1,800.
+bool sigma_pays(const SpinTables &ta, const SpinTables &tb, int R) {
+    const auto pad = [](int64_t d) { return (d + kTile - 1) / kTile * kTile; };
+    const int64_t tiles = pad(ta.D) / kTile * (pad(tb.D) / kTile), sms = sm_count();
+    const int64_t slabs = sigma_slabs(tiles, R, sms), passes = (R / kC + slabs - 1) / slabs;
+    const int64_t waves = (2 * tiles * slabs + sms - 1) / sms;
+    const double op = 22.0 + (double)(waves * passes) * (5.0 + 0.43 * (ta.ns + tb.ns));
+    const double width = 1.0 + ta.ns + tb.ns + ta.nd + tb.nd + (double)ta.ns * tb.ns;
+    return op <= 4.0 * (double)ta.D * (double)pad(tb.D) * width / 5.5e6;
+}
 
 }  // namespace
 
@@ -625,9 +640,8 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
     const int rank = (int)vecs.size();
     const int R = std::max(kSigmaChunk, (rank + kSigmaChunk - 1) / kSigmaChunk * kSigmaChunk);
     if (!any_grid && small && R > 2 * kC && ta.D * tb.D < kSigmaMinRowsAnyRank) return false;
-    if (R > kSigmaMaxRank ||
-        sizeof(float) * N * (R + 1) + sizeof(uint2) * (size_t)kTile * (ta.ns + tb.ns) > kSigmaMaxTables ||
-        opposite_smem(L) > kSigmaMaxSmem || ta.D * std::max(ta.ns, 1) > (int64_t)UINT32_MAX)
+    if (!any_grid && !small && !sigma_pays(ta, tb, R)) return false;
+    if (R > kSigmaMaxRank || opposite_smem(L) > kSigmaMaxSmem || ta.D * std::max(ta.ns, 1) > (int64_t)UINT32_MAX)
         return false;
     // [R / 16][L^2][16]
     std::vector<float> F(N * R, 0.f), G(N * R, 0.f);

@@ -401,3 +401,20 @@ def test_sigma_one_panel(L, na, nb, monkeypatch):
     torch.cuda.synchronize()
     y = yd.cpu().numpy().astype(np.float64)
     assert np.abs(y - y_ref).max() <= 2e-5 * np.abs(y_ref).max()
+
+
+@pytest.mark.parametrize("L,na,nb,rank,padded", [(15, 3, 3, 105, 112), (16, 4, 2, 90, 96), (20, 3, 2, 60, 64)])
+def test_sigma_serves_high_ranks(L, na, nb, rank, padded):
+    """The factorised FP32 product at high ranks in many orbitals, where it is the faster
+    one: taken without being forced, and equal to the FP64 product of the stored matrix to
+    the bound of test_sigma_fp32_matvec."""
+    torch = pytest.importorskip("torch")
+    m = build(FCI, make_integrals(L, na, nb, nchol=rank, seed=L), A.MIXED).get_mat()
+    kind, _, got = A.fp32_product(m.handle)
+    assert (kind, got) == (A.FP32_SIGMA, padded)
+    x = torch.randn(m.n, dtype=torch.float32, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    y, y64 = torch.full_like(x, float("nan")), torch.empty(m.n, dtype=torch.float64, device="cuda")
+    m.mvprod_device(x, y)
+    m.mvprod_device(x.double(), y64)
+    torch.cuda.synchronize()
+    assert float((y.double() - y64).abs().max()) <= 2e-5 * float(y64.abs().max())
