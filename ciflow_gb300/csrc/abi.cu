@@ -241,8 +241,7 @@ static int64_t binom64(int n, int k) { return d_binom(n, k); }
 
 // The mixed FCI method's FP32 product, read at every build from CIGPU_FP32_PRODUCT:
 // "slots" takes the stored FP32 slot values, "sigma" the factorised sigma operator
-// on any space it supports, anything else the sigma operator where its tile grid
-// fills the GPU. Both are complete products; the choice exists to compare them.
+// on any space it supports, anything else the faster one by the strings and the rank. Both are complete products; the choice exists to compare them.
 enum SigmaMode { kSigmaOff = 0, kSigmaAuto = 1, kSigmaForced = 2 };
 int sigma_mode() {
     const char *e = std::getenv("CIGPU_FP32_PRODUCT");

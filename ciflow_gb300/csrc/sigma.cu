@@ -522,31 +522,36 @@ int sigma_slabs(int64_t tiles, int R, int64_t sms) {
 
 constexpr size_t kSigmaMaxSmem = 200 * 1024;
 constexpr size_t kSigmaMaxPanel = 192 * 1024;  // a same-spin panel held in shared memory
-// Spaces of fewer 32 x 32 string tiles than SMs: the operator's three launches take about
-// 40 us one after the other, the stored values a time by size; with other products beside
-// them only the work counts. Measured per product alone, and among others, operator |
-// stored: L=10 4a4b, 44,100 rows, rank 12, 40 | 38 and 12 | 28 us, rank 20, 42 | 38 and
-// 15 | 28, rank 60, 47 | 38 (whole mixed solve 27.8 | 25.5 ms; rank 20: 19.4 | 20.7);
-// L=10 5a5b, 63,504, rank 60, 50 | 67 and 32 | 39 (solve 25.4 | 28.3 ms); L=9 4a4b,
-// 15,876, 37 | 16 and 11 | 7.
-constexpr int64_t kSigmaMinRows = 40000;
-constexpr int64_t kSigmaMinRowsAnyRank = 50000;  // ranks above two passes of factors
+// A grid of fewer 32 x 32 string tiles than SMs.
+bool sigma_small_grid(const SpinTables &ta, const SpinTables &tb) {
+    return ((ta.D + 31) / 32) * ((tb.D + 31) / 32) < sm_count();
+}
 
-// Whether the operator is the faster product on a grid that fills the GPU. Its time (us): 22
-// for the launches and the same-spin part, and for every pass of 16 factors and wave of
-// blocks 5 and 0.43 per single excitation of a row (fitted to 27.5 to 43 us a pass at 52
-// to 88 excitations). The stored values come at about 5.5 TB/s, rows padded to whole tiles
-// of beta strings. Measured, operator | stored, among others: L=15 3a3b (207,025 rows)
-// padded rank 112 272 | 311 us, 128 308 | 311; L=16 4a2b (218,400) 96 252 | 299, 128 326 |
-// 299; L=20 3a2b (216,600) 64 198 | 398, 128 364 | 398; L=12 6a6b 32 316 | 1,800.
+// Whether the operator is the faster product, alone on the GPU. Its time (us): 22 for the
+// launches and the same-spin part, and for every pass of 16 factors and wave of blocks 5
+// and 0.43 per single excitation of a row (fitted to 27.5 to 43 us a pass at 52 to 88
+// excitations). The stored values come at about 5.5 TB/s, rows padded to whole tiles of
+// beta strings; on small grids at about 3.3 TB/s of the rows' own. Measured, operator |
+// stored, among others:
+//   L=15 3a3b (207,025 rows) padded rank 112 272 | 311 us, 128 308 | 311; L=16 4a2b (218,400)
+//   96 252 | 299, 128 326 | 299; L=20 3a2b (216,600) 64 198 | 398, 128 364 | 398; L=12 6a6b 32
+//   316 | 1,800;
+//   small grids: L=10 4a4b (44,100) 16 42 | 38, 64 47 | 39; L=10 5a4b (52,920) 16 43 | 64, 64
+//   49 | 64; L=12 3a3b (48,400) 16 45 | 48, 80 78 | 48; L=11 4a3b (54,450) 32 45 | 66, 80 74 |
+//   66; L=12 5a2b (52,272) 32 53 | 74, 80 108 | 74; L=11 4a4b (108,900) 80 107 | 125; L=13
+//   5a2b (100,386) 96 213 | 139; L=9 4a4b (15,876) 16 37 | 16.
+// With other solves beside, where only the work counts, any grid takes it (L=10 4a4b 12 | 28
+// us, L=9 4a4b 11 | 7).
 bool sigma_pays(const SpinTables &ta, const SpinTables &tb, int R) {
     const auto pad = [](int64_t d) { return (d + kTile - 1) / kTile * kTile; };
     const int64_t tiles = pad(ta.D) / kTile * (pad(tb.D) / kTile), sms = sm_count();
     const int64_t slabs = sigma_slabs(tiles, R, sms), passes = (R / kC + slabs - 1) / slabs;
     const int64_t waves = (2 * tiles * slabs + sms - 1) / sms;
     const double op = 22.0 + (double)(waves * passes) * (5.0 + 0.43 * (ta.ns + tb.ns));
+    const bool small = sigma_small_grid(ta, tb);
     const double width = 1.0 + ta.ns + tb.ns + ta.nd + tb.nd + (double)ta.ns * tb.ns;
-    return op <= 4.0 * (double)ta.D * (double)pad(tb.D) * width / 5.5e6;
+    const double bytes = 4.0 * (double)ta.D * (double)(small ? tb.D : pad(tb.D)) * width;
+    return op <= bytes / (small ? 3.3e6 : 5.5e6);
 }
 
 }  // namespace
@@ -567,8 +572,10 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
                    const SpinTables &tb, const FciParams &p, bool any_grid, cudaStream_t s) {
     op.R = 0;
     if (!sigma_applies(L) || ta.D < 1 || tb.D < 1) return false;
-    const bool small = ((ta.D + 31) / 32) * ((tb.D + 31) / 32) < sm_count();
-    if (!any_grid && small && ta.D * tb.D < kSigmaMinRows) return false;
+    // the padded ranks the space takes: none, and the factorisation need not begin
+    int most = kSigmaMaxRank;
+    while (!any_grid && most > 0 && !sigma_pays(ta, tb, most)) most -= kC;
+    if (most == 0) return false;
     const int L2 = L * L;
     const size_t N = (size_t)L2;
     // The factors, in the space of orbital pairs p >= q: with c = 1 on the diagonal
@@ -618,6 +625,7 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
             }
             vecs.push_back(std::move(l));
             sgn.push_back(1.0);
+            if ((int)vecs.size() > most) return false;  // so many positive pivots: the rank is no lower
             if (!psd) break;
         }
         if (!psd) {  // indefinite: eigenpairs of the pair matrix
@@ -639,9 +647,7 @@ bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const
     }
     const int rank = (int)vecs.size();
     const int R = std::max(kSigmaChunk, (rank + kSigmaChunk - 1) / kSigmaChunk * kSigmaChunk);
-    if (!any_grid && small && R > 2 * kC && ta.D * tb.D < kSigmaMinRowsAnyRank) return false;
-    if (!any_grid && !small && !sigma_pays(ta, tb, R)) return false;
-    if (R > kSigmaMaxRank || opposite_smem(L) > kSigmaMaxSmem || ta.D * std::max(ta.ns, 1) > (int64_t)UINT32_MAX)
+    if (R > most || opposite_smem(L) > kSigmaMaxSmem || ta.D * std::max(ta.ns, 1) > (int64_t)UINT32_MAX)
         return false;
     // [R / 16][L^2][16]
     std::vector<float> F(N * R, 0.f), G(N * R, 0.f);

@@ -31,9 +31,9 @@ inline bool sigma_applies(int L) { return L >= 1 && L <= kSigmaMaxL; }
 // Factorises (pq|rs) = sum_k s_k F^k_pq F^k_rs (a pivoted Cholesky factor of the
 // pair matrix to 1e-10 of its largest diagonal; eigenpairs when it is indefinite),
 // forms the per-string tables (p: the string tables on the device) and allocates the
-// work buffers. False (op.R = 0) when the space does not qualify (too many orbitals,
-// or fewer 32 x 32 string tiles than SMs unless any_grid) or the rank exceeds
-// kSigmaMaxRank.
+// work buffers. False (op.R = 0) when the space does not qualify (too many orbitals, or a
+// rank past kSigmaMaxRank or, unless any_grid, past the one to which the operator is faster
+// than the stored values).
 bool sigma_prepare(SigmaOp &op, int L, const double *h, const double *eri, const SpinTables &ta,
                    const SpinTables &tb, const FciParams &p, bool any_grid, cudaStream_t s);
 

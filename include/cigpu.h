@@ -153,7 +153,7 @@ int cigpu_crs_layout(const cigpu_crs *crs, int *layout, int64_t *stored);
  * stored matrix. rank and padded are 0 for the stored product. FP64 matrices
  * report CIGPU_FP32_STORED. The environment variable CIGPU_FP32_PRODUCT, read at
  * each build, selects "slots" or "sigma"; by default the sigma product is taken
- * where its 32 x 32 string tiles outnumber the SMs. */
+ * where, by the space's strings and the rank, it is the faster one. */
 enum { CIGPU_FP32_STORED = 0, CIGPU_FP32_SIGMA = 1 };
 int cigpu_crs_fp32_product(const cigpu_crs *crs, int *kind, int *rank, int *padded);
 /* Upper triangle in the reference layout (SparseMatrix_CRS::row/col/data,

@@ -418,3 +418,13 @@ def test_sigma_serves_high_ranks(L, na, nb, rank, padded):
     m.mvprod_device(x.double(), y64)
     torch.cuda.synchronize()
     assert float((y.double() - y64).abs().max()) <= 2e-5 * float(y64.abs().max())
+
+
+@pytest.mark.parametrize("L,na,nb,rank,sigma", [(10, 4, 4, 12, False), (10, 4, 4, 30, False), (10, 5, 4, 16, True),
+                                                (10, 5, 5, 55, True), (12, 3, 3, 16, True), (11, 4, 3, 66, False),
+                                                (11, 4, 3, 30, True), (12, 5, 2, 78, False), (9, 4, 4, 16, False)])
+def test_fp32_product_choice(L, na, nb, rank, sigma):
+    """The FP32 product by strings and rank on small grids: the factorised one only where
+    it was measured to be the faster."""
+    m = build(FCI, make_integrals(L, na, nb, nchol=rank, seed=rank), A.MIXED).get_mat()
+    assert A.fp32_product(m.handle)[0] == (A.FP32_SIGMA if sigma else A.FP32_STORED)
