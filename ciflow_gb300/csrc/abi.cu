@@ -640,7 +640,8 @@ void crs_mv64(cigpu_crs &c, const double *x, double *y, cudaStream_t s) {
         return;
     }
     if (c.precision == CIGPU_FP64) {
-        spmv_f64(c.dim, c.nnz_full, c.row_ptr.p, c.col.p, c.val64.p, x, y, s, c.method == CIGPU_FCI);
+        const RowKind kind = c.method == CIGPU_FCI ? RowKind::kFci : c.method == CIGPU_DOCI ? RowKind::kDoci : RowKind::kList;
+        spmv_f64(c.dim, c.nnz_full, c.row_ptr.p, c.col.p, c.val64.p, x, y, s, kind);
         return;
     }
     if (c.val32lo.p || c.nnz_full == 0) {

@@ -131,36 +131,23 @@ int sm_count_spmv() {
     return sms;
 }
 
-// Lanes per row from the mean row length (in 4-element chunks), and chunks per lane and
-// round. FP64 products are bound by the FP64 pipe as much as by memory: a lane without an
-// element in a round, and every step of a row's final sum, costs the pipe a full warp.
-//   * DOCI rows (18-36 chunks): 4 lanes in FP64 from 12,000 rows (L=20 8 pairs, 125,970
-//     rows: 52 us with 8 lanes, 41 with 4; L=24: 1,241 and 1,068; L=14, 3,432 rows, 5.2
-//     and 6.2: too few warps), else 8, five chunks each (one round covers a row's 36).
-//   * longer rows: 32 lanes, four chunks each; FCI rows, all of one length, two in FP64
-//     (fewer registers: L=9 4a3b, 504 elements, 22.7 -> 18.6 us, L=8 4a4b 12.4 -> 11.3;
-//     determinant lists' uneven rows lose by it: 20.6 and 24.5 at 595).
-// The grid covers the rows once (at most a full persistent grid), so a small matrix
-// leaves SMs free for the kernels of concurrent solves on other streams.
-constexpr int64_t kFourLaneRows = 12000;
-
+// The shape by row_shape. The grid covers the rows once (at most a full persistent grid),
+// so a small matrix leaves SMs free for the kernels of concurrent solves on other streams.
 template <typename F>
 static void launch_rows(int64_t n, int64_t nnz, const int64_t *row_ptr, const uint32_t *col, const F &f0,
-                        typename F::X *y, cudaStream_t s, bool equal_rows = false) {
+                        typename F::X *y, cudaStream_t s, RowKind kind = RowKind::kList) {
     F f = f0;
     f.nx = (uint64_t)n;
     f.err = check_word_device();
-    constexpr bool kFp64 = std::is_same<F, Plain<double>>::value;
-    const double chunks = n > 0 ? (double)nnz / n / 4.0 : 0;
-    const int G = chunks >= 48 ? 32 : (kFp64 && n >= kFourLaneRows) ? 4 : 8;
-    const int64_t need = (n * G + kSpmvThreads - 1) / kSpmvThreads;
+    const RowShape shape = row_shape(n, nnz, std::is_same<F, Plain<double>>::value, kind);
+    const int64_t need = (n * shape.lanes + kSpmvThreads - 1) / kSpmvThreads;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(spmv_grid(), need));
-    if (G == 32) {
-        if (kFp64 && equal_rows)
+    if (shape.lanes == 32) {
+        if (shape.chunks == 2)
             k_spmv_rows<F, 32, 2><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
         else
             k_spmv_rows<F, 32, 4><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
-    } else if (G == 4) {
+    } else if (shape.lanes == 4) {
         k_spmv_rows<F, 4, 2><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
     } else {
         k_spmv_rows<F, 8, 5><<<grid, kSpmvThreads, 0, s>>>(n, row_ptr, col, f, y);
@@ -196,8 +183,8 @@ void spmv_f64_shape(int64_t n, const int64_t *row_ptr, const uint32_t *col, cons
 }
 
 void spmv_f64(int64_t n, int64_t nnz, const int64_t *row_ptr, const uint32_t *col, const double *val, const double *x,
-              double *y, cudaStream_t s, bool equal_rows) {
-    launch_rows(n, nnz, row_ptr, col, Plain<double>{val, x}, y, s, equal_rows);
+              double *y, cudaStream_t s, RowKind kind) {
+    launch_rows(n, nnz, row_ptr, col, Plain<double>{val, x}, y, s, kind);
 }
 
 void spmv_f32(int64_t n, int64_t nnz, const int64_t *row_ptr, const uint32_t *col, const float *val, const float *x,

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "cigpu_internal.h"
+#include "row_shape.h"
 
 namespace cigpu {
 
@@ -11,7 +12,7 @@ constexpr int kSpmvBlocksPerSM = 8;
 int sm_count_spmv();
 int spmv_grid();
 void spmv_f64(int64_t n, int64_t nnz, const int64_t *row_ptr, const uint32_t *col, const double *val, const double *x, double *y,
-              cudaStream_t s, bool equal_rows = false);
+              cudaStream_t s, RowKind kind = RowKind::kList);
 // FP64 CRS matvec with an explicit shape: `lanes` (4, 8, 16 or 32) lanes per row,
 // `grid` blocks of kSpmvThreads (the batched solver's autotuner picks both). With
 // row_prob non-null, row r is skipped when status[row_prob[r]] != 0 (finished
