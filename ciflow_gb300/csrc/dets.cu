@@ -728,8 +728,8 @@ __global__ void __launch_bounds__(32, 32) k_dets_scan(const DetParams p) {
 // The build where no integral is dropped (every |(pq|rs)| > 1e-14: molecules without
 // symmetry, rotated orbitals). The row structure is then the connected pairs, so the
 // count pass evaluates nothing: it scans, tests the pairs that pass exactly in place and,
-// while they fit kMaskBytes, leaves the 32-column masks (n^2 / 8 bytes) for the fill. The
-// fill reads the masks (or scans again), and every element's place follows from its row's
+// while they fit kMaskBytes and the device's memory, leaves the 32-column masks (n^2 / 8
+// bytes) for the fill. The fill reads the masks (or scans again), and every element's place follows from its row's
 // count as it is queued, so doubles and singles are written as they are evaluated. An
 // element that vanishes all the same (a difference of equal integrals) is counted, and
 // the build starts again with the passes above, which evaluate twice. L=32 8a8b CISD
@@ -1684,7 +1684,12 @@ int build_dets(cigpu_ham *ham, int64_t ndet, int words, const uint64_t *up, cons
         auto passes = [&](bool structure) {
             DevBuf<uint32_t> masks;
             const size_t words = (size_t)((nb + 31) / 32);
-            if (structure && words * words * 32 * sizeof(uint32_t) <= kMaskBytes) masks.alloc(words * words * 32);
+            if (structure && words * words * 32 * sizeof(uint32_t) <= kMaskBytes) {
+                try {
+                    masks.alloc(words * words * 32);
+                } catch (const std::bad_alloc &) {  // the fill scans again
+                }
+            }
             p.masks = masks.p;
             CIGPU_CUDA(cudaMemsetAsync(count.p, 0, count.bytes(), s));
             CIGPU_CUDA(cudaMemsetAsync(c->upper_off.p, 0, c->upper_off.bytes(), s));
@@ -1705,17 +1710,28 @@ int build_dets(cigpu_ham *ham, int64_t ndet, int words, const uint64_t *up, cons
             CIGPU_CUDA(cudaStreamSynchronize(s));
             c->nnz_full = nnz;
             c->nnz_upper = nnz - (int64_t)nlow;
-            c->col.alloc(std::max<int64_t>(nnz, 1));
-            p.col = c->col.p;
-            if (precision == CIGPU_FP64) {
-                c->val64.alloc(std::max<int64_t>(nnz, 1));
-                p.val64 = c->val64.p;
-            } else {
-                c->val32.alloc(std::max<int64_t>(nnz, 1));
-                c->val32lo.alloc(std::max<int64_t>(nnz, 1));
-                p.val32 = c->val32.p;
-                p.val32lo = c->val32lo.p;
+            const auto storage = [&] {
+                const size_t n = (size_t)std::max<int64_t>(nnz, 1);
+                c->col.alloc(n);
+                if (precision == CIGPU_FP64) {
+                    c->val64.alloc(n);
+                } else {
+                    c->val32.alloc(n);
+                    c->val32lo.alloc(n);
+                }
+            };
+            try {
+                storage();
+            } catch (const std::bad_alloc &) {  // without the masks' memory held beside it
+                if (!masks.p) throw;
+                masks.release();
+                p.masks = nullptr;
+                storage();
             }
+            p.col = c->col.p;
+            p.val64 = c->val64.p;
+            p.val32 = c->val32.p;
+            p.val32lo = c->val32lo.p;
             if (structure && precision == CIGPU_FP64)
                 pairs<kDetFill64>(p, W, s);
             else if (structure)
