@@ -541,13 +541,20 @@ void build_crs(cigpu_crs &c, cudaStream_t s) {
         // pairs 745 against 1,068 us, L=26, 8 pairs (1,562,275) 469 against 607; L=20, 10
         // pairs (184,756), whose rows lie in L2 in part, 60.3 against 63.5, L=30, 5 pairs
         // (142,506) 80 against 57.
+        // Only where no pair hop is dropped: every row then holds all its hops. With dropped
+        // ones (K_jk <= 1e-14, a lattice's) the stored rows are shorter, and a vector's
+        // infinity or NaN reaches the rows that hold an element of its column and no others
+        // (a hop of value 0 would carry it). L=24, 12 pairs, no hop kept: 272 us from the
+        // rows, 744 by the hops.
         if (c.allow_compact && c.precision == CIGPU_FP64 && dim >= kSplitPlainRows) {
             c.kpair64.alloc((size_t)c.L * c.L);
-            c.kpair32.alloc((size_t)c.L * c.L);
-            doci_pair_table_launch(c.L, h.d_eri.p, c.kpair64.p, c.kpair32.p, s);
-            doci_split_make(c.L, c.nup, dim, c.split, s);
-            c.split_tried = true;
+            doci_pair_table_launch(c.L, h.d_eri.p, c.kpair64.p, nullptr, s);
+            if (count_nonzero(c.kpair64.p, (int64_t)c.L * c.L, s) == (int64_t)c.L * (c.L - 1)) {
+                doci_split_make(c.L, c.nup, dim, c.split, s);
+                c.split_tried = true;
+            }
             c.split_product = (bool)c.split;
+            if (!c.split_product) c.kpair64.release();
         }
     }
     if (c.side) {

@@ -483,7 +483,8 @@ void launch_split(const DociSplit &sp, const T *K, const T *diag, const T *x, T 
     count_launch();
 }
 
-// K_jk = (jk|jk) (chemist), zero where |v| <= 1e-14 and on the diagonal; FP64 and FP32.
+// K_jk = (jk|jk) (chemist), zero where |v| <= 1e-14 and on the diagonal; FP64, and FP32
+// where K32 is given.
 __global__ void k_doci_pair_table(int L, const double *__restrict__ eri, double *__restrict__ K64,
                                   float *__restrict__ K32) {
     const int L1 = L;
@@ -494,7 +495,7 @@ __global__ void k_doci_pair_table(int L, const double *__restrict__ eri, double 
         double v = (j == k) ? 0.0 : eri[lo * L3 + hi * L2 + lo * L1 + hi];
         if (!(v > kZero || v < -kZero)) v = 0.0;
         K64[t] = v;
-        K32[t] = (float)v;
+        if (K32) K32[t] = (float)v;
     }
 }
 

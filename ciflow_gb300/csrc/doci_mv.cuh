@@ -58,7 +58,7 @@ struct DociSplit {
 void doci_split_make(int L, int n, int64_t D, DociSplit &plan, cudaStream_t s);
 
 // K_jk = (jk|jk) for j != k, zero where |v| <= 1e-14 (and on the diagonal): the
-// pair-hop values, FP64 and FP32 (L*L each, device).
+// pair-hop values, FP64 and (K32 may be null) FP32 (L*L each, device).
 void doci_pair_table_launch(int L, const double *eri, double *K64, float *K32, cudaStream_t s);
 // Entries of v with |v| > 1e-14 (synchronises s).
 int64_t count_nonzero(const double *v, int64_t n, cudaStream_t s);

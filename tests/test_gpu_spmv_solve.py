@@ -428,3 +428,34 @@ def test_fp32_product_choice(L, na, nb, rank, sigma):
     it was measured to be the faster."""
     m = build(FCI, make_integrals(L, na, nb, nchol=rank, seed=rank), A.MIXED).get_mat()
     assert A.fp32_product(m.handle)[0] == (A.FP32_SIGMA if sigma else A.FP32_STORED)
+
+
+def test_plain_doci_dropped_hops():
+    """A large plain DOCI matrix with dropped pair hops (exchange integrals of zero)
+    multiplies its stored elements: a NaN and an infinity in x reach the rows that hold an
+    element of their columns, and no others."""
+    torch = pytest.importorskip("torch")
+    import scipy.sparse as sp
+    L, n = 24, 8  # 735,471 rows
+    ints = make_integrals(L, n, n, nchol=4, seed=3)
+    chain = np.abs(np.arange(L)[:, None] - np.arange(L)) == 1
+    for j in range(L):
+        for k in range(L):
+            if j != k and not chain[j, k]:
+                ints.eri[j, k, j, k] = ints.eri[j, k, k, j] = 0.0
+    m = build(DOCI, ints).get_mat()
+    row, col, val = m.full()
+    H = sp.csr_matrix((val, col.astype(np.int64), row.astype(np.int64)), shape=(m.n, m.n))
+    x = np.random.default_rng(1).standard_normal(m.n)
+    x[[5, 400000]] = np.nan, np.inf
+    y = torch.empty(m.n, dtype=torch.float64, device="cuda")
+    m.mvprod_device(torch.tensor(x, device="cuda"), y)
+    torch.cuda.synchronize()
+    y = y.cpu().numpy()
+    with np.errstate(invalid="ignore"):
+        y_ref = H @ x
+    met = np.asarray(abs(H)[:, [5, 400000]].sum(1)).ravel() > 0
+    assert np.array_equal(~np.isfinite(y), met) and np.array_equal(np.isnan(y), np.isnan(y_ref))
+    most = abs(H) @ np.where(np.isfinite(x), np.abs(x), 0.0)
+    ok = ~met
+    assert np.all(np.abs(y[ok] - y_ref[ok]) <= 2 * (2 * L + 3) * 2.0 ** -53 * most[ok])
