@@ -585,6 +585,10 @@ def run_cigpu(args, rank: int, world: int, dist):
             roof[tag]["fp64_pipe"] = {"dfma_per_launch": fmas, "achieved_dfma_per_s": fmas / t,
                                       "peak_dfma_per_s": peak_fma, "frac": fmas / t / peak_fma,
                                       "note": "2 FP64 FMA per clock per SM x SMs x 2070 MHz"}
+            if A.hop_product(crs) == A.HOPS_SPLIT:  # reads no matrix: the FP64 pipe is its bound
+                roof[tag].update({"bound": "fp64", "achieved": 2 * fmas / t / 1e12, "peak": 2 * peak_fma / 1e12,
+                                  "unit": "TFLOP/s", "frac": fmas / t / peak_fma,
+                                  "peak_source": "nominal FP64 FMA rate: SMs x 2 lanes x 2 flops x 2070 MHz"})
         lib.cigpu_crs_destroy(crs)
 
     # e2e through the C ABI with host buffers, H2D of the integrals and D2H of c inside the region

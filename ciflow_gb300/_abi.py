@@ -20,6 +20,7 @@ DETS_CRS, DETS_ONTHEFLY = 0, 1
 FP64, MIXED = 0, 1
 LAYOUT_CRS, LAYOUT_SLOTS, LAYOUT_ONTHEFLY, LAYOUT_PAIRS = 0, 1, 2, 3
 FP32_STORED, FP32_SIGMA = 0, 1
+HOPS_STORED, HOPS_ROWS, HOPS_SPLIT = 0, 1, 2
 
 _P = ctypes.c_void_p
 _I = ctypes.c_int
@@ -101,6 +102,7 @@ SIGNATURES = {
     "cigpu_crs_dims": (_I, [_P, _P, _P, _P]),
     "cigpu_crs_layout": (_I, [_P, _P, _P]),
     "cigpu_crs_fp32_product": (_I, [_P, _P, _P, _P]),
+    "cigpu_crs_hop_product": (_I, [_P, _P]),
     "cigpu_crs_export_upper": (_I, [_P, _P, _P, _P]),
     "cigpu_crs_export_full": (_I, [_P, _P, _P, _P]),
     "cigpu_mvprod": (_I, [_P, _P, _P, _P]),
@@ -211,6 +213,13 @@ def fp32_product(handle) -> tuple[int, int, int]:
     return kind.value, rank.value, padded.value
 
 
+def hop_product(handle) -> int:
+    """How a DOCI matrix's products form the pair hops (cigpu_crs_hop_product)."""
+    kind = ctypes.c_int()
+    check(lib().cigpu_crs_hop_product(handle, ctypes.byref(kind)))
+    return kind.value
+
+
 def sigma_work(L: int, nup: int, ndown: int, rank: int, padded: int) -> dict:
     """Algorithmic work of one FP32 sigma product on the FCI space (nup, ndown) of L
     orbitals with `rank` factors: FP32 FMAs per determinant (the same-spin elements of
@@ -228,18 +237,20 @@ def sigma_work(L: int, nup: int, ndown: int, rank: int, padded: int) -> dict:
 
 
 def matvec_bytes(handle, fp32: bool) -> tuple[int, str]:
-    """Algorithmic bytes of one matvec for the stored layout: one read of the stored
-    matrix and of x, one write of y. FP32: FP32 values/x/y; FP64: FP64 x/y with FP64
-    values (plain CRS) or the split hi + lo values (MIXED). Plain DOCI matrices from
-    500,000 rows keep their CRS but multiply matrix-free: these are the bytes of the rows
-    that such a product does not read."""
+    """Algorithmic bytes of one matvec for the form that multiplies: one read of the
+    stored matrix and of x, one write of y. FP32: FP32 values/x/y; FP64: FP64 x/y with
+    FP64 values (plain CRS) or the split hi + lo values (MIXED). DOCI products that
+    generate the pair hops read the diagonal and x (and, row by row, the strings)."""
     dim, nu, nf = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int64()
     check(lib().cigpu_crs_dims(handle, ctypes.byref(dim), ctypes.byref(nu), ctypes.byref(nf)))
     lay, stored = ctypes.c_int(), ctypes.c_int64()
     check(lib().cigpu_crs_layout(handle, ctypes.byref(lay), ctypes.byref(stored)))
+    hops = hop_product(handle)
     n, m = dim.value, stored.value
     sx = 4 if fp32 else 8
-    if lay.value == LAYOUT_PAIRS:  # matrix-free DOCI: strings, diagonal, x, y (hop gathers hit x in L2)
+    if hops == HOPS_SPLIT:  # diagonal, x, y (the hop gathers hit x in L2)
+        return 3 * n * sx, "doci-split-fp32" if fp32 else "doci-split-fp64"
+    if hops == HOPS_ROWS:  # and the strings
         return n * (8 + 3 * sx), "doci-pairs-fp32" if fp32 else "doci-pairs-fp64"
     if lay.value == LAYOUT_SLOTS:
         sv = 4 if fp32 else 8  # FP32 values, or FP64 values / FP32 hi + lo

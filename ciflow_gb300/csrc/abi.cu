@@ -969,6 +969,15 @@ int cigpu_crs_fp32_product(const cigpu_crs *crs, int *kind, int *rank, int *padd
     return CIGPU_OK;
 }
 
+int cigpu_crs_hop_product(const cigpu_crs *crs, int *kind) {
+    if (!crs || !kind) return CIGPU_EINVAL;
+    if (crs->pairs)
+        *kind = crs->split ? CIGPU_HOPS_SPLIT : CIGPU_HOPS_ROWS;
+    else
+        *kind = crs->split_product ? CIGPU_HOPS_SPLIT : CIGPU_HOPS_STORED;
+    return CIGPU_OK;
+}
+
 int cigpu_crs_export_upper(cigpu_crs *crs, uint32_t *row, uint32_t *col, double *val) {
     if (!crs || !row || !col || !val) return CIGPU_EINVAL;
     if (crs->onthefly) return CIGPU_ENOTSUP;

@@ -156,6 +156,14 @@ int cigpu_crs_layout(const cigpu_crs *crs, int *layout, int64_t *stored);
  * where, by the space's strings and the rank, it is the faster one. */
 enum { CIGPU_FP32_STORED = 0, CIGPU_FP32_SIGMA = 1 };
 int cigpu_crs_fp32_product(const cigpu_crs *crs, int *kind, int *rank, int *padded);
+/* How a DOCI matrix's products form the pair hops (no reference counterpart; reported
+ * with matvec measurements). CIGPU_HOPS_STORED: they read the stored elements (and every
+ * matrix of another method). CIGPU_HOPS_ROWS: generated row by row from the pair strings.
+ * CIGPU_HOPS_SPLIT: generated by low and high orbitals, from x, the diagonal and tables of
+ * the orbitals; plain matrices of 500,000 rows and more whose pair hops are all kept
+ * multiply so too, and keep their CRS (CIGPU_LAYOUT_CRS) for the exports. */
+enum { CIGPU_HOPS_STORED = 0, CIGPU_HOPS_ROWS = 1, CIGPU_HOPS_SPLIT = 2 };
+int cigpu_crs_hop_product(const cigpu_crs *crs, int *kind);
 /* Upper triangle in the reference layout (SparseMatrix_CRS::row/col/data,
  * SparseMatrix_CRS.h:107-111): row[dim+1], col[nnz_upper], val[nnz_upper]. Host buffers. */
 int cigpu_crs_export_upper(cigpu_crs *crs, uint32_t *row, uint32_t *col, double *val);

@@ -459,3 +459,20 @@ def test_plain_doci_dropped_hops():
     most = abs(H) @ np.where(np.isfinite(x), np.abs(x), 0.0)
     ok = ~met
     assert np.all(np.abs(y[ok] - y_ref[ok]) <= 2 * (2 * L + 3) * 2.0 ** -53 * most[ok])
+
+
+def test_matvec_bytes_follow_the_product():
+    """The bytes reported with a matvec are those of the form that multiplies: a large
+    plain DOCI matrix keeps its CRS and reads none of it."""
+    for L, n, precision, hops, per_row in [(23, 8, A.FP64, A.HOPS_STORED, None), (24, 8, A.FP64, A.HOPS_SPLIT, 24),
+                                           (24, 8, A.MIXED, A.HOPS_SPLIT, 24), (14, 7, A.MIXED, A.HOPS_ROWS, 32)]:
+        m = build(DOCI, make_integrals(L, n, n, nchol=4, seed=L), precision).get_mat()
+        assert A.hop_product(m.handle) == hops
+        nbytes, layout = A.matvec_bytes(m.handle, False)
+        if per_row is None:
+            assert layout == "crs-fp64" and nbytes == 12 * m.nnz_full + 8 * (m.n + 1) + 16 * m.n
+        else:
+            assert layout == {A.HOPS_SPLIT: "doci-split-fp64", A.HOPS_ROWS: "doci-pairs-fp64"}[hops]
+            assert nbytes == per_row * m.n
+    m = build(FCI, make_integrals(8, 4, 4, nchol=4, seed=1)).get_mat()
+    assert A.hop_product(m.handle) == A.HOPS_STORED
