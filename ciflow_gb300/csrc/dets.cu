@@ -930,10 +930,36 @@ struct MatvecWarp {
     uint16_t at[kQueue], single[kQueue];  // row << 9 | word << 5 | column; queue positions of the singles
 };
 
+// Rows of the matvec's groups of 32, in runs of 2^shift consecutive ones from as many places
+// of the list: in a list ordered by excitation the best connected rows stand together, and
+// a block with 32 of them (a CISD list's reference and first singles) ends long after the
+// others. Whole runs keep the words that many of a group's rows meet. Rows of one word in
+// runs of 16, of two in runs of 8 (their elements take longer), in order from 8 groups
+// per SM, where other groups fill the wait. Alone and among other products, runs | in
+// order: L=70 4a4b, 6,100 rows 302 and 172 | 517 and 180 us, 14,000 822 and 728 | 1,067
+// and 773 (the matvec of a warp per row and element it replaced: 368 and 1,268 alone);
+// L=24 6a6b, 16,471 513 and 394 | 540 and 398; L=28 7a7b, 21,500 885 and 480 | 1,159 and
+// 500; L=32 8a8b, 35,000 1,485 and 1,134 | 2,211 and 1,273, 52,705 3,071 and 2,629 | 2,898
+// and 2,504. Lists in no order take the same time either way, but for where the group of
+// their best connected row stands in the grid.
+// The rows of the stored block make groups of their own, which skip its columns; its last
+// ones, short of a group, go with the rest.
+struct MvRows {
+    int64_t inside, outside;  // groups of the stored block's rows, and of the others
+    int shift;
+    // the place in the list of a group's row `lane`: n or more where there is none
+    __device__ int64_t place(int64_t group, int lane) const {
+        const bool in = group < inside;
+        const int64_t groups = in ? inside : outside, g = in ? group : group - inside;
+        const int64_t i = (((lane >> shift) * groups + g) << shift) + (lane & ((1 << shift) - 1));
+        return in ? i : inside * kScanRows + i;
+    }
+};
+
 // Evaluates the queued words (n pairs in all, `mine` of the lane's row) and adds them.
 template <int W, int NW>
-__device__ __noinline__ double matvec_flush(const DetParams &p, MatvecWarp<W, NW> &q, const ScanRow<W> &rows, int64_t r0,
-                                            int span, int n, int mine, const double *__restrict__ x, double acc) {
+__device__ __noinline__ double matvec_flush(const DetParams &p, MatvecWarp<W, NW> &q, const ScanRow<W> &rows,
+                                            const int64_t *at, int span, int n, int mine, const double *__restrict__ x, double acc) {
     using U = std::conditional_t<NW == 2, uint32_t, uint64_t>;
     const int lane = threadIdx.x & 31;
     int start = mine;
@@ -961,7 +987,7 @@ __device__ __noinline__ double matvec_flush(const DetParams &p, MatvecWarp<W, NW
             int64_t j;
             place(k, row, j);
             const double xj = __ldg(x + j);
-            const double v = pair_of<W, U>(p, rows.s[row], r0 + row, j, single);
+            const double v = pair_of<W, U>(p, rows.s[row], at[row], j, single);
             if (!single) q.val[k] = v;
             q.xv[k] = xj;
         }
@@ -989,15 +1015,17 @@ __device__ __noinline__ double matvec_flush(const DetParams &p, MatvecWarp<W, NW
 }
 
 template <int W, int NW, bool RANGED, int CL>
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * kMvWarps, 3) k_dets_matvec(const DetParams p, const double *__restrict__ x,
-                                                                  double *__restrict__ y) {
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * kMvWarps, 3)
+    k_dets_matvec(const DetParams p, const MvRows map, const double *__restrict__ x, double *__restrict__ y) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ScanRow<W> rows;
+    __shared__ int64_t at[kScanRows];  // the rows' places in the list
     __shared__ double part[kMvWarps][kScanRows];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x % CL;  // of the rows' blocks
     MatvecWarp<W, NW> &q = reinterpret_cast<MatvecWarp<W, NW> *>(smem)[warp];
-    const int64_t r0 = (int64_t)(blockIdx.x / CL) * kScanRows, i = r0 + lane;
+    const int64_t group = blockIdx.x / CL;
+    const int64_t i = map.place(group, lane);
     const bool active = i < p.n;
     uint64_t rec[2 * W];
 #pragma unroll
@@ -1005,11 +1033,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * kMvWarps, 3) k
     uint32_t rk[NW];
     scan_key<W, NW>(rec, rk);
     if (warp == 0) {
+        at[lane] = i;
 #pragma unroll
         for (int w = 0; w < 2 * W; ++w) rows.s[lane][w] = rec[w];
     }
     __syncthreads();
-    const int64_t c_lo = (RANGED && r0 + kScanRows <= p.block) ? p.block : 0;  // the stored rows' pairs outside the block
+    const int64_t c_lo = (RANGED && group < map.inside) ? p.block : 0;  // the stored rows' pairs outside the block
     const int64_t words = (p.n - c_lo + 31) / 32;
     const uint32_t one = p.one;
     uint64_t next[2 * W];
@@ -1021,7 +1050,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * kMvWarps, 3) k
     int span = 0, n = 0, mine = 0;
     double acc = 0;
     auto flush = [&] {
-        acc = matvec_flush<W, NW>(p, q, rows, r0, span, n, mine, x, acc);
+        acc = matvec_flush<W, NW>(p, q, rows, at, span, n, mine, x, acc);
         span = n = mine = 0;
     };
     auto add = [&](int64_t base, uint32_t m, int total) {
@@ -1081,7 +1110,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * kMvWarps, 3) k
 // the kernel above, whose 32 rows to a warp leave a short list's blocks too few. Alone,
 // and among other products, this | that: 1,577 rows of L=36 44 | 126 and 17 | 46 us; 5,665
 // of L=20 133 | 280 and 107 | 123; 6,189 of L=24 236 | 138 and 129 | 76; 12,290 of L=28
-// 623 | 262 and 400 | 173.
+// 623 | 262 and 400 | 173; longer strings the same (ordered lists, one right after another):
+// 6,100 rows of L=60 195 | 220, 8,000 290 | 286, of L=70 (two words) 3,000 141 | 129, 6,100
+// 335 | 296, 10,000 683 | 548.
 constexpr int64_t kMvShort = 6000;
 
 template <int W>
@@ -1222,12 +1253,16 @@ void matvec(const DetParams &p, int W, const double *x, double *y, cudaStream_t 
                 k_dets_matvec_rows<w(), nw(), false><<<blocks, 32 * kMvWarps, 0, s>>>(p, x, y);
             return;
         }
-        const unsigned groups = (unsigned)((p.n + kScanRows - 1) / kScanRows);
+        MvRows map;
+        map.inside = ranged ? p.block / kScanRows : 0;
+        map.outside = (p.n - map.inside * kScanRows + kScanRows - 1) / kScanRows;
+        const unsigned groups = (unsigned)(map.inside + map.outside);
+        map.shift = groups >= 8 * (unsigned)sm_count() ? 5 : w() == 2 ? 3 : 4;
         constexpr int smem = (int)sizeof(MatvecWarp<w(), nw()>) * kMvWarps;
         auto go = [&](auto kern, unsigned blocks) {
             // the same value at every call: concurrent callers never lower it
             CIGPU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            kern<<<blocks, 32 * kMvWarps, smem, s>>>(p, x, y);
+            kern<<<blocks, 32 * kMvWarps, smem, s>>>(p, map, x, y);
         };
         const bool two = groups < 4 * (unsigned)sm_count();
         if (ranged && two)

@@ -262,3 +262,42 @@ def test_matvec_of_a_longer_list(L, na, nb, n, repeat):
     tol = 2.0 ** -52 * (len(up) + 2) * float(np.abs(val).max() * np.abs(x).max()) * np.sqrt(len(up))
     for keep in (0, 777):
         assert np.abs(CI_Big(ham, up=up, down=down, keep=keep).get_mat().mvprod(x) - y).max() <= tol
+
+
+def cisd_list(L, na, nb):
+    """(up, down) strings as Python integers: the lowest determinant, its singles and its
+    doubles, in the order a program writes them."""
+    import itertools
+
+    def excited(n, k):
+        ref = (1 << n) - 1
+        return [ref ^ sum(1 << o for o in hs + ps) for hs in itertools.combinations(range(n), k)
+                for ps in itertools.combinations(range(n, L), k)]
+
+    ra, rb, a1, b1 = (1 << na) - 1, (1 << nb) - 1, excited(na, 1), excited(nb, 1)
+    pairs = [(ra, rb)] + [(a, rb) for a in a1] + [(ra, b) for b in b1]
+    pairs += [(a, rb) for a in excited(na, 2)] + [(ra, b) for b in excited(nb, 2)]
+    return pairs + [(a, b) for a in a1 for b in b1]
+
+
+@pytest.mark.parametrize("L,na,nb,n", [(70, 3, 2, 6043), (70, 3, 3, 20001), (40, 3, 3, 6100), (24, 4, 4, 6001),
+                                       (36, 6, 6, 40001)])
+def test_matvec_of_an_ordered_list(L, na, nb, n):
+    """The matvec without a stored matrix on lists in order of excitation, whose groups take
+    runs of rows from all over the list: one and two words per string, one and two blocks
+    per group, groups in order (the longest list), whole and with stored leading blocks of
+    whole groups and of a part of one, against the stored CRS."""
+    pairs = cisd_list(L, na, nb)[:n]
+    words = 1 if L <= 64 else 2
+    up, down = (np.array([(s >> (64 * w)) & (2 ** 64 - 1) for s in side for w in range(words)], np.uint64)
+                for side in zip(*pairs))
+    ints = make_integrals(L, na, nb, nchol=2, seed=L)
+    ham = Hamiltonian.from_integrals(ints)
+    x = np.random.default_rng(6).standard_normal(len(pairs))
+    stored = FCI_File(ham, up=up, down=down).get_mat()
+    assert stored.n == len(pairs) > 6000
+    y = stored.mvprod(x)
+    _, _, val = stored.full()
+    tol = 2.0 ** -52 * (len(pairs) + 2) * float(np.abs(val).max() * np.abs(x).max()) * np.sqrt(len(pairs))
+    for keep in (0, 777, 3200):
+        assert np.abs(CI_Big(ham, up=up, down=down, keep=keep).get_mat().mvprod(x) - y).max() <= tol
