@@ -25,10 +25,9 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 PORT_LIB = os.path.join(HERE, "_build", "libcigpu_oracle.so")
 REF_LIB = os.path.join(HERE, "_ref", "libciflow_ref.so")
-# The CIFlow source tree the reference library is compiled from: CIGPU_REFERENCE_ROOT,
-# else the checkout location used where the fixtures were made. Only build_ref()
-# and the fixture generator read it; nothing on a GPU host needs it.
-REF_ROOT = os.environ.get("CIGPU_REFERENCE_ROOT") or "/root/reference"
+# The CIFlow source tree the reference library is compiled from. Only build_ref() and the
+# fixture generator read it; nothing on a GPU host needs it.
+REF_ROOT = os.environ.get("CIGPU_REFERENCE_ROOT", "")
 
 FCI, DOCI = 0, 1
 _P = ctypes.c_void_p
@@ -40,7 +39,7 @@ def build_port() -> str:
 
 
 def build_ref() -> str | None:
-    if not os.path.isdir(os.path.join(REF_ROOT, "src")):
+    if not REF_ROOT or not os.path.isdir(os.path.join(REF_ROOT, "src")):
         return None
     subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF_ROOT={REF_ROOT}", "-j8"], check=True)
     return REF_LIB
