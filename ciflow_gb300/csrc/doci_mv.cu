@@ -205,16 +205,16 @@ __global__ void __launch_bounds__(kMvThreads) k_doci_mv(const DociMv p, const T 
 // A hop is two or three shared-memory reads and a multiply-add where the general
 // kernel forms a rank (two popcounts' worth of lookups and selects, ~110 issue slots
 // per 32 hops). What bounds it: in FP32 the shared-memory gathers, in FP64 the FP64
-// pipe. L=24, 12 pairs (2,704,156 rows, 144 hops): FP32 1122 -> 227 us, FP64
-// 1.70 -> 0.74 ms (the FP64 pipe's share 0.62); L=20, 8 pairs (125,970): 54 -> 19-23 us and
-// 81 -> 39 us.
+// pipe. Among other products: L=24, 12 pairs (2,704,156 rows, 144 hops): FP32 1,072 -> 203
+// us, FP64 1.69 -> 0.74 ms (the FP64 pipe's share 0.62); L=20, 8 pairs (125,970): 54 -> 23
+// us and 81 -> 39 us.
 //
 // A thread block takes `group` consecutive high strings of one sector (number of high
 // pairs); a thread takes whole rows, in eight running sums (two per kind of hop) that
 // meet in a fixed order.
 // Threads per block (and rows it aims at): 256 in FP32, 512 in FP64, whose staged
 // blocks leave room for two thread blocks per SM (L=24: 843 us with 256, 751 with 512;
-// FP32 227 and 348).
+// FP32 227 and 348 in the same measurement).
 template <typename T>
 __host__ __device__ constexpr int split_threads() {
     return sizeof(T) == 4 ? 256 : 512;

@@ -857,7 +857,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_lanczos_steps(int64_t n, doub
 // slices of the basis in shared memory after the residual has read them, and the sums meet
 // through distributed shared memory in a fixed order (FP32 terms, their sums exact to the
 // warp, see add_exact, and FP64 above). Up to kDavRows rows, past which the basis is read faster by all
-// SMs. FCI L=8 4a4b (4,900 rows) to 1e-11: 9.9 -> 6.7 ms.
+// SMs. Solves to 1e-11: FCI L=8 4a4b (4,900 rows) 9.9 -> 6.7 ms, L=9 4a4b (15,876) 12.0 ->
+// 8.6, DOCI L=14 7 pairs (3,432) 3.4 -> 2.4, L=16 8 pairs (12,870) 3.7 -> 2.7; no space just
+// past the line was measured with it.
 constexpr int kDavThreads = 512;
 constexpr int64_t kDavRows = 16384;
 

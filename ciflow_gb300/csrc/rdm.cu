@@ -2,8 +2,9 @@
 //
 // Replaces CIDens::construct_density with DensFCI / DensDOCI (CIDens.cpp:323-334,
 // 1073-1224, 1530-1631). The reference loops over all determinant pairs and
-// classifies each by popcount (O(dim^2)); here only connected pairs contribute and
-// every sum has a fixed order (no atomics, bit-reproducible).
+// classifies each by popcount (O(dim^2)); here only connected pairs contribute. FCI sums
+// have a fixed order (no atomics); DOCI sums are fixed-point integers collected by
+// integer atomics, the same in any order. Both are bit-reproducible.
 //
 // FCI. Write C[Ia][Ib] for the CI vector. Every contribution of fill_density_matrix
 // (CIDens.cpp:676-881) with a pair (I, J), I <= J in row order, is one of
@@ -20,14 +21,15 @@
 // excitation (ar < ac) the string sums
 //        g_x[Ib] = sum_(Ia -> Ja) s_a C[Ia][Ib] C[Ja][x(Ib)]
 // over its string pairs, x the identity or one of Ib's single excitations, one thread
-// per Ib with its sums in registers; then the sums of s_b g_x[Ib] over the Ib that
+// per Ib with 36 or 12 of its sums in registers; then the sums of s_b g_x[Ib] over the Ib that
 // belong to each (br, bc). The identity's sums, over the Ib that hold z, are the
 // elements with beta occupation z; the mirror pass (identity only) gives those with
 // alpha occupation.
 //
-// DOCI: one block of L*L threads per slice of pair strings; thread (j, k)
-// accumulates c_I^2 n_j n_k and the pair-hop products c_I c_J (DensDOCI,
-// CIDens.cpp:1073-1224).
+// DOCI (DensDOCI, CIDens.cpp:1073-1224): the sums of c_I^2 n_j n_k and of the pair-hop
+// products c_I c_J, on larger spaces as dot products of the blocks of strings with one
+// set of high pairs (k_doci_rdm_split, a thread block per block of strings), else by a
+// thread per orbital pair j <= k over a slice of the pair strings (k_doci_rdm).
 //
 // Storage follows CIDens: the 1-RDM and each 2-RDM block are symmetric pair
 // matrices (Vector2d, matrix.cpp:674-690), accumulated on (min, max) and mirrored.
@@ -706,7 +708,8 @@ __global__ void k_doci_rdm(const double *__restrict__ c, const uint64_t *__restr
 // sums of squares, per block and per low string. The products and sums are the
 // fixed-point integers above, so the result is the same bit for bit in any order:
 // integer atomics collect them. Bound by instruction issue (49 for 32
-// products, ALU 41%) and, at three blocks per SM, the barriers around the staging. L=24,
+// products, ALU 41%) and the barriers around the staging (three blocks per SM: 65 KB of
+// shared memory each at L=24). L=24,
 // 12 pairs: 3.80 -> 0.74 ms per cigpu_rdm with a sum at a time for every warp, 0.66 with
 // four and in digits, 0.65 without the block's own matrices of sums (the kernel 490 -> 418
 // us; the vector's way from host memory is 150).
