@@ -38,7 +38,6 @@
 #include "doci_mv.cuh"
 
 #include <algorithm>
-#include <vector>
 
 namespace cigpu {
 
@@ -398,7 +397,10 @@ __global__ void __launch_bounds__(split_threads<T>()) k_doci_split(const DociSpl
     }
 }
 
-// The plan's tables. Sector q's low strings, by m pairs: thread per low string.
+// The plan's tables, one launch on the build's stream and no wait: with a copy of the
+// binomials from the host, two launches that read them from memory and a wait, the plan was
+// a third of a small space's build (L=18 9 pairs, mixed build 107 us without it, 144 so, 116
+// now).
 __device__ __forceinline__ uint32_t low_rank(uint32_t b, const uint32_t *binom) {
     uint32_t r = 0;
     for (int k = 1; b; b &= b - 1, ++k) r += binom[(__ffs((int)b) - 1) * kSplitBinomRow + k];
@@ -411,63 +413,83 @@ __device__ __forceinline__ uint32_t squeeze(uint32_t b, int j) {
     return (b & low) | ((b >> 1) & ~low);
 }
 
-constexpr int kSplitLowThreads = 128;
+struct SplitBinom {
+    uint32_t c[64 * kSplitBinomRow];  // C(p, k) mod 2^32, 0 past the space's orbitals and pairs
+};
+struct SplitTables {  // what the launch writes, in DociSplit's block
+    uint64_t *hbits;
+    uint32_t *hbase, *binom, *ll, *one, *two;
+    uint16_t *lminus, *lplus, *lowbits;
+};
 
-__global__ void __launch_bounds__(kSplitLowThreads) k_split_low(const DociSplitView p, uint32_t *__restrict__ ll,
-                                                                uint16_t *__restrict__ lminus,
-                                                                uint16_t *__restrict__ lplus,
-                                                                uint32_t *__restrict__ one, uint32_t *__restrict__ two,
-                                                                uint16_t *__restrict__ lowbits) {
+constexpr int kSplitThreads = 256;
+constexpr int kSplitLowBlocks = 16, kSplitHighBlocks = 32;  // per sector
+
+// Blocks of sector blockIdx.y: a thread per low string (by m pairs) and orbital, or per high
+// string.
+__global__ void __launch_bounds__(kSplitThreads)
+    k_split_tables(const __grid_constant__ DociSplitView p, const __grid_constant__ SplitBinom table, const SplitTables out) {
+    __shared__ uint32_t binom[64 * kSplitBinomRow];
     __shared__ uint16_t rank[1 << kSplitMaxLow];  // of every low string among those of its size
     const DociSector &c = p.sec[blockIdx.y];
     const int s = p.s, m = c.m;
-    for (int b = threadIdx.x; b < (1 << s); b += kSplitLowThreads) rank[b] = (uint16_t)low_rank((uint32_t)b, p.binom);
+    const bool low = blockIdx.x < kSplitLowBlocks;
+    const int used = (low ? s + 1 : p.L + 1) * kSplitBinomRow;
+    for (int i = threadIdx.x; i < used; i += kSplitThreads) binom[i] = table.c[i];
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < 64 * kSplitBinomRow; i += kSplitThreads) out.binom[i] = table.c[i];
     __syncthreads();
-    for (uint32_t l = blockIdx.x * kSplitLowThreads + threadIdx.x; l < c.nlow; l += gridDim.x * kSplitLowThreads) {
+    if (!low) {  // high strings and block starts
+        const int Lh = p.L - s;
+        for (uint32_t i = (blockIdx.x - kSplitLowBlocks) * kSplitThreads + threadIdx.x; i < c.nhigh;
+             i += (gridDim.x - kSplitLowBlocks) * kSplitThreads) {
+            uint64_t b = 0;
+            uint32_t rest = i, r = 0;
+            for (int k = c.nh, o = Lh - 1; k > 0; --o)
+                if (binom[o * kSplitBinomRow + k] <= rest) {
+                    rest -= binom[o * kSplitBinomRow + k];
+                    b |= (uint64_t)1 << o;
+                    r += binom[(s + o) * kSplitBinomRow + m + k];
+                    --k;
+                }
+            out.hbits[c.high0 + i] = b;
+            out.hbase[c.high0 + i] = r;
+        }
+        return;
+    }
+    for (int b = threadIdx.x; b < (1 << s); b += kSplitThreads) rank[b] = (uint16_t)low_rank((uint32_t)b, binom);
+    __syncthreads();
+    const uint32_t all = (1u << s) - 1u;
+    for (uint32_t it = blockIdx.x * kSplitThreads + threadIdx.x; it < c.nlow * (uint32_t)s; it += kSplitLowBlocks * kSplitThreads) {
+        const int j = (int)(it / c.nlow);
+        const uint32_t l = it - (uint32_t)j * c.nlow;
         uint32_t b = 0, rest = l;  // the low string of rank l
         for (int k = m, o = s - 1; k > 0; --o)
-            if (p.binom[o * kSplitBinomRow + k] <= rest) {
-                rest -= p.binom[o * kSplitBinomRow + k];
+            if (binom[o * kSplitBinomRow + k] <= rest) {
+                rest -= binom[o * kSplitBinomRow + k];
                 b |= 1u << o;
                 --k;
             }
-        lowbits[c.low0 + l] = (uint16_t)b;
-        int e = 0, em = 0, ep = 0;
-        for (int j = s - 1; j >= 0; --j) {
-            const uint32_t bj = b ^ (1u << j), at = rank[bj];
-            if (!((b >> j) & 1u)) {
-                lplus[c.plus0 + (uint32_t)ep++ * c.nlow + l] = (uint16_t)(at | ((uint32_t)j << 10));
-                continue;
-            }
-            lminus[c.minus0 + (uint32_t)em++ * c.nlow + l] = (uint16_t)(at | ((uint32_t)j << 10));
-            one[c.one0 + (uint32_t)j * c.n1 + rank[squeeze(bj, j)]] = l | (at << 16);
-            for (int k = j + 1, q = j * s - j * (j + 1) / 2; k < s; ++k, ++q)  // pair (j, k): row-major, j < k
-                if (!((b >> k) & 1u))
-                    two[c.two0 + (uint32_t)q * c.n2 + rank[squeeze(squeeze(bj, k), j)]] =
-                        l | ((uint32_t)rank[bj ^ (1u << k)] << 16);
-            for (int k = s - 1; k >= 0; --k)
-                if (!((b >> k) & 1u))
-                    ll[c.ll0 + (uint32_t)e++ * c.nlow + l] = rank[bj ^ (1u << k)] | ((uint32_t)(j * s + k) << 10);
+        if (j == 0) out.lowbits[c.low0 + l] = (uint16_t)b;
+        // entries run down the orbitals: those of the orbitals above j come first
+        const uint32_t above = all & ~((2u << j) - 1u), bj = b ^ (1u << j), at = rank[bj];
+        const uint32_t held = __popc(b & above), empty = __popc(~b & above);
+        if (!((b >> j) & 1u)) {
+            out.lplus[c.plus0 + empty * c.nlow + l] = (uint16_t)(at | ((uint32_t)j << 10));
+            continue;
         }
-    }
-}
-
-// High strings and block starts, sector by sector.
-__global__ void k_split_high(const DociSplitView p, uint64_t *__restrict__ hbits, uint32_t *__restrict__ hbase) {
-    const DociSector &c = p.sec[blockIdx.y];
-    const int Lh = p.L - p.s;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.nhigh; i += gridDim.x * blockDim.x) {
-        uint64_t b = 0;
-        uint32_t rest = i, r = 0;
-        for (int k = c.nh, o = Lh - 1; k > 0; --o)
-            if (p.binom[o * kSplitBinomRow + k] <= rest) {
-                rest -= p.binom[o * kSplitBinomRow + k];
-                b |= (uint64_t)1 << o;
-                r += p.binom[(p.s + o) * kSplitBinomRow + c.m + k];
-                --k;
+        out.lminus[c.minus0 + held * c.nlow + l] = (uint16_t)(at | ((uint32_t)j << 10));
+        out.one[c.one0 + (uint32_t)j * c.n1 + rank[squeeze(bj, j)]] = l | (at << 16);
+        uint32_t e = held * (uint32_t)(s - m);
+        for (int k = s - 1; k >= 0; --k) {
+            if ((b >> k) & 1u) continue;
+            const uint32_t to = rank[bj ^ (1u << k)];
+            out.ll[c.ll0 + e++ * c.nlow + l] = to | ((uint32_t)(j * s + k) << 10);
+            if (k > j) {  // pair (j, k): row-major, j < k
+                const uint32_t q = (uint32_t)(j * s - j * (j + 1) / 2 + k - j - 1);
+                out.two[c.two0 + q * c.n2 + rank[squeeze(squeeze(bj, k), j)]] = l | (to << 16);
             }
-        hbits[c.high0 + i] = b;
-        hbase[c.high0 + i] = r;
+        }
     }
 }
 
@@ -613,35 +635,37 @@ void doci_split_make(int L, int n, int64_t D, DociSplit &sp, cudaStream_t st) {
         }
     }
     if (v.s == 0 || (int64_t)nhi * kSplitMinBlock > D) return;
-    std::vector<uint32_t> bin((size_t)64 * kSplitBinomRow);
-    for (int p = 0; p < 64; ++p)
-        for (int k = 0; k < kSplitBinomRow; ++k) bin[(size_t)p * kSplitBinomRow + k] = p <= L && k <= n + 1 ? (uint32_t)d_binom(p, k) : 0u;
-    sp.binom.alloc(bin.size());
-    CIGPU_CUDA(cudaMemcpyAsync(sp.binom.p, bin.data(), bin.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    sp.hbits.alloc(nhi);
-    sp.hbase.alloc(nhi);
-    sp.ll.alloc(std::max(nll, 1u));
-    sp.lminus.alloc(std::max(nmi, 1u));
-    sp.lplus.alloc(std::max(npl, 1u));
-    sp.one.alloc(std::max(none, 1u));
-    sp.two.alloc(std::max(ntwo, 1u));
-    sp.lowbits.alloc(nlo);
+    SplitBinom table{};  // Pascal's triangle; p <= L and k <= n + 1 are read
+    for (int p = 0; p <= L; ++p)
+        for (int k = 0; k <= std::min(n + 1, p); ++k)
+            table.c[p * kSplitBinomRow + k] =
+                k == 0 ? 1u : table.c[(p - 1) * kSplitBinomRow + k - 1] + table.c[(p - 1) * kSplitBinomRow + k];
+    // one block: an allocation and its release cost a build a microsecond or two each
+    size_t words = 0;
+    const auto place = [&](size_t n, size_t size) {
+        const size_t at = words;
+        words += (n * size + 7) / 8;
+        return at;
+    };
+    const size_t at[] = {place(nhi, 8), place(nhi, 4),  place((size_t)64 * kSplitBinomRow, 4), place(nll, 4), place(none, 4),
+                         place(ntwo, 4), place(nmi, 2), place(npl, 2), place(nlo, 2)};
+    sp.tables.alloc(words);
+    const auto u32 = [&](int i) { return reinterpret_cast<uint32_t *>(sp.tables.p + at[i]); };
+    const auto u16 = [&](int i) { return reinterpret_cast<uint16_t *>(sp.tables.p + at[i]); };
+    const SplitTables out{sp.tables.p + at[0], u32(1), u32(2), u32(3), u32(4), u32(5), u16(6), u16(7), u16(8)};
     sp.nlowbits = nlo;
-    v.one = sp.one.p;
-    v.two = sp.two.p;
-    v.lowbits = sp.lowbits.p;
-    v.hbits = sp.hbits.p;
-    v.hbase = sp.hbase.p;
-    v.binom = sp.binom.p;
-    v.ll = sp.ll.p;
-    v.lminus = sp.lminus.p;
-    v.lplus = sp.lplus.p;
-    k_split_low<<<dim3(8, v.nsec), kSplitLowThreads, 0, st>>>(v, sp.ll.p, sp.lminus.p, sp.lplus.p, sp.one.p, sp.two.p,
-                                               sp.lowbits.p);
-    k_split_high<<<dim3(64, v.nsec), 256, 0, st>>>(v, sp.hbits.p, sp.hbase.p);
+    v.hbits = out.hbits;
+    v.hbase = out.hbase;
+    v.binom = out.binom;
+    v.ll = out.ll;
+    v.one = out.one;
+    v.two = out.two;
+    v.lminus = out.lminus;
+    v.lplus = out.lplus;
+    v.lowbits = out.lowbits;
+    k_split_tables<<<dim3(kSplitLowBlocks + kSplitHighBlocks, v.nsec), kSplitThreads, 0, st>>>(v, table, out);
     CIGPU_CUDA(cudaGetLastError());
-    count_launch(2);
-    CIGPU_CUDA(cudaStreamSynchronize(st));  // the binomial table goes out of scope
+    count_launch();
     sp.view = v;
 }
 

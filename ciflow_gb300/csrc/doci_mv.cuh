@@ -48,13 +48,12 @@ constexpr int kSplitBinomRow = 34;
 struct DociSplit {
     DociSplitView view{};
     size_t smem[2] = {0, 0};          // the product's shared memory, FP32 and FP64
-    DevBuf<uint64_t> hbits;
-    DevBuf<uint32_t> hbase, binom, ll, one, two;
-    DevBuf<uint16_t> lminus, lplus, lowbits;
+    DevBuf<uint64_t> tables;          // all of the view's, in one block
     uint32_t nlowbits = 0;
     explicit operator bool() const { return view.s > 0; }
 };
-// Makes the plan where the split product is the faster one (plan.view.s stays 0 elsewhere).
+// Makes the plan where the split product is the faster one (plan.view.s stays 0 elsewhere);
+// its tables are complete when the work queued on s is.
 void doci_split_make(int L, int n, int64_t D, DociSplit &plan, cudaStream_t s);
 
 // K_jk = (jk|jk) for j != k, zero where |v| <= 1e-14 (and on the diagonal): the

@@ -996,6 +996,7 @@ const DociSplit *doci_split_of(cigpu_crs &c, cudaStream_t s) {
     std::lock_guard<std::mutex> lock(mu);
     if (!c.split_tried) {
         doci_split_make(c.L, c.nup, c.dim, c.split, s);
+        CIGPU_CUDA(cudaStreamSynchronize(s));  // for callers on other streams
         c.split_tried = true;
     }
     return c.split && (int64_t)split_blocks(c.split.view) * kSplitRdmBlock <= c.dim &&
