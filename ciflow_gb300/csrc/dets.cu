@@ -53,6 +53,7 @@ struct DetParams {
     // stored block: count / fill take columns below `block` (n for a whole CRS); the
     // matvec takes the pairs outside the block (row i < block: columns >= block)
     int64_t nrows = 0, block = 0;
+    int group = 32;        // rows of a warp in the count and fill passes (32, fewer in short lists)
     const uint64_t *dets;  // [n][2W]
     const double *eri;     // chemist (pq|rs), L^4
     const double *h;       // L^2
@@ -426,6 +427,23 @@ __device__ __forceinline__ void mark(uint32_t &m, uint32_t x, uint32_t bit, uint
         : "r"((uint32_t)__popc(x)), "r"(one), "r"(bit));
 }
 
+// Where a segment's kept elements of the lane's row begin: the row's start and the counts of
+// the segments before it, the warp summing a row at a time (a lane's own 63 counts lie 256
+// bytes from its neighbour's).
+__device__ __forceinline__ int64_t segment_start(const DetParams &p, int64_t r0, int seg) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = r0 + lane;
+    const int rows = (int)min((int64_t)p.group, p.nrows - r0);
+    int64_t at = lane < rows ? p.row_ptr[i] : 0;
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
+        const uint32_t *c = p.seg_count + (r0 + r) * kSegs;
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, (lane < seg ? c[lane] : 0u) + (lane + 32 < seg ? c[lane + 32] : 0u));
+        if (lane == r) at += sum;
+    }
+    return at;
+}
+
 // Shared memory of one warp.
 template <int W, int NW>
 struct ScanWarp {
@@ -643,9 +661,9 @@ __global__ void __launch_bounds__(32, 32) k_dets_scan(const DetParams p) {
     const int lane = threadIdx.x;
     const int64_t group = blockIdx.x / kSegs;
     const int seg = (int)(blockIdx.x - group * kSegs);
-    const int64_t r0 = group * kScanRows;
+    const int64_t r0 = group * p.group;
     const int64_t i = r0 + lane;
-    const bool active = i < p.nrows;
+    const bool active = lane < p.group && i < p.nrows;
     uint64_t rec[2 * W];
 #pragma unroll
     for (int w = 0; w < 2 * W; ++w) rec[w] = active ? p.dets[i * 2 * W + w] : 0;
@@ -655,14 +673,11 @@ __global__ void __launch_bounds__(32, 32) k_dets_scan(const DetParams p) {
     for (int w = 0; w < 2 * W; ++w) rows.s[lane][w] = rec[w];
     q.run[lane] = q.low[lane] = 0;
     const int64_t words = (p.block + 31) / 32, w0 = words * seg / kSegs, w1 = words * (seg + 1) / kSegs;
-    if (MODE == kDetFill64 || MODE == kDetFill32) {
-        int64_t at = 0;
-        if (active) {
-            at = p.row_ptr[i];
-            for (int w = 0; w < seg; ++w) at += p.seg_count[i * kSegs + w];
-        }
-        rowpos[lane] = at;
+    if (w0 == w1) {  // a short list has fewer words than segments
+        if (MODE == kDetCount && active) p.seg_count[i * kSegs + seg] = 0;
+        return;
     }
+    if (MODE == kDetFill64 || MODE == kDetFill32) rowpos[lane] = segment_start(p, r0, seg);
     __syncwarp();
     const uint32_t one = p.one;
     int qn = 0;
@@ -735,6 +750,10 @@ __global__ void __launch_bounds__(32, 32) k_dets_scan(const DetParams p) {
 // the build starts again with the passes above, which evaluate twice. L=32 8a8b CISD
 // list, list to CRS and one product: 4.64 -> 3.22 ms.
 constexpr size_t kMaskBytes = size_t(1) << 30;
+// Lists shorter than this evaluate twice all the same: a wait for the count of vanished
+// elements, and the masks' passes, cost as much as their few elements (60 determinants 125
+// against 121 us, 442 136 and 132, 1,000 151 and 149).
+constexpr int64_t kShortList = 1000;
 
 template <int W, int NW>
 struct FillWarp {
@@ -796,9 +815,9 @@ template <int W, int NW, int MODE, bool MASKS>
 __global__ void __launch_bounds__(32, 32) k_dets_pairs(const DetParams p) {
     __shared__ FillWarp<W, NW> q;
     const int lane = threadIdx.x;
-    const int64_t group = blockIdx.x / kSegs, r0 = group * kScanRows, i = r0 + lane;
+    const int64_t group = blockIdx.x / kSegs, r0 = group * p.group, i = r0 + lane;
     const int seg = (int)(blockIdx.x - group * kSegs);
-    const bool active = i < p.nrows;
+    const bool active = lane < p.group && i < p.nrows;
     uint64_t rec[2 * W];
 #pragma unroll
     for (int w = 0; w < 2 * W; ++w) q.rows.s[lane][w] = rec[w] = active ? p.dets[i * 2 * W + w] : 0;
@@ -806,14 +825,11 @@ __global__ void __launch_bounds__(32, 32) k_dets_pairs(const DetParams p) {
     scan_key<W, NW>(rec, rk);
     const int64_t words = (p.block + 31) / 32, w0 = words * seg / kSegs, w1 = words * (seg + 1) / kSegs;
     uint32_t run = 0, low = 0;
-    if (MODE != kDetCount) {
-        int64_t at = 0;
-        if (active) {
-            at = p.row_ptr[i];
-            for (int w = 0; w < seg; ++w) at += p.seg_count[i * kSegs + w];
-        }
-        q.rowpos[lane] = at;
+    if (w0 == w1) {  // a short list has fewer words than segments
+        if (MODE == kDetCount && active) p.seg_count[i * kSegs + seg] = 0;
+        return;
     }
+    if (MODE != kDetCount) q.rowpos[lane] = segment_start(p, r0, seg);
     __syncwarp();
     const uint32_t one = p.one;
     uint32_t *masks = p.masks + group * words * 32 + lane;
@@ -1206,8 +1222,16 @@ int rows_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + kDetWarps - 1) / kDetWarps, (int64_t)sm_count() * 16));
 }
 
+// Rows of a warp in the build's passes. A short list has few words of columns and few
+// groups of 32 rows, each a long queue of connected pairs on one warp; fewer rows make more
+// warps. List to CRS in us, 32 | 16 | 8 | 4 rows: 60 determinants of L=8 150 | 137 | 128 | 125,
+// 442 of L=10 170 | 145 | 137 | 136, 1,486 of L=14 190 | 169 | 164 | 168, 5,000 of L=20 322 |
+// 292 | 298 | 335, 8,000 of L=24 444 | 413 | 435 | 537 and, with vanishing integrals, 632 | 535 |
+// 530 | 649.
+int build_group(int64_t n) { return n < kShortList ? 4 : n < 10000 ? 8 : 32; }
+
 unsigned segment_blocks(const DetParams &p) {
-    const int64_t blocks = (p.nrows + kScanRows - 1) / kScanRows * kSegs;
+    const int64_t blocks = (p.nrows + p.group - 1) / p.group * kSegs;
     if (blocks > (int64_t)INT32_MAX) throw std::invalid_argument("determinant list too long");
     return (unsigned)blocks;
 }
@@ -1706,42 +1730,44 @@ int build_dets(cigpu_ham *ham, int64_t ndet, int words, const uint64_t *up, cons
         const int64_t nb = c->det_block;
         p.nrows = nb;
         p.block = nb;
-        DevBuf<uint32_t> count(nb), segs((size_t)nb * kSegs), dropped(1);
-        DevBuf<unsigned long long> lower(1);
+        p.group = build_group(nb);
+        // the sums that start at zero in one block: elements below the diagonal (64 bits),
+        // vanished elements, each row's count
+        DevBuf<uint32_t> sums((size_t)nb + 4), segs((size_t)nb * kSegs);
+        unsigned long long *const lower = reinterpret_cast<unsigned long long *>(sums.p);
+        uint32_t *const dropped = sums.p + 2, *const count = sums.p + 4;
         c->upper_off.alloc(nb);
         c->row_ptr.alloc(nb + 1);
-        p.row_count = count.p;
+        p.row_count = count;
+        p.dropped = dropped;
         p.upper_off = c->upper_off.p;
         p.seg_count = segs.p;
         p.row_ptr = c->row_ptr.p;
-        p.dropped = dropped.p;
         // structure: the row structure is the connected pairs (see k_dets_pairs)
         auto passes = [&](bool structure) {
             DevBuf<uint32_t> masks;
-            const size_t words = (size_t)((nb + 31) / 32);
-            if (structure && words * words * 32 * sizeof(uint32_t) <= kMaskBytes) {
+            const size_t words = (size_t)((nb + 31) / 32), groups = (size_t)((nb + p.group - 1) / p.group);
+            if (structure && groups * words * 32 * sizeof(uint32_t) <= kMaskBytes) {
                 try {
-                    masks.alloc(words * words * 32);
+                    masks.alloc(groups * words * 32);
                 } catch (const std::bad_alloc &) {  // the fill scans again
                 }
             }
             p.masks = masks.p;
-            CIGPU_CUDA(cudaMemsetAsync(count.p, 0, count.bytes(), s));
+            CIGPU_CUDA(cudaMemsetAsync(sums.p, 0, sums.bytes(), s));
             CIGPU_CUDA(cudaMemsetAsync(c->upper_off.p, 0, c->upper_off.bytes(), s));
-            CIGPU_CUDA(cudaMemsetAsync(lower.p, 0, sizeof(unsigned long long), s));
-            CIGPU_CUDA(cudaMemsetAsync(dropped.p, 0, sizeof(uint32_t), s));
             if (structure)
                 pairs<kDetCount>(p, W, s);
             else
                 rows<kDetCount>(p, W, s);
-            exclusive_scan_u32(count.p, c->row_ptr.p, nb, s);
-            k_sum_u32<<<(int)std::min<int64_t>((nb + 255) / 256, 1024), 256, 0, s>>>(c->upper_off.p, nb, lower.p);
+            exclusive_scan_u32(count, c->row_ptr.p, nb, s);
+            k_sum_u32<<<(int)std::min<int64_t>((nb + 255) / 256, 1024), 256, 0, s>>>(c->upper_off.p, nb, lower);
             CIGPU_CUDA(cudaGetLastError());
             count_launch();
             int64_t nnz = 0;
             unsigned long long nlow = 0;
             CIGPU_CUDA(cudaMemcpyAsync(&nnz, c->row_ptr.p + nb, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-            CIGPU_CUDA(cudaMemcpyAsync(&nlow, lower.p, sizeof(nlow), cudaMemcpyDeviceToHost, s));
+            CIGPU_CUDA(cudaMemcpyAsync(&nlow, lower, sizeof(nlow), cudaMemcpyDeviceToHost, s));
             CIGPU_CUDA(cudaStreamSynchronize(s));
             c->nnz_full = nnz;
             c->nnz_upper = nnz - (int64_t)nlow;
@@ -1777,11 +1803,11 @@ int build_dets(cigpu_ham *ham, int64_t ndet, int words, const uint64_t *up, cons
                 rows<kDetFill32>(p, W, s);
             if (!structure) return true;
             uint32_t d = 0;
-            CIGPU_CUDA(cudaMemcpyAsync(&d, dropped.p, sizeof(d), cudaMemcpyDeviceToHost, s));
+            CIGPU_CUDA(cudaMemcpyAsync(&d, dropped, sizeof(d), cudaMemcpyDeviceToHost, s));
             CIGPU_CUDA(cudaStreamSynchronize(s));
             return d == 0;
         };
-        if (ham->eri_zero || !passes(true)) passes(false);
+        if (ham->eri_zero || nb < kShortList || !passes(true)) passes(false);
     }
     CIGPU_CUDA(cudaStreamSynchronize(s));
     c->build_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

@@ -301,3 +301,19 @@ def test_matvec_of_an_ordered_list(L, na, nb, n):
     tol = 2.0 ** -52 * (len(pairs) + 2) * float(np.abs(val).max() * np.abs(x).max()) * np.sqrt(len(pairs))
     for keep in (0, 777, 3200):
         assert np.abs(CI_Big(ham, up=up, down=down, keep=keep).get_mat().mvprod(x) - y).max() <= tol
+
+
+@pytest.mark.parametrize("kind", ["no zero", "zeros", "vanishing differences"])
+@pytest.mark.parametrize("n", [3, 45, 999, 1001, 1999])
+def test_build_groups(n, kind):
+    """List builds by groups of 4, 8 and 32 rows, evaluated twice (short lists, vanishing
+    integrals), from the structure, and from the structure in vain: the oracle's CRS."""
+    ints = make_integrals(13, 3, 3, nchol=4, seed=n)
+    if kind == "zeros":
+        odd = np.arange(13) % 2
+        ints.eri[((odd[:, None, None, None] + odd[:, None, None] + odd[:, None] + odd) % 2) == 1] = 0.0
+    elif kind == "vanishing differences":
+        ints.eri[...] = 0.125
+    up, down = random_list(13, 3, 3, n, seed=n)
+    m = O.build_dets(ints, up, down)
+    assert upper_sha(FCI_File(Hamiltonian.from_integrals(ints), up=up, down=down)) == crs_sha256(m.row, m.col, m.val)
