@@ -642,9 +642,9 @@ void doci_split_make(int L, int n, int64_t D, DociSplit &sp, cudaStream_t st) {
                 k == 0 ? 1u : table.c[(p - 1) * kSplitBinomRow + k - 1] + table.c[(p - 1) * kSplitBinomRow + k];
     // one block: an allocation and its release cost a build a microsecond or two each
     size_t words = 0;
-    const auto place = [&](size_t n, size_t size) {
+    const auto place = [&](size_t n, size_t size) {  // each on 256 bytes, as an allocation
         const size_t at = words;
-        words += (n * size + 7) / 8;
+        words += (n * size + 255) / 256 * 32;
         return at;
     };
     const size_t at[] = {place(nhi, 8), place(nhi, 4),  place((size_t)64 * kSplitBinomRow, 4), place(nll, 4), place(none, 4),
